@@ -156,97 +156,130 @@ __device__ __forceinline__ void norm_pieces(float v, int storage, uint16_t (&out
 constexpr int kPlanesBf16x3 = 0;
 constexpr int kPlanesFp16x2 = 1;
 
-template <int STORAGE>
-__global__ void store_rows_kernel(const float* __restrict__ src, int64_t src_pitch, int64_t n, int d,
-                                  void* __restrict__ dst, int64_t dst_pitch,
-                                  uint16_t* __restrict__ planes, int64_t plane_pitch,
-                                  int64_t plane_stride, int plane_format, float plane_scale,
-                                  int32_t* __restrict__ range_flag, float* __restrict__ norms, int norm_cols) {
-    const int lane = threadIdx.x & 31;
-    const int d8 = (d + 7) & ~7;
-    const int64_t warps_total = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t r = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < n;
-         r += warps_total) {
-        const float* row = src + r * src_pitch;
-        float s = 0.f;
-        if (STORAGE == B200F_STORAGE_F32) {
-            float* out = reinterpret_cast<float*>(dst) + r * dst_pitch;
-            if (out != row) {   // a re-split reads the stored rows themselves
-                for (int j = lane; j < dst_pitch; j += 32) {
-                    float v = (j < d) ? row[j] : 0.f;
-                    out[j] = v;
-                    s = fmaf(v, v, s);
-                }
-            } else {
-                for (int j = lane; j < d; j += 32) s = fmaf(row[j], row[j], s);
-            }
-            if (planes && plane_format == kPlanesFp16x2) {
-                uint16_t* p0 = planes + r * plane_pitch;
-                uint16_t* p1 = p0 + plane_stride;
-                float amax = 0.f;
-                for (int j = lane; j < plane_pitch; j += 32) {
-                    const float v = (j < d) ? row[j] * plane_scale : 0.f;
-                    amax = fmaxf(amax, fabsf(v));
-                    const uint16_t h0 = float_to_fp16_bits(v);
-                    const float r1 = v - fp16_bits_to_float(h0);   // exact in fp32
-                    p0[j] = h0;
-                    p1[j] = float_to_fp16_bits(r1);
-                }
+// V consecutive elements of a row per lane and access: 4 (or 8, load_rows_kernel) where the row
+// length and every pitch and base allow it, else 2 or 1.
+template <int V>
+struct alignas(V * 4) FloatVec {
+    float v[V];
+};
+template <int V>
+struct alignas(V * 2) HalfVec {
+    uint16_t v[V];
+};
+template <int V>
+__device__ __forceinline__ void store_bits(uint16_t* p, const uint16_t (&b)[V]) {
+    HalfVec<V> h;
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-                if (lane == 0 && range_flag && (amax >= 32768.f || (amax > 0.f && amax < 0.0625f)))
-                    atomicOr(range_flag, 1);
-            } else if (planes) {
-                uint16_t* p0 = planes + r * plane_pitch;
-                uint16_t* p1 = p0 + plane_stride;
-                uint16_t* p2 = p1 + plane_stride;
-                for (int j = lane; j < plane_pitch; j += 32) {
-                    float v = (j < d) ? row[j] : 0.f;
-                    uint16_t b0 = float_to_bf16_bits(v);
-                    float r1 = v - bf16_bits_to_float(b0);
-                    uint16_t b1 = float_to_bf16_bits(r1);
-                    float r2 = r1 - bf16_bits_to_float(b1);
-                    uint16_t b2 = float_to_bf16_bits(r2);
-                    p0[j] = b0;
-                    p1[j] = b1;
-                    p2[j] = b2;
-                }
+    for (int e = 0; e < V; e++) h.v[e] = b[e];
+    *reinterpret_cast<HalfVec<V>*>(p) = h;
+}
+
+// HBM-bound: 4 d bytes read and (fp32 rows, two fp16 planes) 8 d written per row.  A row belongs to
+// lpr lanes of a warp (all 32 from d = 4 V 8 on, fewer for short rows, so that no lane idles), each
+// lane keeps U vectors in flight and the row is read ONCE: squares, conversions and the plane split
+// all come from the same registers.  1,000,003 rows of d = 384, fp32 with fp16 planes: 720 us
+// (6.5 TB/s); element by element with a second read of the row for the planes it took 940 us.
+template <int STORAGE, int V>
+__global__ void __launch_bounds__(ROW_THREADS)
+store_rows_kernel(const float* __restrict__ src, int64_t src_pitch, int64_t n, int d, int lpr,
+                  void* __restrict__ dst, int64_t dst_pitch, uint16_t* __restrict__ planes, int64_t plane_pitch,
+                  int64_t plane_stride, int plane_format, float plane_scale, int32_t* __restrict__ range_flag,
+                  float* __restrict__ norms, int norm_cols) {
+    constexpr int U = V == 4 ? 4 : 8;
+    const int lane = threadIdx.x & 31;
+    const int sub = lane / lpr, cl = lane & (lpr - 1);
+    const int d8 = (d + 7) & ~7;
+    const int64_t rows_per_step = 32 / lpr;
+    const int64_t warps_total = (int64_t)gridDim.x * (blockDim.x >> 5);
+    // columns written: the stored row and the plane rows, pads included
+    const int64_t width = (planes && plane_pitch > dst_pitch) ? plane_pitch : dst_pitch;
+    for (int64_t r0 = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * rows_per_step; r0 < n;
+         r0 += warps_total * rows_per_step) {
+        const int64_t r = r0 + sub;
+        const bool live = r < n;
+        const float* row = src + r * src_pitch;
+        float* const outf = reinterpret_cast<float*>(dst) + r * dst_pitch;
+        uint16_t* const outh = reinterpret_cast<uint16_t*>(dst) + r * dst_pitch;
+        uint16_t* const p0 = planes + r * plane_pitch;
+        const bool copy_row = STORAGE != B200F_STORAGE_F32 || outf != row;   // a re-split reads the stored rows themselves
+        float s = 0.f, amax = 0.f;
+        for (int64_t base = 0; base < width; base += (int64_t)lpr * V * U) {
+            FloatVec<V> x[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int64_t j = base + ((int64_t)u * lpr + cl) * V;
+#pragma unroll
+                for (int e = 0; e < V; e++) x[u].v[e] = 0.f;
+                if (live && j < d) x[u] = *reinterpret_cast<const FloatVec<V>*>(row + j);
             }
-        } else {
-            uint16_t* out = reinterpret_cast<uint16_t*>(dst) + r * dst_pitch;
-            for (int j = lane; j < dst_pitch; j += 32) {
-                float v = (j < d) ? row[j] : 0.f;
-                uint16_t b;
-                float back;
-                if (STORAGE == B200F_STORAGE_F16) {
-                    b = float_to_fp16_bits(v);
-                    back = fp16_bits_to_float(b);
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int64_t j = base + ((int64_t)u * lpr + cl) * V;
+                if (!live || j >= width) continue;
+                const bool ncol = norm_cols && j >= d8 && j < d8 + 8;   // written below
+                if (STORAGE == B200F_STORAGE_F32) {
+#pragma unroll
+                    for (int e = 0; e < V; e++) s = fmaf(x[u].v[e], x[u].v[e], s);
+                    if (copy_row && j < dst_pitch) *reinterpret_cast<FloatVec<V>*>(outf + j) = x[u];
+                    if (!planes || j >= plane_pitch) continue;
+                    uint16_t h0[V], h1[V], h2[V];
+                    if (plane_format == kPlanesFp16x2) {
+#pragma unroll
+                        for (int e = 0; e < V; e++) {
+                            const float v = x[u].v[e] * plane_scale;
+                            amax = fmaxf(amax, fabsf(v));
+                            h0[e] = float_to_fp16_bits(v);
+                            h1[e] = float_to_fp16_bits(v - fp16_bits_to_float(h0[e]));   // the difference is exact
+                        }
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < V; e++) {
+                            h0[e] = float_to_bf16_bits(x[u].v[e]);
+                            const float r1 = x[u].v[e] - bf16_bits_to_float(h0[e]);
+                            h1[e] = float_to_bf16_bits(r1);
+                            h2[e] = float_to_bf16_bits(r1 - bf16_bits_to_float(h1[e]));
+                        }
+                        store_bits<V>(p0 + 2 * plane_stride + j, h2);
+                    }
+                    if (!ncol) store_bits<V>(p0 + j, h0);
+                    store_bits<V>(p0 + plane_stride + j, h1);
                 } else {
-                    b = float_to_bf16_bits(v);
-                    back = bf16_bits_to_float(b);
+                    uint16_t h[V];
+#pragma unroll
+                    for (int e = 0; e < V; e++) {
+                        float back;
+                        if (STORAGE == B200F_STORAGE_F16) {
+                            h[e] = float_to_fp16_bits(x[u].v[e]);
+                            back = fp16_bits_to_float(h[e]);
+                        } else {
+                            h[e] = float_to_bf16_bits(x[u].v[e]);
+                            back = bf16_bits_to_float(h[e]);
+                        }
+                        s = fmaf(back, back, s);
+                    }
+                    if (!ncol) store_bits<V>(outh + j, h);
                 }
-                out[j] = b;
-                s = fmaf(back, back, s);
             }
         }
-        s = warp_sum(s);
-        if (norms && lane == 0) norms[r] = s;
+        for (int o = lpr >> 1; o > 0; o >>= 1) {
+            s += __shfl_xor_sync(0xffffffffu, s, o);
+            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        }
+        if (!live || cl != 0) continue;
+        if (range_flag && planes && plane_format == kPlanesFp16x2 && (amax >= 32768.f || (amax > 0.f && amax < 0.0625f)))
+            atomicOr(range_flag, 1);
+        if (norms) norms[r] = s;
         if (norm_cols) {
-            __syncwarp();
-            if (lane == 0) {
-                uint16_t pc[8];
-                if (STORAGE == B200F_STORAGE_F32 && plane_format == kPlanesFp16x2)
-                    // in the scaled units of the planes: (s x).(s x) / 2, fp16 pieces
-                    norm_pieces(-0.5f * s * plane_scale * plane_scale, B200F_STORAGE_F16, pc);
-                else
-                    norm_pieces(-0.5f * s, STORAGE == B200F_STORAGE_F32 ? B200F_STORAGE_BF16 : STORAGE, pc);
-                uint16_t* o = (STORAGE == B200F_STORAGE_F32)
-                                      ? (planes ? planes + r * plane_pitch + d8 : nullptr)
-                                      : reinterpret_cast<uint16_t*>(dst) + r * dst_pitch + d8;
-                if (o) {
+            uint16_t pc[8];
+            if (STORAGE == B200F_STORAGE_F32 && plane_format == kPlanesFp16x2)
+                // in the scaled units of the planes: (s x).(s x) / 2, fp16 pieces
+                norm_pieces(-0.5f * s * plane_scale * plane_scale, B200F_STORAGE_F16, pc);
+            else
+                norm_pieces(-0.5f * s, STORAGE == B200F_STORAGE_F32 ? B200F_STORAGE_BF16 : STORAGE, pc);
+            uint16_t* o = (STORAGE == B200F_STORAGE_F32) ? (planes ? p0 + d8 : nullptr) : outh + d8;
+            if (o) {
 #pragma unroll
-                    for (int i = 0; i < 8; i++) o[i] = pc[i];
-                }
+                for (int i = 0; i < 8; i++) o[i] = pc[i];
             }
         }
     }
@@ -271,15 +304,55 @@ __global__ void rows_absmax_kernel(const float* __restrict__ src, int64_t pitch,
     if (lane == 0 && amax > 0.f) atomicMax(out_max_bits, __float_as_uint(amax));
 }
 
-template <int STORAGE>
-__global__ void load_rows_kernel(const void* __restrict__ rows, int64_t n, int d, int64_t pitch,
-                                 float* __restrict__ dst) {
-    const int64_t total = n * (int64_t)d;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = i / d;
-        const int j = (int)(i - r * d);
-        dst[i] = load_elem<STORAGE>(rows, r * pitch + j);
+// Stored rows back to fp32, HBM-bound; lanes and vectors as in store_rows_kernel (fp32, 1,000,003 rows
+// of d = 384: 480 us, 6.4 TB/s; one element per thread with a 64-bit division each: 935 us).
+template <int STORAGE, int V>
+__global__ void __launch_bounds__(ROW_THREADS)
+load_rows_kernel(const void* __restrict__ rows, int64_t n, int d, int lpr, int64_t pitch, float* __restrict__ dst) {
+    constexpr int U = 4;
+    const int lane = threadIdx.x & 31;
+    const int sub = lane / lpr, cl = lane & (lpr - 1);
+    const int64_t rows_per_step = 32 / lpr;
+    const int64_t warps_total = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t r0 = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * rows_per_step; r0 < n;
+         r0 += warps_total * rows_per_step) {
+        const int64_t r = r0 + sub;
+        if (r >= n) continue;
+        float* const out = dst + r * (int64_t)d;
+        for (int base = 0; base < d; base += lpr * V * U) {
+            if constexpr (STORAGE == B200F_STORAGE_F32) {
+                const float* row = reinterpret_cast<const float*>(rows) + r * pitch;
+                FloatVec<V> x[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int j = base + (u * lpr + cl) * V;
+                    if (j < d) x[u] = *reinterpret_cast<const FloatVec<V>*>(row + j);
+                }
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int j = base + (u * lpr + cl) * V;
+                    if (j < d) *reinterpret_cast<FloatVec<V>*>(out + j) = x[u];
+                }
+            } else {
+                const uint16_t* row = reinterpret_cast<const uint16_t*>(rows) + r * pitch;
+                HalfVec<V> h[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int j = base + (u * lpr + cl) * V;
+                    if (j < d) h[u] = *reinterpret_cast<const HalfVec<V>*>(row + j);
+                }
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int j = base + (u * lpr + cl) * V;
+                    if (j >= d) continue;
+                    FloatVec<V> x;
+#pragma unroll
+                    for (int e = 0; e < V; e++)
+                        x.v[e] = STORAGE == B200F_STORAGE_F16 ? fp16_bits_to_float(h[u].v[e]) : bf16_bits_to_float(h[u].v[e]);
+                    *reinterpret_cast<FloatVec<V>*>(out + j) = x;
+                }
+            }
+        }
     }
 }
 
@@ -408,6 +481,18 @@ __global__ void fill_synthetic_kernel(float* __restrict__ dst, int64_t n, int d,
     }
 }
 
+// Lanes that share a row of d elements read V at a time.
+int lanes_for_row(int d, int v) {
+    int lpr = 1;
+    while (lpr < 32 && lpr * v < d) lpr <<= 1;
+    return lpr;
+}
+
+// True when every offset (in elements) and the base (in elements of `bytes` bytes) are multiples of v.
+bool vec_ok(const void* base, int bytes, int v, int64_t a, int64_t b = 0) {
+    return (reinterpret_cast<uintptr_t>(base) % (size_t)(bytes * v)) == 0 && a % v == 0 && b % v == 0;
+}
+
 int grid_for_rows(int64_t n) {
     int64_t g = ceil_div64(n, ROW_THREADS / 32);
     int64_t cap = (int64_t)cached_sm_count() * 16;
@@ -499,25 +584,37 @@ int store_rows_impl(const float* src, int64_t src_pitch, int64_t n, int d, int s
     }
     if (n == 0) return B200F_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int g = grid_for_rows(n);
     const float scale = std::ldexp(1.f, plane_scale_log2);
-    switch (storage) {
-        case B200F_STORAGE_F32:
-            store_rows_kernel<B200F_STORAGE_F32><<<g, ROW_THREADS, 0, st>>>(
-                    src, src_pitch, n, d, dst_rows, dst_pitch, planes, plane_pitch, plane_stride, plane_format, scale,
-                    range_flag, norms_or_null, norm_cols);
-            break;
-        case B200F_STORAGE_F16:
-            store_rows_kernel<B200F_STORAGE_F16><<<g, ROW_THREADS, 0, st>>>(
-                    src, src_pitch, n, d, dst_rows, dst_pitch, nullptr, 0, 0, 0, 1.f, nullptr, norms_or_null, norm_cols);
-            break;
-        case B200F_STORAGE_BF16:
-            store_rows_kernel<B200F_STORAGE_BF16><<<g, ROW_THREADS, 0, st>>>(
-                    src, src_pitch, n, d, dst_rows, dst_pitch, nullptr, 0, 0, 0, 1.f, nullptr, norms_or_null, norm_cols);
-            break;
-        default:
-            return B200F_ERR_BAD_ARG;
+    const bool fp32 = storage == B200F_STORAGE_F32;
+    if (!fp32) {
+        planes = nullptr;
+        plane_pitch = plane_stride = 0;
     }
+    int v = 4;
+    while (v > 1 && !(d % v == 0 && vec_ok(src, 4, v, src_pitch) && vec_ok(dst_rows, fp32 ? 4 : 2, v, dst_pitch) &&
+                      (!planes || vec_ok(planes, 2, v, plane_pitch, plane_stride))))
+        v >>= 1;
+    const int lpr = lanes_for_row(d, v);
+    const int g = grid_for_rows(ceil_div64(n, 32 / lpr));
+    // macro: the kernel is a template over (storage, elements per access)
+#define B200F_STORE_ROWS(ST, V)                                                                          \
+    store_rows_kernel<ST, V><<<g, ROW_THREADS, 0, st>>>(src, src_pitch, n, d, lpr, dst_rows, dst_pitch,   \
+                                                        planes, plane_pitch, plane_stride, plane_format, \
+                                                        scale, range_flag, norms_or_null, norm_cols)
+#define B200F_STORE_ROWS_V(ST)                    \
+    do {                                          \
+        if (v == 4) B200F_STORE_ROWS(ST, 4);      \
+        else if (v == 2) B200F_STORE_ROWS(ST, 2); \
+        else B200F_STORE_ROWS(ST, 1);             \
+    } while (0)
+    switch (storage) {
+        case B200F_STORAGE_F32: B200F_STORE_ROWS_V(B200F_STORAGE_F32); break;
+        case B200F_STORAGE_F16: B200F_STORE_ROWS_V(B200F_STORAGE_F16); break;
+        case B200F_STORAGE_BF16: B200F_STORE_ROWS_V(B200F_STORAGE_BF16); break;
+        default: return B200F_ERR_BAD_ARG;
+    }
+#undef B200F_STORE_ROWS_V
+#undef B200F_STORE_ROWS
     count_launch();
     B200F_LAUNCH_CHECK();
     return B200F_OK;
@@ -557,23 +654,32 @@ extern "C" int b200f_load_rows(const void* rows, int storage, int64_t n, int d, 
     if (n < 0 || d <= 0 || pitch_elems < d || (n > 0 && (!rows || !dst))) return B200F_ERR_BAD_ARG;
     if (n == 0) return B200F_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    int64_t total = n * (int64_t)d;
-    int64_t g = ceil_div64(total, 256);
-    int64_t cap = (int64_t)cached_sm_count() * 32;
-    if (g > cap) g = cap;
+    const bool fp32 = storage == B200F_STORAGE_F32;
+    int v = fp32 ? 4 : 8;
+    while (v > 1 && !(d % v == 0 && vec_ok(rows, fp32 ? 4 : 2, v, pitch_elems) && vec_ok(dst, 4, v, 0))) v >>= 1;
+    const int lpr = lanes_for_row(d, v);
+    const int g = grid_for_rows(ceil_div64(n, 32 / lpr));
+#define B200F_LOAD_ROWS(ST, V) load_rows_kernel<ST, V><<<g, ROW_THREADS, 0, st>>>(rows, n, d, lpr, pitch_elems, dst)
     switch (storage) {
         case B200F_STORAGE_F32:
-            load_rows_kernel<B200F_STORAGE_F32><<<(int)g, 256, 0, st>>>(rows, n, d, pitch_elems, dst);
+            if (v == 4) B200F_LOAD_ROWS(B200F_STORAGE_F32, 4);
+            else if (v == 2) B200F_LOAD_ROWS(B200F_STORAGE_F32, 2);
+            else B200F_LOAD_ROWS(B200F_STORAGE_F32, 1);
             break;
         case B200F_STORAGE_F16:
-            load_rows_kernel<B200F_STORAGE_F16><<<(int)g, 256, 0, st>>>(rows, n, d, pitch_elems, dst);
+            if (v == 8) B200F_LOAD_ROWS(B200F_STORAGE_F16, 8);
+            else if (v >= 2) B200F_LOAD_ROWS(B200F_STORAGE_F16, 2);
+            else B200F_LOAD_ROWS(B200F_STORAGE_F16, 1);
             break;
         case B200F_STORAGE_BF16:
-            load_rows_kernel<B200F_STORAGE_BF16><<<(int)g, 256, 0, st>>>(rows, n, d, pitch_elems, dst);
+            if (v == 8) B200F_LOAD_ROWS(B200F_STORAGE_BF16, 8);
+            else if (v >= 2) B200F_LOAD_ROWS(B200F_STORAGE_BF16, 2);
+            else B200F_LOAD_ROWS(B200F_STORAGE_BF16, 1);
             break;
         default:
             return B200F_ERR_BAD_ARG;
     }
+#undef B200F_LOAD_ROWS
     count_launch();
     B200F_LAUNCH_CHECK();
     return B200F_OK;

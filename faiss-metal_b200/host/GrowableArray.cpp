@@ -8,6 +8,7 @@
 #include <mutex>
 #include <stdexcept>
 #include <string>
+#include <utility>
 
 namespace faiss_b200 {
 
@@ -132,6 +133,7 @@ void GrowableDeviceArray::back(size_t offset, size_t bytes) {
         const size_t off = g * granule_, size = (e - g) * granule_;
         CUmemGenericAllocationHandle h = 0;
         CUresult r = api().create(&h, size, &prop, 0);
+        if (r == CUDA_ERROR_OUT_OF_MEMORY && trimRetainedStorage(device_) > 0) r = api().create(&h, size, &prop, 0);
         if (r != CUDA_SUCCESS)
             throw std::runtime_error("faiss-b200: failed to allocate " + std::to_string(size) +
                                      " bytes of device memory for the index (driver error " +
@@ -166,6 +168,74 @@ void GrowableDeviceArray::release() {
     reserved_ = 0;
     backedBytes_ = 0;
     device_ = -1;
+}
+
+// ---- storage kept between reset() and the next add() ------------------------------------------
+namespace {
+
+struct Registry {
+    std::mutex mu;
+    std::vector<std::pair<const void*, std::unique_ptr<IndexArrays>>> held;   // oldest first
+};
+Registry& registry() {
+    static Registry* r = new Registry;   // never destroyed: indexes may outlive static destructors
+    return *r;
+}
+
+}  // namespace
+
+void retainStorage(const void* owner, std::unique_ptr<IndexArrays> arrays) {
+    if (!arrays) return;
+    const int device = arrays->device;
+    std::vector<std::unique_ptr<IndexArrays>> drop;   // unmapped outside the lock
+    {
+        Registry& r = registry();
+        std::lock_guard<std::mutex> g(r.mu);
+        r.held.emplace_back(owner, std::move(arrays));
+        size_t total = 0;
+        for (auto& h : r.held)
+            if (h.second->device == device) total += h.second->backedBytes();
+        for (size_t i = 0; i < r.held.size() && total > kRetainBytes;) {
+            if (r.held[i].second->device != device) {
+                i++;
+                continue;
+            }
+            total -= r.held[i].second->backedBytes();
+            drop.push_back(std::move(r.held[i].second));
+            r.held.erase(r.held.begin() + (long)i);
+        }
+    }
+}
+
+std::unique_ptr<IndexArrays> takeRetainedStorage(const void* owner) {
+    Registry& r = registry();
+    std::lock_guard<std::mutex> g(r.mu);
+    for (size_t i = 0; i < r.held.size(); i++)
+        if (r.held[i].first == owner) {
+            std::unique_ptr<IndexArrays> a = std::move(r.held[i].second);
+            r.held.erase(r.held.begin() + (long)i);
+            return a;
+        }
+    return nullptr;
+}
+
+size_t trimRetainedStorage(int device) {
+    std::vector<std::unique_ptr<IndexArrays>> drop;
+    {
+        Registry& r = registry();
+        std::lock_guard<std::mutex> g(r.mu);
+        for (size_t i = 0; i < r.held.size();) {
+            if (r.held[i].second->device != device) {
+                i++;
+                continue;
+            }
+            drop.push_back(std::move(r.held[i].second));
+            r.held.erase(r.held.begin() + (long)i);
+        }
+    }
+    size_t bytes = 0;
+    for (auto& a : drop) bytes += a->backedBytes();
+    return bytes;
 }
 
 }  // namespace faiss_b200

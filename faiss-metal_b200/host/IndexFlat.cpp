@@ -29,6 +29,7 @@ namespace faiss_b200 {
 namespace {
 
 constexpr size_t kStageBytes = 32ull << 20;   // fp32 staging chunk of add / reconstruct_n (two in flight)
+constexpr int64_t kScaleSampleRows = 8192;    // rows an fp32 index takes its plane scale from
 constexpr int64_t kGraphMaxQueries = 8;        // searches this small are replayed from a CUDA graph
 constexpr size_t kMaxGraphs = 8;               // graphs kept per index (least recently used goes)
 constexpr int64_t kFusedBatch = 16384;        // queries per launch, k <= 1024 (fused kernel, lists)
@@ -156,12 +157,9 @@ struct B200IndexFlat::Impl {
     // added; see GrowableArray.h).  When the driver calls are not available, or
     // B200F_NO_VMM=1 is set in the environment (testing), plain allocations with the
     // reference's allocate-copy-free growth are used instead.
-    GrowableDeviceArray vRows, vPlanes, vNorms;
-    bool inPlace = false;
-    int64_t maxRows = 0;          // rows the reserved ranges can hold
-    int64_t planeStrideFixed = 0;  // elements between split planes when inPlace
+    std::unique_ptr<IndexArrays> arrays;   // null: plain allocations, or no storage at all
 
-    int64_t planeStride() const { return inPlace ? planeStrideFixed : capacity * planePitch; }
+    int64_t planeStride() const { return arrays ? arrays->planeStride : capacity * planePitch; }
     int growthMode = -1;           // -1: process default, 0: in place, 1: allocate-copy-free
 
     // FP32 storage: format of the split planes (B200F_PLANES_*).  An index starts with two fp16
@@ -213,12 +211,11 @@ struct B200IndexFlat::Impl {
         seenShapes.clear();
     }
 
-    void freeStorage() {
-        if (inPlace) {
-            vRows.release();
-            vPlanes.release();
-            vNorms.release();
-            inPlace = false;
+    // keep: the mapped memory stays reachable for this index's next add() (see retainStorage)
+    void freeStorage(bool keep = false) {
+        if (arrays) {
+            if (keep) retainStorage(this, std::move(arrays));
+            arrays.reset();
         } else {
             if (rows) res->deallocBuffer(rows);
             if (planes) res->deallocBuffer(planes);
@@ -230,57 +227,56 @@ struct B200IndexFlat::Impl {
         capacity = 0;
     }
 
-    // First allocation of an empty index: reserve the address ranges.  Returns false (nothing
-    // reserved) when in-place growth cannot be used.
+    // First allocation of an empty index: reserve the address ranges, or take back what reset()
+    // left mapped.  Returns false (nothing reserved) when in-place growth cannot be used.
     bool reserveInPlace() {
+        std::unique_ptr<IndexArrays> a = takeRetainedStorage(this);
         if (growthMode == 1 || (growthMode < 0 && growthByCopyDefault())) return false;
         const int dev = res->getDevice();
-        if (!GrowableDeviceArray::supported(dev)) return false;
-        const size_t es = elemBytes(storage);
-        const size_t rowBytes = (size_t)pitch * es;
-        // no shard can hold more rows than fit the device memory (or the int32 row numbers)
-        size_t freeB = 0, totalB = 0;
-        if (cudaMemGetInfo(&freeB, &totalB) != cudaSuccess) {
-            (void)cudaGetLastError();
-            return false;
+        if (!a) {
+            if (!GrowableDeviceArray::supported(dev)) return false;
+            const size_t rowBytes = (size_t)pitch * elemBytes(storage);
+            // no shard can hold more rows than fit the device memory (or the int32 row numbers)
+            size_t freeB = 0, totalB = 0;
+            if (cudaMemGetInfo(&freeB, &totalB) != cudaSuccess) {
+                (void)cudaGetLastError();
+                return false;
+            }
+            int64_t cap = (int64_t)(totalB / rowBytes);
+            cap = std::min<int64_t>(cap, B200DeviceCapabilities::kMaxVectorsPerShard);
+            cap = std::max<int64_t>(cap, 1024);
+            // planes start on 2 MiB multiples of a common stride, so that each one is backed on its own
+            const size_t planeBytes = roundUp((int64_t)((size_t)cap * planePitch * 2), 2ll << 20);
+            a.reset(new IndexArrays);
+            a->device = dev;
+            a->maxRows = cap;
+            a->planeStride = (int64_t)(planeBytes / 2);
+            bool ok = a->rows.reserve(dev, (size_t)cap * rowBytes);
+            if (ok && storage == StorageType::Float32) ok = a->planes.reserve(dev, 3 * planeBytes);
+            if (ok && l2) ok = a->norms.reserve(dev, (size_t)cap * 4);
+            if (!ok) return false;
         }
-        int64_t cap = (int64_t)(totalB / rowBytes);
-        cap = std::min<int64_t>(cap, B200DeviceCapabilities::kMaxVectorsPerShard);
-        cap = std::max<int64_t>(cap, 1024);
-        // planes start on 2 MiB multiples of a common stride, so that each one is backed on its own
-        const size_t planeBytes = roundUp((int64_t)((size_t)cap * planePitch * 2), 2ll << 20);
-        bool ok = vRows.reserve(dev, (size_t)cap * rowBytes);
-        if (ok && storage == StorageType::Float32) ok = vPlanes.reserve(dev, 3 * planeBytes);
-        if (ok && l2) ok = vNorms.reserve(dev, (size_t)cap * 4);
-        if (!ok) {
-            vRows.release();
-            vPlanes.release();
-            vNorms.release();
-            return false;
-        }
-        maxRows = cap;
-        planeStrideFixed = (int64_t)(planeBytes / 2);
-        rows = vRows.data();
-        planes = storage == StorageType::Float32 ? static_cast<uint16_t*>(vPlanes.data()) : nullptr;
-        norms = l2 ? static_cast<float*>(vNorms.data()) : nullptr;
-        inPlace = true;
+        arrays = std::move(a);
+        rows = arrays->rows.data();
+        planes = storage == StorageType::Float32 ? static_cast<uint16_t*>(arrays->planes.data()) : nullptr;
+        norms = l2 ? static_cast<float*>(arrays->norms.data()) : nullptr;
         return true;
     }
 
     // Grow to hold at least `want` rows; keeps the first `keep` rows.
     void grow(int64_t want, int64_t keep) {
         if (want <= capacity) return;
-        if (capacity == 0 && !rows && !inPlace) (void)reserveInPlace();
-        if (inPlace) {
-            if (want > maxRows)
+        if (capacity == 0 && !rows && !arrays) (void)reserveInPlace();
+        if (arrays) {
+            if (want > arrays->maxRows)
                 throw B200RuntimeError(B200F_ERR_OOM, "faiss-b200: the index cannot hold " + std::to_string(want) +
                                                               " rows on this device");
             const size_t es = elemBytes(storage);
-            vRows.back(0, (size_t)want * pitch * es);
+            arrays->rows.back(0, (size_t)want * pitch * es);
             if (planes)
                 for (int p = 0; p < planesBacked(); p++)
-                    vPlanes.back((size_t)p * planeStrideFixed * 2, (size_t)want * planePitch * 2);
-            if (norms) vNorms.back(0, (size_t)want * 4);
+                    arrays->planes.back((size_t)p * arrays->planeStride * 2, (size_t)want * planePitch * 2);
+            if (norms) arrays->norms.back(0, (size_t)want * 4);
             capacity = want;
             return;
         }
@@ -404,6 +400,7 @@ B200IndexFlat::~B200IndexFlat() {
         (void)cudaStreamSynchronize(impl_->stream());
         impl_->invalidateGraphs();
         impl_->freeStorage();
+        (void)takeRetainedStorage(impl_.get());   // unmapped here
         impl_->res->deallocBuffer(impl_->status);
         impl_->res->deallocBuffer(impl_->oneRow);
         free_pinned(impl_->hostStatus);
@@ -463,6 +460,29 @@ void B200IndexFlat::add(faiss::idx_t n, const float* x) {
     const size_t es = elemBytes(impl_->storage);
     const bool fp32 = impl_->storage == StorageType::Float32;
     if (fp32) cudaCheck(cudaMemsetAsync(impl_->rangeFlag(), 0, 4, st), "add: clear range flag");
+    bool scaleFromSample = false;
+    auto setPlaneScale = [&](const float* src, int64_t nr, int64_t pitch) {
+        uint32_t* bits = reinterpret_cast<uint32_t*>(impl_->rangeFlag() + 1);
+        abiCheck(b200f_rows_absmax(src, nr, d, pitch, bits, st), "add: rows absmax");
+        cudaCheck(cudaMemcpyAsync(impl_->hostStatus + 8, bits, 4, cudaMemcpyDeviceToHost, st), "add: absmax copy");
+        cudaCheck(cudaStreamSynchronize(st), "add: synchronize");
+        float amax;
+        std::memcpy(&amax, impl_->hostStatus + 8, 4);
+        int e = 0;
+        if (amax > 0.f) (void)std::frexp(amax, &e);
+        impl_->planeScaleLog2 = amax > 0.f ? std::max(-120, std::min(120, 7 - e)) : 0;
+        impl_->planeScaleKnown = amax > 0.f;   // all-zero rows say nothing: ask the next block again
+        return impl_->planeScaleKnown;
+    };
+    // the stored fp32 rows split again (their planes only), in the index's present format and scale
+    auto resplit = [&](int64_t nr) {
+        abiCheck(b200f_store_rows_fp32(static_cast<const float*>(impl_->rows), impl_->pitch, nr, d,
+                                       static_cast<float*>(impl_->rows), impl_->pitch, impl_->planes, impl_->planePitch,
+                                       impl_->planeStride(), impl_->planeFormat,
+                                       impl_->planeFormat == B200F_PLANES_FP16X2 ? impl_->planeScaleLog2 : 0,
+                                       impl_->rangeFlag(), impl_->norms, impl_->l2 ? 1 : 0, st),
+                 "add: re-split rows");
+    };
     auto store = [&](const float* src, int64_t r0, int64_t nr) {
         const int64_t row = ntotal + r0;
         if (!fp32) {
@@ -474,17 +494,13 @@ void B200IndexFlat::add(faiss::idx_t n, const float* x) {
             return;
         }
         if (impl_->planeFormat == B200F_PLANES_FP16X2 && !impl_->planeScaleKnown) {
-            // the index's scale: the largest element of the first rows it is given goes to [2^6, 2^7)
-            uint32_t* bits = reinterpret_cast<uint32_t*>(impl_->rangeFlag() + 1);
-            abiCheck(b200f_rows_absmax(src, nr, d, d, bits, st), "add: rows absmax");
-            cudaCheck(cudaMemcpyAsync(impl_->hostStatus + 8, bits, 4, cudaMemcpyDeviceToHost, st), "add: absmax copy");
-            cudaCheck(cudaStreamSynchronize(st), "add: synchronize");
-            float amax;
-            std::memcpy(&amax, impl_->hostStatus + 8, 4);
-            int e = 0;
-            if (amax > 0.f) (void)std::frexp(amax, &e);
-            impl_->planeScaleLog2 = amax > 0.f ? std::max(-120, std::min(120, 7 - e)) : 0;
-            impl_->planeScaleKnown = amax > 0.f;   // all-zero rows say nothing: ask the next block again
+            // The index's scale: the largest element of the first rows it is given goes to [2^6, 2^7).  A
+            // few thousand rows spread over the block tell it (a pass over all of them costs a quarter of
+            // what storing them does: 242 us of 1.5 GB); rows that do not fit it raise the range flag.
+            const int64_t stride = std::max<int64_t>(1, nr / kScaleSampleRows);
+            if (!setPlaneScale(src, (nr + stride - 1) / stride, (int64_t)d * stride) && stride > 1)
+                (void)setPlaneScale(src, nr, d);   // nothing but zeros in the sample
+            scaleFromSample = stride > 1;
         }
         abiCheck(b200f_store_rows_fp32(src, d, nr, d, static_cast<float*>(impl_->rows) + (size_t)row * impl_->pitch,
                                        impl_->pitch, impl_->planes + (size_t)row * impl_->planePitch, impl_->planePitch,
@@ -566,17 +582,23 @@ void B200IndexFlat::add(faiss::idx_t n, const float* x) {
     cudaCheck(cudaStreamSynchronize(st), "add: synchronize");
     ntotal = newTotal;
     impl_->mirrorValid = false;
-    if (fp32 && impl_->planeFormat == B200F_PLANES_FP16X2 && impl_->hostStatus[9] != 0) {
-        // a row of this add does not fit fp16's range at the index's scale: three bf16 planes
-        // from now on, re-split from the stored fp32 rows
+    auto flagged = [&] { return fp32 && impl_->planeFormat == B200F_PLANES_FP16X2 && impl_->hostStatus[9] != 0; };
+    if (flagged() && scaleFromSample) {
+        // the sample missed the largest rows: the scale of all of them, if there is one
+        cudaCheck(cudaMemsetAsync(impl_->rangeFlag(), 0, 4, st), "add: clear range flag");
+        (void)setPlaneScale(static_cast<const float*>(impl_->rows), ntotal, impl_->pitch);
+        resplit(ntotal);
+        cudaCheck(cudaMemcpyAsync(impl_->hostStatus + 9, impl_->rangeFlag(), 4, cudaMemcpyDeviceToHost, st),
+                  "add: range flag copy");
+        cudaCheck(cudaStreamSynchronize(st), "add: synchronize");
+    }
+    if (flagged()) {
+        // a row does not fit fp16's range at the index's scale: three bf16 planes from now on
         impl_->planeFormat = B200F_PLANES_BF16X3;
-        if (impl_->inPlace)
-            impl_->vPlanes.back((size_t)2 * impl_->planeStrideFixed * 2, (size_t)impl_->capacity * impl_->planePitch * 2);
-        abiCheck(b200f_store_rows_fp32(static_cast<const float*>(impl_->rows), impl_->pitch, ntotal, d,
-                                       static_cast<float*>(impl_->rows), impl_->pitch, impl_->planes, impl_->planePitch,
-                                       impl_->planeStride(), B200F_PLANES_BF16X3, 0, nullptr, impl_->norms,
-                                       impl_->l2 ? 1 : 0, st),
-                 "add: re-split rows");
+        if (impl_->arrays)
+            impl_->arrays->planes.back((size_t)2 * impl_->arrays->planeStride * 2,
+                                       (size_t)impl_->capacity * impl_->planePitch * 2);
+        resplit(ntotal);
         cudaCheck(cudaStreamSynchronize(st), "add: synchronize");
     }
 }
@@ -585,7 +607,7 @@ void B200IndexFlat::reset() {
     DeviceGuard g(impl_->res->getDevice());
     cudaCheck(cudaStreamSynchronize(impl_->stream()), "reset: synchronize");
     impl_->invalidateGraphs();
-    impl_->freeStorage();
+    impl_->freeStorage(true);
     impl_->planeFormat = impl_->planeFormatWanted;
     impl_->planeScaleKnown = false;
     impl_->planeScaleLog2 = 0;

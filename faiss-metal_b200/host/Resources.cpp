@@ -13,6 +13,7 @@
 #include "../../include/b200_flat.h"
 #include "../include/faiss-b200/B200Exception.h"
 #include "../include/faiss-b200/StandardB200Resources.h"
+#include "GrowableArray.h"
 
 namespace faiss_b200 {
 
@@ -37,6 +38,16 @@ struct DeviceGuard {
         if (prev >= 0 && cudaGetDevice(&cur) == cudaSuccess && cur != prev) (void)cudaSetDevice(prev);
     }
 };
+
+// cudaMalloc; when the device is full, once more after reset() indexes have given up what they retain
+cudaError_t mallocOrTrim(void** p, size_t bytes, int device) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && trimRetainedStorage(device) > 0) {
+        (void)cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
 
 }  // namespace
 
@@ -277,7 +288,7 @@ void StandardB200Resources::waitStream(StreamHandle producer) {
 void* StandardB200Resources::allocBuffer(size_t size) {
     DeviceGuard g(impl_->device);
     void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, size ? size : 256);
+    cudaError_t e = mallocOrTrim(&p, size ? size : 256, impl_->device);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
         throw B200RuntimeError(e == cudaErrorMemoryAllocation ? B200F_ERR_OOM : B200F_ERR_CUDA,
@@ -295,9 +306,10 @@ void StandardB200Resources::deallocBuffer(void* buf) {
 
 void* StandardB200Resources::acquireDeviceTemp(size_t size) {
     DeviceGuard g(impl_->device);
-    void* p = impl_->devicePool.acquire(size, [](size_t n) -> void* {
+    const int device = impl_->device;
+    void* p = impl_->devicePool.acquire(size, [device](size_t n) -> void* {
         void* q = nullptr;
-        if (cudaMalloc(&q, n) != cudaSuccess) {
+        if (mallocOrTrim(&q, n, device) != cudaSuccess) {
             (void)cudaGetLastError();
             return nullptr;
         }
@@ -342,7 +354,7 @@ void* StandardB200Resources::getScratch(size_t bytes) {
         if (e != cudaSuccess) {
             (void)cudaGetLastError();
             want = (bytes + 255) & ~(size_t)255;
-            check(cudaMalloc(&impl_->scratch, want), "cudaMalloc(scratch)");
+            check(mallocOrTrim(&impl_->scratch, want, impl_->device), "cudaMalloc(scratch)");
         }
         impl_->scratchBytes = want;
     }

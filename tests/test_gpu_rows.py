@@ -1,0 +1,92 @@
+"""store_rows / load_rows at the row lengths where their vector width, lanes per row and pads change,
+and the storage an index keeps between reset() and the next add()."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import helpers as H
+from oracle import flat_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+@pytest.mark.parametrize("storage", [0, 1, 2])
+@pytest.mark.parametrize("d", [1, 2, 4, 6, 7, 8, 12, 31, 32, 36, 66, 100, 127, 132, 520, 770, 1028])
+def test_store_and_load_rows(fm, res, storage, d):
+    from test_gpu_ops import Stored, cur_stream, vp
+    n = 61 if d > 64 else 1003   # not a multiple of the rows a warp takes
+    xb = H.uniform_pm1(n, d, d)
+    st = Stored(fm, xb, storage)
+    eff = O.round_storage(xb, storage)
+    # squares of d values <= 1 summed in fp32 in any order: d * 2^-24 relative, below 1e-4 for d <= 1028
+    np.testing.assert_allclose(st.norms[:n].cpu().numpy(), O.row_norms(eff), rtol=(d + 4) * 2.0 ** -24)
+    back = torch.full((n, d), float("nan"), device="cuda:0")
+    fm.abi.check_op(fm.lib().b200f_load_rows(vp(st.rows), storage, n, d, st.pitch, vp(back), cur_stream()), "load_rows")
+    assert np.array_equal(back.cpu().numpy().view(np.uint32), eff.view(np.uint32))
+    if storage == 0:
+        assert not st.rows.view(torch.float32).reshape(n, st.pitch)[:, d:].any()       # pads are zero
+        planes = st.planes.view(torch.bfloat16).reshape(3, n, st.ppitch).to(torch.float64)
+        np.testing.assert_allclose(planes[:, :, :d].sum(0).cpu().numpy(), xb.astype(np.float64), rtol=2.0 ** -22, atol=1e-30)
+        assert not planes[:, :, d:st.ppitch - 8].any() and not planes[1:, :, d:].any()
+    else:
+        bits = st.rows.view(torch.int16).reshape(n, st.pitch)
+        assert not bits[:, d:st.pitch - 8].any() and not bits[:, st.pitch - 4:].any()
+
+
+@pytest.mark.parametrize("storage", [0, 1])
+def test_storage_kept_by_reset(fm, res, storage):
+    # refilled with fewer, more and equally many rows, beside a second index that resets in between
+    d = 72
+    xb = H.uniform_pm1(9000, d, 3)
+    xq = H.uniform_pm1(12, d, 4)
+    a = fm.B200IndexFlat(res, d, O.METRIC_L2, storage)
+    b = fm.B200IndexFlat(res, d, O.METRIC_INNER_PRODUCT, storage)
+    for n in (5000, 1200, 9000, 9000):
+        a.add(xb[:n])
+        b.add(xb[:n // 2])
+        b.reset()
+        assert b.ntotal == 0 and b.device_rows() == 0
+        assert np.array_equal(a.reconstruct_n(0, n), O.round_storage(xb[:n], storage))
+        D, I = a.search(xq, 10)
+        H.check_against_oracle(O.METRIC_L2, storage, True, xb[:n], xq, 10, D, I)
+        a.reset()
+        assert a.ntotal == 0 and a.device_rows() == 0
+    a.set_growth_mode(1)           # retained storage is dropped when the index changes its growth mode
+    a.add(xb)
+    assert np.array_equal(a.reconstruct_n(0, 9000), O.round_storage(xb, storage))
+    a.close()
+    b.close()
+
+
+def test_reset_gives_back_what_exceeds_the_bound(fm, res):
+    # 9.2 GB of rows: more than an index may keep, so reset() returns the memory to the device
+    d = 768
+    n = 3_000_000
+    x = torch.zeros((250_000, d), device="cuda:0")
+    idx = fm.B200IndexFlat(res, d, O.METRIC_INNER_PRODUCT, 0)
+    free0 = torch.cuda.mem_get_info()[0]
+    idx.reserve(n)
+    idx.add(x)
+    assert free0 - torch.cuda.mem_get_info()[0] > 8 << 30
+    idx.reset()
+    assert free0 - torch.cuda.mem_get_info()[0] < 1 << 30
+    idx.close()
+
+
+@pytest.mark.parametrize("n", [8192, 30_000])
+def test_plane_scale_from_a_sample(fm, res, n):
+    # one row 600 times larger than the others: over fp16's range at a scale made for them (2^7), while they
+    # stay inside it (0.95 / 8 >= 2^-4) at the scale made for it; of 30,000 rows the sample takes every third
+    d = 48
+    xb = H.uniform_pm1(n, d, 11)
+    xb[n - 2] *= np.float32(600.0)
+    idx = fm.B200IndexFlat(res, d, O.METRIC_L2, 0)
+    idx.add(xb)
+    assert idx.fp32_planes == fm.abi.PLANES_FP16X2
+    xq = H.uniform_pm1(40, d, 12)
+    D, I = idx.search(xq, 10)
+    H.check_against_oracle(O.METRIC_L2, 0, True, xb, xq, 10, D, I)
+    idx.close()
