@@ -170,7 +170,6 @@ int launch_select_candidates(const float* cand_key, const int32_t* cand_idx, con
 // select_rank.cu: the same selection / merge for inputs of at most 8192 entries per row, sorted in
 // registers and placed by binary search; results identical to the kernels of select.cu.
 bool rank_select_enabled();
-bool rank_select_fits(int cap, int k);
 int launch_rank_select(const float* cand_key, const int32_t* cand_idx, const int32_t* cand_cnt, int cap,
                        int64_t nb, int64_t nq, int k, int metric, const float* qnorm, int64_t label_base,
                        float* out_dist, int64_t* out_labels, int32_t* dirty, cudaStream_t stream);

@@ -15,7 +15,6 @@
 //    Sources: a key matrix chunk, sorted lists of other ranks, the fused kernel's 32-entry
 //    lists, or a threshold-filtered candidate buffer; the last two also report rows whose
 //    result is not proven exact.
-//  * select_small: k <= 32 from a candidate buffer, one warp per query.
 //  * compact_rows / gather_rows: the rows to redo, counted and gathered on the device.
 //
 // Keys are "smaller is better" everywhere: L2 key = distance, inner product key = -dot.
@@ -514,57 +513,7 @@ __global__ void __launch_bounds__(SS_THREADS) sort_select_kernel(const SortSelec
     }
 }
 
-// k <= 32 from an unordered candidate buffer of a few hundred to a few thousand entries per
-// row: one WARP per row.  The lanes read 32 candidates at a time; those that beat the current
-// k-th best are inserted one after the other into the warp's sorted list (lane j = rank j).
-// About 32 ln(n / 32) + 32 insertions per row; a 1024-thread bitonic sort per row would cost
-// fifty barrier rounds for the same result.
 constexpr int SEL_WARPS = 8;
-__global__ void __launch_bounds__(SEL_WARPS * 32) select_small_kernel(const SortSelectParams p) {
-    const int lane = threadIdx.x & 31;
-    const int64_t warp0 = (int64_t)blockIdx.x * SEL_WARPS + (threadIdx.x >> 5);
-    const int64_t nwarps = (int64_t)gridDim.x * SEL_WARPS;
-    const int64_t nq_live = p.nq_dev ? min((int64_t)*p.nq_dev, p.nq) : p.nq;
-    for (int64_t q = warp0; q < nq_live; q += nwarps) {
-        const int64_t cnt = __ldg(p.cand_cnt + q);
-        const int n = (int)min(cnt, p.ld);
-        const float* keys = p.keys + q * p.ld;
-        const int32_t* ids = p.part_idx + q * p.ld;
-        float lk = CUDART_INF_F;
-        int32_t li = -1;
-        float thr = CUDART_INF_F;
-        int32_t thr_id = -1;
-        for (int base = 0; base < n; base += 32) {
-            const int c = base + lane;
-            const float key = c < n ? p.key_sign * __ldg(keys + c) : CUDART_INF_F;
-            const int32_t id = c < n ? __ldg(ids + c) : -1;
-            unsigned m = __ballot_sync(FULL, id >= 0 && before_id<int32_t>(key, id, thr, thr_id));
-            while (m) {
-                const int src = __ffs(m) - 1;
-                m &= m - 1;
-                const float s = __shfl_sync(FULL, key, src);
-                const int32_t sid = __shfl_sync(FULL, id, src);
-                if (before_id<int32_t>(s, sid, thr, thr_id)) {  // the bound moved since the ballot
-                    warp_insert_id<int32_t>(lk, li, s, sid, lane);
-                    thr = __shfl_sync(FULL, lk, p.k - 1);
-                    thr_id = __shfl_sync(FULL, li, p.k - 1);
-                }
-            }
-        }
-        if (lane < p.k) {
-            float dist = p.pad;
-            int64_t label = -1;
-            if (li >= 0) {
-                dist = p.out_sign * lk + (p.qnorm ? p.qnorm[q] : 0.f);
-                if (p.clamp && dist < 0.f) dist = 0.f;
-                label = (int64_t)li + p.label_base;
-            }
-            p.out_dist[q * p.k + lane] = dist;
-            p.out_labels[q * p.k + lane] = label;
-        }
-        if (lane == 0 && p.dirty) p.dirty[q] = ((cnt > p.ld) || (cnt < p.k && cnt < p.nb_total)) ? 1 : 0;
-    }
-}
 
 // The r <= 32 smallest keys of a matrix row (the pilot sample of the threshold filter): one warp
 // per row reads 128 columns at a time; a key under the current r-th best is inserted into the
@@ -707,42 +656,6 @@ __global__ void finalize_lists_kernel(const float* __restrict__ run_key,
 
 }  // namespace
 
-int launch_merge_partials(const float* part_key, const int32_t* part_idx, int P, int64_t nq, int k,
-                          int metric, const float* qnorm, int64_t label_base, float* out_dist,
-                          int64_t* out_labels, const int* nq_dev, const int32_t* row_map,
-                          cudaStream_t stream) {
-    if (nq <= 0) return B200F_OK;
-    if (k < 1 || k > 32 || P < 1) return B200F_ERR_UNSUPPORTED;
-    MergeSmallParams<int32_t> p{};
-    p.nq_dev = nq_dev;
-    p.row_map = row_map;
-    p.in_key = part_key;
-    p.in_id = part_idx;
-    p.q_stride = (int64_t)P * k;
-    p.p_stride = k;
-    p.p_stride_id = k;
-    p.P = P;
-    p.nq = nq;
-    p.k = k;
-    p.key_sign = 1.f;
-    const bool l2 = metric == B200F_METRIC_L2;
-    p.out_sign = l2 ? 1.f : -1.f;
-    p.qnorm = l2 ? qnorm : nullptr;
-    p.clamp = l2 ? 1 : 0;
-    p.pad = l2 ? kHostInf : -kHostInf;
-    p.label_base = label_base;
-    p.out_dist = out_dist;
-    p.out_labels = out_labels;
-    int64_t g = nq;
-    const int64_t cap = (int64_t)cached_sm_count() * 32;
-    if (g > cap) g = cap;
-    if (nq_dev && g > cached_sm_count()) g = cached_sm_count();
-    merge_small_kernel<int32_t><<<(int)g, MS_THREADS, 0, stream>>>(p);
-    count_launch();
-    B200F_LAUNCH_CHECK();
-    return B200F_OK;
-}
-
 int launch_merge_keys(const float* part_key, const int32_t* part_idx, int P, int64_t nq, int k,
                       float* out_key, cudaStream_t stream) {
     if (nq <= 0) return B200F_OK;
@@ -832,7 +745,7 @@ int launch_select_candidates(const float* cand_key, const int32_t* cand_idx, con
                              int64_t label_base, float* out_dist, int64_t* out_labels, int32_t* dirty,
                              cudaStream_t stream) {
     if (cap < 1 || !cand_cnt) return B200F_ERR_BAD_ARG;
-    if (rank_select_enabled() && rank_select_fits(cap, k) && dirty)
+    if (rank_select_enabled() && dirty)
         return launch_rank_select(cand_key, cand_idx, cand_cnt, cap, nb, nq, k, metric, qnorm, label_base,
                                   out_dist, out_labels, dirty, stream);
     const bool l2 = metric == B200F_METRIC_L2;
@@ -854,16 +767,6 @@ int launch_select_candidates(const float* cand_key, const int32_t* cand_idx, con
     p.out_dist = out_dist;
     p.out_labels = out_labels;
     p.dirty = dirty;
-    if (k <= 32) {
-        if (nq <= 0) return B200F_OK;
-        int64_t g = ceil_div64(nq, SEL_WARPS);
-        const int64_t gcap = (int64_t)cached_sm_count() * 8;
-        if (g > gcap) g = gcap;
-        select_small_kernel<<<(int)g, SEL_WARPS * 32, 0, stream>>>(p);
-        count_launch();
-        B200F_LAUNCH_CHECK();
-        return B200F_OK;
-    }
     return launch_sort_select<SRC_PARTS>(p, stream);
 }
 

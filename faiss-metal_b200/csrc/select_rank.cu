@@ -4,14 +4,8 @@
 // list merge of the fused kernels (shaders/fused_l2_topk.metal:88-131) for the two inputs that
 // are small enough to need no streaming:
 //
-//  * rank_select: the k best (32 < k <= 4096) of a row's threshold-filtered candidates, an
-//    unordered buffer of at most 8192 (key, id) pairs, typically several times k.  A CTA of W
-//    warps takes one row.  (1) The k-th smallest key is found exactly by a radix select over the
-//    keys' spread (8 bits a pass, histogram in shared memory).  (2) The candidates up to that key
-//    (k of them plus ties) are compacted.  (3) Every warp sorts its share of them in registers
-//    (bitonic network over 32 R elements, R per lane: strides below R are register swaps, the
-//    others one shuffle pair), the sorted runs go to shared memory, and every element finds its
-//    final position as its own index plus its lower bounds in the other runs.
+//  * row_select: the k best of a row's few hundred to few thousand (key, id) pairs in any order:
+//    threshold-filtered candidates, or the partial lists the fused kernels leave.  See the kernel.
 //  * rank_merge: P sorted result lists of k entries (other shards' answers), P k <= 8192.
 //    The lists are runs already.  Only entries up to the largest of the lists' (k / P)-th keys
 //    can belong to the result; each of those finds its position by binary search in the other
@@ -31,7 +25,6 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 constexpr uint64_t RS_EMPTY = ~0ull;
-constexpr int RS_MAX_WARPS = 8;
 constexpr int RS_RUN = 512;    // most elements one warp sorts (16 per lane)
 
 std::atomic<int> g_rank_select{1};
@@ -76,14 +69,18 @@ __device__ __forceinline__ void warp_sort(uint64_t (&v)[R], int lane) {
     }
 }
 
-struct RankSelectParams {
-    const float* keys;        // [nq][ld] candidate keys, smaller is better
-    const int32_t* ids;       // [nq][ld] row ids (-1 = empty)
-    const int32_t* cnt;       // [nq] candidates counted (may exceed ld: overflow)
+struct RowSelectParams {
+    const float* keys;        // [nq][ld] keys, smaller is better
+    const int32_t* ids;       // [nq][ld] row ids (-1 = empty); null: the id is the column, NaN keys are empty
+    const int32_t* cnt;       // candidates counted per row (may exceed ld: overflow); null: n
     int64_t ld;
-    int64_t nb_total;
+    int64_t n;
+    int64_t nb_total;         // rows in the shard (dirty)
     int64_t nq;
+    const int* nq_dev;        // optional: live rows (<= nq), read on the device
+    const int32_t* row_map;   // optional: row j belongs to query row_map[j]
     int k;
+    int bound;                // words of the staging area
     float out_sign;
     const float* qnorm;
     int clamp;
@@ -91,20 +88,20 @@ struct RankSelectParams {
     int64_t label_base;
     float* out_dist;
     int64_t* out_labels;
-    int32_t* dirty;
+    int32_t* dirty;           // optional: 1 when the result is not proven complete
 };
 
-__device__ __forceinline__ void rs_write(const RankSelectParams& p, int64_t q, int rank, uint64_t w) {
-    float dist = p.out_sign * ordered_to_float((uint32_t)(w >> 32)) + (p.qnorm ? p.qnorm[q] : 0.f);
+__device__ __forceinline__ void rs_write(const RowSelectParams& p, int64_t qo, int rank, uint64_t w) {
+    float dist = p.out_sign * ordered_to_float((uint32_t)(w >> 32)) + (p.qnorm ? p.qnorm[qo] : 0.f);
     if (p.clamp && dist < 0.f) dist = 0.f;
-    p.out_dist[q * p.k + rank] = dist;
-    p.out_labels[q * p.k + rank] = (int64_t)(uint32_t)w + p.label_base;
+    p.out_dist[qo * p.k + rank] = dist;
+    p.out_labels[qo * p.k + rank] = (int64_t)(uint32_t)w + p.label_base;
 }
 
 // Sort and place the c words staged in `runs` (all distinct); warp w takes words [w m, w m + m).
 // The staging area becomes the sorted runs, 32 R words per warp.
 template <int R>
-__device__ __forceinline__ void rank_place(const RankSelectParams& p, int64_t q, int c, int m,
+__device__ __forceinline__ void rank_place(const RowSelectParams& p, int64_t qo, int c, int m,
                                            uint64_t* runs, int W) {
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -121,165 +118,259 @@ __device__ __forceinline__ void rank_place(const RankSelectParams& p, int64_t q,
 #pragma unroll
     for (int r = 0; r < R; r++) runs[warp * N + lane * R + r] = v[r];
     __syncthreads();
+    int rank[R];
 #pragma unroll
-    for (int r = 0; r < R; r++) {
-        const int e = lane * R + r;
-        const uint64_t w = v[r];
-        if (w != RS_EMPTY && e < p.k) {
-            int rank = e;
-            for (int o = 0; o < W && rank < p.k; o++) {
-                if (o == warp) continue;
-                const uint64_t* run = runs + o * N;
-                int lo = 0, hi = N;       // words are distinct: the lower bound is the count
-                while (lo < hi) {
-                    const int mid = (lo + hi) >> 1;
-                    if (run[mid] < w) lo = mid + 1; else hi = mid;
-                }
-                rank += lo;
-            }
-            if (rank < p.k) rs_write(p, q, rank, w);
+    for (int r = 0; r < R; r++) rank[r] = lane * R + r;
+    for (int o = 0; o < W; o++) {
+        if (o == warp) continue;
+        // words are distinct: the lower bound is the count.  A fixed number of steps, so that the R
+        // searches of a lane run side by side instead of one after the other.
+        const uint64_t* run = runs + o * N;
+        int lo[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) lo[r] = 0;
+#pragma unroll
+        for (int step = N / 2; step > 0; step >>= 1) {
+#pragma unroll
+            for (int r = 0; r < R; r++) lo[r] += (run[lo[r] + step - 1] < v[r]) ? step : 0;
         }
+#pragma unroll
+        for (int r = 0; r < R; r++) rank[r] += lo[r] + (run[lo[r]] < v[r] ? 1 : 0);
     }
+#pragma unroll
+    for (int r = 0; r < R; r++)
+        if (v[r] != RS_EMPTY && rank[r] < p.k) rs_write(p, qo, rank[r], v[r]);
 }
 
-// W warps; at most W * RS_RUN candidates up to the k-th key are sorted here.  A row with more
-// (k-th key shared by hundreds of candidates) is reported through dirty[] like an overflowed
-// one, and the caller's exact redo pass takes it.
-__global__ void __launch_bounds__(RS_MAX_WARPS * 32, 4) rank_select_kernel(const RankSelectParams p) {
-    extern __shared__ __align__(16) uint64_t rs_runs[];   // W * RS_RUN words
+// The kk-th smallest x = key - mn of what `visit` enumerates (a callable that calls its argument with
+// the ordered key of every live element of this thread), 8 bits a pass over `bits` significant
+// bits, stopping when at most `slack` low bits are undecided: returns an upper bound of it that is
+// exact for slack = 0; kk is left at how many elements equal to it are among the kk smallest.  All
+// threads of the CTA call it; s_hist and s_sel are shared.
+template <typename Visit>
+__device__ __forceinline__ uint32_t radix_kth(Visit visit, uint32_t mn, int bits, int slack, int& kk,
+                                              int* s_hist, int* s_sel) {
+    const int tid = threadIdx.x, lane = tid & 31, T = blockDim.x;
+    uint32_t prefix = 0;
+    int hi = bits;
+    while (hi > slack) {
+        const int lo = hi > 8 ? hi - 8 : 0;
+        const uint32_t mask = (1u << (hi - lo)) - 1u;
+        for (int i = tid; i < 256; i += T) s_hist[i] = 0;
+        __syncthreads();
+        visit([&](uint32_t key) {
+            const uint32_t x = key - mn;
+            if ((uint32_t)((uint64_t)x >> hi) == prefix) atomicAdd(&s_hist[(x >> lo) & mask], 1);
+        });
+        __syncthreads();
+        if (tid < 32) {
+            int h[8], sum = 0;
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                h[i] = s_hist[lane * 8 + i];
+                sum += h[i];
+            }
+            int incl = sum;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int up = __shfl_up_sync(FULL, incl, o);
+                if (lane >= o) incl += up;
+            }
+            int below = incl - sum;
+            if (below < kk && kk <= incl) {   // exactly one lane
+                int digit = 0;
+#pragma unroll
+                for (int i = 0; i < 7; i++) {
+                    if (digit == i && below + h[i] < kk) {
+                        below += h[i];
+                        digit = i + 1;
+                    }
+                }
+                s_sel[0] = lane * 8 + digit;
+                s_sel[1] = kk - below;
+            }
+        }
+        __syncthreads();
+        prefix = (prefix << (hi - lo)) | (uint32_t)s_sel[0];
+        kk = s_sel[1];
+        hi = lo;
+    }
+    return hi > 0 ? (uint32_t)((((uint64_t)prefix + 1) << hi) - 1) : prefix;
+}
+
+// Block-wide live count, smallest and largest key.
+struct Spread {
+    int live;
+    uint32_t mn, mx;
+};
+__device__ __forceinline__ Spread block_spread(int live, uint32_t mn, uint32_t mx, int* s_live, uint32_t* s_min,
+                                               uint32_t* s_max) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        live += __shfl_xor_sync(FULL, live, o);
+        mn = min(mn, __shfl_xor_sync(FULL, mn, o));
+        mx = max(mx, __shfl_xor_sync(FULL, mx, o));
+    }
+    if (lane == 0) {
+        s_live[warp] = live;
+        s_min[warp] = mn;
+        s_max[warp] = mx;
+    }
+    __syncthreads();
+    live = lane < W ? s_live[lane] : 0;
+    mn = lane < W ? s_min[lane] : 0xffffffffu;
+    mx = lane < W ? s_max[lane] : 0u;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        live += __shfl_xor_sync(FULL, live, o);
+        mn = min(mn, __shfl_xor_sync(FULL, mn, o));
+        mx = max(mx, __shfl_xor_sync(FULL, mx, o));
+    }
+    return Spread{live, mn, mx};
+}
+
+constexpr int RS_COUNT_MAX = 256;   // so few words are placed by counting the smaller ones
+
+// One CTA per row, latency-bound (a row is a few KB in L1 / L2).  A pass over the keys leaves every
+// thread with the smallest key of its share; with k <= T / 2 the k-th smallest of those T minima
+// bounds the row's k-th key from above and admits little more than k keys (2 histogram passes over
+// T register values instead of 4 over the row).  Otherwise, or when that bound admits more than the
+// staging area holds, the k-th key is found exactly by radix select over the row.  The words up to
+// the bound are compacted and placed: by counting the smaller ones up to 256 of them, else sorted per
+// warp and placed by binary search.  Where even the exact k-th key is shared by more than fit (hundreds
+// of ties), a second radix select over the ids of those finds the ones that belong to the result.
+__global__ void __launch_bounds__(1024) row_select_kernel(const RowSelectParams p) {
+    extern __shared__ __align__(16) uint64_t rs_runs[];   // bound words
     __shared__ int s_hist[256];
-    __shared__ uint32_t s_min[RS_MAX_WARPS], s_max[RS_MAX_WARPS];
-    __shared__ int s_live[RS_MAX_WARPS];
+    __shared__ uint32_t s_min[32], s_max[32];
+    __shared__ int s_live[32];
     __shared__ int s_sel[2];
     __shared__ int s_count;
     const int W = blockDim.x >> 5;
     const int T = blockDim.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int bound = W * RS_RUN;
-    for (int64_t q = blockIdx.x; q < p.nq; q += gridDim.x) {
-        const int64_t cnt = __ldg(p.cnt + q);
+    const int64_t nq_live = p.nq_dev ? min((int64_t)*p.nq_dev, p.nq) : p.nq;
+    for (int64_t q = blockIdx.x; q < nq_live; q += gridDim.x) {
+        const int64_t cnt = p.cnt ? (int64_t)__ldg(p.cnt + q) : p.n;
         const int n = (int)min(cnt, p.ld);
         const float* keys = p.keys + q * p.ld;
-        const int32_t* ids = p.ids + q * p.ld;
-        // spread of the live keys (the row's few KB stay in L1 for the passes below)
+        const int32_t* ids = p.ids ? p.ids + q * p.ld : nullptr;
+        // (ordered key, live) of column c; both loads are issued before either is used
+        auto load = [&](int c, uint32_t& key, int32_t& id) {
+            const float f = __ldg(keys + c) + 0.f;   // -0 becomes +0: the two tie
+            id = ids ? __ldg(ids + c) : (f == f ? c : -1);
+            key = float_to_ordered(f);
+        };
         int live = 0;
         uint32_t mn = 0xffffffffu, mx = 0;
-#pragma unroll 4
+#pragma unroll 8
         for (int c = tid; c < n; c += T) {
-            const int32_t id = __ldg(ids + c);     // both loads issued before either is used
-            const uint32_t key = float_to_ordered(__ldg(keys + c));
+            uint32_t key;
+            int32_t id;
+            load(c, key, id);
             if (id >= 0) {
                 live++;
                 mn = min(mn, key);
                 mx = max(mx, key);
             }
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            live += __shfl_xor_sync(FULL, live, o);
-            mn = min(mn, __shfl_xor_sync(FULL, mn, o));
-            mx = max(mx, __shfl_xor_sync(FULL, mx, o));
-        }
-        if (lane == 0) {
-            s_live[warp] = live;
-            s_min[warp] = mn;
-            s_max[warp] = mx;
-        }
+        const uint32_t my_min = mn;
+        const int my_live = live;
         if (tid == 0) s_count = 0;
-        __syncthreads();
-        live = 0;
-        for (int w = 0; w < W; w++) {
-            live += s_live[w];
-            mn = min(mn, s_min[w]);
-            mx = max(mx, s_max[w]);
-        }
-        // x = key - mn; the k-th smallest x of the live candidates, exactly
-        uint32_t thr_x = live > 0 ? mx - mn : 0;
-        if (live > p.k) {
-            int hi = 32 - __clz(thr_x);   // significant bits of the spread; 0: all keys equal
-            uint32_t prefix = 0;
-            int kk = p.k;
-            while (hi > 0) {
-                const int lo = hi > 8 ? hi - 8 : 0;
-                const uint32_t mask = (1u << (hi - lo)) - 1u;
-                for (int i = tid; i < 256; i += T) s_hist[i] = 0;
-                __syncthreads();
+        const Spread sp = block_spread(live, mn, mx, s_live, s_min, s_max);
+        live = sp.live;
+        mn = sp.mn;
+        auto visit_all = [&](auto f) {
 #pragma unroll 4
-                for (int c = tid; c < n; c += T) {
-                    const int32_t id = __ldg(ids + c);
-                    const uint32_t x = float_to_ordered(__ldg(keys + c)) - mn;
-                    if (id >= 0 && (uint32_t)((uint64_t)x >> hi) == prefix)
-                        atomicAdd(&s_hist[(x >> lo) & mask], 1);
+            for (int c = tid; c < n; c += T) {
+                uint32_t key;
+                int32_t id;
+                load(c, key, id);
+                if (id >= 0) f(key);
+            }
+        };
+        const int bits = 32 - __clz(sp.mx - mn);   // significant bits of the spread (live > 0)
+        uint32_t thr_x = live > 0 ? sp.mx - mn : 0;
+        uint32_t tie_id = 0x7fffffffu;             // of the keys equal to thr_x: ids up to this one
+        bool loose = false;
+        if (live > p.k) {
+            loose = 2 * p.k <= T && __syncthreads_count(my_live > 0) >= p.k;
+            if (loose) {
+                int kk = p.k;
+                thr_x = radix_kth([&](auto f) { if (my_live > 0) f(my_min); }, mn, bits, bits > 16 ? bits - 16 : 0, kk,
+                                  s_hist, s_sel);
+            } else {
+                int kk = p.k;
+                thr_x = radix_kth(visit_all, mn, bits, 0, kk, s_hist, s_sel);
+            }
+        }
+        // compaction of the candidates up to the threshold (k of them plus a few, or all)
+        int c = 0;
+        for (int pass = 0; pass < 2; pass++) {
+            for (int c0 = warp * 32; c0 < n; c0 += T) {
+                const int cc = c0 + lane;
+                bool keep = false;
+                uint64_t word = 0;
+                if (cc < n) {
+                    uint32_t key;
+                    int32_t id;
+                    load(cc, key, id);
+                    const uint32_t x = key - mn;           // live keys are >= mn
+                    keep = id >= 0 && (x < thr_x || (x == thr_x && (uint32_t)id <= tie_id));
+                    word = ((uint64_t)key << 32) | (uint32_t)id;
                 }
-                __syncthreads();
-                if (warp == 0) {
-                    int h[8], sum = 0;
-#pragma unroll
-                    for (int i = 0; i < 8; i++) {
-                        h[i] = s_hist[lane * 8 + i];
-                        sum += h[i];
-                    }
-                    int incl = sum;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const int up = __shfl_up_sync(FULL, incl, o);
-                        if (lane >= o) incl += up;
-                    }
-                    int below = incl - sum;
-                    if (below < kk && kk <= incl) {   // exactly one lane
-                        int digit = 0;
-#pragma unroll
-                        for (int i = 0; i < 7; i++) {
-                            if (digit == i && below + h[i] < kk) {
-                                below += h[i];
-                                digit = i + 1;
-                            }
+                const unsigned b = __ballot_sync(FULL, keep);
+                int base = 0;
+                if (lane == 0 && b) base = atomicAdd(&s_count, __popc(b));
+                base = __shfl_sync(FULL, base, 0);
+                const int pos = base + __popc(b & ((1u << lane) - 1u));
+                if (keep && pos < p.bound) rs_runs[pos] = word;
+            }
+            __syncthreads();
+            c = s_count;
+            if (c <= p.bound || pass == 1) break;
+            // more than fit: the exact k-th key, and of the keys equal to it the ids that are wanted
+            // (exactly k words are kept the second time)
+            __syncthreads();   // everybody has read the count
+            if (tid == 0) s_count = 0;
+            int kk = p.k;
+            thr_x = radix_kth(visit_all, mn, bits, 0, kk, s_hist, s_sel);
+            tie_id = radix_kth(
+                    [&](auto f) {
+                        for (int cc = tid; cc < n; cc += T) {
+                            uint32_t key;
+                            int32_t id;
+                            load(cc, key, id);
+                            if (id >= 0 && key - mn == thr_x) f((uint32_t)id);
                         }
-                        s_sel[0] = lane * 8 + digit;
-                        s_sel[1] = kk - below;
-                    }
-                }
-                __syncthreads();
-                prefix = (prefix << (hi - lo)) | (uint32_t)s_sel[0];
-                kk = s_sel[1];
-                hi = lo;
-            }
-            thr_x = prefix;
+                    },
+                    0u, 31, 0, kk, s_hist, s_sel);
         }
-        // compaction of the candidates up to the threshold (k of them plus ties, or all)
-        for (int c0 = warp * 32; c0 < n; c0 += T) {
-            const int c = c0 + lane;
-            bool keep = false;
-            uint64_t word = 0;
-            if (c < n) {
-                const int32_t id = __ldg(ids + c);
-                const uint32_t key = float_to_ordered(__ldg(keys + c));
-                keep = id >= 0 && key - mn <= thr_x;   // live keys are >= mn
-                word = ((uint64_t)key << 32) | (uint32_t)id;
+        c = min(c, p.bound);   // ids are distinct: the second pass keeps k words
+        const int64_t qo = p.row_map ? (int64_t)p.row_map[q] : q;
+        if (c <= RS_COUNT_MAX) {
+            for (int i = tid; i < c; i += T) {
+                const uint64_t w = rs_runs[i];
+                int rank = 0;
+#pragma unroll 8
+                for (int j = 0; j < c; j++) rank += rs_runs[j] < w ? 1 : 0;
+                if (rank < p.k) rs_write(p, qo, rank, w);
             }
-            const unsigned b = __ballot_sync(FULL, keep);
-            int base = 0;
-            if (lane == 0 && b) base = atomicAdd(&s_count, __popc(b));
-            base = __shfl_sync(FULL, base, 0);
-            const int pos = base + __popc(b & ((1u << lane) - 1u));
-            if (keep && pos < bound) rs_runs[pos] = word;
-        }
-        __syncthreads();
-        const int c = s_count;
-        const bool too_many = c > bound;
-        if (!too_many) {
+        } else {
             const int m = (c + W - 1) / W;    // <= RS_RUN
-            if (m <= 32) rank_place<1>(p, q, c, m, rs_runs, W);
-            else if (m <= 64) rank_place<2>(p, q, c, m, rs_runs, W);
-            else if (m <= 128) rank_place<4>(p, q, c, m, rs_runs, W);
-            else if (m <= 256) rank_place<8>(p, q, c, m, rs_runs, W);
-            else rank_place<16>(p, q, c, m, rs_runs, W);
-            for (int j = c + tid; j < p.k; j += T) {
-                p.out_dist[q * p.k + j] = p.pad;
-                p.out_labels[q * p.k + j] = -1;
-            }
+            if (m <= 32) rank_place<1>(p, qo, c, m, rs_runs, W);
+            else if (m <= 64) rank_place<2>(p, qo, c, m, rs_runs, W);
+            else if (m <= 128) rank_place<4>(p, qo, c, m, rs_runs, W);
+            else if (m <= 256) rank_place<8>(p, qo, c, m, rs_runs, W);
+            else rank_place<16>(p, qo, c, m, rs_runs, W);
         }
-        if (tid == 0) p.dirty[q] = (too_many || (cnt > p.ld) || (cnt < p.k && cnt < p.nb_total)) ? 1 : 0;
+        for (int j = c + tid; j < p.k; j += T) {
+            p.out_dist[qo * p.k + j] = p.pad;
+            p.out_labels[qo * p.k + j] = -1;
+        }
+        if (tid == 0 && p.dirty)
+            p.dirty[q] = ((cnt > p.ld) || (live < p.k && live < p.nb_total)) ? 1 : 0;
         __syncthreads();   // the shared arrays are rewritten by the next row
     }
 }
@@ -469,22 +560,43 @@ __global__ void __launch_bounds__(512, 2) rank_merge_kernel(const RankMergeParam
 
 bool rank_select_enabled() { return g_rank_select.load(std::memory_order_relaxed) != 0; }
 
-bool rank_select_fits(int cap, int k) { return k > 32 && k <= 1024 && cap >= 1; }
+namespace {
 
-int launch_rank_select(const float* cand_key, const int32_t* cand_idx, const int32_t* cand_cnt, int cap,
-                       int64_t nb, int64_t nq, int k, int metric, const float* qnorm, int64_t label_base,
-                       float* out_dist, int64_t* out_labels, int32_t* dirty, cudaStream_t stream) {
-    if (!rank_select_fits(cap, k) || !cand_cnt || !dirty) return B200F_ERR_BAD_ARG;
-    if (nq <= 0) return B200F_OK;
+// Threads per row: few for many rows of few candidates, many for few long rows.  The staging area
+// holds 4 k words and at least 1024, 8192 at most: W warps sort at most RS_RUN words each.
+int launch_row_select(RowSelectParams& p, int64_t n_typical, cudaStream_t stream) {
+    if (p.nq <= 0) return B200F_OK;
+    if (p.k < 1 || p.k > B200F_MAX_K) return B200F_ERR_UNSUPPORTED;
+    const int64_t sm = cached_sm_count();
+    int bound = 1024;
+    while (bound < 4 * p.k && bound < 8192) bound <<= 1;
+    int T = 128;
+    while (T < 1024 && (T * RS_RUN < 32 * bound ||                         // the area must be sortable
+                        (p.nq * T < sm * 512 && T * 4 < n_typical)))        // rows alone do not fill the SMs
+        T <<= 1;
+    if (p.k > 64 && T < 256) T = 256;
+    p.bound = bound;
+    const int smem = bound * 8;
+    static bool attr_set[kMaxDevices] = {false};
+    const int slot = device_slot();
+    if (!attr_set[slot]) {
+        B200F_CUDA_TRY(cudaFuncSetAttribute(row_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 8192 * 8));
+        attr_set[slot] = true;
+    }
+    int64_t g = p.nq;
+    const int64_t gcap = sm * (2048 / T);
+    if (g > gcap) g = gcap;
+    // rows counted on the device are usually few or none: idle CTAs leave at once
+    if (p.nq_dev && g > sm) g = sm;
+    row_select_kernel<<<(int)g, T, smem, stream>>>(p);
+    count_launch();
+    B200F_LAUNCH_CHECK();
+    return B200F_OK;
+}
+
+void set_output(RowSelectParams& p, int metric, const float* qnorm, int64_t label_base, float* out_dist,
+                int64_t* out_labels) {
     const bool l2 = metric == B200F_METRIC_L2;
-    RankSelectParams p{};
-    p.keys = cand_key;
-    p.ids = cand_idx;
-    p.cnt = cand_cnt;
-    p.ld = cap;
-    p.nb_total = nb;
-    p.nq = nq;
-    p.k = k;
     p.out_sign = l2 ? 1.f : -1.f;
     p.qnorm = l2 ? qnorm : nullptr;
     p.clamp = l2 ? 1 : 0;
@@ -492,17 +604,45 @@ int launch_rank_select(const float* cand_key, const int32_t* cand_idx, const int
     p.label_base = label_base;
     p.out_dist = out_dist;
     p.out_labels = out_labels;
+}
+
+}  // namespace
+
+int launch_rank_select(const float* cand_key, const int32_t* cand_idx, const int32_t* cand_cnt, int cap,
+                       int64_t nb, int64_t nq, int k, int metric, const float* qnorm, int64_t label_base,
+                       float* out_dist, int64_t* out_labels, int32_t* dirty, cudaStream_t stream) {
+    if (cap < 1 || !cand_cnt || !dirty) return B200F_ERR_BAD_ARG;
+    RowSelectParams p{};
+    p.keys = cand_key;
+    p.ids = cand_idx;
+    p.cnt = cand_cnt;
+    p.ld = cap;
+    p.nb_total = nb;
+    p.nq = nq;
+    p.k = k;
     p.dirty = dirty;
-    // room for 4 k candidates up to the k-th key: 2048 (4 warps) or 4096 (8 warps)
-    const int W = k <= 512 ? 4 : RS_MAX_WARPS;
-    const int smem = W * RS_RUN * 8;
-    int64_t g = nq;
-    const int64_t gcap = (int64_t)cached_sm_count() * 8;
-    if (g > gcap) g = gcap;
-    rank_select_kernel<<<(int)g, W * 32, smem, stream>>>(p);
-    count_launch();
-    B200F_LAUNCH_CHECK();
-    return B200F_OK;
+    set_output(p, metric, qnorm, label_base, out_dist, out_labels);
+    return launch_row_select(p, cap / 4, stream);
+}
+
+int launch_merge_partials(const float* part_key, const int32_t* part_idx, int P, int64_t nq, int k,
+                          int metric, const float* qnorm, int64_t label_base, float* out_dist,
+                          int64_t* out_labels, const int* nq_dev, const int32_t* row_map,
+                          cudaStream_t stream) {
+    if (nq <= 0) return B200F_OK;
+    if (k < 1 || k > 32 || P < 1) return B200F_ERR_UNSUPPORTED;
+    RowSelectParams p{};
+    p.keys = part_key;
+    p.ids = part_idx;
+    p.ld = (int64_t)P * k;
+    p.n = (int64_t)P * k;
+    p.nb_total = 0;
+    p.nq = nq;
+    p.nq_dev = nq_dev;
+    p.row_map = row_map;
+    p.k = k;
+    set_output(p, metric, qnorm, label_base, out_dist, out_labels);
+    return launch_row_select(p, p.n, stream);
 }
 
 bool rank_merge_fits(int P, int k) { return k > 32 && P >= 1 && (int64_t)P * k <= 8192; }
