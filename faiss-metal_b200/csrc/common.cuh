@@ -74,11 +74,19 @@ ScanPlan plan_scan(int64_t nq, int64_t nb, int d, int storage, int sm_count);
 // *out_P receives the number of partial lists per query actually written (<= plan.grid).
 // stream_f32: FP32 rows may take the streaming tf32 kernel (up to 8 queries); the caller must pass
 // the same value for every query group of a search, since the kernels write different list counts.
+// thr (optional, [nq]): the lists only take keys up to it.  guard (optional): when *guard is 0 in
+// device memory the kernel does nothing.
 int launch_scan_topk(const B200FSearchArgs& a, const ScanPlan& plan, float* part_key,
-                     int32_t* part_idx, int* out_P, bool stream_f32, cudaStream_t stream);
-// Scan that stores keys (smaller = better) to a matrix [nq][ld] for columns [col0, col0+ncols).
-int launch_scan_store(const B200FSearchArgs& a, int64_t col0, int64_t ncols, float* out,
-                      int64_t ld, int sm_count, cudaStream_t stream);
+                     int32_t* part_idx, int* out_P, bool stream_f32, const float* thr, const int* guard,
+                     cudaStream_t stream);
+// Scan that stores keys (smaller = better) to a matrix [nq][ld] for columns [col0, col0+ncols); with
+// stride > 1 column c is row (col0 + c) * stride of the shard.
+int launch_scan_store(const B200FSearchArgs& a, int64_t col0, int64_t ncols, int64_t stride, float* out,
+                      int64_t ld, int sm_count, const int* guard, cudaStream_t stream);
+// Scan that appends every row whose key is <= thr[q] to the query's candidate buffer
+// cand_key / cand_idx [nq][cap]; cand_cnt[q] (zeroed by the caller) counts every hit.
+int launch_scan_filter(const B200FSearchArgs& a, const float* thr, float* cand_key, int32_t* cand_idx,
+                       int32_t* cand_cnt, int cap, int sm_count, cudaStream_t stream);
 
 // gemm_topk.cu
 struct GemmPlan {
@@ -130,11 +138,12 @@ int launch_gemm_store(const GemmOperands& op, const GemmPlan& plan, int64_t col0
 // Merge P sorted partial lists (key smaller=better, int32 local ids; -1 = empty) per
 // query and finalise: L2 dist = max(key + qnorm, 0), IP dist = -key; labels = id + base.
 // nq_dev / row_map (optional): live rows counted on the device; lists of row j belong to query
-// row_map[j].  out_labels may be null (keys only).
+// row_map[j].  dirty (optional): dirty[q] = 1 when the lists hold fewer than k entries although the
+// shard has nb rows (lists that were cut at a threshold).
 int launch_merge_partials(const float* part_key, const int32_t* part_idx, int P, int64_t nq, int k,
                           int metric, const float* qnorm, int64_t label_base, float* out_dist,
                           int64_t* out_labels, const int* nq_dev, const int32_t* row_map,
-                          cudaStream_t stream);
+                          int64_t nb, int32_t* dirty, cudaStream_t stream);
 // Running top-k over a key matrix chunk: run lists [nq][k] (key, int32 id) are read
 // (if has_prev) and rewritten with the best k of (previous list U chunk columns).
 // Merged raw keys only: out_key[q][k], best first, +INF where fewer than k entries exist.
@@ -173,6 +182,16 @@ bool rank_select_enabled();
 int launch_rank_select(const float* cand_key, const int32_t* cand_idx, const int32_t* cand_cnt, int cap,
                        int64_t nb, int64_t nq, int k, int metric, const float* qnorm, int64_t label_base,
                        float* out_dist, int64_t* out_labels, int32_t* dirty, cudaStream_t stream);
+// The k best of every row of a key matrix (n columns, column c is row c of the shard), finalised.
+int launch_matrix_select(const float* keys, int64_t nq, int64_t n, int64_t ld, int k, int metric, const float* qnorm,
+                         int64_t label_base, float* out_dist, int64_t* out_labels, const int* nq_dev,
+                         const int32_t* row_map, cudaStream_t stream);
+// out[q]: an upper bound, close to it, of the r-th smallest (r <= 512) of the n keys of row q; +INF when
+// there are too few.  NaN keys are skipped.
+int launch_row_bound(const float* keys, int64_t nq, int64_t n, int64_t ld, int r, float* out, cudaStream_t stream);
+// *count = nq when any of dirty[0 .. nq) is set, else 0 (also to *count_copy): the streaming scans redo
+// all of their few queries or none.
+int launch_any_dirty(const int32_t* dirty, int64_t nq, int32_t* count, int32_t* count_copy, cudaStream_t stream);
 bool rank_merge_fits(int P, int k);
 int launch_rank_merge(const float* dist, const int64_t* labels, int64_t stride_d, int64_t stride_l, int P,
                       int64_t nq, int k, int metric, float* out_dist, int64_t* out_labels,

@@ -47,8 +47,15 @@ struct ScanParams {
     float nscale[4];        // scales the query side puts into those columns
     float* part_key;        // top-k mode: [nq][P][k]
     int32_t* part_idx;
+    const float* thr;       // top-k mode, optional: [nq] upper bounds the lists start from; filter mode: thresholds
+    const int* guard;       // optional: *guard == 0 in device memory leaves at once
     float* out;             // store mode: [nq][ld]
     int64_t ld;
+    int64_t norm_stride;    // floats between the norms of consecutive rows (store mode over a sample)
+    float* cand_key;        // filter mode: [nq][cand_cap]
+    int32_t* cand_idx;
+    int32_t* cand_cnt;      // [nq]
+    int cand_cap;
     // bulk-copy pipeline (scan_bulk_kernel)
     int rb;                 // rows per consumer warp per stage
     int stage_rows;         // rows per stage = SB_NW * rb
@@ -127,16 +134,31 @@ __device__ __forceinline__ void warp_insert(float& lk, int& li, float s, int id,
     }
 }
 
-template <int STORAGE, int NQ, bool STORE>
+// The bound of a warp list after an insertion: its k-th entry once it has one in front of the bound the
+// list started from (a threshold, or none).
+__device__ __forceinline__ void take_bound(float& thr, int& thr_id, float lk, int li, int k) {
+    const float t = __shfl_sync(FULL, lk, k - 1);
+    const int tid = __shfl_sync(FULL, li, k - 1);
+    if (before(t, tid, thr, thr_id)) {
+        thr = t;
+        thr_id = tid;
+    }
+}
+
+enum { SCAN_TOPK = 0, SCAN_STORE = 1, SCAN_FILTER = 2 };
+
+template <int STORAGE, int NQ, int MODE>
 // Three CTAs per SM where 80 registers suffice; four queries, and two queries on fp32 rows (paired
 // accumulators), take 128 registers and two CTAs; the grid is exactly one such wave.  Measured on
 // 12.5 M fp32 rows of d = 128: 6.90 / 5.64 / 4.06 TB/s for one / two / four queries (4.98 / 4.58 /
 // 3.53 with plain FMAs and a grid of four CTAs per SM, whose last wave ran a third full).
-__global__ void __launch_bounds__(SCAN_THREADS, (NQ == 4 || (NQ == 2 && STORAGE == B200F_STORAGE_F32 && !STORE)) ? 2 : 3)
+__global__ void __launch_bounds__(SCAN_THREADS, (NQ == 4 || (NQ == 2 && STORAGE == B200F_STORAGE_F32 && MODE == SCAN_TOPK)) ? 2 : 3)
 scan_kernel(const ScanParams p) {
+    constexpr bool STORE = MODE == SCAN_STORE;
+    if (p.guard && *p.guard == 0) return;
     constexpr int E = Piece<STORAGE>::E;
     // rows per lane and block; fp32 rows keep two partial sums per (row, query), so fewer rows fit the registers
-    constexpr int U = (STORAGE == B200F_STORAGE_F32 && !STORE && NQ == 4) ? 6 : SCAN_U;
+    constexpr int U = (STORAGE == B200F_STORAGE_F32 && MODE == SCAN_TOPK && NQ == 4) ? 6 : SCAN_U;
     extern __shared__ __align__(16) float sq[];  // [NQ][qstride] queries, then merge area
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -175,7 +197,7 @@ scan_kernel(const ScanParams p) {
     for (int qi = 0; qi < NQ; qi++) {
         lk[qi] = CUDART_INF_F;
         li[qi] = -1;
-        thr[qi] = CUDART_INF_F;
+        thr[qi] = (MODE != SCAN_STORE && p.thr && qi < p.nq) ? p.thr[qi] : CUDART_INF_F;
         thr_id[qi] = -1;
     }
 
@@ -270,6 +292,27 @@ scan_kernel(const ScanParams p) {
         // lane cl == 0 of each row group owns the row's candidates.  With several queries the
         // dot products are first turned into keys and ONE vote decides whether any row of the block
         // has a candidate for any query (a single query measured slower with the extra pass).
+        if constexpr (MODE == SCAN_FILTER) {
+            // a few rows in a thousand at most pass their query's threshold: each takes a slot by itself
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int64_t row = row_base + u * rps + sub;
+                if (cl != 0 || row >= p.col1) continue;
+                const float nrm = l2 ? __ldg(p.norms + row) : 0.f;
+#pragma unroll
+                for (int qi = 0; qi < NQ; qi++) {
+                    const float key = l2 ? fmaf(-2.f, acc[u][qi], nrm) : -acc[u][qi];
+                    if (key <= thr[qi] && qi < p.nq) {
+                        const int pos = atomicAdd(p.cand_cnt + qi, 1);
+                        if (pos < p.cand_cap) {
+                            p.cand_key[(int64_t)qi * p.cand_cap + pos] = key;
+                            p.cand_idx[(int64_t)qi * p.cand_cap + pos] = (int32_t)row;
+                        }
+                    }
+                }
+            }
+            continue;
+        }
         constexpr bool PREVOTE = (NQ > 1) && !STORE;
         if (PREVOTE) {
             bool any_hit = false;
@@ -292,7 +335,7 @@ scan_kernel(const ScanParams p) {
             const int64_t row = row_base + u * rps + sub;
             const bool owner = (cl == 0) && row < p.col1;
             float nrm = 0.f;
-            if (!PREVOTE && owner && l2) nrm = __ldg(p.norms + row);
+            if (!PREVOTE && owner && l2) nrm = __ldg(p.norms + (STORE ? row * p.norm_stride : row));
 #pragma unroll
             for (int qi = 0; qi < NQ; qi++) {
                 const float key = PREVOTE ? acc[u][qi] : (l2 ? fmaf(-2.f, acc[u][qi], nrm) : -acc[u][qi]);
@@ -308,8 +351,7 @@ scan_kernel(const ScanParams p) {
                         const int id = __shfl_sync(FULL, (int)row, src);
                         if (before(s, id, thr[qi], thr_id[qi])) {
                             warp_insert(lk[qi], li[qi], s, id, lane);
-                            thr[qi] = __shfl_sync(FULL, lk[qi], p.k - 1);
-                            thr_id[qi] = __shfl_sync(FULL, li[qi], p.k - 1);
+                            take_bound(thr[qi], thr_id[qi], lk[qi], li[qi], p.k);
                         }
                     }
                 }
@@ -317,7 +359,7 @@ scan_kernel(const ScanParams p) {
         }
     }
 
-    if (STORE) return;
+    if constexpr (MODE != SCAN_TOPK) return;
 
     // CTA merge: every warp publishes its lists, warp qi folds them for query qi.
     __syncthreads();  // queries in shared memory are no longer needed
@@ -400,6 +442,7 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
 template <bool BF16, int NW>
 __global__ void __launch_bounds__(32 * (1 + NW), 1) scan_mma_kernel(const ScanParams p) {
     extern __shared__ __align__(128) uint8_t sm[];
+    if (p.guard && *p.guard == 0) return;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const uint32_t sbase = smem_u32(sm);
@@ -449,7 +492,7 @@ __global__ void __launch_bounds__(32 * (1 + NW), 1) scan_mma_kernel(const ScanPa
     for (int qi = 0; qi < SM_NQ; qi++) {
         lk[qi] = CUDART_INF_F;
         li[qi] = -1;
-        thr[qi] = CUDART_INF_F;
+        thr[qi] = (p.thr && qi < p.nq) ? p.thr[qi] : CUDART_INF_F;
         thr_id[qi] = -1;
     }
 
@@ -566,8 +609,7 @@ __global__ void __launch_bounds__(32 * (1 + NW), 1) scan_mma_kernel(const ScanPa
                             const int id = __shfl_sync(FULL, row, src);
                             if (before(s, id, thr[qi], thr_id[qi])) {
                                 warp_insert(lk[qi], li[qi], s, id, lane);
-                                thr[qi] = __shfl_sync(FULL, lk[qi], p.k - 1);
-                                thr_id[qi] = __shfl_sync(FULL, li[qi], p.k - 1);
+                                take_bound(thr[qi], thr_id[qi], lk[qi], li[qi], p.k);
                             }
                         }
                     }
@@ -655,6 +697,7 @@ constexpr int ST_THREADS = 32 * (1 + ST_NW);
 
 __global__ void __launch_bounds__(ST_THREADS, 1) scan_tf32_kernel(const ScanParams p) {
     extern __shared__ __align__(128) uint8_t sm[];
+    if (p.guard && *p.guard == 0) return;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const uint32_t sbase = smem_u32(sm);
@@ -704,7 +747,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tf32_kernel(const ScanPara
     for (int qi = 0; qi < SM_NQ; qi++) {
         lk[qi] = CUDART_INF_F;
         li[qi] = -1;
-        thr[qi] = CUDART_INF_F;
+        thr[qi] = (p.thr && qi < p.nq) ? p.thr[qi] : CUDART_INF_F;
         thr_id[qi] = -1;
     }
 
@@ -861,8 +904,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tf32_kernel(const ScanPara
                             const int id = __shfl_sync(FULL, row, src);
                             if (before(s, id, thr[qi], thr_id[qi])) {
                                 warp_insert(lk[qi], li[qi], s, id, lane);
-                                thr[qi] = __shfl_sync(FULL, lk[qi], p.k - 1);
-                                thr_id[qi] = __shfl_sync(FULL, li[qi], p.k - 1);
+                                take_bound(thr[qi], thr_id[qi], lk[qi], li[qi], p.k);
                             }
                         }
                     }
@@ -964,16 +1006,16 @@ void fill_geometry(ScanParams& p, int storage, int d, int64_t row_pitch, int nor
     p.qstride = p.C * E;
 }
 
-template <int STORAGE, bool STORE>
+template <int STORAGE, int MODE>
 int launch_nq(const ScanParams& p, int grid, size_t smem, cudaStream_t stream) {
 #define B200F_SCAN_CASE(NQ)                                                                      \
     {                                                                                            \
         if (smem > 48 * 1024)                                                                    \
-            B200F_CUDA_TRY(cudaFuncSetAttribute(scan_kernel<STORAGE, NQ, STORE>,                 \
+            B200F_CUDA_TRY(cudaFuncSetAttribute(scan_kernel<STORAGE, NQ, MODE>,                 \
                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,     \
                                                 (int)smem));                                     \
         main_kernel_begin(stream);                                                               \
-        scan_kernel<STORAGE, NQ, STORE><<<grid, SCAN_THREADS, smem, stream>>>(p);                \
+        scan_kernel<STORAGE, NQ, MODE><<<grid, SCAN_THREADS, smem, stream>>>(p);                \
         main_kernel_end(stream);                                                                 \
         count_launch();                                                                          \
     }
@@ -985,15 +1027,15 @@ int launch_nq(const ScanParams& p, int grid, size_t smem, cudaStream_t stream) {
     return B200F_OK;
 }
 
-template <bool STORE>
+template <int MODE>
 int launch_storage(const ScanParams& p, int storage, int grid, cudaStream_t stream) {
     const int nq_t = p.nq == 1 ? 1 : (p.nq == 2 ? 2 : 4);
     const size_t smem = scan_smem_bytes(nq_t, p.qstride);
     if (smem > 200 * 1024) return B200F_ERR_UNSUPPORTED;
     switch (storage) {
-        case B200F_STORAGE_F32: return launch_nq<B200F_STORAGE_F32, STORE>(p, grid, smem, stream);
-        case B200F_STORAGE_F16: return launch_nq<B200F_STORAGE_F16, STORE>(p, grid, smem, stream);
-        case B200F_STORAGE_BF16: return launch_nq<B200F_STORAGE_BF16, STORE>(p, grid, smem, stream);
+        case B200F_STORAGE_F32: return launch_nq<B200F_STORAGE_F32, MODE>(p, grid, smem, stream);
+        case B200F_STORAGE_F16: return launch_nq<B200F_STORAGE_F16, MODE>(p, grid, smem, stream);
+        case B200F_STORAGE_BF16: return launch_nq<B200F_STORAGE_BF16, MODE>(p, grid, smem, stream);
     }
     return B200F_ERR_BAD_ARG;
 }
@@ -1055,7 +1097,8 @@ ScanPlan plan_scan(int64_t nq, int64_t nb, int d, int storage, int sm_count) {
 }
 
 int launch_scan_topk(const B200FSearchArgs& a, const ScanPlan& plan, float* part_key,
-                     int32_t* part_idx, int* out_P, bool stream_f32, cudaStream_t stream) {
+                     int32_t* part_idx, int* out_P, bool stream_f32, const float* thr, const int* guard,
+                     cudaStream_t stream) {
     if (a.nq < 1 || a.nq > 8 || a.k < 1 || a.k > 32) return B200F_ERR_UNSUPPORTED;
     ScanParams p{};
     fill_geometry(p, a.storage, a.d, a.row_pitch, a.metric == B200F_METRIC_L2 ? a.norm_cols : 0,
@@ -1072,6 +1115,8 @@ int launch_scan_topk(const B200FSearchArgs& a, const ScanPlan& plan, float* part
     p.metric = a.metric;
     p.part_key = part_key;
     p.part_idx = part_idx;
+    p.thr = thr;
+    p.guard = guard;
     p.status = a.status;
     const int sm = cached_sm_count();
     {
@@ -1128,19 +1173,20 @@ int launch_scan_topk(const B200FSearchArgs& a, const ScanPlan& plan, float* part
     }
     if (a.nq > 4) return B200F_ERR_UNSUPPORTED;
     *out_P = plan.grid;
-    return launch_storage<false>(p, a.storage, plan.grid, stream);
+    return launch_storage<SCAN_TOPK>(p, a.storage, plan.grid, stream);
 }
 
-int launch_scan_store(const B200FSearchArgs& a, int64_t col0, int64_t ncols, float* out, int64_t ld,
-                      int sm_count, cudaStream_t stream) {
-    if (a.nq < 1 || a.nq > 4) return B200F_ERR_UNSUPPORTED;
+int launch_scan_store(const B200FSearchArgs& a, int64_t col0, int64_t ncols, int64_t stride, float* out, int64_t ld,
+                      int sm_count, const int* guard, cudaStream_t stream) {
+    if (a.nq < 1 || a.nq > 4 || stride < 1) return B200F_ERR_UNSUPPORTED;
     if (ncols <= 0) return B200F_OK;
     ScanParams p{};
-    fill_geometry(p, a.storage, a.d, a.row_pitch, a.metric == B200F_METRIC_L2 ? a.norm_cols : 0,
+    fill_geometry(p, a.storage, a.d, a.row_pitch * stride, a.metric == B200F_METRIC_L2 ? a.norm_cols : 0,
                   lanes_per_row_cap(a.nq));
     p.queries = a.queries;
     p.rows = a.rows;
     p.norms = a.norms;
+    p.norm_stride = stride;
     p.nb = a.nb;
     p.col0 = col0;
     p.col1 = col0 + ncols;
@@ -1148,12 +1194,40 @@ int launch_scan_store(const B200FSearchArgs& a, int64_t col0, int64_t ncols, flo
     p.nq = (int)a.nq;
     p.k = 1;
     p.metric = a.metric;
+    p.guard = guard;
     p.out = out;
     p.ld = ld;
-    return launch_storage<true>(p, a.storage,
-                                scan_grid(ncols, a.d, a.storage, sm_count, lanes_per_row_cap(a.nq),
-                                          resident_ctas(a.nq, a.storage, true)),
-                                stream);
+    return launch_storage<SCAN_STORE>(p, a.storage,
+                                      scan_grid(ncols, a.d, a.storage, sm_count, lanes_per_row_cap(a.nq),
+                                                resident_ctas(a.nq, a.storage, true)),
+                                      stream);
+}
+
+int launch_scan_filter(const B200FSearchArgs& a, const float* thr, float* cand_key, int32_t* cand_idx,
+                       int32_t* cand_cnt, int cap, int sm_count, cudaStream_t stream) {
+    if (a.nq < 1 || a.nq > 4 || !thr || !cand_key || !cand_idx || !cand_cnt || cap < 1) return B200F_ERR_BAD_ARG;
+    ScanParams p{};
+    fill_geometry(p, a.storage, a.d, a.row_pitch, a.metric == B200F_METRIC_L2 ? a.norm_cols : 0,
+                  lanes_per_row_cap(a.nq));
+    p.queries = a.queries;
+    p.rows = a.rows;
+    p.norms = a.norms;
+    p.nb = a.nb;
+    p.col0 = 0;
+    p.col1 = a.nb;
+    p.d = a.d;
+    p.nq = (int)a.nq;
+    p.k = 1;
+    p.metric = a.metric;
+    p.thr = thr;
+    p.cand_key = cand_key;
+    p.cand_idx = cand_idx;
+    p.cand_cnt = cand_cnt;
+    p.cand_cap = cap;
+    return launch_storage<SCAN_FILTER>(p, a.storage,
+                                       scan_grid(a.nb, a.d, a.storage, sm_count, lanes_per_row_cap(a.nq),
+                                                 resident_ctas(a.nq, a.storage, true)),
+                                       stream);
 }
 
 }  // namespace b200f

@@ -35,6 +35,7 @@ namespace {
 
 constexpr int64_t MATRIX_BUDGET_BYTES = 1024ll << 20;  // key-matrix chunk of the k > 32 path
 constexpr int SCAN_GROUP = 4;
+constexpr int64_t MATRIX_SELECT_MAX_COLS = 1 << 19;
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -58,6 +59,8 @@ struct SearchPlan {
     bool lists;       // k > 32 selected from the fused kernel's 32-entry lists, matrix fallback per row
     int gslots;       // words per query row in the shared bound array
     bool filter;      // pilot threshold + candidate buffers, fused / matrix fallback per row
+    bool sample;      // scan path: thresholds from a sample of the rows (lists cut at them, or candidate buffers)
+    int64_t nsample;  // rows in that sample
     int fstride;      // pilot pass: every fstride-th column tile
     int frank;        // threshold = frank-th best key of the pilot sample
     int fcap;         // candidate buffer entries per query
@@ -72,6 +75,7 @@ struct SearchPlan {
     size_t off_qscale;
     size_t off_qnorm, off_gthr, off_a, off_part_key, off_part_idx, off_matrix, off_run_key, off_run_idx;
     size_t off_dirty, off_rows, off_count, off_a2;
+    size_t off_sample;
     size_t off_pilot_key, off_pilot_idx, off_thr, off_cand_key, off_cand_idx, off_cand_cnt;
     size_t total;
     // debug canaries: a 256-byte guard behind every slice of the scratch region
@@ -124,6 +128,38 @@ static int64_t matrix_chunk_cols(int64_t nq, int64_t nb) {
     if (cols > nb_pad) cols = nb_pad;
     return cols;
 }
+
+// Sample of every stride-th row of a shard, from which a threshold for a query's k best is taken: the
+// sample holds on average e = k / stride of them, and its r-th best key, r = e + 4.5 sqrt(e) + 3, has
+// fewer than k rows of the shard under it only if the sample caught r of the k best (about one query in a
+// million).  About r * stride rows do lie under it; more than stride (r + 6 sqrt(r) + 12), what the
+// candidate buffers hold, for one query in 10^8.  Of about `target` rows, more where that admits
+// thousands of candidates beyond 2 k, fewer where r would be beyond 400.  False: shard too small.
+bool choose_sample(int64_t nb, int k, int64_t target, int* stride_out, int* rank_out, int* cap_out) {
+    auto rank_of = [k](int stride) {
+        const double e = (double)k / stride;
+        return (int)(e + 4.5 * std::sqrt(e) + 3.0 + 0.999);
+    };
+    int stride = 1;
+    while (stride < 1024 && nb / (2 * stride) >= target) stride *= 2;
+    while (stride > 2 && (int64_t)rank_of(stride) * stride > 2 * (int64_t)k + 2048) stride /= 2;
+    while (rank_of(stride) > 400) stride *= 2;
+    const int r = rank_of(stride);
+    if (stride < 2 || nb / stride < 8 * (int64_t)r) return false;
+    *stride_out = stride;
+    *rank_out = r;
+    *cap_out = (int)round_up64((int64_t)(stride * (r + 6.0 * std::sqrt((double)r) + 12.0)), 256);
+    return true;
+}
+
+// Scan path.  Lists of k <= 32: every insertion is a serial step of its warp, about k (1 + ln(rows per
+// warp / k)) of them per query and warp; measured on 2.5 M fp32 rows of d = 128, k = 32: 197 / 246 / 297 / 346
+// us for 1 / 2 / 4 / 6 queries with lists from empty, against about 190 - 206 with none.  Two launches
+// for the thresholds cost ~10 us.  k > 32: candidates instead of the key matrix from 32 Ki rows on.
+constexpr int64_t SCAN_SAMPLE_ROWS = 8192;
+constexpr int64_t SCAN_LIST_THR_MIN_ROWS = 1 << 19;
+constexpr int64_t SCAN_LIST_THR_MIN_WORK = 24;      // queries x k
+constexpr int64_t SCAN_FILTER_MIN_ROWS = 1 << 15;
 
 bool make_plan(int64_t nq, int64_t nb, int d, int k, int storage, int path, bool pairwise,
                SearchPlan& pl) {
@@ -195,6 +231,31 @@ bool make_plan(int64_t nq, int64_t nb, int d, int k, int storage, int path, bool
         if ((int64_t)2 * g.P * B200F_FUSED_MAX_K >= 4 * (int64_t)k) {
             pl.lists = true;
             pl.gslots = (k + B200F_FUSED_MAX_K - 1) / B200F_FUSED_MAX_K;
+        }
+    }
+    if (!pairwise && pl.path == B200F_PATH_SCAN && nq <= 2 * SCAN_GROUP && !filter_disabled()) {
+        const bool wanted = pl.fused ? (nb >= SCAN_LIST_THR_MIN_ROWS && nq * k >= SCAN_LIST_THR_MIN_WORK)
+                                     : nb >= SCAN_FILTER_MIN_ROWS;
+        pl.sample = wanted && choose_sample(nb, k, SCAN_SAMPLE_ROWS, &pl.fstride, &pl.frank, &pl.fcap);
+        if (pl.sample) {
+            pl.nsample = nb / pl.fstride;
+            const int64_t n1 = nq > 0 ? nq : 1;
+            pl.off_sample = off;
+            adv((size_t)n1 * pl.nsample * 4);
+            pl.off_thr = off;
+            adv((size_t)n1 * 4);
+            pl.off_dirty = off;
+            adv((size_t)n1 * 4);
+            pl.off_count = off;
+            adv(256);
+            if (!pl.fused) {
+                pl.off_cand_key = off;
+                adv((size_t)n1 * pl.fcap * 4);
+                pl.off_cand_idx = off;
+                adv((size_t)n1 * pl.fcap * 4);
+                pl.off_cand_cnt = off;
+                adv((size_t)n1 * 4);
+            }
         }
     }
     pl.off_gthr = off;
@@ -694,9 +755,54 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
         if (rc != B200F_OK) return rc;
     }
 
+    // scan path: thresholds from a sample of the rows
+    float* thr = reinterpret_cast<float*>(scratch + pl.off_thr);
+    int32_t* dirty = reinterpret_cast<int32_t*>(scratch + pl.off_dirty);
+    int32_t* any_count = reinterpret_cast<int32_t*>(scratch + pl.off_count);
+    auto query_group = [&](int64_t q0, int64_t group) {
+        B200FSearchArgs sub = *a;
+        sub.queries = a->queries + q0 * (int64_t)a->d;
+        sub.nq = (a->nq - q0) < group ? (a->nq - q0) : group;
+        return sub;
+    };
+    if (pl.sample) {
+        float* keys = reinterpret_cast<float*>(scratch + pl.off_sample);
+        for (int64_t q0 = 0; q0 < a->nq; q0 += SCAN_GROUP) {
+            rc = launch_scan_store(query_group(q0, SCAN_GROUP), 0, pl.nsample, pl.fstride, keys + q0 * pl.nsample,
+                                   pl.nsample, sm, nullptr, st);
+            if (rc != B200F_OK) return rc;
+        }
+        rc = launch_row_bound(keys, a->nq, pl.nsample, pl.nsample, pl.frank, thr, st);
+        if (rc != B200F_OK) return rc;
+    }
+
     if (pl.fused) {
         float* part_key = reinterpret_cast<float*>(scratch + pl.off_part_key);
         int32_t* part_idx = reinterpret_cast<int32_t*>(scratch + pl.off_part_idx);
+        // Every group of queries writes the same number of lists (same shard, same geometry); the
+        // first launch reports it.  Groups of 8 where a streaming kernel applies (shard large enough),
+        // else of 4.  FP32 rows: the streaming tf32 kernel for two queries and more (7.1 - 6.1 TB/s for
+        // 2 - 8 per pass; the FMA kernel: 6.9 / 5.6 / 4.1 TB/s for 1 / 2 / 4).
+        auto scan_lists = [&](const float* from, const int* guard, int& P) -> int {
+            P = pl.scan.grid;
+            const bool stream_f32 = a->nq >= 2;
+            int64_t group = a->nq > SCAN_GROUP ? 2 * SCAN_GROUP : SCAN_GROUP;
+            for (int64_t q0 = 0; q0 < a->nq;) {
+                const B200FSearchArgs sub = query_group(q0, group);
+                int Pg = P;
+                const int r2 = launch_scan_topk(sub, pl.scan, part_key + q0 * (int64_t)P * a->k,
+                                                part_idx + q0 * (int64_t)P * a->k, &Pg, stream_f32,
+                                                from ? from + q0 : nullptr, guard, st);
+                if (r2 == B200F_ERR_UNSUPPORTED && q0 == 0 && group > SCAN_GROUP) {
+                    group = SCAN_GROUP;  // no streaming kernel for this shape: nothing was launched
+                    continue;
+                }
+                if (r2 != B200F_OK) return r2;
+                if (q0 == 0) P = Pg;
+                q0 += sub.nq;
+            }
+            return B200F_OK;
+        };
         int P;
         if (pl.path == B200F_PATH_TENSOR) {
             P = 2 * pl.gemm.P;
@@ -704,32 +810,21 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
                                   a->status, st);
             if (rc != B200F_OK) return rc;
         } else {
-            // every group of queries writes the same number of lists (same shard, same
-            // geometry); the first launch reports it.  Groups of 8 where a streaming kernel
-            // applies (shard large enough), else of 4.
-            P = pl.scan.grid;
-            // FP32 rows: the streaming tf32 kernel for two queries and more (7.1 - 6.1 TB/s for 2 - 8
-            // per pass; the FMA kernel: 6.9 / 5.6 / 4.1 TB/s for 1 / 2 / 4)
-            const bool stream_f32 = a->nq >= 2;
-            int64_t group = a->nq > SCAN_GROUP ? 2 * SCAN_GROUP : SCAN_GROUP;
-            for (int64_t q0 = 0; q0 < a->nq;) {
-                B200FSearchArgs sub = *a;
-                sub.queries = a->queries + q0 * (int64_t)a->d;
-                sub.nq = (a->nq - q0) < group ? (a->nq - q0) : group;
-                int Pg = P;
-                rc = launch_scan_topk(sub, pl.scan, part_key + q0 * (int64_t)P * a->k,
-                                      part_idx + q0 * (int64_t)P * a->k, &Pg, stream_f32, st);
-                if (rc == B200F_ERR_UNSUPPORTED && q0 == 0 && group > SCAN_GROUP) {
-                    group = SCAN_GROUP;  // no streaming kernel for this shape: nothing was launched
-                    continue;
-                }
+            rc = scan_lists(pl.sample ? thr : nullptr, nullptr, P);
+            if (rc != B200F_OK) return rc;
+            if (pl.sample) {
+                rc = launch_merge_partials(part_key, part_idx, P, a->nq, a->k, a->metric, qnorm, a->label_base,
+                                           a->out_dist, a->out_labels, nullptr, nullptr, a->nb, dirty, st);
                 if (rc != B200F_OK) return rc;
-                if (q0 == 0) P = Pg;
-                q0 += sub.nq;
+                rc = launch_any_dirty(dirty, a->nq, any_count, a->status ? a->status + 1 : nullptr, st);
+                if (rc != B200F_OK) return rc;
+                nq_dev = any_count;
+                rc = scan_lists(nullptr, any_count, P);
+                if (rc != B200F_OK) return rc;
             }
         }
         return launch_merge_partials(part_key, part_idx, P, a->nq, a->k, a->metric, qnorm,
-                                     a->label_base, a->out_dist, a->out_labels, nq_dev, row_map, st);
+                                     a->label_base, a->out_dist, a->out_labels, nq_dev, row_map, 0, nullptr, st);
     }
 
     // k > 32 from 32-entry lists: select, find the rows that are not proven exact, and send only
@@ -737,7 +832,6 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
     if (pl.lists) {
         float* part_key = reinterpret_cast<float*>(scratch + pl.off_part_key);
         int32_t* part_idx = reinterpret_cast<int32_t*>(scratch + pl.off_part_idx);
-        int32_t* dirty = reinterpret_cast<int32_t*>(scratch + pl.off_dirty);
         rc = launch_gemm_topk(op, pl.gemm, 0, a->nb, 1, kscale, B200F_FUSED_MAX_K, pl.gslots, part_key,
                               part_idx, gthr, a->status, st);
         if (rc != B200F_OK) return rc;
@@ -746,6 +840,25 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
         if (rc != B200F_OK) return rc;
         rc = redo_setup(dirty);
         if (rc != B200F_OK) return rc;
+    }
+
+    // scan path, k > 32: the rows under the threshold, k best of them
+    if (pl.sample) {
+        float* ckey = reinterpret_cast<float*>(scratch + pl.off_cand_key);
+        int32_t* cidx = reinterpret_cast<int32_t*>(scratch + pl.off_cand_idx);
+        int32_t* ccnt = reinterpret_cast<int32_t*>(scratch + pl.off_cand_cnt);
+        B200F_CUDA_TRY(cudaMemsetAsync(ccnt, 0, (size_t)a->nq * sizeof(int32_t), st));
+        for (int64_t q0 = 0; q0 < a->nq; q0 += SCAN_GROUP) {
+            rc = launch_scan_filter(query_group(q0, SCAN_GROUP), thr + q0, ckey + q0 * pl.fcap, cidx + q0 * pl.fcap,
+                                    ccnt + q0, pl.fcap, sm, st);
+            if (rc != B200F_OK) return rc;
+        }
+        rc = launch_select_candidates(ckey, cidx, ccnt, pl.fcap, a->nb, a->nq, a->k, a->metric, qnorm,
+                                      a->label_base, a->out_dist, a->out_labels, dirty, st);
+        if (rc != B200F_OK) return rc;
+        rc = launch_any_dirty(dirty, a->nq, any_count, a->status ? a->status + 1 : nullptr, st);
+        if (rc != B200F_OK) return rc;
+        nq_dev = any_count;
     }
 
     // k > 32: distance keys per column chunk + running selection
@@ -761,15 +874,16 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
                                    a->status, st);
             if (rc != B200F_OK) return rc;
         } else {
-            for (int64_t g = 0; g < pl.ngroups; g++) {
-                B200FSearchArgs sub = *a;
-                sub.queries = a->queries + g * SCAN_GROUP * (int64_t)a->d;
-                sub.nq = (a->nq - g * SCAN_GROUP) < SCAN_GROUP ? (a->nq - g * SCAN_GROUP) : SCAN_GROUP;
-                rc = launch_scan_store(sub, c0, nc, matrix + g * SCAN_GROUP * pl.chunk_cols,
-                                       pl.chunk_cols, sm, st);
+            for (int64_t q0 = 0; q0 < a->nq; q0 += SCAN_GROUP) {
+                rc = launch_scan_store(query_group(q0, SCAN_GROUP), c0, nc, 1, matrix + q0 * pl.chunk_cols,
+                                       pl.chunk_cols, sm, nq_dev, st);
                 if (rc != B200F_OK) return rc;
             }
         }
+        // the whole shard in one chunk: select from it at once (a few passes over a row that stays in L2)
+        if (nc == a->nb && nc <= MATRIX_SELECT_MAX_COLS && rank_select_enabled())
+            return launch_matrix_select(matrix, a->nq, nc, pl.chunk_cols, a->k, a->metric, qnorm, a->label_base,
+                                        a->out_dist, a->out_labels, nq_dev, row_map, st);
         rc = launch_select_chunk(matrix, a->nq, nc, pl.chunk_cols, c0, a->k, has_prev, run_key,
                                  run_idx, nq_dev, st);
         if (rc != B200F_OK) return rc;
@@ -833,7 +947,7 @@ extern "C" int b200f_pairwise(const B200FSearchArgs* a, float* out_matrix, int64
         B200FSearchArgs sub = *a;
         sub.queries = a->queries + g * SCAN_GROUP * (int64_t)a->d;
         sub.nq = (a->nq - g * SCAN_GROUP) < SCAN_GROUP ? (a->nq - g * SCAN_GROUP) : SCAN_GROUP;
-        rc = launch_scan_store(sub, 0, a->nb, out_matrix + g * SCAN_GROUP * ld_out, ld_out, sm, st);
+        rc = launch_scan_store(sub, 0, a->nb, 1, out_matrix + g * SCAN_GROUP * ld_out, ld_out, sm, nullptr, st);
         if (rc != B200F_OK) return rc;
     }
     const int64_t total = a->nq * a->nb;

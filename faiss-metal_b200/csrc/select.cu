@@ -590,6 +590,16 @@ __global__ void __launch_bounds__(1024) compact_rows_kernel(const int32_t* __res
     }
 }
 
+__global__ void any_dirty_kernel(const int32_t* __restrict__ dirty, int nq, int32_t* __restrict__ count,
+                                 int32_t* __restrict__ count_copy) {
+    const bool d = (int)threadIdx.x < nq && dirty[threadIdx.x] != 0;
+    const int n = __any_sync(FULL, d) ? nq : 0;
+    if (threadIdx.x == 0) {
+        *count = n;
+        if (count_copy) *count_copy = n;
+    }
+}
+
 __global__ void gather_rows_kernel(const uint16_t* __restrict__ a, int npl, int64_t plane_stride,
                                    int64_t pitch, const int32_t* __restrict__ rows,
                                    const int32_t* __restrict__ count, uint16_t* __restrict__ out) {
@@ -774,6 +784,14 @@ int launch_compact_rows(const int32_t* dirty, int64_t nq, int32_t* rows, int32_t
                         int32_t* count_copy, cudaStream_t stream) {
     if (nq <= 0) return B200F_OK;
     compact_rows_kernel<<<1, 1024, 0, stream>>>(dirty, nq, rows, count, count_copy);
+    count_launch();
+    B200F_LAUNCH_CHECK();
+    return B200F_OK;
+}
+
+int launch_any_dirty(const int32_t* dirty, int64_t nq, int32_t* count, int32_t* count_copy, cudaStream_t stream) {
+    if (nq < 1 || nq > 32) return B200F_ERR_BAD_ARG;
+    any_dirty_kernel<<<1, 32, 0, stream>>>(dirty, (int)nq, count, count_copy);
     count_launch();
     B200F_LAUNCH_CHECK();
     return B200F_OK;

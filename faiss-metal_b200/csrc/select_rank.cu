@@ -375,6 +375,48 @@ __global__ void __launch_bounds__(1024) row_select_kernel(const RowSelectParams 
     }
 }
 
+// Threshold of the filters: an upper bound of the r-th smallest of a row's n sample keys, the r-th
+// smallest of the T thread minima (T several times r keeps it close; +INF where fewer than r threads
+// have a key, which lets every row pass).  One CTA per row; out[q] may be exceeded by no key that
+// belongs to the r smallest.
+__global__ void __launch_bounds__(1024) row_bound_kernel(const float* __restrict__ keys, int64_t ld, int64_t n,
+                                                         int64_t nq, int r, float* __restrict__ out) {
+    __shared__ int s_hist[256];
+    __shared__ uint32_t s_min[32], s_max[32];
+    __shared__ int s_live[32];
+    __shared__ int s_sel[2];
+    const int tid = threadIdx.x, T = blockDim.x;
+    const bool vec = (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(keys) & 15) == 0;
+    for (int64_t q = blockIdx.x; q < nq; q += gridDim.x) {
+        const float* row = keys + q * ld;
+        float best = CUDART_INF_F;   // fminf drops NaN
+        if (vec) {
+#pragma unroll 4
+            for (int64_t c = (int64_t)tid * 4; c + 4 <= n; c += (int64_t)T * 4) {
+                const float4 f = __ldg(reinterpret_cast<const float4*>(row + c));
+                best = fminf(best, fminf(fminf(f.x, f.y), fminf(f.z, f.w)));
+            }
+            if (tid < (n & 3)) best = fminf(best, __ldg(row + (n & ~(int64_t)3) + tid));
+        } else {
+#pragma unroll 4
+            for (int64_t c = tid; c < n; c += T) best = fminf(best, __ldg(row + c));
+        }
+        const bool have = best < CUDART_INF_F;
+        const uint32_t key = float_to_ordered(best + 0.f);
+        const Spread sp = block_spread(have ? 1 : 0, have ? key : 0xffffffffu, have ? key : 0u, s_live, s_min, s_max);
+        float bound = CUDART_INF_F;
+        if (sp.live >= r) {
+            const int bits = 32 - __clz(sp.mx - sp.mn);
+            int kk = r;
+            const uint32_t x = radix_kth([&](auto f) { if (have) f(key); }, sp.mn, bits, bits > 16 ? bits - 16 : 0, kk,
+                                         s_hist, s_sel);
+            bound = ordered_to_float(sp.mn + min(x, sp.mx - sp.mn));
+        }
+        if (tid == 0) out[q] = bound;
+        __syncthreads();   // the shared arrays are rewritten by the next row
+    }
+}
+
 // ---------------------------------------------------------------------------------------
 // rank_merge
 // ---------------------------------------------------------------------------------------
@@ -608,6 +650,21 @@ void set_output(RowSelectParams& p, int metric, const float* qnorm, int64_t labe
 
 }  // namespace
 
+int launch_row_bound(const float* keys, int64_t nq, int64_t n, int64_t ld, int r, float* out, cudaStream_t stream) {
+    if (r < 1 || r > 512 || n < 0 || ld < n || !keys || !out) return B200F_ERR_BAD_ARG;
+    if (nq <= 0) return B200F_OK;
+    const int64_t sm = cached_sm_count();
+    int T = 128;
+    while (T < 1024 && (T < 8 * r || (nq * T < sm * 512 && T * 8 < n))) T <<= 1;
+    int64_t g = nq;
+    const int64_t gcap = sm * (2048 / T);
+    if (g > gcap) g = gcap;
+    row_bound_kernel<<<(int)g, T, 0, stream>>>(keys, ld, n, nq, r, out);
+    count_launch();
+    B200F_LAUNCH_CHECK();
+    return B200F_OK;
+}
+
 int launch_rank_select(const float* cand_key, const int32_t* cand_idx, const int32_t* cand_cnt, int cap,
                        int64_t nb, int64_t nq, int k, int metric, const float* qnorm, int64_t label_base,
                        float* out_dist, int64_t* out_labels, int32_t* dirty, cudaStream_t stream) {
@@ -628,7 +685,7 @@ int launch_rank_select(const float* cand_key, const int32_t* cand_idx, const int
 int launch_merge_partials(const float* part_key, const int32_t* part_idx, int P, int64_t nq, int k,
                           int metric, const float* qnorm, int64_t label_base, float* out_dist,
                           int64_t* out_labels, const int* nq_dev, const int32_t* row_map,
-                          cudaStream_t stream) {
+                          int64_t nb, int32_t* dirty, cudaStream_t stream) {
     if (nq <= 0) return B200F_OK;
     if (k < 1 || k > 32 || P < 1) return B200F_ERR_UNSUPPORTED;
     RowSelectParams p{};
@@ -636,13 +693,30 @@ int launch_merge_partials(const float* part_key, const int32_t* part_idx, int P,
     p.ids = part_idx;
     p.ld = (int64_t)P * k;
     p.n = (int64_t)P * k;
-    p.nb_total = 0;
+    p.nb_total = nb;
+    p.dirty = dirty;
     p.nq = nq;
     p.nq_dev = nq_dev;
     p.row_map = row_map;
     p.k = k;
     set_output(p, metric, qnorm, label_base, out_dist, out_labels);
     return launch_row_select(p, p.n, stream);
+}
+
+int launch_matrix_select(const float* keys, int64_t nq, int64_t n, int64_t ld, int k, int metric, const float* qnorm,
+                         int64_t label_base, float* out_dist, int64_t* out_labels, const int* nq_dev,
+                         const int32_t* row_map, cudaStream_t stream) {
+    if (n < 0 || n > 0x7fffffffLL || ld < n) return B200F_ERR_BAD_ARG;
+    RowSelectParams p{};
+    p.keys = keys;
+    p.ld = ld;
+    p.n = n;
+    p.nq = nq;
+    p.nq_dev = nq_dev;
+    p.row_map = row_map;
+    p.k = k;
+    set_output(p, metric, qnorm, label_base, out_dist, out_labels);
+    return launch_row_select(p, n, stream);
 }
 
 bool rank_merge_fits(int P, int k) { return k > 32 && P >= 1 && (int64_t)P * k <= 8192; }

@@ -1,0 +1,49 @@
+"""Streaming scans whose thresholds come from a sample of the rows: candidate buffers (k > 32) and lists
+cut at a threshold (k <= 32), at the row counts where they begin, on rows the sample misjudges and on ties."""
+import numpy as np
+import pytest
+
+import helpers as H
+from oracle import flat_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("storage,metric", [(0, O.METRIC_L2), (1, O.METRIC_INNER_PRODUCT), (2, O.METRIC_L2)])
+@pytest.mark.parametrize("nb", [32_767, 32_768, 100_003])
+@pytest.mark.parametrize("nq,k", [(1, 33), (3, 200), (4, 4096), (8, 1000)])
+def test_candidates(fm, res, storage, metric, nb, nq, k):
+    d = 40
+    xb = H.gaussian(nb, d, 1)
+    xq = H.gaussian(nq, d, 2)
+    idx = fm.B200IndexFlat(res, d, metric, storage)
+    idx.add(xb)
+    idx.set_path(1)
+    D, I = idx.search(xq, k)
+    H.check_against_oracle(metric, storage, False, xb, xq, k, D, I, loose=False)
+    idx.close()
+
+
+@pytest.mark.parametrize("storage", [0, 2])
+@pytest.mark.parametrize("nq,k", [(1, 24), (1, 100), (5, 32), (8, 100)])
+def test_rows_the_sample_misjudges(fm, res, storage, nq, k):
+    # every row the sample takes (row numbers that are multiples of its stride) is nearer to the first query
+    # than any other: its threshold admits far fewer than k rows; for the second query one row is repeated
+    # 40,000 times, more than its candidate buffer holds.  Both must come out exactly.
+    nb, d = 600_000, 16
+    xb = H.gaussian(nb, d, 3)
+    xb[::4] = 6.0 + 0.1 * H.gaussian(nb // 4, d, 4)
+    xb[::64] = 3.0 + 0.1 * H.gaussian(len(xb[::64]), d, 5)
+    xb[1:160_001:4] = xb[1]
+    xq = H.gaussian(nq, d, 6)
+    xq[0] = 2.5
+    if nq > 1:
+        xq[1] = xb[1] + 0.2
+    for use_path in (0, 1):
+        idx = fm.B200IndexFlat(res, d, O.METRIC_L2, storage)
+        idx.add(xb)
+        idx.set_path(use_path)
+        D, I = idx.search(xq, k)
+        tensor = storage != 0 and k <= 32    # the streaming kernel rounds the query like the tensor path
+        H.check_against_oracle(O.METRIC_L2, storage, tensor, xb, xq, k, D, I, loose=False)
+        idx.close()
