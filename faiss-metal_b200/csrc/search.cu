@@ -133,16 +133,18 @@ static int64_t matrix_chunk_cols(int64_t nq, int64_t nb) {
 // sample holds on average e = k / stride of them, and its r-th best key, r = e + 4.5 sqrt(e) + 3, has
 // fewer than k rows of the shard under it only if the sample caught r of the k best (about one query in a
 // million).  About r * stride rows do lie under it; more than stride (r + 6 sqrt(r) + 12), what the
-// candidate buffers hold, for one query in 10^8.  Of about `target` rows, more where that admits
-// thousands of candidates beyond 2 k, fewer where r would be beyond 400.  False: shard too small.
-bool choose_sample(int64_t nb, int k, int64_t target, int* stride_out, int* rank_out, int* cap_out) {
+// candidate buffers hold, for one query in 10^8.  Of about `target` rows, fewer where r would be beyond
+// 400.  buffers: more where that admits thousands of candidates beyond 2 k (lists spread what the
+// threshold admits over every warp of the GPU and keep the sample small: it has to fit the scratch of
+// the search without allocation at any shard size).  False: shard too small.
+bool choose_sample(int64_t nb, int k, int64_t target, bool buffers, int* stride_out, int* rank_out, int* cap_out) {
     auto rank_of = [k](int stride) {
         const double e = (double)k / stride;
         return (int)(e + 4.5 * std::sqrt(e) + 3.0 + 0.999);
     };
     int stride = 1;
-    while (stride < 1024 && nb / (2 * stride) >= target) stride *= 2;
-    while (stride > 2 && (int64_t)rank_of(stride) * stride > 2 * (int64_t)k + 2048) stride /= 2;
+    while (nb / (2 * stride) >= target) stride *= 2;
+    while (buffers && stride > 2 && (int64_t)rank_of(stride) * stride > 2 * (int64_t)k + 2048) stride /= 2;
     while (rank_of(stride) > 400) stride *= 2;
     const int r = rank_of(stride);
     if (stride < 2 || nb / stride < 8 * (int64_t)r) return false;
@@ -236,7 +238,7 @@ bool make_plan(int64_t nq, int64_t nb, int d, int k, int storage, int path, bool
     if (!pairwise && pl.path == B200F_PATH_SCAN && nq <= 2 * SCAN_GROUP && !filter_disabled()) {
         const bool wanted = pl.fused ? (nb >= SCAN_LIST_THR_MIN_ROWS && nq * k >= SCAN_LIST_THR_MIN_WORK)
                                      : nb >= SCAN_FILTER_MIN_ROWS;
-        pl.sample = wanted && choose_sample(nb, k, SCAN_SAMPLE_ROWS, &pl.fstride, &pl.frank, &pl.fcap);
+        pl.sample = wanted && choose_sample(nb, k, SCAN_SAMPLE_ROWS, !pl.fused, &pl.fstride, &pl.frank, &pl.fcap);
         if (pl.sample) {
             pl.nsample = nb / pl.fstride;
             const int64_t n1 = nq > 0 ? nq : 1;

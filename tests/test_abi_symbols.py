@@ -99,6 +99,16 @@ def test_library_switches_without_gpu(fm):
     assert L.b200f_search_scratch_bytes(64, 100000, 128, 10, 2, 2) == plain
 
 
+def test_built_in_scratch_holds_small_searches_of_any_shard(fm):
+    # 4 queries, k = 32: the largest search the entry point without scratch takes, whatever the rows
+    L = fm.lib()
+    for storage in (0, 1, 2):
+        for nb in (1, 1000, 524_288, 1_000_003, 50_000_000, 400_000_001, 2 ** 31 - 1):
+            for d in (1, 128, 1536):
+                for nq, k in ((1, 32), (4, 6), (4, 32)):
+                    assert L.b200f_search_scratch_bytes(nq, nb, d, k, storage, 1) <= L.b200f_noalloc_scratch_capacity()
+
+
 def test_python_mirror_validates_arrays(fm):
     # dtype / shape errors are caught before a pointer reaches the C side
     import numpy as np
