@@ -7,6 +7,7 @@
 // (src/MetalIndexFlat.mm:224-255).  One warp owns one row; lanes read 128-bit
 // vectors and reduce with shuffles.  Squares are formed in fp32 (the reference's
 // "f16" norm kernels square in half precision, which is not reproduced).
+#include <algorithm>
 #include <cmath>
 
 #include "common.cuh"
@@ -175,10 +176,12 @@ __device__ __forceinline__ void store_bits(uint16_t* p, const uint16_t (&b)[V]) 
 }
 
 // HBM-bound: 4 d bytes read and (fp32 rows, two fp16 planes) 8 d written per row.  A row belongs to
-// lpr lanes of a warp (all 32 from d = 4 V 8 on, fewer for short rows, so that no lane idles), each
-// lane keeps U vectors in flight and the row is read ONCE: squares, conversions and the plane split
-// all come from the same registers.  1,000,003 rows of d = 384, fp32 with fp16 planes: 720 us
-// (6.5 TB/s); element by element with a second read of the row for the planes it took 940 us.
+// lpr lanes of a warp, as many as leave each lane up to U vectors of it: they are loaded together, the row
+// is read ONCE, and squares, conversions and the plane split all come from the same registers.
+// 1,000,003 rows of d = 384, fp32 with fp16 planes: 720 us (6.5 TB/s); element by element with a second
+// read of the row for the planes it took 940 us.  One vector per lane (a whole warp on a row of 128) kept
+// too few loads in flight and a single lane busy with the norm pieces: add() of 1 GiB to an fp16 index of
+// d = 128 took 0.63 ms (element by element 0.50), now 0.29 ms (5.7 TB/s read and written).
 template <int STORAGE, int V>
 __global__ void __launch_bounds__(ROW_THREADS)
 store_rows_kernel(const float* __restrict__ src, int64_t src_pitch, int64_t n, int d, int lpr,
@@ -203,7 +206,7 @@ store_rows_kernel(const float* __restrict__ src, int64_t src_pitch, int64_t n, i
         uint16_t* const p0 = planes + r * plane_pitch;
         const bool copy_row = STORAGE != B200F_STORAGE_F32 || outf != row;   // a re-split reads the stored rows themselves
         float s = 0.f, amax = 0.f;
-        for (int64_t base = 0; base < width; base += (int64_t)lpr * V * U) {
+        for (int64_t base = 0; base < d; base += (int64_t)lpr * V * U) {
             FloatVec<V> x[U];
 #pragma unroll
             for (int u = 0; u < U; u++) {
@@ -215,13 +218,12 @@ store_rows_kernel(const float* __restrict__ src, int64_t src_pitch, int64_t n, i
 #pragma unroll
             for (int u = 0; u < U; u++) {
                 const int64_t j = base + ((int64_t)u * lpr + cl) * V;
-                if (!live || j >= width) continue;
-                const bool ncol = norm_cols && j >= d8 && j < d8 + 8;   // written below
+                if (!live || j >= d) continue;
                 if (STORAGE == B200F_STORAGE_F32) {
 #pragma unroll
                     for (int e = 0; e < V; e++) s = fmaf(x[u].v[e], x[u].v[e], s);
-                    if (copy_row && j < dst_pitch) *reinterpret_cast<FloatVec<V>*>(outf + j) = x[u];
-                    if (!planes || j >= plane_pitch) continue;
+                    if (copy_row) *reinterpret_cast<FloatVec<V>*>(outf + j) = x[u];
+                    if (!planes) continue;
                     uint16_t h0[V], h1[V], h2[V];
                     if (plane_format == kPlanesFp16x2) {
 #pragma unroll
@@ -241,7 +243,7 @@ store_rows_kernel(const float* __restrict__ src, int64_t src_pitch, int64_t n, i
                         }
                         store_bits<V>(p0 + 2 * plane_stride + j, h2);
                     }
-                    if (!ncol) store_bits<V>(p0 + j, h0);
+                    store_bits<V>(p0 + j, h0);
                     store_bits<V>(p0 + plane_stride + j, h1);
                 } else {
                     uint16_t h[V];
@@ -257,8 +259,22 @@ store_rows_kernel(const float* __restrict__ src, int64_t src_pitch, int64_t n, i
                         }
                         s = fmaf(back, back, s);
                     }
-                    if (!ncol) store_bits<V>(outh + j, h);
+                    store_bits<V>(outh + j, h);
                 }
+            }
+        }
+        // pads behind the row's elements (a few columns), except the norm columns, which are written below
+        for (int64_t j = d + (int64_t)cl * V; live && j < width; j += (int64_t)lpr * V) {
+            const uint16_t z[V] = {};
+            const bool ncol = norm_cols && j >= d8 && j < d8 + 8;
+            if (STORAGE == B200F_STORAGE_F32) {
+                if (copy_row && j < dst_pitch) *reinterpret_cast<FloatVec<V>*>(outf + j) = FloatVec<V>{};
+                if (!planes || j >= plane_pitch) continue;
+                if (!ncol) store_bits<V>(p0 + j, z);
+                store_bits<V>(p0 + plane_stride + j, z);
+                if (plane_format != kPlanesFp16x2) store_bits<V>(p0 + 2 * plane_stride + j, z);
+            } else if (!ncol) {
+                store_bits<V>(outh + j, z);
             }
         }
         for (int o = lpr >> 1; o > 0; o >>= 1) {
@@ -277,7 +293,9 @@ store_rows_kernel(const float* __restrict__ src, int64_t src_pitch, int64_t n, i
             else
                 norm_pieces(-0.5f * s, STORAGE == B200F_STORAGE_F32 ? B200F_STORAGE_BF16 : STORAGE, pc);
             uint16_t* o = (STORAGE == B200F_STORAGE_F32) ? (planes ? p0 + d8 : nullptr) : outh + d8;
-            if (o) {
+            if (o && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
+                store_bits<8>(o, pc);
+            } else if (o) {
 #pragma unroll
                 for (int i = 0; i < 8; i++) o[i] = pc[i];
             }
@@ -594,7 +612,9 @@ int store_rows_impl(const float* src, int64_t src_pitch, int64_t n, int d, int s
     while (v > 1 && !(d % v == 0 && vec_ok(src, 4, v, src_pitch) && vec_ok(dst_rows, fp32 ? 4 : 2, v, dst_pitch) &&
                       (!planes || vec_ok(planes, 2, v, plane_pitch, plane_stride))))
         v >>= 1;
-    const int lpr = lanes_for_row(d, v);
+    // four vectors per lane, at least four lanes on rows that have as many (whole 32-byte sectors of
+    // 16-bit elements per store)
+    const int lpr = v == 4 ? std::max(lanes_for_row(d, 16), std::min(4, lanes_for_row(d, 4))) : lanes_for_row(d, 2 * v);
     const int g = grid_for_rows(ceil_div64(n, 32 / lpr));
     // macro: the kernel is a template over (storage, elements per access)
 #define B200F_STORE_ROWS(ST, V)                                                                          \
