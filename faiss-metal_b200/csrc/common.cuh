@@ -110,6 +110,7 @@ struct GemmOperands {
     const int32_t* rowscale_map;  // optional: row j of A is row rowscale_map[j] of rowscale (redone rows)
     int64_t nq, nb;
     int d_pad;                 // K extent (multiple of 8), norm columns included
+    int d_data;                // K extent without them
     const int* nq_dev;         // optional: live rows of A (<= nq) left in device memory by a kernel
 };
 // Fused top-k (k <= 32): partial lists part_key/part_idx [nq][2 * P][k] (two per column range).

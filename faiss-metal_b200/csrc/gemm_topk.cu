@@ -110,8 +110,11 @@ struct GemmParams {
     int64_t tiles_per_range;
     int nqb;
     int P;
-    int kb_per_pass;     // k-blocks of 64 per plane product
-    int k_extent;        // valid K elements per plane product (multiple of 8)
+    // k-blocks of 64 and valid K elements (multiple of 8) of a plane product.  The norm columns are zero in
+    // every plane but the first, so only the last product, of the two first planes, takes them (d = 128,
+    // three products: 25 MMAs a tile instead of 27, 7 k-blocks instead of 9).
+    int kb_per_pass, kb_last_pass;
+    int k_extent, k_extent_last;
     int npass;
     uint32_t pass_a;     // 4 bits per pass: plane index of A
     uint32_t pass_b;
@@ -420,7 +423,7 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
     const int64_t nq_live = p.nq_dev ? min((int64_t)*p.nq_dev, p.nq) : p.nq;
     const int nqb = p.nq_dev ? (int)((nq_live + C::QB - 1) / C::QB) : p.nqb;
     const int64_t nitems = (int64_t)nqb * p.P;
-    const int kb_total = p.kb_per_pass * p.npass;
+    const int kb_total = p.kb_per_pass * (p.npass - 1) + p.kb_last_pass;
 
     if (warp == 0) {
         // ------------------------------ TMA producer ------------------------------
@@ -440,7 +443,7 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
                             ok = false;
                             break;
                         }
-                        const int pass = kb / p.kb_per_pass;
+                        const int pass = min(kb / p.kb_per_pass, p.npass - 1);
                         const int kk = (kb - pass * p.kb_per_pass) * BK;
                         const int pa = (p.pass_a >> (4 * pass)) & 15;
                         const int pb = (p.pass_b >> (4 * pass)) & 15;
@@ -502,8 +505,8 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
             const uint32_t tfull1 = PAIR ? map_to_cta(bar_tfull, 1) : 0;
             // the last k-block of a plane product may hold fewer than 64 valid K elements
             // (TMA zero-fills the rest): skip the all-zero sub-steps
-            const int klast_valid = p.k_extent - (p.kb_per_pass - 1) * BK;
-            const int nk4_last = klast_valid >= BK ? BK / UMMA_K : (klast_valid + UMMA_K - 1) / UMMA_K;
+            const int nk4_pass = (p.k_extent - (p.kb_per_pass - 1) * BK + UMMA_K - 1) / UMMA_K;
+            const int nk4_end = (p.k_extent_last - (p.kb_last_pass - 1) * BK + UMMA_K - 1) / UMMA_K;
             for (int64_t item = unit; item < nitems && ok; item += nunits) {
                 const int64_t xr = item / nqb;
                 const int64_t t0 = xr * p.tiles_per_range;
@@ -517,6 +520,7 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
                     tc_fence_after();
                     const uint32_t d_tmem = tmem_base + acc * TILE_N;
                     int kin = 0;
+                    const int kb_early = kb_total - p.kb_last_pass;   // k-blocks of the products before the last
                     uint32_t accumulate = 0;
                     for (int kb = 0; kb < kb_total; kb++) {
                         if (!mbar_try_wait(bar_full + stage * 8, phase) &&
@@ -526,9 +530,15 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
                         }
                         const uint64_t da = da0 + (uint64_t)(stage * (A_STAGE_BYTES >> 4));
                         const uint64_t db = db0 + (uint64_t)(stage * (B_STAGE_BYTES >> 4));
-                        const bool last = ++kin == p.kb_per_pass;
-                        if (last) kin = 0;
-                        const int nk4 = last ? nk4_last : BK / UMMA_K;
+                        int nk4 = BK / UMMA_K;
+                        if (kb < kb_early) {
+                            if (++kin == p.kb_per_pass) {
+                                kin = 0;
+                                nk4 = nk4_pass;
+                            }
+                        } else if (kb == kb_total - 1) {
+                            nk4 = nk4_end;
+                        }
 #pragma unroll
                         for (int k4 = 0; k4 < BK / UMMA_K; k4++) {
                             // advance 32 bytes (16 elements) along K inside the swizzle row
@@ -672,44 +682,51 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
                             for (int c = 0; c < CW; c++)
                                 if (cbase + c >= p.ncols_end) r[c] = 0xff800000u;  // -INF
                         }
-                        // one max per column (tree), one compare per CW columns
-                        float m[CW / 2];
+                        // one max per column: of every group of eight columns, then of all
+                        constexpr int NG = CW / 8;
+                        float gm[NG];
 #pragma unroll
-                        for (int c = 0; c < CW / 2; c++)
-                            m[c] = fmaxf(__uint_as_float(r[c]), __uint_as_float(r[c + CW / 2]));
+                        for (int g = 0; g < NG; g++) {
+                            float m4[4];
 #pragma unroll
-                        for (int w2 = CW / 4; w2 > 0; w2 >>= 1)
+                            for (int c = 0; c < 4; c++)
+                                m4[c] = fmaxf(__uint_as_float(r[8 * g + c]), __uint_as_float(r[8 * g + 4 + c]));
+                            gm[g] = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+                        }
+                        float m[NG];
 #pragma unroll
-                            for (int c = 0; c < w2; c++) m[c] = fmaxf(m[c], m[c + w2]);
-                        // Slow path, entered by the whole warp when any row has a candidate in
-                        // this chunk: a lane marks its hit columns and moves them to its stage.
-                        const bool any_hit = row_live && (-m[0] < thr_eff);
-                        if (__any_sync(0xffffffffu, any_hit)) {
-                            if (any_hit) {
+                        for (int g = 0; g < NG; g++) m[g] = gm[g];
 #pragma unroll
-                                for (int h = 0; h < CW / 32; h++) {
-                                    uint32_t mask = 0;
+                        for (int w2 = NG / 2; w2 > 0; w2 >>= 1)
 #pragma unroll
-                                    for (int c = 0; c < 32; c++)
-                                        mask |= (-__uint_as_float(r[h * 32 + c]) < thr_eff ? 1u : 0u) << c;
-                                    while (mask != 0) {
-                                        const int cc = __ffs(mask) - 1;
-                                        mask &= mask - 1;
-                                        uint32_t bits = 0;
+                            for (int g = 0; g < w2; g++) m[g] = fmaxf(m[g], m[g + w2]);
+                        // Slow path, entered by the whole warp when any row has a candidate in this chunk:
+                        // the groups that hold one, column by column, each hit to its thread's stage (1,000
+                        // queries, 100,000 fp32 rows of d = 128, 320 candidates a query: 243 us a search with a
+                        // mask over all columns and a select chain per hit, 222 with this).
+                        if (__any_sync(0xffffffffu, row_live && -m[0] < thr_eff)) {
 #pragma unroll
-                                        for (int c = 0; c < 32; c++) bits = (c == cc) ? r[h * 32 + c] : bits;
-                                        if (nstaged == STAGE_N) {  // rare: list warm-up, massive ties
-                                            if (MODE == MODE_TOPK)
-                                                drain_to_list(lk, li, stage_key, stage_idx, nstaged, thr, thr_eff);
-                                            else
-                                                drain_to_buffer(p.cand_cnt + grow, p.cand_key + grow * p.cand_cap,
-                                                                p.cand_idx + grow * p.cand_cap, p.cand_cap,
-                                                                ksc, stage_key, stage_idx, nstaged);
-                                            nstaged = 0;
+                            for (int g = 0; g < NG; g++) {
+                                const bool hit = row_live && -gm[g] < thr_eff;
+                                if (!__any_sync(0xffffffffu, hit)) continue;
+                                if (hit) {
+                                    if (nstaged > STAGE_N - 8) {  // rare: list warm-up, massive ties
+                                        if (MODE == MODE_TOPK)
+                                            drain_to_list(lk, li, stage_key, stage_idx, nstaged, thr, thr_eff);
+                                        else
+                                            drain_to_buffer(p.cand_cnt + grow, p.cand_key + grow * p.cand_cap,
+                                                            p.cand_idx + grow * p.cand_cap, p.cand_cap,
+                                                            ksc, stage_key, stage_idx, nstaged);
+                                        nstaged = 0;
+                                    }
+#pragma unroll
+                                    for (int c = 0; c < 8; c++) {
+                                        const float sc = -__uint_as_float(r[8 * g + c]);
+                                        if (sc < thr_eff) {
+                                            stage_key[nstaged * STAGE_LD] = sc;
+                                            stage_idx[nstaged * STAGE_LD] = (int32_t)cbase + 8 * g + c;
+                                            nstaged++;
                                         }
-                                        stage_key[nstaged * STAGE_LD] = -__uint_as_float(bits);
-                                        stage_idx[nstaged * STAGE_LD] = (int32_t)cbase + h * 32 + cc;
-                                        nstaged++;
                                     }
                                 }
                             }
@@ -876,8 +893,10 @@ int launch_common(const GemmOperands& op, const GemmPlan& plan, GemmParams& p, i
     p.tiles_per_range = plan.tiles_per_range;
     p.nqb = plan.nqb;
     p.P = plan.P;
-    p.kb_per_pass = (int)ceil_div64(op.d_pad, BK);
-    p.k_extent = op.d_pad;
+    p.kb_per_pass = (int)ceil_div64(op.d_data, BK);
+    p.k_extent = op.d_data;
+    p.kb_last_pass = (int)ceil_div64(op.d_pad, BK);
+    p.k_extent_last = op.d_pad;
     p.rowscale = op.rowscale;
     p.rowscale_map = op.rowscale_map;
     if (op.npl == 1) {

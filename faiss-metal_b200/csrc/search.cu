@@ -402,7 +402,8 @@ int fill_operands(const B200FSearchArgs& a, const SearchPlan& pl, uint8_t* scrat
     op.nb = a.nb;
     const bool l2 = a.metric == B200F_METRIC_L2;
     if (l2 && !a.norm_cols) return B200F_ERR_BAD_ARG;  // the tensor path takes ||x||^2 from the rows
-    op.d_pad = (int)round_up64(a.d, 8) + (l2 ? 8 : 0);
+    op.d_data = (int)round_up64(a.d, 8);
+    op.d_pad = op.d_data + (l2 ? 8 : 0);
     if (a.storage == B200F_STORAGE_F32) {
         if (!a.planes || a.plane_pitch < op.d_pad || (a.plane_pitch % 8) != 0 ||
             (a.plane_stride % 8) != 0)
