@@ -97,6 +97,7 @@ struct GemmPlan {
     int P;               // column ranges == partial lists per query
     int64_t tiles_per_range;
     int grid;
+    int units;           // CTAs (CTA pairs) that run at once
 };
 GemmPlan plan_gemm(int64_t nq, int64_t ncols, int sm_count);
 struct GemmOperands {
@@ -150,10 +151,6 @@ int launch_merge_partials(const float* part_key, const int32_t* part_idx, int P,
 // Merged raw keys only: out_key[q][k], best first, +INF where fewer than k entries exist.
 int launch_merge_keys(const float* part_key, const int32_t* part_idx, int P, int64_t nq, int k,
                       float* out_key, cudaStream_t stream);
-// The r <= 32 smallest keys of every row of a key matrix (no ids): out_key[q][r], best first,
-// +INF where the row has fewer.  One warp per row.
-int launch_select_keys(const float* keys, int64_t nq, int64_t ncols, int64_t ld, int r, float* out_key,
-                       cudaStream_t stream);
 // nq_dev (optional): number of live rows, read on the device.
 int launch_select_chunk(const float* keys, int64_t nq, int64_t ncols, int64_t ld, int64_t col0,
                         int k, int has_prev, float* run_key, int32_t* run_idx, const int* nq_dev,

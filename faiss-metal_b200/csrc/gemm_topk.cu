@@ -1018,6 +1018,7 @@ GemmPlan plan_gemm(int64_t nq, int64_t ncols, int sm_count) {
     g.pair = ov >= 0 ? ov : (nq > BM ? 1 : 0);       // a pair covers 256 query rows
     const int qb = g.pair ? 2 * BM : BM;
     const int units = g.pair ? max_active_pairs(sm_count) : sm_count;  // CTAs or CTA pairs that run at once
+    g.units = units;
     g.nqb = (int)ceil_div64(nq, qb);
     g.tile_n = g.pair ? Cfg<true>::TILE_N : Cfg<false>::TILE_N;
     g.ntiles = ceil_div64(ncols, g.tile_n);

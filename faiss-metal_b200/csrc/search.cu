@@ -58,6 +58,7 @@ struct SearchPlan {
     bool fused;       // k <= 32
     bool lists;       // k > 32 selected from the fused kernel's 32-entry lists, matrix fallback per row
     int gslots;       // words per query row in the shared bound array
+    bool direct;      // tensor path: the keys of all rows as one matrix, selected from directly
     bool filter;      // pilot threshold + candidate buffers, fused / matrix fallback per row
     bool sample;      // scan path: thresholds from a sample of the rows (lists cut at them, or candidate buffers)
     int64_t nsample;  // rows in that sample
@@ -107,16 +108,24 @@ bool filter_disabled() { const int m = select_mode(); return m == B200F_SELECT_N
 bool filter_forced() { return select_mode() == B200F_SELECT_FILTER; }
 bool lists_disabled() { return select_mode() == B200F_SELECT_MATRIX; }
 
-// The pilot pass costs 0.1 - 0.2 ms whatever the size (a handful of work items, each warming up
-// its lists on a single tile).  Measured: at 2.6e8 (query, row) pairs the filter path is 19 - 47 %
-// faster than the lists (d = 768 / 1536, 16-bit rows), at 1e8 - 4e8 pairs of fp32 rows with
-// d = 128 the two are level; below this many pairs the lists are used.
 // fp32 rows: five to eight queries take the scan path where the tf32 streaming scan pays and fits (three
 // stages of 16 rows and two query matrices in shared memory: d up to 768)
 constexpr int64_t F32_STREAM_MIN_ROWS = 65536;
 constexpr int F32_STREAM_MAX_D = 768;
+// A pilot pass made of lists costs 0.1 - 0.2 ms whatever the size (a handful of work items, each warming
+// up its lists on a single tile).  Measured: at 2.6e8 (query, row) pairs the filter path is 19 - 47 %
+// faster than the lists (d = 768 / 1536, 16-bit rows), at 1e8 - 4e8 pairs of fp32 rows with
+// d = 128 the two are level; below FILTER_MIN_PAIRS the lists are used.  A pilot kept as a key matrix
+// costs 20 us and pays wherever the matrix of all keys is too large (DIRECT_MAX_*).
 constexpr int64_t FILTER_MIN_PAIRS = 1ll << 27;
-constexpr int64_t FILTER_MIN_PAIRS_MATRIX = 1ll << 22;
+constexpr int64_t FILTER_MIN_PAIRS_MATRIX = 1ll << 18;
+constexpr int PILOT_MAX_RANK = 400;
+// Few pairs: the whole key matrix fits the L2 cache and one row of it a CTA's few passes, so store and
+// select it, two launches (100 queries, 10,000 rows, k = 10: 64 us a search, 158 with the fused lists, whose
+// first tiles insert nearly every key).  Beyond, the filter (50 queries, 300,007 rows, k = 2048: 174 us, 476
+// with the matrix and a CTA per row of it).
+constexpr int64_t DIRECT_MAX_ROWS = 32768;
+constexpr int64_t DIRECT_MAX_PAIRS = 16ll << 20;
 constexpr int64_t PILOT_MATRIX_BYTES = 256ll << 20;   // k <= 32: largest pilot sample kept as a key matrix
 
 // columns of the key matrix slice: at most MATRIX_BUDGET_BYTES, at least 1024, never more than the shard
@@ -197,36 +206,56 @@ bool make_plan(int64_t nq, int64_t nb, int d, int k, int storage, int path, bool
     pl.off_qscale = off;   // per-row key scales of the fp16x2 plane format
     adv((size_t)(nq > 0 ? nq : 1) * 4);
     pl.gslots = 1;
-    if (!pairwise && pl.path == B200F_PATH_TENSOR && k <= B200F_LIST_MAX_K && !filter_disabled()) {
+    if (!pairwise && pl.path == B200F_PATH_TENSOR && rank_select_enabled() && select_mode() == B200F_SELECT_AUTO &&
+        nb <= DIRECT_MAX_ROWS && nq * nb <= DIRECT_MAX_PAIRS) {
+        pl.fused = false;   // all keys as one matrix, selected from by row_select
+        pl.direct = true;
+    }
+    if (!pl.direct && !pairwise && pl.path == B200F_PATH_TENSOR && !filter_disabled()) {
         // The pilot sample holds nb / stride rows and, on average, e = k / stride of a query's k
         // best.  The threshold is the sample's r-th best key with r = e + 4.5 sqrt(e) + 3: fewer
         // than k rows of the shard lie under it only if the sample caught r of the k best, which
         // is about one row in a million; about r * stride rows do lie under it.
-        const int stride = k <= 128 ? 64 : 128;
-        // with the pilot sample kept as a key matrix (no list warm-up) the filter wins from far
-        // fewer pairs: measured 26 - 36 % faster than the lists at 3e7 - 1.3e8 pairs (d = 128, k = 10)
-        int64_t min_pairs = FILTER_MIN_PAIRS;
-        if (nb >= (int64_t)stride * 1024 && rank_select_enabled()) {
-            const GemmPlan g0 = plan_gemm(nq, nb, sm);
-            const int64_t pcols = ceil_div64(g0.ntiles, stride) * g0.tile_n;
-            const int64_t n1 = nq > 0 ? nq : 1;
-            const bool as_matrix = (k <= B200F_FUSED_MAX_K) ? n1 * pcols * 4 <= PILOT_MATRIX_BYTES
-                                                            : pcols <= matrix_chunk_cols(nq, nb);
-            if (as_matrix) min_pairs = FILTER_MIN_PAIRS_MATRIX;
-        }
-        if (nb >= (int64_t)stride * 1024 && (nq * nb >= min_pairs || filter_forced())) {
+        auto rank_of = [k](int stride) {
             const double e = (double)k / stride;
-            int r = (int)(e + 4.5 * std::sqrt(e) + 3.0 + 0.999);
-            if (r > B200F_FUSED_MAX_K) r = B200F_FUSED_MAX_K;
+            return (int)(e + 4.5 * std::sqrt(e) + 3.0 + 0.999);
+        };
+        const GemmPlan g0 = plan_gemm(nq, nb, sm);
+        const int64_t n1 = nq > 0 ? nq : 1;
+        // A list starts empty and takes every key of its first tile: ~0.1 ms per work item, and a small
+        // shard's pilot is all first tiles.  Where the sample's keys fit the matrix slice they are
+        // written out instead and a selection kernel bounds the r-th best.
+        auto as_matrix = [&](int stride) {
+            const int64_t pcols = ceil_div64(g0.ntiles, stride) * g0.tile_n;
+            return rank_select_enabled() && (k <= B200F_FUSED_MAX_K ? n1 * pcols * 4 <= PILOT_MATRIX_BYTES
+                                                                    : pcols <= matrix_chunk_cols(nq, nb));
+        };
+        int stride = k <= 128 ? 64 : 128;
+        const bool matrix = as_matrix(stride);
+        if (matrix) {
+            // A sample that the GPU's CTAs take in one wave costs the same whatever its size, so it may as
+            // well be larger: a closer threshold, fewer candidates (1,000 queries, 100,000 rows: one
+            // row in 16 instead of 64, 128 candidates instead of 320).  Forced, the filter keeps its sparse
+            // sample, which misjudges more rows.
+            while (!filter_forced() && stride > 8 && ceil_div64(g0.ntiles, stride / 2) * g0.nqb <= g0.units && as_matrix(stride / 2) &&
+                   rank_of(stride / 2) <= PILOT_MAX_RANK)
+                stride /= 2;
+        }
+        const int r = rank_of(stride);
+        const int64_t least = 8 * (int64_t)r > 1024 ? 8 * (int64_t)r : 1024;   // rows of a sample worth having
+        const int64_t min_pairs = matrix ? FILTER_MIN_PAIRS_MATRIX : FILTER_MIN_PAIRS;
+        if ((r <= B200F_FUSED_MAX_K || matrix) && nb >= stride * least && (nq * nb >= min_pairs || filter_forced())) {
+            const int bound = (int)round_up64((int64_t)(stride * (r + 6.0 * std::sqrt((double)r) + 12.0)), 256);
             int cap = 1024;
             while (cap < 4 * r * stride && cap < 8192) cap <<= 1;
             pl.filter = true;
+            pl.pilot_matrix = matrix;
             pl.fstride = stride;
             pl.frank = r;
-            pl.fcap = cap;
+            pl.fcap = cap > bound ? cap : bound;
         }
     }
-    if (!pl.filter && !pl.fused && !pairwise && pl.path == B200F_PATH_TENSOR && k <= B200F_LIST_MAX_K &&
+    if (!pl.direct && !pl.filter && !pl.fused && !pairwise && pl.path == B200F_PATH_TENSOR && k <= B200F_LIST_MAX_K &&
         !lists_disabled()) {
         // lists must be able to hold the result four times over, else the fallback would be the rule
         const GemmPlan g = plan_gemm(nq, nb, sm);
@@ -292,10 +321,12 @@ bool make_plan(int64_t nq, int64_t nb, int d, int k, int storage, int path, bool
         const int64_t n1 = nq > 0 ? nq : 1;
         if (!pl.fused) pl.gemm = plan_gemm(nq, nb, sm);
         pl.pilot = plan_gemm(nq, ceil_div64(pl.gemm.ntiles, pl.fstride) * pl.gemm.tile_n, sm);
-        pl.off_pilot_key = off;
-        adv((size_t)n1 * 2 * (pl.pilot.P > 0 ? pl.pilot.P : 1) * pl.frank * 4);
-        pl.off_pilot_idx = off;
-        adv((size_t)n1 * 2 * (pl.pilot.P > 0 ? pl.pilot.P : 1) * pl.frank * 4);
+        if (!pl.pilot_matrix) {
+            pl.off_pilot_key = off;
+            adv((size_t)n1 * 2 * (pl.pilot.P > 0 ? pl.pilot.P : 1) * pl.frank * 4);
+            pl.off_pilot_idx = off;
+            adv((size_t)n1 * 2 * (pl.pilot.P > 0 ? pl.pilot.P : 1) * pl.frank * 4);
+        }
         pl.off_thr = off;
         adv((size_t)n1 * pl.frank * 4);
         pl.off_cand_key = off;
@@ -305,16 +336,11 @@ bool make_plan(int64_t nq, int64_t nb, int d, int k, int storage, int path, bool
         pl.off_cand_cnt = off;
         adv((size_t)n1 * 4);
     }
-    if (pl.filter && pl.fused && rank_select_enabled()) {
+    if (pl.pilot_matrix && pl.fused) {
         // k <= 32 has no matrix slice of its own: a small one for the pilot sample alone (the lists'
         // first-tile cost, ~0.1 ms per work item, is most of a small search)
-        const int64_t pcols = pl.pilot.ntiles * pl.pilot.tile_n;
-        const int64_t n1 = nq > 0 ? nq : 1;
-        if (pcols > 0 && n1 * pcols * 4 <= PILOT_MATRIX_BYTES) {
-            pl.pilot_matrix = true;
-            pl.off_matrix = off;
-            adv((size_t)(n1 * pcols * 4));
-        }
+        pl.off_matrix = off;
+        adv((size_t)(nq > 0 ? nq : 1) * pl.pilot.ntiles * pl.pilot.tile_n * 4);
     }
     if (pl.lists || pl.filter) {
         pl.off_dirty = off;
@@ -330,11 +356,6 @@ bool make_plan(int64_t nq, int64_t nb, int d, int k, int storage, int path, bool
         const int64_t cols = matrix_chunk_cols(nq, nb);
         pl.chunk_cols = cols;
         if (!pl.lists && !pl.filter) pl.gemm = plan_gemm(nq, cols, sm);
-        // A list starts empty and takes every key of its first tile: ~0.1 ms per work item, and a
-        // small shard's pilot is all first tiles.  Where the sample's keys fit the matrix slice
-        // they are written out instead and the frank best picked by a selection kernel.
-        pl.pilot_matrix = pl.filter && rank_select_enabled() &&
-                          pl.pilot.ntiles * pl.pilot.tile_n <= cols;
         pl.off_matrix = off;
         adv((size_t)(nq > 0 ? nq : 1) * cols * 4);
         pl.off_run_key = off;
@@ -738,7 +759,7 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
             rc = launch_gemm_store(op, pl.pilot, 0, a->nb, pl.fstride, kscale, 1.f, nullptr, matrix, pcols,
                                    a->status, st);
             if (rc != B200F_OK) return rc;
-            rc = launch_select_keys(matrix, a->nq, valid, pcols, pl.frank, thr, st);
+            rc = launch_row_bound(matrix, a->nq, valid, pcols, pl.frank, thr, st);
             if (rc != B200F_OK) return rc;
         } else {
             rc = launch_gemm_topk(op, pl.pilot, 0, a->nb, pl.fstride, kscale, pl.frank, 1, pkey, pidx, gthr,
@@ -747,9 +768,10 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
             rc = launch_merge_keys(pkey, pidx, 2 * pl.pilot.P, a->nq, pl.frank, thr, st);
             if (rc != B200F_OK) return rc;
         }
-        // candidates per row ~ frank * fstride: a few hundred for k <= 128, thousands beyond
-        rc = launch_gemm_filter(op, pl.gemm, kscale, thr, pl.frank, pl.frank - 1, ckey, cidx, ccnt,
-                                pl.fcap, pl.fstride == 64 ? 1 : 0, a->status, st);
+        // about frank * fstride candidates per row; wide TMEM loads where fewer than one row in 1024 is one
+        rc = launch_gemm_filter(op, pl.gemm, kscale, thr, pl.pilot_matrix ? 1 : pl.frank,
+                                pl.pilot_matrix ? 0 : pl.frank - 1, ckey, cidx, ccnt, pl.fcap,
+                                (int64_t)pl.frank * pl.fstride * 1024 < a->nb ? 1 : 0, a->status, st);
         if (rc != B200F_OK) return rc;
         rc = launch_select_candidates(ckey, cidx, ccnt, pl.fcap, a->nb, a->nq, a->k, a->metric, qnorm,
                                       a->label_base, a->out_dist, a->out_labels, dirty, st);

@@ -408,7 +408,9 @@ __global__ void __launch_bounds__(1024) row_bound_kernel(const float* __restrict
         if (sp.live >= r) {
             const int bits = 32 - __clz(sp.mx - sp.mn);
             int kk = r;
-            const uint32_t x = radix_kth([&](auto f) { if (have) f(key); }, sp.mn, bits, bits > 16 ? bits - 16 : 0, kk,
+            // three digits: with keys of both signs the spread has 32 bits, and two would leave the bound
+            // 2^-7 of the key loose
+            const uint32_t x = radix_kth([&](auto f) { if (have) f(key); }, sp.mn, bits, bits > 24 ? bits - 24 : 0, kk,
                                          s_hist, s_sel);
             bound = ordered_to_float(sp.mn + min(x, sp.mx - sp.mn));
         }
@@ -617,6 +619,8 @@ int launch_row_select(RowSelectParams& p, int64_t n_typical, cudaStream_t stream
                         (p.nq * T < sm * 512 && T * 4 < n_typical)))        // rows alone do not fill the SMs
         T <<= 1;
     if (p.k > 64 && T < 256) T = 256;
+    // long rows: enough minima to bound the k-th key without histogram passes over the row
+    while (T < 1024 && T < 2 * p.k && 16 * (int64_t)T < n_typical) T <<= 1;
     p.bound = bound;
     const int smem = bound * 8;
     static bool attr_set[kMaxDevices] = {false};

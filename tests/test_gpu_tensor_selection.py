@@ -1,0 +1,45 @@
+"""Selection on the tensor path at the sizes where its stages change: the whole key matrix (up to 32,768 rows
+and 16 Mi pairs), thresholds from samples of different density, and k beyond 1024."""
+import numpy as np
+import pytest
+
+import helpers as H
+from oracle import flat_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("storage,metric", [(0, O.METRIC_L2), (1, O.METRIC_INNER_PRODUCT), (2, O.METRIC_L2)])
+@pytest.mark.parametrize("nq,nb,k", [(9, 1, 3), (130, 255, 300), (17, 32_768, 10), (17, 32_769, 10), (512, 32_768, 33),
+                                     (40, 32_768, 1500), (11, 32_769, 1025), (300, 60_000, 4096), (129, 140_001, 100)])
+def test_stages(fm, res, storage, metric, nq, nb, k):
+    d = 40
+    xb = H.gaussian(nb, d, 1)
+    xq = H.gaussian(nq, d, 2)
+    idx = fm.B200IndexFlat(res, d, metric, storage)
+    idx.add(xb)
+    D, I = idx.search(xq, k)
+    H.check_against_oracle(metric, storage, True, xb, xq[:40], k, D[:40], I[:40], loose=False)
+    H.check_against_oracle(metric, storage, True, xb, xq[-3:], k, D[-3:], I[-3:], loose=False)
+    idx.close()
+
+
+@pytest.mark.parametrize("storage", [0, 2])
+@pytest.mark.parametrize("k", [10, 100, 2000])
+def test_rows_the_sample_misjudges(fm, res, storage, k):
+    # the first tiles hold every near row of query 0 (the sample sees them all, or too few of them), and query 1
+    # finds one row 30,000 times, more than its candidate buffer holds
+    # ||q||^2 + ||x||^2 - 2 q.x in 22 bits leaves 2^-22 (||q|| + ||x||)^2 of a distance: 9e-5 of 0.24 d / 24 for
+    # query 1, 7e-5 of about 1.3 for query 0 (a cluster of sigma 0.3 around 2; of sigma 0.1 around 5 it would be 6e-3)
+    nb, nq, d = 120_000, 64, 24
+    xb = H.gaussian(nb, d, 3)
+    xb[:512] = 2.0 + 0.3 * H.gaussian(512, d, 4)
+    xb[80_000:110_000] = xb[80_000]
+    xq = H.gaussian(nq, d, 5)
+    xq[0] = 2.0
+    xq[1] = xb[80_000] + np.float32(0.1)
+    idx = fm.B200IndexFlat(res, d, O.METRIC_L2, storage)
+    idx.add(xb)
+    D, I = idx.search(xq, k)
+    H.check_against_oracle(O.METRIC_L2, storage, True, xb, xq[:8], k, D[:8], I[:8], loose=False)
+    idx.close()
