@@ -110,6 +110,11 @@ struct GemmParams {
     int64_t tiles_per_range;
     int nqb;
     int P;
+    // single CTA: rows of a query box, the live ones rounded up to 8.  Rows beyond the queries are never
+    // fetched: zero-filling 104 of 128 rows held the ring back to one k-block per 1,900 cycles whatever
+    // it cost to read X (24 queries, 1,000,003 fp16 rows of d = 770: 354 us a launch, 242 without).  What the
+    // tile holds there instead reaches only accumulator rows that nobody reads.
+    int a_rows;
     // k-blocks of 64 and valid K elements (multiple of 8) of a plane product.  The norm columns are zero in
     // every plane but the first, so only the last product, of the two first planes, takes them (d = 128,
     // three products: 25 MMAs a tile instead of 27, 7 k-blocks instead of 9).
@@ -460,7 +465,7 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
                                 tma_load_3d_pair(sbase + SM_B + stage * B_STAGE_BYTES + sub * C::B_SUB_BYTES,
                                                  &tmap_b, fb, kk, xrow + sub * BN + (int)cta_rank * C::B_ROWS, pb);
                         } else {
-                            mbar_arrive_expect_tx(bar_full + stage * 8, A_STAGE_BYTES + B_STAGE_BYTES);
+                            mbar_arrive_expect_tx(bar_full + stage * 8, p.a_rows * BK * 2 + B_STAGE_BYTES);
                             tma_load_3d(sbase + SM_A + stage * A_STAGE_BYTES, &tmap_a,
                                         bar_full + stage * 8, kk, qb * BM, pa);
                             tma_load_3d(sbase + SM_B + stage * B_STAGE_BYTES, &tmap_b,
@@ -877,8 +882,9 @@ int launch_common(const GemmOperands& op, const GemmPlan& plan, GemmParams& p, i
     if (op.nq <= 0 || ncols <= 0) return B200F_OK;
     if (col0 + ncols > op.nb || op.nb > 0x7fffffffLL) return B200F_ERR_BAD_ARG;
     CUtensorMap ma, mb;
+    p.a_rows = plan.pair || op.nq >= BM ? BM : (int)round_up64(op.nq, 8);
     int rc = make_operand_map(&ma, op.a_planes, op.is_bf16, op.d_pad, op.nq, op.a_pitch, op.npl,
-                              op.a_plane_stride, BM);
+                              op.a_plane_stride, p.a_rows);
     if (rc != B200F_OK) return rc;
     rc = make_operand_map(&mb, op.b_planes, op.is_bf16, op.d_pad, op.nb, op.b_pitch, op.npl,
                           op.b_plane_stride, plan.pair ? Cfg<true>::B_ROWS : Cfg<false>::B_ROWS);

@@ -17,6 +17,7 @@
 //                      through the key matrix only when a full list could have dropped one of
 //                      its k results (rows counted and compacted on the device, no host sync)
 //   k   > 32 otherwise distance keys written per column chunk, running sort-select
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <cmath>
@@ -120,6 +121,10 @@ constexpr int F32_STREAM_MAX_D = 768;
 constexpr int64_t FILTER_MIN_PAIRS = 1ll << 27;
 constexpr int64_t FILTER_MIN_PAIRS_MATRIX = 1ll << 18;
 constexpr int PILOT_MAX_RANK = 400;
+// Lists of one or two entries hardly insert: on small shards they beat the matrix and the filter (10,000
+// queries, 60,000 fp16 rows of d = 64: 314 / 414 us for k = 1 / 2, 541 / 562 with the filter; 580 against 565
+// for k = 4).
+constexpr int SHORT_LIST = 2;
 // Few pairs: the whole key matrix fits the L2 cache and one row of it a CTA's few passes, so store and
 // select it, two launches (100 queries, 10,000 rows, k = 10: 64 us a search, 158 with the fused lists, whose
 // first tiles insert nearly every key).  Beyond, the filter (50 queries, 300,007 rows, k = 2048: 174 us, 476
@@ -207,7 +212,7 @@ bool make_plan(int64_t nq, int64_t nb, int d, int k, int storage, int path, bool
     adv((size_t)(nq > 0 ? nq : 1) * 4);
     pl.gslots = 1;
     if (!pairwise && pl.path == B200F_PATH_TENSOR && rank_select_enabled() && select_mode() == B200F_SELECT_AUTO &&
-        nb <= DIRECT_MAX_ROWS && nq * nb <= DIRECT_MAX_PAIRS) {
+        k > SHORT_LIST && nb <= DIRECT_MAX_ROWS && nq * nb <= DIRECT_MAX_PAIRS) {
         pl.fused = false;   // all keys as one matrix, selected from by row_select
         pl.direct = true;
     }
@@ -237,14 +242,18 @@ bool make_plan(int64_t nq, int64_t nb, int d, int k, int storage, int path, bool
             // well be larger: a closer threshold, fewer candidates (1,000 queries, 100,000 rows: one
             // row in 16 instead of 64, 128 candidates instead of 320).  Forced, the filter keeps its sparse
             // sample, which misjudges more rows.
-            while (!filter_forced() && stride > 8 && ceil_div64(g0.ntiles, stride / 2) * g0.nqb <= g0.units && as_matrix(stride / 2) &&
+            while (!filter_forced() && stride > 8 && (k > SHORT_LIST || nb >= 65536) && ceil_div64(g0.ntiles, stride / 2) * g0.nqb <= g0.units && as_matrix(stride / 2) &&
                    rank_of(stride / 2) <= PILOT_MAX_RANK)
                 stride /= 2;
         }
+        // rows of a sample worth having
+        auto least = [&](int stride) { return std::max<int64_t>(1024, 8 * (int64_t)rank_of(stride)); };
+        while (!filter_forced() && k > SHORT_LIST && matrix && stride > 8 && nb < stride * least(stride) && as_matrix(stride / 2) &&
+               rank_of(stride / 2) <= PILOT_MAX_RANK)
+            stride /= 2;
         const int r = rank_of(stride);
-        const int64_t least = 8 * (int64_t)r > 1024 ? 8 * (int64_t)r : 1024;   // rows of a sample worth having
-        const int64_t min_pairs = matrix ? FILTER_MIN_PAIRS_MATRIX : FILTER_MIN_PAIRS;
-        if ((r <= B200F_FUSED_MAX_K || matrix) && nb >= stride * least && (nq * nb >= min_pairs || filter_forced())) {
+        const int64_t min_pairs = !matrix ? FILTER_MIN_PAIRS : k > SHORT_LIST ? FILTER_MIN_PAIRS_MATRIX : 16 * FILTER_MIN_PAIRS_MATRIX;
+        if ((r <= B200F_FUSED_MAX_K || matrix) && nb >= stride * least(stride) && (nq * nb >= min_pairs || filter_forced())) {
             const int bound = (int)round_up64((int64_t)(stride * (r + 6.0 * std::sqrt((double)r) + 12.0)), 256);
             int cap = 1024;
             while (cap < 4 * r * stride && cap < 8192) cap <<= 1;
