@@ -60,9 +60,26 @@ __device__ __forceinline__ float warp_sum(float v) {
 // FP32 storage, plane_format B200F_PLANES_FP16X2: two fp16 planes of the row scaled by its own
 // power of two, and rowscale[r] = 1 / (row scale * 2^x_scale_log2) (what turns the kernel's
 // accumulator back into key units).  Otherwise rowscale is not written.
+// zero_word (optional) is cleared.
 int launch_prepare_queries(const float* q, int64_t nq, int d, int storage, uint16_t* a_planes,
                            int64_t a_pitch, int64_t a_plane_stride, float* qnorm, int norm_cols,
-                           int plane_format, int x_scale_log2, float* rowscale, cudaStream_t stream);
+                           int plane_format, int x_scale_log2, float* rowscale, int32_t* zero_word,
+                           cudaStream_t stream);
+
+// A filter whose keys are only bounds of the true ones (L2): a row's key ||x||^2 - 2 q.x is at least
+// (1 - eps) ||x||^2 - 2 (q.x as computed) - eps ||q||^2 when eps (||x||^2 + ||q||^2) covers twice the error
+// of the product (2 |e| <= 2 u |q| |x| <= u (||q||^2 + ||x||^2)).  What passes a threshold that way contains
+// every row under it; the candidates are scored again in fp32 (launch_rescore) before they are selected.
+// `bad` counts the queries for which that would admit too many (rows far from the origin and near
+// to each other); beyond bad_limit of them the exact filter runs instead.
+struct BoundFilter {
+    float eps = 0.f;               // 0: keys are exact
+    const float* qnorm = nullptr;  // ||q||^2
+    float thr_abs = 0.f;           // added to every threshold
+    const int32_t* bad = nullptr;
+    int bad_limit = 0;
+    int run_if_bad = 0;            // leave at once unless (*bad > bad_limit) == run_if_bad
+};
 
 // scan.cu: streaming search for small nq, k <= 32.  Writes P = *out_P partial lists.
 struct ScanPlan {
@@ -86,7 +103,16 @@ int launch_scan_store(const B200FSearchArgs& a, int64_t col0, int64_t ncols, int
 // Scan that appends every row whose key is <= thr[q] to the query's candidate buffer
 // cand_key / cand_idx [nq][cap]; cand_cnt[q] (zeroed by the caller) counts every hit.
 int launch_scan_filter(const B200FSearchArgs& a, const float* thr, float* cand_key, int32_t* cand_idx,
-                       int32_t* cand_cnt, int cap, int sm_count, cudaStream_t stream);
+                       int32_t* cand_cnt, int cap, int sm_count, const BoundFilter& bf, cudaStream_t stream);
+// The same by the streaming kernels (up to 8 queries, L2, keys that are bounds); false: no such kernel for this shape.
+bool scan_bound_filter_fits(const B200FSearchArgs& a);
+// eps of those kernels for a storage type
+float scan_bound_eps(int storage);
+int launch_scan_bound_filter(const B200FSearchArgs& a, const float* thr, float* cand_key, int32_t* cand_idx,
+                             int32_t* cand_cnt, int cap, const BoundFilter& bf, cudaStream_t stream);
+// ckey[q][c] = ||x||^2 - 2 q.x in fp32 for every candidate of a query whose buffer did not overflow.
+int launch_rescore(const B200FSearchArgs& a, const int32_t* cand_idx, const int32_t* cand_cnt, int cap,
+                   float* cand_key, const BoundFilter& bf, cudaStream_t stream);
 
 // gemm_topk.cu
 struct GemmPlan {
@@ -170,23 +196,27 @@ int launch_select_parts(const float* part_key, const int32_t* part_idx, int nlis
 // Selection of the k best of a row's threshold-filtered candidates (unordered buffer of
 // min(cand_cnt[q], cap) entries).  dirty[q] = 1 when entries were lost to overflow or fewer than
 // k candidates were found although the shard has more rows.
+// thr (optional, [nq]): also when the k-th key found is beyond it.
 int launch_select_candidates(const float* cand_key, const int32_t* cand_idx, const int32_t* cand_cnt,
                              int cap, int64_t nb, int64_t nq, int k, int metric, const float* qnorm,
                              int64_t label_base, float* out_dist, int64_t* out_labels, int32_t* dirty,
-                             cudaStream_t stream);
+                             const float* thr, cudaStream_t stream);
 // select_rank.cu: the same selection / merge for inputs of at most 8192 entries per row, sorted in
 // registers and placed by binary search; results identical to the kernels of select.cu.
 bool rank_select_enabled();
 int launch_rank_select(const float* cand_key, const int32_t* cand_idx, const int32_t* cand_cnt, int cap,
                        int64_t nb, int64_t nq, int k, int metric, const float* qnorm, int64_t label_base,
-                       float* out_dist, int64_t* out_labels, int32_t* dirty, cudaStream_t stream);
+                       float* out_dist, int64_t* out_labels, int32_t* dirty, const float* thr,
+                       cudaStream_t stream);
 // The k best of every row of a key matrix (n columns, column c is row c of the shard), finalised.
 int launch_matrix_select(const float* keys, int64_t nq, int64_t n, int64_t ld, int k, int metric, const float* qnorm,
                          int64_t label_base, float* out_dist, int64_t* out_labels, const int* nq_dev,
                          const int32_t* row_map, cudaStream_t stream);
 // out[q]: an upper bound, close to it, of the r-th smallest (r <= 512) of the n keys of row q; +INF when
-// there are too few.  NaN keys are skipped.
-int launch_row_bound(const float* keys, int64_t nq, int64_t n, int64_t ld, int r, float* out, cudaStream_t stream);
+// there are too few.  NaN keys are skipped.  bad (optional): one more for every row with more than about
+// `most` keys up to its bound + margin * qnorm[q], or with qnorm[q] >= qnorm_max.
+int launch_row_bound(const float* keys, int64_t nq, int64_t n, int64_t ld, int r, float* out, int32_t* bad,
+                     const float* qnorm, float margin, float qnorm_max, double most, cudaStream_t stream);
 // *count = nq when any of dirty[0 .. nq) is set, else 0 (also to *count_copy): the streaming scans redo
 // all of their few queries or none.
 int launch_any_dirty(const int32_t* dirty, int64_t nq, int32_t* count, int32_t* count_copy, cudaStream_t stream);

@@ -382,7 +382,8 @@ __global__ void prepare_queries_kernel(const float* __restrict__ q, int64_t nq, 
                                        uint16_t* __restrict__ a, int64_t a_pitch,
                                        int64_t a_plane_stride, float* __restrict__ qnorm,
                                        int norm_cols, int plane_format, int x_scale_log2,
-                                       float* __restrict__ rowscale) {
+                                       float* __restrict__ rowscale, int32_t* __restrict__ zero_word) {
+    if (zero_word && blockIdx.x == 0 && threadIdx.x == 0) *zero_word = 0;
     const int lane = threadIdx.x & 31;
     const int d8 = (d + 7) & ~7;
     const int fmt = storage == B200F_STORAGE_F16 ? B200F_STORAGE_F16 : B200F_STORAGE_BF16;
@@ -548,11 +549,12 @@ int cached_sm_count() {
 
 int launch_prepare_queries(const float* q, int64_t nq, int d, int storage, uint16_t* a_planes,
                            int64_t a_pitch, int64_t a_plane_stride, float* qnorm, int norm_cols,
-                           int plane_format, int x_scale_log2, float* rowscale, cudaStream_t stream) {
+                           int plane_format, int x_scale_log2, float* rowscale, int32_t* zero_word,
+                           cudaStream_t stream) {
     if (nq <= 0) return B200F_OK;
     prepare_queries_kernel<<<grid_for_rows(nq), ROW_THREADS, 0, stream>>>(
             q, nq, d, storage, a_planes, a_pitch, a_plane_stride, qnorm, norm_cols, plane_format, x_scale_log2,
-            rowscale);
+            rowscale, zero_word);
     count_launch();
     B200F_LAUNCH_CHECK();
     return B200F_OK;

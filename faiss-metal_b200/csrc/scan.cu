@@ -56,6 +56,7 @@ struct ScanParams {
     int32_t* cand_idx;
     int32_t* cand_cnt;      // [nq]
     int cand_cap;
+    BoundFilter bf;         // filter mode of the streaming kernels: keys that are bounds
     // bulk-copy pipeline (scan_bulk_kernel)
     int rb;                 // rows per consumer warp per stage
     int stage_rows;         // rows per stage = SB_NW * rb
@@ -63,6 +64,14 @@ struct ScanParams {
     int nstage;
     int32_t* status;
 };
+
+__device__ __forceinline__ bool filter_leaves(const BoundFilter& bf) {
+    return bf.bad && (*bf.bad > bf.bad_limit) != (bf.run_if_bad != 0);
+}
+// threshold of query qi for keys that are bounds
+__device__ __forceinline__ float filter_thr(const ScanParams& p, int qi) {
+    return fmaf(p.bf.eps, __ldg(p.bf.qnorm + qi), p.thr[qi] + p.bf.thr_abs);
+}
 
 template <int STORAGE>
 struct Piece {
@@ -145,6 +154,15 @@ __device__ __forceinline__ void take_bound(float& thr, int& thr_id, float lk, in
     }
 }
 
+// one row of a filter's result
+__device__ __forceinline__ void filter_append(const ScanParams& p, int qi, float key, int row) {
+    const int pos = atomicAdd(p.cand_cnt + qi, 1);
+    if (pos < p.cand_cap) {
+        p.cand_key[(int64_t)qi * p.cand_cap + pos] = key;
+        p.cand_idx[(int64_t)qi * p.cand_cap + pos] = row;
+    }
+}
+
 enum { SCAN_TOPK = 0, SCAN_STORE = 1, SCAN_FILTER = 2 };
 
 template <int STORAGE, int NQ, int MODE>
@@ -156,6 +174,7 @@ __global__ void __launch_bounds__(SCAN_THREADS, (NQ == 4 || (NQ == 2 && STORAGE 
 scan_kernel(const ScanParams p) {
     constexpr bool STORE = MODE == SCAN_STORE;
     if (p.guard && *p.guard == 0) return;
+    if (MODE == SCAN_FILTER && filter_leaves(p.bf)) return;
     constexpr int E = Piece<STORAGE>::E;
     // rows per lane and block; fp32 rows keep two partial sums per (row, query), so fewer rows fit the registers
     constexpr int U = (STORAGE == B200F_STORAGE_F32 && MODE == SCAN_TOPK && NQ == 4) ? 6 : SCAN_U;
@@ -302,13 +321,7 @@ scan_kernel(const ScanParams p) {
 #pragma unroll
                 for (int qi = 0; qi < NQ; qi++) {
                     const float key = l2 ? fmaf(-2.f, acc[u][qi], nrm) : -acc[u][qi];
-                    if (key <= thr[qi] && qi < p.nq) {
-                        const int pos = atomicAdd(p.cand_cnt + qi, 1);
-                        if (pos < p.cand_cap) {
-                            p.cand_key[(int64_t)qi * p.cand_cap + pos] = key;
-                            p.cand_idx[(int64_t)qi * p.cand_cap + pos] = (int32_t)row;
-                        }
-                    }
+                    if (key <= thr[qi] && qi < p.nq) filter_append(p, qi, key, (int)row);
                 }
             }
             continue;
@@ -439,10 +452,15 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
 
 // NW consumer warps: 8 for one or two queries (6.80 / 6.62 TB/s on 25 M fp16 rows; 12 warps: 6.55 at
 // one), 12 beyond (four queries 6.24 -> 6.53 TB/s, eight 5.44 -> 6.08).
-template <bool BF16, int NW>
+// FILTER: no lists; every row whose bound (see BoundFilter; the queries are rounded to the rows' format) is
+// under the query's threshold goes to its candidate buffer.  ||x||^2 then comes from the norm array, copied
+// into the ring behind the rows: norm columns have fp16's range.  Four queries, k = 200, on 1 M bf16 rows of
+// d = 384: 313 -> 238 us a search (216 us of it the FMA kernel before).
+template <bool BF16, int NW, bool FILTER>
 __global__ void __launch_bounds__(32 * (1 + NW), 1) scan_mma_kernel(const ScanParams p) {
     extern __shared__ __align__(128) uint8_t sm[];
     if (p.guard && *p.guard == 0) return;
+    if (FILTER && filter_leaves(p.bf)) return;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const uint32_t sbase = smem_u32(sm);
@@ -483,6 +501,7 @@ __global__ void __launch_bounds__(32 * (1 + NW), 1) scan_mma_kernel(const ScanPa
     const int64_t nchunks = ceil_div64(nrows_total, p.stage_rows);
     const uint8_t* base = reinterpret_cast<const uint8_t*>(p.rows);
     const float kmul = p.metric == B200F_METRIC_L2 ? -2.f : -1.f;
+    const uint32_t norm_off = (uint32_t)p.stage_rows * (uint32_t)p.pitch_bytes;   // FILTER: norms of a stage, behind its rows
 
     float lk[SM_NQ];
     int li[SM_NQ];
@@ -492,7 +511,7 @@ __global__ void __launch_bounds__(32 * (1 + NW), 1) scan_mma_kernel(const ScanPa
     for (int qi = 0; qi < SM_NQ; qi++) {
         lk[qi] = CUDART_INF_F;
         li[qi] = -1;
-        thr[qi] = (p.thr && qi < p.nq) ? p.thr[qi] : CUDART_INF_F;
+        thr[qi] = (p.thr && qi < p.nq) ? (FILTER ? filter_thr(p, qi) : p.thr[qi]) : CUDART_INF_F;
         thr_id[qi] = -1;
     }
 
@@ -510,9 +529,17 @@ __global__ void __launch_bounds__(32 * (1 + NW), 1) scan_mma_kernel(const ScanPa
                 const int64_t row0 = p.col0 + c * p.stage_rows;
                 const int64_t nr = min((int64_t)p.stage_rows, p.col1 - row0);
                 const uint32_t bytes = (uint32_t)(nr * p.pitch_bytes);
-                mbar_arrive_expect_tx(bar_full + stage * 8, bytes);
+                const uint32_t nbytes = FILTER ? (uint32_t)(nr * 4) & ~15u : 0u;
+                if (FILTER) {   // the up to three norms left of a ragged last stage by plain stores
+                    float* sn = reinterpret_cast<float*>(sm + stage * p.stage_stride + norm_off);
+                    for (int64_t r = nbytes / 4; r < nr; r++) sn[r] = __ldg(p.norms + row0 + r);
+                }
+                mbar_arrive_expect_tx(bar_full + stage * 8, bytes + nbytes);
                 bulk_load(sbase + stage * p.stage_stride, base + row0 * p.pitch_bytes, bytes,
                           bar_full + stage * 8);
+                if (nbytes)
+                    bulk_load(sbase + stage * p.stage_stride + norm_off, p.norms + row0, nbytes,
+                              bar_full + stage * 8);
                 if (++stage == p.nstage) {
                     stage = 0;
                     phase ^= 1;
@@ -585,9 +612,25 @@ __global__ void __launch_bounds__(32 * (1 + NW), 1) scan_mma_kernel(const ScanPa
                 float key[4];
 #pragma unroll
                 for (int j = 0; j < 4; j++) key[j] = kmul * acc[j];
+                if constexpr (FILTER) {
+                    const float* sn = reinterpret_cast<const float*>(sm + stage * p.stage_stride + norm_off);
+                    const float keep = 1.f - p.bf.eps;
+                    const float n0 = v0 ? sn[r0] : 0.f, n1 = v1 ? sn[r1] : 0.f;
+                    key[0] = fmaf(keep, n0, key[0]);
+                    key[1] = fmaf(keep, n0, key[1]);
+                    key[2] = fmaf(keep, n1, key[2]);
+                    key[3] = fmaf(keep, n1, key[3]);
+                }
                 const bool h0 = v0 && before(key[0], row_a, mta, mia), h1 = v0 && before(key[1], row_a, mtb, mib);
                 const bool h2 = v1 && before(key[2], row_b, mta, mia), h3 = v1 && before(key[3], row_b, mtb, mib);
                 if (!__any_sync(FULL, h0 || h1 || h2 || h3)) continue;  // the usual case: nothing for any query
+                if constexpr (FILTER) {
+                    if (h0) filter_append(p, 2 * t, key[0], row_a);
+                    if (h1) filter_append(p, 2 * t + 1, key[1], row_a);
+                    if (h2) filter_append(p, 2 * t, key[2], row_b);
+                    if (h3) filter_append(p, 2 * t + 1, key[3], row_b);
+                    continue;
+                }
                 unsigned mj[4];
                 mj[0] = __ballot_sync(FULL, h0);
                 mj[1] = __ballot_sync(FULL, h1);
@@ -626,6 +669,7 @@ __global__ void __launch_bounds__(32 * (1 + NW), 1) scan_mma_kernel(const ScanPa
         }
     }
 
+    if constexpr (FILTER) return;   // every copy has landed: the consumers waited for all of them
     // CTA merge in the (now idle) ring memory: consumer warp wc publishes its lists,
     // warp 1 + qi folds them for query qi.
     __syncthreads();
@@ -695,9 +739,11 @@ constexpr int ST_QPAD = 16;   // floats between query rows beyond kq: rows 64 by
 constexpr int ST_NW = 15;     // consumer warps: the split and the three MMA chains of a tile are latency, not issue, bound
 constexpr int ST_THREADS = 32 * (1 + ST_NW);
 
+template <bool FILTER>
 __global__ void __launch_bounds__(ST_THREADS, 1) scan_tf32_kernel(const ScanParams p) {
     extern __shared__ __align__(128) uint8_t sm[];
     if (p.guard && *p.guard == 0) return;
+    if (FILTER && filter_leaves(p.bf)) return;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const uint32_t sbase = smem_u32(sm);
@@ -747,7 +793,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tf32_kernel(const ScanPara
     for (int qi = 0; qi < SM_NQ; qi++) {
         lk[qi] = CUDART_INF_F;
         li[qi] = -1;
-        thr[qi] = (p.thr && qi < p.nq) ? p.thr[qi] : CUDART_INF_F;
+        thr[qi] = (p.thr && qi < p.nq) ? (FILTER ? filter_thr(p, qi) : p.thr[qi]) : CUDART_INF_F;
         thr_id[qi] = -1;
     }
 
@@ -830,6 +876,10 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tf32_kernel(const ScanPara
                 if (l2) {
                     if (v0) n0 = snorm[r0];
                     if (v1) n1 = snorm[r1];
+                    if (FILTER) {
+                        n0 *= 1.f - p.bf.eps;
+                        n1 *= 1.f - p.bf.eps;
+                    }
                 }
                 const uint32_t a_row0 = sstage + (uint32_t)r0 * (uint32_t)p.pitch_bytes + t * 16;
                 const uint32_t a_row1 = sstage + (uint32_t)r1 * (uint32_t)p.pitch_bytes + t * 16;
@@ -883,6 +933,13 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tf32_kernel(const ScanPara
                 const bool h0 = v0 && before(key[0], row_a, mta, mia), h1 = v0 && before(key[1], row_a, mtb, mib);
                 const bool h2 = v1 && before(key[2], row_b, mta, mia), h3 = v1 && before(key[3], row_b, mtb, mib);
                 if (!__any_sync(FULL, h0 || h1 || h2 || h3)) continue;  // the usual case: nothing for any query
+                if constexpr (FILTER) {
+                    if (h0) filter_append(p, 2 * t, key[0], row_a);
+                    if (h1) filter_append(p, 2 * t + 1, key[1], row_a);
+                    if (h2) filter_append(p, 2 * t, key[2], row_b);
+                    if (h3) filter_append(p, 2 * t + 1, key[3], row_b);
+                    continue;
+                }
                 unsigned mj[4];
                 mj[0] = __ballot_sync(FULL, h0);
                 mj[1] = __ballot_sync(FULL, h1);
@@ -921,6 +978,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tf32_kernel(const ScanPara
         }
     }
 
+    if constexpr (FILTER) return;
     // CTA merge in the (now idle) ring memory, as in scan_mma_kernel
     __syncthreads();
     float* mk = reinterpret_cast<float*>(sm);                        // [ST_NW][SM_NQ][32]
@@ -953,6 +1011,61 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tf32_kernel(const ScanPara
             const int64_t o = ((int64_t)qi * gridDim.x + blockIdx.x) * p.k + lane;
             p.part_key[o] = k0;
             p.part_idx[o] = i0;
+        }
+    }
+}
+
+// Candidates of a filter whose keys are bounds, scored again in fp32 (L2): eight lanes share a candidate's row
+// and two rows are in flight per lane group; a few us, bound by latency.  blockIdx.x is the query, blockIdx.y its share of the candidates.
+constexpr int RC_THREADS = 256;
+template <int STORAGE>
+__global__ void __launch_bounds__(RC_THREADS) rescore_kernel(const ScanParams p) {
+    constexpr int E = Piece<STORAGE>::E;
+    constexpr int LPR = 8, U = 2, PER_CTA = RC_THREADS / LPR;
+    if (filter_leaves(p.bf)) return;
+    const int q = blockIdx.x;
+    const int n = p.cand_cnt[q];
+    if (n > p.cand_cap || (int)blockIdx.y * PER_CTA * U >= n) return;   // overflow: the query is redone
+    extern __shared__ __align__(16) float sq[];   // the query, zero padded to whole pieces
+    for (int j = threadIdx.x; j < p.qstride; j += RC_THREADS) sq[j] = j < p.d ? p.queries[(int64_t)q * p.d + j] : 0.f;
+    __syncthreads();
+    const int cl = threadIdx.x & (LPR - 1), grp = threadIdx.x / LPR;
+    const int32_t* idx = p.cand_idx + (int64_t)q * p.cand_cap;
+    float* out = p.cand_key + (int64_t)q * p.cand_cap;
+    const uint8_t* base = reinterpret_cast<const uint8_t*>(p.rows);
+    for (int c0 = blockIdx.y * PER_CTA * U; c0 < n; c0 += gridDim.y * PER_CTA * U) {
+        int row[U];
+        float acc[U], nrm[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int c = c0 + u * PER_CTA + grp;
+            row[u] = c < n ? __ldg(idx + c) : -1;
+            nrm[u] = row[u] >= 0 ? __ldg(p.norms + row[u]) : 0.f;
+            acc[u] = 0.f;
+        }
+#pragma unroll 3
+        for (int piece = cl; piece < p.C; piece += LPR) {
+            uint4 v[U];
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                v[u] = row[u] >= 0 ? __ldg(reinterpret_cast<const uint4*>(base + (int64_t)row[u] * p.pitch_bytes) + piece)
+                                   : make_uint4(0, 0, 0, 0);
+            float qf[E];
+#pragma unroll
+            for (int e = 0; e < E; e++) qf[e] = sq[piece * E + e];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                float x[E];
+                unpack<STORAGE>(v[u], x);
+#pragma unroll
+                for (int e = 0; e < E; e++) acc[u] = fmaf(qf[e], x[e], acc[u]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+#pragma unroll
+            for (int o = LPR / 2; o > 0; o >>= 1) acc[u] += __shfl_xor_sync(FULL, acc[u], o);
+            if (cl == 0 && row[u] >= 0) out[c0 + u * PER_CTA + grp] = fmaf(-2.f, acc[u], nrm[u]);
         }
     }
 }
@@ -1042,7 +1155,7 @@ int launch_storage(const ScanParams& p, int storage, int grid, cudaStream_t stre
 
 
 // Stage geometry of the streaming pipeline; returns false when it does not apply.
-bool plan_stream(ScanParams& p, int storage, int d, int norm_cols) {
+bool plan_stream(ScanParams& p, int storage, int d, int norm_cols, bool norms_behind = false) {
     if (storage == B200F_STORAGE_F32 || (p.pitch_bytes % 16) != 0) return false;
     const int d8 = (d + 7) & ~7;
     const int kext = d8 + (norm_cols ? 8 : 0);
@@ -1054,7 +1167,7 @@ bool plan_stream(ScanParams& p, int storage, int d, int norm_cols) {
     if (rows > 256) rows = 256;
     p.stage_rows = (int)rows;
     p.rb = 16;
-    p.stage_stride = (int)round_up64((int64_t)p.stage_rows * p.pitch_bytes + 64, 128);
+    p.stage_stride = (int)round_up64((int64_t)p.stage_rows * (p.pitch_bytes + (norms_behind ? 4 : 0)) + 64, 128);
     const int64_t fixed = (int64_t)SM_NQ * p.iters * 32 * 2 + 2 * SM_MAX_STAGES * 8 + 16;
     int64_t ns = (220 * 1024 - fixed) / p.stage_stride;
     if (ns > SM_MAX_STAGES) ns = SM_MAX_STAGES;
@@ -1133,10 +1246,10 @@ int launch_scan_topk(const B200FSearchArgs& a, const ScanPlan& plan, float* part
             // macro: the kernel is a template over (format, consumer warps)
 #define B200F_SCAN_MMA(BF, NW)                                                                            \
     {                                                                                                     \
-        B200F_CUDA_TRY(cudaFuncSetAttribute(scan_mma_kernel<BF, NW>,                                      \
+        B200F_CUDA_TRY(cudaFuncSetAttribute(scan_mma_kernel<BF, NW, false>,                               \
                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));     \
         main_kernel_begin(stream);                                                                        \
-        scan_mma_kernel<BF, NW><<<grid, 32 * (1 + NW), smem, stream>>>(ps);                               \
+        scan_mma_kernel<BF, NW, false><<<grid, 32 * (1 + NW), smem, stream>>>(ps);                               \
     }
             const bool bf = a.storage == B200F_STORAGE_BF16;
             if (a.nq <= 2) {
@@ -1161,10 +1274,10 @@ int launch_scan_topk(const B200FSearchArgs& a, const ScanPlan& plan, float* part
             const size_t smem = (size_t)ps.nstage * ps.stage_stride +
                                 (size_t)2 * SM_NQ * (ps.iters * 16 + ST_QPAD) * 4 + 2 * SM_MAX_STAGES * 8 + 16;
             *out_P = grid;
-            B200F_CUDA_TRY(cudaFuncSetAttribute(scan_tf32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            B200F_CUDA_TRY(cudaFuncSetAttribute(scan_tf32_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                 (int)smem));
             main_kernel_begin(stream);
-            scan_tf32_kernel<<<grid, ST_THREADS, smem, stream>>>(ps);
+            scan_tf32_kernel<false><<<grid, ST_THREADS, smem, stream>>>(ps);
             main_kernel_end(stream);
             count_launch();
             B200F_LAUNCH_CHECK();
@@ -1204,7 +1317,7 @@ int launch_scan_store(const B200FSearchArgs& a, int64_t col0, int64_t ncols, int
 }
 
 int launch_scan_filter(const B200FSearchArgs& a, const float* thr, float* cand_key, int32_t* cand_idx,
-                       int32_t* cand_cnt, int cap, int sm_count, cudaStream_t stream) {
+                       int32_t* cand_cnt, int cap, int sm_count, const BoundFilter& bf, cudaStream_t stream) {
     if (a.nq < 1 || a.nq > 4 || !thr || !cand_key || !cand_idx || !cand_cnt || cap < 1) return B200F_ERR_BAD_ARG;
     ScanParams p{};
     fill_geometry(p, a.storage, a.d, a.row_pitch, a.metric == B200F_METRIC_L2 ? a.norm_cols : 0,
@@ -1224,10 +1337,106 @@ int launch_scan_filter(const B200FSearchArgs& a, const float* thr, float* cand_k
     p.cand_idx = cand_idx;
     p.cand_cnt = cand_cnt;
     p.cand_cap = cap;
+    p.bf = bf;
     return launch_storage<SCAN_FILTER>(p, a.storage,
                                        scan_grid(a.nb, a.d, a.storage, sm_count, lanes_per_row_cap(a.nq),
                                                  resident_ctas(a.nq, a.storage, true)),
                                        stream);
+}
+
+namespace {
+bool plan_bound_filter(const B200FSearchArgs& a, ScanParams& p) {
+    if (a.metric != B200F_METRIC_L2 || !a.norms || (reinterpret_cast<uintptr_t>(a.norms) & 15) != 0 || a.nq < 1 || a.nq > 8)
+        return false;
+    fill_geometry(p, a.storage, a.d, a.row_pitch, 0, 8);
+    p.rows = a.rows;
+    p.norms = a.norms;
+    if (a.storage == B200F_STORAGE_F32) return plan_stream_f32(p, a.d);
+    return plan_stream(p, a.storage, a.d, 0, true) && a.nb >= (int64_t)p.stage_rows * cached_sm_count();
+}
+}  // namespace
+
+bool scan_bound_filter_fits(const B200FSearchArgs& a) {
+    ScanParams p{};
+    return plan_bound_filter(a, p);
+}
+
+// Twice the rounding of the queries (bf16 2^-9, fp16 2^-11 relative; the tf32 split and its sums stay below
+// 2^-14): the other half covers the sums, and fp16's subnormals together with thr_abs.
+float scan_bound_eps(int storage) {
+    return storage == B200F_STORAGE_BF16 ? 0.00390625f : storage == B200F_STORAGE_F16 ? 0.0009765625f : 0.000244140625f;
+}
+
+int launch_scan_bound_filter(const B200FSearchArgs& a, const float* thr, float* cand_key, int32_t* cand_idx,
+                             int32_t* cand_cnt, int cap, const BoundFilter& bf, cudaStream_t stream) {
+    if (!thr || !cand_key || !cand_idx || !cand_cnt || cap < 1 || !bf.qnorm) return B200F_ERR_BAD_ARG;
+    ScanParams p{};
+    if (!plan_bound_filter(a, p)) return B200F_ERR_UNSUPPORTED;
+    p.queries = a.queries;
+    p.nb = a.nb;
+    p.col0 = 0;
+    p.col1 = a.nb;
+    p.d = a.d;
+    p.nq = (int)a.nq;
+    p.k = 1;
+    p.metric = a.metric;
+    p.thr = thr;
+    p.cand_key = cand_key;
+    p.cand_idx = cand_idx;
+    p.cand_cnt = cand_cnt;
+    p.cand_cap = cap;
+    p.bf = bf;
+    p.status = a.status;
+    const int64_t nchunks = ceil_div64(a.nb, p.stage_rows);
+    const int sm = cached_sm_count();
+    const int grid = (int)(nchunks < sm ? nchunks : sm);
+    const bool f32 = a.storage == B200F_STORAGE_F32;
+    const size_t query_bytes = f32 ? (size_t)2 * SM_NQ * (p.iters * 16 + ST_QPAD) * 4 : (size_t)SM_NQ * p.iters * 32 * 2;
+    const size_t smem = (size_t)p.nstage * p.stage_stride + query_bytes + 2 * SM_MAX_STAGES * 8 + 16;
+    typedef void (*KernelFn)(const ScanParams);
+    const KernelFn kernel = f32 ? scan_tf32_kernel<true>
+                                : a.storage == B200F_STORAGE_BF16 ? scan_mma_kernel<true, SM_NW_MANY, true>
+                                                                  : scan_mma_kernel<false, SM_NW_MANY, true>;
+    B200F_CUDA_TRY(cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)smem));
+    main_kernel_begin(stream);
+    kernel<<<grid, f32 ? ST_THREADS : 32 * (1 + SM_NW_MANY), smem, stream>>>(p);
+    main_kernel_end(stream);
+    count_launch();
+    B200F_LAUNCH_CHECK();
+    return B200F_OK;
+}
+
+int launch_rescore(const B200FSearchArgs& a, const int32_t* cand_idx, const int32_t* cand_cnt, int cap,
+                   float* cand_key, const BoundFilter& bf, cudaStream_t stream) {
+    if (a.metric != B200F_METRIC_L2 || !a.norms || !cand_idx || !cand_cnt || !cand_key) return B200F_ERR_BAD_ARG;
+    if (a.nq <= 0) return B200F_OK;
+    ScanParams p{};
+    fill_geometry(p, a.storage, a.d, a.row_pitch, 0, 8);
+    p.queries = a.queries;
+    p.rows = a.rows;
+    p.norms = a.norms;
+    p.d = a.d;
+    p.cand_key = cand_key;
+    p.cand_idx = const_cast<int32_t*>(cand_idx);
+    p.cand_cnt = const_cast<int32_t*>(cand_cnt);
+    p.cand_cap = cap;
+    p.bf = bf;
+    const size_t smem = (size_t)p.qstride * 4;
+    if (smem > 48 * 1024) return B200F_ERR_UNSUPPORTED;
+    // eight CTAs per SM; a CTA takes 64 candidates at a time
+    int64_t split = ceil_div64((int64_t)cached_sm_count() * 8, a.nq);
+    const int64_t most = ceil_div64(cap, 2 * RC_THREADS / 8);
+    if (split > most) split = most;
+    const dim3 grid((unsigned)a.nq, (unsigned)split);
+    switch (a.storage) {
+        case B200F_STORAGE_F32: rescore_kernel<B200F_STORAGE_F32><<<grid, RC_THREADS, smem, stream>>>(p); break;
+        case B200F_STORAGE_F16: rescore_kernel<B200F_STORAGE_F16><<<grid, RC_THREADS, smem, stream>>>(p); break;
+        default: rescore_kernel<B200F_STORAGE_BF16><<<grid, RC_THREADS, smem, stream>>>(p); break;
+    }
+    count_launch();
+    B200F_LAUNCH_CHECK();
+    return B200F_OK;
 }
 
 }  // namespace b200f

@@ -177,6 +177,11 @@ constexpr int64_t SCAN_LIST_THR_MIN_ROWS = 1 << 19;
 constexpr int64_t SCAN_LIST_THR_MIN_WORK = 24;      // queries x k
 constexpr int64_t SCAN_FILTER_MIN_ROWS = 1 << 15;
 
+// A filter with keys that are bounds has two more launches (about 8 us) and pays on large shards: four queries,
+// k = 200, 1 M bf16 rows of d = 384: 313 -> 238 us.
+constexpr int64_t BOUND_MIN_ELEMS = 32ll << 20;    // stored elements
+constexpr int BOUND_MAX_D = 8192;                  // a query in a rescoring CTA's shared memory
+
 bool make_plan(int64_t nq, int64_t nb, int d, int k, int storage, int path, bool pairwise,
                SearchPlan& pl) {
     // the query operand always reserves the 8 norm columns (used for L2 only)
@@ -714,6 +719,21 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
     const float kscale = l2 ? 2.f : 1.f;
     const int qnc = l2 ? 1 : 0;
 
+    // scans with k > 32: filter with keys that are bounds (see BoundFilter) where it pays
+    BoundFilter bf;
+    if (pl.sample && !pl.fused && l2 && rank_select_enabled() && a->nq >= 2 && a->d <= BOUND_MAX_D &&
+        a->nb * a->row_pitch >= BOUND_MIN_ELEMS && scan_bound_filter_fits(*a)) {
+        bf.eps = scan_bound_eps(a->storage);
+        bf.qnorm = qnorm;
+        if (a->storage == B200F_STORAGE_F16) bf.thr_abs = std::ldexp((float)a->d, -38);
+        bf.bad = reinterpret_cast<const int32_t*>(scratch + pl.off_count) + 16;
+    }
+    int32_t* const bad = const_cast<int32_t*>(bf.bad);
+    // what a query's sample may hold under its widened threshold: 0.7 of what its buffer takes; the
+    // margin there is that of a row as long as the query.  fp16 queries: elements below 2^15.
+    const double most = pl.sample ? 0.7 * pl.fcap / pl.fstride : 0.0;
+    const float margin = 2.5f * bf.eps, qnorm_max = a->storage == B200F_STORAGE_F16 ? 1073741824.f : kHostInf;
+
     GemmOperands op{};
     if (pl.path == B200F_PATH_TENSOR) {
         rc = fill_operands(*a, pl, scratch, op);
@@ -721,9 +741,9 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
         rc = launch_prepare_queries(a->queries, a->nq, a->d, a->storage,
                                     reinterpret_cast<uint16_t*>(scratch + pl.off_a), pl.a_pitch,
                                     pl.a_plane_stride, qnorm, qnc, a->plane_format, a->plane_scale_log2,
-                                    reinterpret_cast<float*>(scratch + pl.off_qscale), st);
+                                    reinterpret_cast<float*>(scratch + pl.off_qscale), nullptr, st);
     } else {
-        rc = launch_prepare_queries(a->queries, a->nq, a->d, a->storage, nullptr, 0, 0, qnorm, 0, 0, 0, nullptr, st);
+        rc = launch_prepare_queries(a->queries, a->nq, a->d, a->storage, nullptr, 0, 0, qnorm, 0, 0, 0, nullptr, bad, st);
     }
     if (rc != B200F_OK) return rc;
 
@@ -768,7 +788,7 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
             rc = launch_gemm_store(op, pl.pilot, 0, a->nb, pl.fstride, kscale, 1.f, nullptr, matrix, pcols,
                                    a->status, st);
             if (rc != B200F_OK) return rc;
-            rc = launch_row_bound(matrix, a->nq, valid, pcols, pl.frank, thr, st);
+            rc = launch_row_bound(matrix, a->nq, valid, pcols, pl.frank, thr, nullptr, nullptr, 0.f, 0.f, 0.0, st);
             if (rc != B200F_OK) return rc;
         } else {
             rc = launch_gemm_topk(op, pl.pilot, 0, a->nb, pl.fstride, kscale, pl.frank, 1, pkey, pidx, gthr,
@@ -778,12 +798,12 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
             if (rc != B200F_OK) return rc;
         }
         // about frank * fstride candidates per row; wide TMEM loads where fewer than one row in 1024 is one
+        const int wide = (int64_t)pl.frank * pl.fstride * 1024 < a->nb ? 1 : 0;
         rc = launch_gemm_filter(op, pl.gemm, kscale, thr, pl.pilot_matrix ? 1 : pl.frank,
-                                pl.pilot_matrix ? 0 : pl.frank - 1, ckey, cidx, ccnt, pl.fcap,
-                                (int64_t)pl.frank * pl.fstride * 1024 < a->nb ? 1 : 0, a->status, st);
+                                pl.pilot_matrix ? 0 : pl.frank - 1, ckey, cidx, ccnt, pl.fcap, wide, a->status, st);
         if (rc != B200F_OK) return rc;
         rc = launch_select_candidates(ckey, cidx, ccnt, pl.fcap, a->nb, a->nq, a->k, a->metric, qnorm,
-                                      a->label_base, a->out_dist, a->out_labels, dirty, st);
+                                      a->label_base, a->out_dist, a->out_labels, dirty, nullptr, st);
         if (rc != B200F_OK) return rc;
         rc = redo_setup(dirty);
         if (rc != B200F_OK) return rc;
@@ -806,7 +826,7 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
                                    pl.nsample, sm, nullptr, st);
             if (rc != B200F_OK) return rc;
         }
-        rc = launch_row_bound(keys, a->nq, pl.nsample, pl.nsample, pl.frank, thr, st);
+        rc = launch_row_bound(keys, a->nq, pl.nsample, pl.nsample, pl.frank, thr, bad, qnorm, margin, qnorm_max, most, st);
         if (rc != B200F_OK) return rc;
     }
 
@@ -882,13 +902,23 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
         int32_t* cidx = reinterpret_cast<int32_t*>(scratch + pl.off_cand_idx);
         int32_t* ccnt = reinterpret_cast<int32_t*>(scratch + pl.off_cand_cnt);
         B200F_CUDA_TRY(cudaMemsetAsync(ccnt, 0, (size_t)a->nq * sizeof(int32_t), st));
+        BoundFilter exact;
+        if (bad) {
+            rc = launch_scan_bound_filter(*a, thr, ckey, cidx, ccnt, pl.fcap, bf, st);
+            if (rc != B200F_OK) return rc;
+            rc = launch_rescore(*a, cidx, ccnt, pl.fcap, ckey, bf, st);
+            if (rc != B200F_OK) return rc;
+            exact.bad = bf.bad;
+            exact.bad_limit = bf.bad_limit;
+            exact.run_if_bad = 1;
+        }
         for (int64_t q0 = 0; q0 < a->nq; q0 += SCAN_GROUP) {
             rc = launch_scan_filter(query_group(q0, SCAN_GROUP), thr + q0, ckey + q0 * pl.fcap, cidx + q0 * pl.fcap,
-                                    ccnt + q0, pl.fcap, sm, st);
+                                    ccnt + q0, pl.fcap, sm, exact, st);
             if (rc != B200F_OK) return rc;
         }
         rc = launch_select_candidates(ckey, cidx, ccnt, pl.fcap, a->nb, a->nq, a->k, a->metric, qnorm,
-                                      a->label_base, a->out_dist, a->out_labels, dirty, st);
+                                      a->label_base, a->out_dist, a->out_labels, dirty, bad ? thr : nullptr, st);
         if (rc != B200F_OK) return rc;
         rc = launch_any_dirty(dirty, a->nq, any_count, a->status ? a->status + 1 : nullptr, st);
         if (rc != B200F_OK) return rc;
@@ -970,12 +1000,12 @@ extern "C" int b200f_pairwise(const B200FSearchArgs* a, float* out_matrix, int64
         rc = launch_prepare_queries(a->queries, a->nq, a->d, a->storage,
                                     reinterpret_cast<uint16_t*>(scratch + pl.off_a), pl.a_pitch,
                                     pl.a_plane_stride, qnorm, l2 ? 1 : 0, a->plane_format, a->plane_scale_log2,
-                                    reinterpret_cast<float*>(scratch + pl.off_qscale), st);
+                                    reinterpret_cast<float*>(scratch + pl.off_qscale), nullptr, st);
         if (rc != B200F_OK) return rc;
         return launch_gemm_store(op, pl.gemm, 0, a->nb, 1, kscale, l2 ? 1.f : -1.f,
                                  l2 ? qnorm : nullptr, out_matrix, ld_out, a->status, st);
     }
-    rc = launch_prepare_queries(a->queries, a->nq, a->d, a->storage, nullptr, 0, 0, qnorm, 0, 0, 0, nullptr, st);
+    rc = launch_prepare_queries(a->queries, a->nq, a->d, a->storage, nullptr, 0, 0, qnorm, 0, 0, 0, nullptr, nullptr, st);
     if (rc != B200F_OK) return rc;
     for (int64_t g = 0; g < pl.ngroups; g++) {
         B200FSearchArgs sub = *a;

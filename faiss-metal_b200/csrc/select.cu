@@ -693,11 +693,12 @@ int launch_select_parts(const float* part_key, const int32_t* part_idx, int nlis
 int launch_select_candidates(const float* cand_key, const int32_t* cand_idx, const int32_t* cand_cnt,
                              int cap, int64_t nb, int64_t nq, int k, int metric, const float* qnorm,
                              int64_t label_base, float* out_dist, int64_t* out_labels, int32_t* dirty,
-                             cudaStream_t stream) {
+                             const float* thr, cudaStream_t stream) {
     if (cap < 1 || !cand_cnt) return B200F_ERR_BAD_ARG;
     if (rank_select_enabled() && dirty)
         return launch_rank_select(cand_key, cand_idx, cand_cnt, cap, nb, nq, k, metric, qnorm, label_base,
-                                  out_dist, out_labels, dirty, stream);
+                                  out_dist, out_labels, dirty, thr, stream);
+    if (thr) return B200F_ERR_BAD_ARG;   // row_select alone compares the k-th key
     const bool l2 = metric == B200F_METRIC_L2;
     SortSelectParams p{};
     p.keys = cand_key;

@@ -16,6 +16,7 @@
 // Both write exactly what sort_select_kernel writes for the same input: ascending key, ties to the
 // lower id / label.
 #include <atomic>
+#include <cmath>
 
 #include "common.cuh"
 
@@ -89,9 +90,11 @@ struct RowSelectParams {
     float* out_dist;
     int64_t* out_labels;
     int32_t* dirty;           // optional: 1 when the result is not proven complete
+    const float* thr;         // optional, [nq]: rows beyond this key may be missing from the input
 };
 
-__device__ __forceinline__ void rs_write(const RowSelectParams& p, int64_t qo, int rank, uint64_t w) {
+__device__ __forceinline__ void rs_write(const RowSelectParams& p, int64_t qo, int rank, uint64_t w, int* s_beyond) {
+    if (p.thr && rank == p.k - 1 && ordered_to_float((uint32_t)(w >> 32)) > p.thr[qo]) *s_beyond = 1;
     float dist = p.out_sign * ordered_to_float((uint32_t)(w >> 32)) + (p.qnorm ? p.qnorm[qo] : 0.f);
     if (p.clamp && dist < 0.f) dist = 0.f;
     p.out_dist[qo * p.k + rank] = dist;
@@ -102,7 +105,7 @@ __device__ __forceinline__ void rs_write(const RowSelectParams& p, int64_t qo, i
 // The staging area becomes the sorted runs, 32 R words per warp.
 template <int R>
 __device__ __forceinline__ void rank_place(const RowSelectParams& p, int64_t qo, int c, int m,
-                                           uint64_t* runs, int W) {
+                                           uint64_t* runs, int W, int* s_beyond) {
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     uint64_t v[R];
@@ -139,7 +142,7 @@ __device__ __forceinline__ void rank_place(const RowSelectParams& p, int64_t qo,
     }
 #pragma unroll
     for (int r = 0; r < R; r++)
-        if (v[r] != RS_EMPTY && rank[r] < p.k) rs_write(p, qo, rank[r], v[r]);
+        if (v[r] != RS_EMPTY && rank[r] < p.k) rs_write(p, qo, rank[r], v[r], s_beyond);
 }
 
 // The kk-th smallest x = key - mn of what `visit` enumerates (a callable that calls its argument with
@@ -248,7 +251,7 @@ __global__ void __launch_bounds__(1024) row_select_kernel(const RowSelectParams 
     __shared__ uint32_t s_min[32], s_max[32];
     __shared__ int s_live[32];
     __shared__ int s_sel[2];
-    __shared__ int s_count, s_have;
+    __shared__ int s_count, s_have, s_beyond;
     const int W = blockDim.x >> 5;
     const int T = blockDim.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -287,7 +290,7 @@ __global__ void __launch_bounds__(1024) row_select_kernel(const RowSelectParams 
         }
         uint32_t mn = best[0];
         const int my_have = min(live, M);
-        if (tid == 0) s_count = s_have = 0;
+        if (tid == 0) s_count = s_have = s_beyond = 0;
         const Spread sp = block_spread(live, mn, mx, s_live, s_min, s_max);
         live = sp.live;
         mn = sp.mn;
@@ -376,22 +379,23 @@ __global__ void __launch_bounds__(1024) row_select_kernel(const RowSelectParams 
                 int rank = 0;
 #pragma unroll 8
                 for (int j = 0; j < c; j++) rank += rs_runs[j] < w ? 1 : 0;
-                if (rank < p.k) rs_write(p, qo, rank, w);
+                if (rank < p.k) rs_write(p, qo, rank, w, &s_beyond);
             }
         } else {
             const int m = (c + W - 1) / W;    // <= RS_RUN
-            if (m <= 32) rank_place<1>(p, qo, c, m, rs_runs, W);
-            else if (m <= 64) rank_place<2>(p, qo, c, m, rs_runs, W);
-            else if (m <= 128) rank_place<4>(p, qo, c, m, rs_runs, W);
-            else if (m <= 256) rank_place<8>(p, qo, c, m, rs_runs, W);
-            else rank_place<16>(p, qo, c, m, rs_runs, W);
+            if (m <= 32) rank_place<1>(p, qo, c, m, rs_runs, W, &s_beyond);
+            else if (m <= 64) rank_place<2>(p, qo, c, m, rs_runs, W, &s_beyond);
+            else if (m <= 128) rank_place<4>(p, qo, c, m, rs_runs, W, &s_beyond);
+            else if (m <= 256) rank_place<8>(p, qo, c, m, rs_runs, W, &s_beyond);
+            else rank_place<16>(p, qo, c, m, rs_runs, W, &s_beyond);
         }
         for (int j = c + tid; j < p.k; j += T) {
             p.out_dist[qo * p.k + j] = p.pad;
             p.out_labels[qo * p.k + j] = -1;
         }
+        if (p.thr) __syncthreads();   // s_beyond is complete
         if (tid == 0 && p.dirty)
-            p.dirty[q] = ((cnt > p.ld) || (live < p.k && live < p.nb_total)) ? 1 : 0;
+            p.dirty[q] = ((cnt > p.ld) || (live < p.k && live < p.nb_total) || s_beyond) ? 1 : 0;
         __syncthreads();   // the shared arrays are rewritten by the next row
     }
 }
@@ -401,7 +405,9 @@ __global__ void __launch_bounds__(1024) row_select_kernel(const RowSelectParams 
 // have a key, which lets every row pass).  One CTA per row; out[q] may be exceeded by no key that
 // belongs to the r smallest.
 __global__ void __launch_bounds__(1024) row_bound_kernel(const float* __restrict__ keys, int64_t ld, int64_t n,
-                                                         int64_t nq, int r, float* __restrict__ out) {
+                                                         int64_t nq, int r, float* __restrict__ out,
+                                                         int32_t* __restrict__ bad, const float* __restrict__ qnorm,
+                                                         float margin, float qnorm_max, int most) {
     __shared__ int s_hist[256];
     __shared__ uint32_t s_min[32], s_max[32];
     __shared__ int s_live[32];
@@ -436,6 +442,11 @@ __global__ void __launch_bounds__(1024) row_bound_kernel(const float* __restrict
             bound = ordered_to_float(sp.mn + min(x, sp.mx - sp.mn));
         }
         if (tid == 0) out[q] = bound;
+        if (bad) {
+            const float qn = __ldg(qnorm + q);
+            const int under = __syncthreads_count(best <= bound + margin * qn);
+            if (tid == 0 && (under > most || !(qn < qnorm_max))) atomicAdd(bad, 1);
+        }
         __syncthreads();   // the shared arrays are rewritten by the next row
     }
 }
@@ -679,7 +690,8 @@ void set_output(RowSelectParams& p, int metric, const float* qnorm, int64_t labe
 
 }  // namespace
 
-int launch_row_bound(const float* keys, int64_t nq, int64_t n, int64_t ld, int r, float* out, cudaStream_t stream) {
+int launch_row_bound(const float* keys, int64_t nq, int64_t n, int64_t ld, int r, float* out, int32_t* bad,
+                     const float* qnorm, float margin, float qnorm_max, double most, cudaStream_t stream) {
     if (r < 1 || r > 512 || n < 0 || ld < n || !keys || !out) return B200F_ERR_BAD_ARG;
     if (nq <= 0) return B200F_OK;
     const int64_t sm = cached_sm_count();
@@ -688,7 +700,9 @@ int launch_row_bound(const float* keys, int64_t nq, int64_t n, int64_t ld, int r
     int64_t g = nq;
     const int64_t gcap = sm * (2048 / T);
     if (g > gcap) g = gcap;
-    row_bound_kernel<<<(int)g, T, 0, stream>>>(keys, ld, n, nq, r, out);
+    // `most` keys in random columns are the minima of this many threads
+    const int most_minima = (int)(T * (1.0 - std::exp(-most / T)));
+    row_bound_kernel<<<(int)g, T, 0, stream>>>(keys, ld, n, nq, r, out, bad, qnorm, margin, qnorm_max, most_minima);
     count_launch();
     B200F_LAUNCH_CHECK();
     return B200F_OK;
@@ -696,7 +710,8 @@ int launch_row_bound(const float* keys, int64_t nq, int64_t n, int64_t ld, int r
 
 int launch_rank_select(const float* cand_key, const int32_t* cand_idx, const int32_t* cand_cnt, int cap,
                        int64_t nb, int64_t nq, int k, int metric, const float* qnorm, int64_t label_base,
-                       float* out_dist, int64_t* out_labels, int32_t* dirty, cudaStream_t stream) {
+                       float* out_dist, int64_t* out_labels, int32_t* dirty, const float* thr,
+                       cudaStream_t stream) {
     if (cap < 1 || !cand_cnt || !dirty) return B200F_ERR_BAD_ARG;
     RowSelectParams p{};
     p.keys = cand_key;
@@ -707,6 +722,7 @@ int launch_rank_select(const float* cand_key, const int32_t* cand_idx, const int
     p.nq = nq;
     p.k = k;
     p.dirty = dirty;
+    p.thr = thr;
     set_output(p, metric, qnorm, label_base, out_dist, out_labels);
     return launch_row_select(p, cap / 4, stream);
 }
