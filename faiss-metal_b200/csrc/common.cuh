@@ -60,11 +60,33 @@ __device__ __forceinline__ float warp_sum(float v) {
 // FP32 storage, plane_format B200F_PLANES_FP16X2: two fp16 planes of the row scaled by its own
 // power of two, and rowscale[r] = 1 / (row scale * 2^x_scale_log2) (what turns the kernel's
 // accumulator back into key units).  Otherwise rowscale is not written.
-// zero_word (optional) is cleared.
+// The kernel also gives a search's counters their first values (every pointer optional): one launch
+// instead of a memset for each.
+struct SearchInit {
+    int32_t* status = nullptr;   // 4 words of 0
+    int32_t* count = nullptr;    // words 0 and 16: 0
+    int32_t* cand_cnt = nullptr; // [nq] 0
+    uint32_t* gthr = nullptr;    // [nq][gslots] all ones (above every ordered float: no bound yet)
+    int gslots = 1;
+};
 int launch_prepare_queries(const float* q, int64_t nq, int d, int storage, uint16_t* a_planes,
                            int64_t a_pitch, int64_t a_plane_stride, float* qnorm, int norm_cols,
-                           int plane_format, int x_scale_log2, float* rowscale, int32_t* zero_word,
+                           int plane_format, int x_scale_log2, float* rowscale, const SearchInit& init,
                            cudaStream_t stream);
+
+// What a selection does with a row whose result it cannot prove complete, beside dirty[q]: the row is
+// appended to rows (any order), its query operand gathered and the count, cleared by the caller,
+// raised; all > 0: the count is set to `all` instead.
+struct RedoRows {
+    int32_t* count = nullptr;        // null: nothing
+    int32_t* count_copy = nullptr;   // optional, the same
+    int all = 0;
+    int32_t* rows = nullptr;
+    const uint16_t* a = nullptr;     // [npl][.][pitch], pitch a multiple of 8
+    uint16_t* out = nullptr;
+    int npl = 0;
+    int64_t plane_stride = 0, pitch = 0;
+};
 
 // A filter whose keys are only bounds of the true ones (L2): a row's key ||x||^2 - 2 q.x is at least
 // (1 - eps) ||x||^2 - 2 (q.x as computed) - eps ||q||^2 when eps (||x||^2 + ||q||^2) covers twice the error
@@ -141,15 +163,17 @@ struct GemmOperands {
     const int* nq_dev;         // optional: live rows of A (<= nq) left in device memory by a kernel
 };
 // Fused top-k (k <= 32): partial lists part_key/part_idx [nq][2 * P][k] (two per column range).
-// gthr holds nq * gslots words; with gslots = s the shared filter bounds the (32 * s)-th best
+// gthr holds nq * gslots words (gthr_ready: all ones already); with gslots = s the shared filter bounds the (32 * s)-th best
 // key of a row, so lists of k = 32 entries can feed a later selection of up to 32 * s results.
 // tile_stride > 1 visits only every tile_stride-th column tile (plan made for that many tiles).
 int launch_gemm_topk(const GemmOperands& op, const GemmPlan& plan, int64_t col0, int64_t ncols,
                      int64_t tile_stride, float kscale, int k, int gslots, float* part_key,
-                     int32_t* part_idx, uint32_t* gthr, int32_t* status, cudaStream_t stream);
+                     int32_t* part_idx, uint32_t* gthr, bool gthr_ready, int32_t* status,
+                     cudaStream_t stream);
 // Threshold filter over the whole shard: column c of row q with scaled key <= thr[q * thr_stride +
 // thr_pos] is appended to the row's candidate buffer cand_key/cand_idx [nq][cand_cap] in any
-// order; cand_cnt[q] counts every hit, also those beyond cand_cap, which are not stored.
+// order; cand_cnt[q] (zeroed by the caller) counts every hit, also those beyond cand_cap, which are
+// not stored.
 // few_hits: the threshold admits well under one column in a thousand (tunes the scan width).
 int launch_gemm_filter(const GemmOperands& op, const GemmPlan& plan, float kscale, const float* thr,
                        int thr_stride, int thr_pos, float* cand_key, int32_t* cand_idx,
@@ -171,7 +195,7 @@ int launch_gemm_store(const GemmOperands& op, const GemmPlan& plan, int64_t col0
 int launch_merge_partials(const float* part_key, const int32_t* part_idx, int P, int64_t nq, int k,
                           int metric, const float* qnorm, int64_t label_base, float* out_dist,
                           int64_t* out_labels, const int* nq_dev, const int32_t* row_map,
-                          int64_t nb, int32_t* dirty, cudaStream_t stream);
+                          int64_t nb, int32_t* dirty, const RedoRows& redo, cudaStream_t stream);
 // Running top-k over a key matrix chunk: run lists [nq][k] (key, int32 id) are read
 // (if has_prev) and rewritten with the best k of (previous list U chunk columns).
 // Merged raw keys only: out_key[q][k], best first, +INF where fewer than k entries exist.
@@ -200,14 +224,14 @@ int launch_select_parts(const float* part_key, const int32_t* part_idx, int nlis
 int launch_select_candidates(const float* cand_key, const int32_t* cand_idx, const int32_t* cand_cnt,
                              int cap, int64_t nb, int64_t nq, int k, int metric, const float* qnorm,
                              int64_t label_base, float* out_dist, int64_t* out_labels, int32_t* dirty,
-                             const float* thr, cudaStream_t stream);
+                             const float* thr, const RedoRows& redo, cudaStream_t stream);
 // select_rank.cu: the same selection / merge for inputs of at most 8192 entries per row, sorted in
 // registers and placed by binary search; results identical to the kernels of select.cu.
 bool rank_select_enabled();
 int launch_rank_select(const float* cand_key, const int32_t* cand_idx, const int32_t* cand_cnt, int cap,
                        int64_t nb, int64_t nq, int k, int metric, const float* qnorm, int64_t label_base,
                        float* out_dist, int64_t* out_labels, int32_t* dirty, const float* thr,
-                       cudaStream_t stream);
+                       const RedoRows& redo, cudaStream_t stream);
 // The k best of every row of a key matrix (n columns, column c is row c of the shard), finalised.
 int launch_matrix_select(const float* keys, int64_t nq, int64_t n, int64_t ld, int k, int metric, const float* qnorm,
                          int64_t label_base, float* out_dist, int64_t* out_labels, const int* nq_dev,
@@ -217,9 +241,6 @@ int launch_matrix_select(const float* keys, int64_t nq, int64_t n, int64_t ld, i
 // `most` keys up to its bound + margin * qnorm[q], or with qnorm[q] >= qnorm_max.
 int launch_row_bound(const float* keys, int64_t nq, int64_t n, int64_t ld, int r, float* out, int32_t* bad,
                      const float* qnorm, float margin, float qnorm_max, double most, cudaStream_t stream);
-// *count = nq when any of dirty[0 .. nq) is set, else 0 (also to *count_copy): the streaming scans redo
-// all of their few queries or none.
-int launch_any_dirty(const int32_t* dirty, int64_t nq, int32_t* count, int32_t* count_copy, cudaStream_t stream);
 bool rank_merge_fits(int P, int k);
 int launch_rank_merge(const float* dist, const int64_t* labels, int64_t stride_d, int64_t stride_l, int P,
                       int64_t nq, int k, int metric, float* out_dist, int64_t* out_labels,

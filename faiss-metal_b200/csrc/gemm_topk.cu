@@ -1059,11 +1059,12 @@ GemmPlan plan_gemm(int64_t nq, int64_t ncols, int sm_count) {
 
 int launch_gemm_topk(const GemmOperands& op, const GemmPlan& plan, int64_t col0, int64_t ncols,
                      int64_t tile_stride, float kscale, int k, int gslots, float* part_key,
-                     int32_t* part_idx, uint32_t* gthr, int32_t* status, cudaStream_t stream) {
+                     int32_t* part_idx, uint32_t* gthr, bool gthr_ready, int32_t* status,
+                     cudaStream_t stream) {
     if (k <= 0 || k > KMAX || gslots < 1) return B200F_ERR_UNSUPPORTED;
     if (!gthr) return B200F_ERR_BAD_ARG;
     // all-ones is above every ordered float: no bound yet
-    B200F_CUDA_TRY(cudaMemsetAsync(gthr, 0xff, (size_t)op.nq * gslots * sizeof(uint32_t), stream));
+    if (!gthr_ready) B200F_CUDA_TRY(cudaMemsetAsync(gthr, 0xff, (size_t)op.nq * gslots * sizeof(uint32_t), stream));
     GemmParams p{};
     p.mode = MODE_TOPK;
     p.tile_stride = tile_stride;
@@ -1086,7 +1087,6 @@ int launch_gemm_filter(const GemmOperands& op, const GemmPlan& plan, float kscal
                        int32_t* cand_cnt, int cand_cap, int few_hits, int32_t* status,
                        cudaStream_t stream) {
     if (!thr || !cand_key || !cand_idx || !cand_cnt || cand_cap < 1) return B200F_ERR_BAD_ARG;
-    B200F_CUDA_TRY(cudaMemsetAsync(cand_cnt, 0, (size_t)op.nq * sizeof(int32_t), stream));
     GemmParams p{};
     p.mode = MODE_FILTER;
     p.kscale = kscale;

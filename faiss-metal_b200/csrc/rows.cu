@@ -382,8 +382,11 @@ __global__ void prepare_queries_kernel(const float* __restrict__ q, int64_t nq, 
                                        uint16_t* __restrict__ a, int64_t a_pitch,
                                        int64_t a_plane_stride, float* __restrict__ qnorm,
                                        int norm_cols, int plane_format, int x_scale_log2,
-                                       float* __restrict__ rowscale, int32_t* __restrict__ zero_word) {
-    if (zero_word && blockIdx.x == 0 && threadIdx.x == 0) *zero_word = 0;
+                                       float* __restrict__ rowscale, const SearchInit init) {
+    if (blockIdx.x == 0) {
+        if (init.status && threadIdx.x < 4) init.status[threadIdx.x] = 0;
+        if (init.count && threadIdx.x < 2) init.count[16 * threadIdx.x] = 0;
+    }
     const int lane = threadIdx.x & 31;
     const int d8 = (d + 7) & ~7;
     const int fmt = storage == B200F_STORAGE_F16 ? B200F_STORAGE_F16 : B200F_STORAGE_BF16;
@@ -392,6 +395,9 @@ __global__ void prepare_queries_kernel(const float* __restrict__ q, int64_t nq, 
     for (int64_t r = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < nq;
          r += warps_total) {
         const float* row = q + r * (int64_t)d;
+        if (init.cand_cnt && lane == 0) init.cand_cnt[r] = 0;
+        if (init.gthr)
+            for (int j = lane; j < init.gslots; j += 32) init.gthr[r * init.gslots + j] = 0xffffffffu;
         // fp16x2 planes: every query row gets its own power-of-two scale (largest element near
         // 2^6, as the stored rows), kept at most 2^3 above the rows' scale so that the norm-column
         // scales below stay inside fp16.  The kernel's accumulator is then (sq * sx) * t, and
@@ -549,12 +555,12 @@ int cached_sm_count() {
 
 int launch_prepare_queries(const float* q, int64_t nq, int d, int storage, uint16_t* a_planes,
                            int64_t a_pitch, int64_t a_plane_stride, float* qnorm, int norm_cols,
-                           int plane_format, int x_scale_log2, float* rowscale, int32_t* zero_word,
+                           int plane_format, int x_scale_log2, float* rowscale, const SearchInit& init,
                            cudaStream_t stream) {
     if (nq <= 0) return B200F_OK;
     prepare_queries_kernel<<<grid_for_rows(nq), ROW_THREADS, 0, stream>>>(
             q, nq, d, storage, a_planes, a_pitch, a_plane_stride, qnorm, norm_cols, plane_format, x_scale_log2,
-            rowscale, zero_word);
+            rowscale, init);
     count_launch();
     B200F_LAUNCH_CHECK();
     return B200F_OK;

@@ -279,8 +279,9 @@ bool make_plan(int64_t nq, int64_t nb, int d, int k, int storage, int path, bool
         }
     }
     if (!pairwise && pl.path == B200F_PATH_SCAN && nq <= 2 * SCAN_GROUP && !filter_disabled()) {
+        // row_select finds the queries to redo
         const bool wanted = pl.fused ? (nb >= SCAN_LIST_THR_MIN_ROWS && nq * k >= SCAN_LIST_THR_MIN_WORK)
-                                     : nb >= SCAN_FILTER_MIN_ROWS;
+                                     : nb >= SCAN_FILTER_MIN_ROWS && rank_select_enabled();
         pl.sample = wanted && choose_sample(nb, k, SCAN_SAMPLE_ROWS, !pl.fused, &pl.fstride, &pl.frank, &pl.fcap);
         if (pl.sample) {
             pl.nsample = nb / pl.fstride;
@@ -685,9 +686,9 @@ extern "C" int b200f_search(const B200FSearchArgs* a) {
     if (rc != B200F_OK) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(a->stream);
     if (a->nq == 0) return B200F_OK;
-    if (a->status) B200F_CUDA_TRY(cudaMemsetAsync(a->status, 0, 4 * sizeof(int32_t), st));
     const bool l2 = a->metric == B200F_METRIC_L2;
     if (a->nb == 0) {
+        if (a->status) B200F_CUDA_TRY(cudaMemsetAsync(a->status, 0, 4 * sizeof(int32_t), st));
         const int64_t n = a->nq * a->k;
         fill_pad_kernel<<<(int)(ceil_div64(n, 256) < 1024 ? ceil_div64(n, 256) : 1024), 256, 0, st>>>(
                 a->out_dist, a->out_labels, n, l2 ? kHostInf : -kHostInf);
@@ -721,7 +722,7 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
 
     // scans with k > 32: filter with keys that are bounds (see BoundFilter) where it pays
     BoundFilter bf;
-    if (pl.sample && !pl.fused && l2 && rank_select_enabled() && a->nq >= 2 && a->d <= BOUND_MAX_D &&
+    if (pl.sample && !pl.fused && l2 && a->nq >= 2 && a->d <= BOUND_MAX_D &&
         a->nb * a->row_pitch >= BOUND_MIN_ELEMS && scan_bound_filter_fits(*a)) {
         bf.eps = scan_bound_eps(a->storage);
         bf.qnorm = qnorm;
@@ -734,6 +735,12 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
     const double most = pl.sample ? 0.7 * pl.fcap / pl.fstride : 0.0;
     const float margin = 2.5f * bf.eps, qnorm_max = a->storage == B200F_STORAGE_F16 ? 1073741824.f : kHostInf;
 
+    SearchInit init;
+    init.status = a->status;
+    if (pl.sample || pl.filter || pl.lists) init.count = reinterpret_cast<int32_t*>(scratch + pl.off_count);
+    if (pl.filter || (pl.sample && !pl.fused)) init.cand_cnt = reinterpret_cast<int32_t*>(scratch + pl.off_cand_cnt);
+    init.gthr = reinterpret_cast<uint32_t*>(scratch + pl.off_gthr);
+    init.gslots = pl.gslots;
     GemmOperands op{};
     if (pl.path == B200F_PATH_TENSOR) {
         rc = fill_operands(*a, pl, scratch, op);
@@ -741,9 +748,9 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
         rc = launch_prepare_queries(a->queries, a->nq, a->d, a->storage,
                                     reinterpret_cast<uint16_t*>(scratch + pl.off_a), pl.a_pitch,
                                     pl.a_plane_stride, qnorm, qnc, a->plane_format, a->plane_scale_log2,
-                                    reinterpret_cast<float*>(scratch + pl.off_qscale), nullptr, st);
+                                    reinterpret_cast<float*>(scratch + pl.off_qscale), init, st);
     } else {
-        rc = launch_prepare_queries(a->queries, a->nq, a->d, a->storage, nullptr, 0, 0, qnorm, 0, 0, 0, nullptr, bad, st);
+        rc = launch_prepare_queries(a->queries, a->nq, a->d, a->storage, nullptr, 0, 0, qnorm, 0, 0, 0, nullptr, init, st);
     }
     if (rc != B200F_OK) return rc;
 
@@ -751,21 +758,32 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
     const int* nq_dev = nullptr;
     const int32_t* row_map = nullptr;
     uint32_t* gthr = reinterpret_cast<uint32_t*>(scratch + pl.off_gthr);
-    auto redo_setup = [&](int32_t* dirty) -> int {
-        int32_t* rows = reinterpret_cast<int32_t*>(scratch + pl.off_rows);
-        int32_t* count = reinterpret_cast<int32_t*>(scratch + pl.off_count);
-        uint16_t* a2 = reinterpret_cast<uint16_t*>(scratch + pl.off_a2);
-        // the number of redone rows is left in status word 1 for whoever wants to know
-        int r2 = launch_compact_rows(dirty, a->nq, rows, count, a->status ? a->status + 1 : nullptr, st);
-        if (r2 != B200F_OK) return r2;
-        r2 = launch_gather_rows(op.a_planes, op.npl, op.a_plane_stride, op.a_pitch, rows, count, a->nq,
-                                a2, st);
-        if (r2 != B200F_OK) return r2;
-        op.a_planes = a2;
-        op.rowscale_map = rows;   // row j of the gathered operand is query rows[j]
-        op.nq_dev = count;
-        nq_dev = count;
-        row_map = rows;
+    // the number of redone rows is left in status word 1 for whoever wants to know
+    RedoRows redo;
+    redo.count_copy = a->status ? a->status + 1 : nullptr;
+    if (pl.lists || pl.filter) {
+        redo.rows = reinterpret_cast<int32_t*>(scratch + pl.off_rows);
+        redo.count = reinterpret_cast<int32_t*>(scratch + pl.off_count);
+        redo.out = reinterpret_cast<uint16_t*>(scratch + pl.off_a2);
+        redo.a = op.a_planes;
+        redo.npl = op.npl;
+        redo.plane_stride = op.a_plane_stride;
+        redo.pitch = op.a_pitch;
+    }
+    // counted: the selection has listed and gathered the rows itself
+    auto redo_setup = [&](int32_t* dirty, bool counted) -> int {
+        if (!counted) {
+            int r2 = launch_compact_rows(dirty, a->nq, redo.rows, redo.count, redo.count_copy, st);
+            if (r2 != B200F_OK) return r2;
+            r2 = launch_gather_rows(op.a_planes, op.npl, op.a_plane_stride, op.a_pitch, redo.rows, redo.count, a->nq,
+                                    redo.out, st);
+            if (r2 != B200F_OK) return r2;
+        }
+        op.a_planes = redo.out;
+        op.rowscale_map = redo.rows;   // row j of the gathered operand is query rows[j]
+        op.nq_dev = redo.count;
+        nq_dev = redo.count;
+        row_map = redo.rows;
         return B200F_OK;
     };
 
@@ -791,7 +809,7 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
             rc = launch_row_bound(matrix, a->nq, valid, pcols, pl.frank, thr, nullptr, nullptr, 0.f, 0.f, 0.0, st);
             if (rc != B200F_OK) return rc;
         } else {
-            rc = launch_gemm_topk(op, pl.pilot, 0, a->nb, pl.fstride, kscale, pl.frank, 1, pkey, pidx, gthr,
+            rc = launch_gemm_topk(op, pl.pilot, 0, a->nb, pl.fstride, kscale, pl.frank, 1, pkey, pidx, gthr, true,
                                   a->status, st);
             if (rc != B200F_OK) return rc;
             rc = launch_merge_keys(pkey, pidx, 2 * pl.pilot.P, a->nq, pl.frank, thr, st);
@@ -803,9 +821,10 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
                                 pl.pilot_matrix ? 0 : pl.frank - 1, ckey, cidx, ccnt, pl.fcap, wide, a->status, st);
         if (rc != B200F_OK) return rc;
         rc = launch_select_candidates(ckey, cidx, ccnt, pl.fcap, a->nb, a->nq, a->k, a->metric, qnorm,
-                                      a->label_base, a->out_dist, a->out_labels, dirty, nullptr, st);
+                                      a->label_base, a->out_dist, a->out_labels, dirty, nullptr,
+                                      rank_select_enabled() ? redo : RedoRows(), st);
         if (rc != B200F_OK) return rc;
-        rc = redo_setup(dirty);
+        rc = redo_setup(dirty, rank_select_enabled());
         if (rc != B200F_OK) return rc;
     }
 
@@ -813,6 +832,10 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
     float* thr = reinterpret_cast<float*>(scratch + pl.off_thr);
     int32_t* dirty = reinterpret_cast<int32_t*>(scratch + pl.off_dirty);
     int32_t* any_count = reinterpret_cast<int32_t*>(scratch + pl.off_count);
+    RedoRows redo_all = redo;   // the streaming scans redo all of their few queries or none
+    redo_all.count = any_count;
+    redo_all.all = (int)a->nq;
+    redo_all.out = nullptr;
     auto query_group = [&](int64_t q0, int64_t group) {
         B200FSearchArgs sub = *a;
         sub.queries = a->queries + q0 * (int64_t)a->d;
@@ -861,16 +884,14 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
         if (pl.path == B200F_PATH_TENSOR) {
             P = 2 * pl.gemm.P;
             rc = launch_gemm_topk(op, pl.gemm, 0, a->nb, 1, kscale, a->k, 1, part_key, part_idx, gthr,
-                                  a->status, st);
+                                  !pl.filter || pl.pilot_matrix, a->status, st);
             if (rc != B200F_OK) return rc;
         } else {
             rc = scan_lists(pl.sample ? thr : nullptr, nullptr, P);
             if (rc != B200F_OK) return rc;
             if (pl.sample) {
                 rc = launch_merge_partials(part_key, part_idx, P, a->nq, a->k, a->metric, qnorm, a->label_base,
-                                           a->out_dist, a->out_labels, nullptr, nullptr, a->nb, dirty, st);
-                if (rc != B200F_OK) return rc;
-                rc = launch_any_dirty(dirty, a->nq, any_count, a->status ? a->status + 1 : nullptr, st);
+                                           a->out_dist, a->out_labels, nullptr, nullptr, a->nb, dirty, redo_all, st);
                 if (rc != B200F_OK) return rc;
                 nq_dev = any_count;
                 rc = scan_lists(nullptr, any_count, P);
@@ -878,7 +899,8 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
             }
         }
         return launch_merge_partials(part_key, part_idx, P, a->nq, a->k, a->metric, qnorm,
-                                     a->label_base, a->out_dist, a->out_labels, nq_dev, row_map, 0, nullptr, st);
+                                     a->label_base, a->out_dist, a->out_labels, nq_dev, row_map, 0, nullptr, RedoRows(),
+                                     st);
     }
 
     // k > 32 from 32-entry lists: select, find the rows that are not proven exact, and send only
@@ -887,12 +909,12 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
         float* part_key = reinterpret_cast<float*>(scratch + pl.off_part_key);
         int32_t* part_idx = reinterpret_cast<int32_t*>(scratch + pl.off_part_idx);
         rc = launch_gemm_topk(op, pl.gemm, 0, a->nb, 1, kscale, B200F_FUSED_MAX_K, pl.gslots, part_key,
-                              part_idx, gthr, a->status, st);
+                              part_idx, gthr, true, a->status, st);
         if (rc != B200F_OK) return rc;
         rc = launch_select_parts(part_key, part_idx, 2 * pl.gemm.P, a->nq, a->k, a->metric, qnorm,
                                  a->label_base, a->out_dist, a->out_labels, dirty, st);
         if (rc != B200F_OK) return rc;
-        rc = redo_setup(dirty);
+        rc = redo_setup(dirty, false);
         if (rc != B200F_OK) return rc;
     }
 
@@ -901,7 +923,6 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
         float* ckey = reinterpret_cast<float*>(scratch + pl.off_cand_key);
         int32_t* cidx = reinterpret_cast<int32_t*>(scratch + pl.off_cand_idx);
         int32_t* ccnt = reinterpret_cast<int32_t*>(scratch + pl.off_cand_cnt);
-        B200F_CUDA_TRY(cudaMemsetAsync(ccnt, 0, (size_t)a->nq * sizeof(int32_t), st));
         BoundFilter exact;
         if (bad) {
             rc = launch_scan_bound_filter(*a, thr, ckey, cidx, ccnt, pl.fcap, bf, st);
@@ -918,9 +939,7 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
             if (rc != B200F_OK) return rc;
         }
         rc = launch_select_candidates(ckey, cidx, ccnt, pl.fcap, a->nb, a->nq, a->k, a->metric, qnorm,
-                                      a->label_base, a->out_dist, a->out_labels, dirty, bad ? thr : nullptr, st);
-        if (rc != B200F_OK) return rc;
-        rc = launch_any_dirty(dirty, a->nq, any_count, a->status ? a->status + 1 : nullptr, st);
+                                      a->label_base, a->out_dist, a->out_labels, dirty, bad ? thr : nullptr, redo_all, st);
         if (rc != B200F_OK) return rc;
         nq_dev = any_count;
     }
@@ -1000,12 +1019,12 @@ extern "C" int b200f_pairwise(const B200FSearchArgs* a, float* out_matrix, int64
         rc = launch_prepare_queries(a->queries, a->nq, a->d, a->storage,
                                     reinterpret_cast<uint16_t*>(scratch + pl.off_a), pl.a_pitch,
                                     pl.a_plane_stride, qnorm, l2 ? 1 : 0, a->plane_format, a->plane_scale_log2,
-                                    reinterpret_cast<float*>(scratch + pl.off_qscale), nullptr, st);
+                                    reinterpret_cast<float*>(scratch + pl.off_qscale), SearchInit(), st);
         if (rc != B200F_OK) return rc;
         return launch_gemm_store(op, pl.gemm, 0, a->nb, 1, kscale, l2 ? 1.f : -1.f,
                                  l2 ? qnorm : nullptr, out_matrix, ld_out, a->status, st);
     }
-    rc = launch_prepare_queries(a->queries, a->nq, a->d, a->storage, nullptr, 0, 0, qnorm, 0, 0, 0, nullptr, nullptr, st);
+    rc = launch_prepare_queries(a->queries, a->nq, a->d, a->storage, nullptr, 0, 0, qnorm, 0, 0, 0, nullptr, SearchInit(), st);
     if (rc != B200F_OK) return rc;
     for (int64_t g = 0; g < pl.ngroups; g++) {
         B200FSearchArgs sub = *a;

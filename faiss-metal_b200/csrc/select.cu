@@ -543,16 +543,6 @@ __global__ void __launch_bounds__(1024) compact_rows_kernel(const int32_t* __res
     }
 }
 
-__global__ void any_dirty_kernel(const int32_t* __restrict__ dirty, int nq, int32_t* __restrict__ count,
-                                 int32_t* __restrict__ count_copy) {
-    const bool d = (int)threadIdx.x < nq && dirty[threadIdx.x] != 0;
-    const int n = __any_sync(FULL, d) ? nq : 0;
-    if (threadIdx.x == 0) {
-        *count = n;
-        if (count_copy) *count_copy = n;
-    }
-}
-
 __global__ void gather_rows_kernel(const uint16_t* __restrict__ a, int npl, int64_t plane_stride,
                                    int64_t pitch, const int32_t* __restrict__ rows,
                                    const int32_t* __restrict__ count, uint16_t* __restrict__ out) {
@@ -693,12 +683,12 @@ int launch_select_parts(const float* part_key, const int32_t* part_idx, int nlis
 int launch_select_candidates(const float* cand_key, const int32_t* cand_idx, const int32_t* cand_cnt,
                              int cap, int64_t nb, int64_t nq, int k, int metric, const float* qnorm,
                              int64_t label_base, float* out_dist, int64_t* out_labels, int32_t* dirty,
-                             const float* thr, cudaStream_t stream) {
+                             const float* thr, const RedoRows& redo, cudaStream_t stream) {
     if (cap < 1 || !cand_cnt) return B200F_ERR_BAD_ARG;
     if (rank_select_enabled() && dirty)
         return launch_rank_select(cand_key, cand_idx, cand_cnt, cap, nb, nq, k, metric, qnorm, label_base,
-                                  out_dist, out_labels, dirty, thr, stream);
-    if (thr) return B200F_ERR_BAD_ARG;   // row_select alone compares the k-th key
+                                  out_dist, out_labels, dirty, thr, redo, stream);
+    if (thr || redo.count) return B200F_ERR_BAD_ARG;   // only row_select knows them
     const bool l2 = metric == B200F_METRIC_L2;
     SortSelectParams p{};
     p.keys = cand_key;
@@ -725,14 +715,6 @@ int launch_compact_rows(const int32_t* dirty, int64_t nq, int32_t* rows, int32_t
                         int32_t* count_copy, cudaStream_t stream) {
     if (nq <= 0) return B200F_OK;
     compact_rows_kernel<<<1, 1024, 0, stream>>>(dirty, nq, rows, count, count_copy);
-    count_launch();
-    B200F_LAUNCH_CHECK();
-    return B200F_OK;
-}
-
-int launch_any_dirty(const int32_t* dirty, int64_t nq, int32_t* count, int32_t* count_copy, cudaStream_t stream) {
-    if (nq < 1 || nq > 32) return B200F_ERR_BAD_ARG;
-    any_dirty_kernel<<<1, 32, 0, stream>>>(dirty, (int)nq, count, count_copy);
     count_launch();
     B200F_LAUNCH_CHECK();
     return B200F_OK;

@@ -91,6 +91,7 @@ struct RowSelectParams {
     int64_t* out_labels;
     int32_t* dirty;           // optional: 1 when the result is not proven complete
     const float* thr;         // optional, [nq]: rows beyond this key may be missing from the input
+    RedoRows redo;
 };
 
 __device__ __forceinline__ void rs_write(const RowSelectParams& p, int64_t qo, int rank, uint64_t w, int* s_beyond) {
@@ -394,8 +395,34 @@ __global__ void __launch_bounds__(1024) row_select_kernel(const RowSelectParams 
             p.out_labels[qo * p.k + j] = -1;
         }
         if (p.thr) __syncthreads();   // s_beyond is complete
-        if (tid == 0 && p.dirty)
-            p.dirty[q] = ((cnt > p.ld) || (live < p.k && live < p.nb_total) || s_beyond) ? 1 : 0;
+        if (tid == 0 && p.dirty) {
+            const bool bad = cnt > p.ld || (live < p.k && live < p.nb_total) || s_beyond;
+            p.dirty[q] = bad ? 1 : 0;
+            s_sel[0] = -1;
+            if (bad && p.redo.count) {
+                if (p.redo.all > 0) {
+                    *p.redo.count = p.redo.all;
+                    if (p.redo.count_copy) *p.redo.count_copy = p.redo.all;
+                } else {
+                    const int j = atomicAdd(p.redo.count, 1);
+                    if (p.redo.count_copy) atomicAdd(p.redo.count_copy, 1);
+                    p.redo.rows[j] = (int32_t)q;
+                    s_sel[0] = j;
+                }
+            }
+        }
+        if (p.redo.out) {   // the query operand of a row to redo
+            __syncthreads();
+            const int j = s_sel[0];
+            if (j >= 0) {
+                const int vec_per_row = (int)(p.redo.pitch / 8);
+                for (int v = tid; v < p.redo.npl * vec_per_row; v += T) {
+                    const int pl = v / vec_per_row, c = v - pl * vec_per_row;
+                    reinterpret_cast<uint4*>(p.redo.out + pl * p.redo.plane_stride + j * p.redo.pitch)[c] =
+                            reinterpret_cast<const uint4*>(p.redo.a + pl * p.redo.plane_stride + q * p.redo.pitch)[c];
+                }
+            }
+        }
         __syncthreads();   // the shared arrays are rewritten by the next row
     }
 }
@@ -711,7 +738,7 @@ int launch_row_bound(const float* keys, int64_t nq, int64_t n, int64_t ld, int r
 int launch_rank_select(const float* cand_key, const int32_t* cand_idx, const int32_t* cand_cnt, int cap,
                        int64_t nb, int64_t nq, int k, int metric, const float* qnorm, int64_t label_base,
                        float* out_dist, int64_t* out_labels, int32_t* dirty, const float* thr,
-                       cudaStream_t stream) {
+                       const RedoRows& redo, cudaStream_t stream) {
     if (cap < 1 || !cand_cnt || !dirty) return B200F_ERR_BAD_ARG;
     RowSelectParams p{};
     p.keys = cand_key;
@@ -723,6 +750,7 @@ int launch_rank_select(const float* cand_key, const int32_t* cand_idx, const int
     p.k = k;
     p.dirty = dirty;
     p.thr = thr;
+    p.redo = redo;
     set_output(p, metric, qnorm, label_base, out_dist, out_labels);
     return launch_row_select(p, cap / 4, stream);
 }
@@ -730,7 +758,7 @@ int launch_rank_select(const float* cand_key, const int32_t* cand_idx, const int
 int launch_merge_partials(const float* part_key, const int32_t* part_idx, int P, int64_t nq, int k,
                           int metric, const float* qnorm, int64_t label_base, float* out_dist,
                           int64_t* out_labels, const int* nq_dev, const int32_t* row_map,
-                          int64_t nb, int32_t* dirty, cudaStream_t stream) {
+                          int64_t nb, int32_t* dirty, const RedoRows& redo, cudaStream_t stream) {
     if (nq <= 0) return B200F_OK;
     if (k < 1 || k > 32 || P < 1) return B200F_ERR_UNSUPPORTED;
     RowSelectParams p{};
@@ -740,6 +768,7 @@ int launch_merge_partials(const float* part_key, const int32_t* part_idx, int P,
     p.n = (int64_t)P * k;
     p.nb_total = nb;
     p.dirty = dirty;
+    p.redo = redo;
     p.nq = nq;
     p.nq_dev = nq_dev;
     p.row_map = row_map;

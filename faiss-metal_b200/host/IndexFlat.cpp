@@ -31,6 +31,7 @@ namespace {
 constexpr size_t kStageBytes = 32ull << 20;   // fp32 staging chunk of add / reconstruct_n (two in flight)
 constexpr int64_t kScaleSampleRows = 8192;    // rows an fp32 index takes its plane scale from
 constexpr int64_t kGraphMaxQueries = 8;        // searches this small are replayed from a CUDA graph
+constexpr int64_t kGraphDirectResults = 512;   // results of a captured search written to host memory by the kernel
 constexpr size_t kMaxGraphs = 8;               // graphs kept per index (least recently used goes)
 constexpr int64_t kFusedBatch = 16384;        // queries per launch, k <= 1024 (fused kernel, lists)
 constexpr int64_t kSelectBatch = 1024;        // queries per launch beyond: few rows, wide column chunks
@@ -882,16 +883,20 @@ bool B200IndexFlat::searchFromGraph(faiss::idx_t n, const float* x, faiss::idx_t
             a.queries = reinterpret_cast<const float*>(region + L.offQueries);
             a.nq = n;
             a.k = (int)k;
-            a.out_dist = reinterpret_cast<float*>(region + L.offDist);
-            a.out_labels = reinterpret_cast<int64_t*>(region + L.offLabels);
+            // a few KB of results: the selection kernel writes them to the pinned slot itself (two copies of
+            // 3 us, with as much between them, were a sixth of a single query's 66 us)
+            const bool direct = n * k <= kGraphDirectResults;
+            a.out_dist = reinterpret_cast<float*>(direct ? e.host + e.hostDistOff : region + L.offDist);
+            a.out_labels = reinterpret_cast<int64_t*>(direct ? e.host + e.hostLabOff : region + L.offLabels);
             a.scratch = region + L.offScratch;
             a.scratch_bytes = L.scratchBytes;
             cudaCheck(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "search: begin capture");
             cudaError_t ce = cudaMemcpyAsync(region + L.offQueries, e.host, (size_t)n * d * 4, cudaMemcpyHostToDevice, st);
             int rc = ce == cudaSuccess ? b200f_search(&a) : B200F_ERR_CUDA;
             if (rc == B200F_OK) {
-                ce = cudaMemcpyAsync(e.host + e.hostDistOff, a.out_dist, (size_t)n * k * 4, cudaMemcpyDeviceToHost, st);
-                if (ce == cudaSuccess)
+                if (!direct)
+                    ce = cudaMemcpyAsync(e.host + e.hostDistOff, a.out_dist, (size_t)n * k * 4, cudaMemcpyDeviceToHost, st);
+                if (!direct && ce == cudaSuccess)
                     ce = cudaMemcpyAsync(e.host + e.hostLabOff, a.out_labels, (size_t)n * k * 8, cudaMemcpyDeviceToHost, st);
                 if (ce == cudaSuccess)
                     ce = cudaMemcpyAsync(e.host + e.hostStatusOff, im.status, 16, cudaMemcpyDeviceToHost, st);
