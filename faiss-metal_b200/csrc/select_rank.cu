@@ -235,6 +235,61 @@ __device__ __forceinline__ Spread block_spread(int live, uint32_t mn, uint32_t m
 }
 
 constexpr int RS_COUNT_MAX = 256;   // so few words are placed by counting the smaller ones
+constexpr int RS_BUCKETS = 2048;
+constexpr int RS_BUCKET_MAX = 64;   // a fuller bucket: sorted runs instead
+
+// The words' positions from 2,048 buckets of equal width in key: a word's rank is the number of words in the
+// buckets before its own plus the smaller ones in it, one or two on average.  Sorted runs and binary
+// searches in the other warps' took half of the 37 us that 2,900 candidates cost (k = 2048), now 18.5.  False, with nothing
+// written, when the keys do not spread (equal keys, infinities).  All threads of the CTA call it.
+__device__ bool bucket_place(const RowSelectParams& p, int64_t qo, int c, float lo, float hi, const uint64_t* words,
+                             int* end, uint16_t* order, int* s_warp, int* s_beyond) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, T = blockDim.x;
+    const float scale = (RS_BUCKETS - 1) / (hi - lo);
+    if (!(scale > 0.f && scale < CUDART_INF_F && hi - lo < CUDART_INF_F)) return false;   // the same for every thread
+    auto bucket = [&](uint64_t w) {   // ascending with the key; clamped against rounding
+        return max(0, min((int)((ordered_to_float((uint32_t)(w >> 32)) - lo) * scale), RS_BUCKETS - 1));
+    };
+    for (int i = tid; i < RS_BUCKETS; i += T) end[i] = 0;
+    __syncthreads();
+    for (int i = tid; i < c; i += T) atomicAdd(&end[bucket(words[i])], 1);
+    __syncthreads();
+    // exclusive prefix sums in place: RS_BUCKETS / T consecutive buckets per thread (T >= 128)
+    const int per = RS_BUCKETS / T;
+    int sum = 0, most = 0;
+    for (int i = 0; i < per; i++) {
+        const int h = end[tid * per + i];
+        sum += h;
+        most = max(most, h);
+    }
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(FULL, incl, o);
+        if (lane >= o) incl += up;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    if (__syncthreads_or(most > RS_BUCKET_MAX)) return false;
+    int start = incl - sum;
+    for (int w = 0; w < warp; w++) start += s_warp[w];
+    for (int i = 0; i < per; i++) {
+        const int h = end[tid * per + i];
+        end[tid * per + i] = start;
+        start += h;
+    }
+    __syncthreads();
+    for (int i = tid; i < c; i += T) order[atomicAdd(&end[bucket(words[i])], 1)] = (uint16_t)i;
+    __syncthreads();
+    for (int i = tid; i < c; i += T) {
+        const uint64_t w = words[i];
+        const int b = bucket(w);
+        const int first = b > 0 ? end[b - 1] : 0;
+        int rank = first;
+        for (int j = first; j < end[b]; j++) rank += words[order[j]] < w ? 1 : 0;
+        if (rank < p.k) rs_write(p, qo, rank, w, s_beyond);
+    }
+    return true;
+}
 
 // One CTA per row, latency-bound (a row is a few KB in L1 / L2).  A pass over the keys leaves every
 // thread with the M smallest keys of its share; with k <= M T / 2 the k-th smallest of those M T bounds the
@@ -242,12 +297,12 @@ constexpr int RS_COUNT_MAX = 256;   // so few words are placed by counting the s
 // of 4 over the row: 10,000 rows of 20,000 keys, k = 1000: 2,415 us with M = 1, which leaves k > T / 2 to
 // the passes over the row, 551 with M = 4).  Otherwise, or when that bound admits more than the
 // staging area holds, the k-th key is found exactly by radix select over the row.  The words up to
-// the bound are compacted and placed: by counting the smaller ones up to 256 of them, else sorted per
-// warp and placed by binary search.  Where even the exact k-th key is shared by more than fit (hundreds
+// the bound are compacted and placed: by counting the smaller ones up to 256 of them, else from buckets of
+// equal width, or sorted per warp and placed by binary search where the keys do not spread.  Where even the exact k-th key is shared by more than fit (hundreds
 // of ties), a second radix select over the ids of those finds the ones that belong to the result.
 template <int M>
 __global__ void __launch_bounds__(1024) row_select_kernel(const RowSelectParams p) {
-    extern __shared__ __align__(16) uint64_t rs_runs[];   // bound words
+    extern __shared__ __align__(16) uint64_t rs_runs[];   // bound words, then the buckets of bucket_place
     __shared__ int s_hist[256];
     __shared__ uint32_t s_min[32], s_max[32];
     __shared__ int s_live[32];
@@ -382,7 +437,9 @@ __global__ void __launch_bounds__(1024) row_select_kernel(const RowSelectParams 
                 for (int j = 0; j < c; j++) rank += rs_runs[j] < w ? 1 : 0;
                 if (rank < p.k) rs_write(p, qo, rank, w, &s_beyond);
             }
-        } else {
+        } else if (!bucket_place(p, qo, c, ordered_to_float(mn), ordered_to_float(mn + min(thr_x, sp.mx - mn)), rs_runs,
+                                 reinterpret_cast<int*>(rs_runs + p.bound),
+                                 reinterpret_cast<uint16_t*>(rs_runs + p.bound) + 2 * RS_BUCKETS, s_live, &s_beyond)) {
             const int m = (c + W - 1) / W;    // <= RS_RUN
             if (m <= 32) rank_place<1>(p, qo, c, m, rs_runs, W, &s_beyond);
             else if (m <= 64) rank_place<2>(p, qo, c, m, rs_runs, W, &s_beyond);
@@ -683,12 +740,13 @@ int launch_row_select(RowSelectParams& p, int64_t n_typical, cudaStream_t stream
     while (T < 1024 && 4 * T < 2 * p.k && 16 * (int64_t)T < n_typical) T <<= 1;
     const bool four = 2 * p.k > T;
     p.bound = bound;
-    const int smem = bound * 8;
+    const int smem = bound * 8 + RS_BUCKETS * 4 + bound * 2;   // words, buckets, order
     static bool attr_set[kMaxDevices] = {false};
     const int slot = device_slot();
     if (!attr_set[slot]) {
         for (auto* fn : {row_select_kernel<1>, row_select_kernel<4>})
-            B200F_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 8192 * 8));
+            B200F_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                8192 * 10 + RS_BUCKETS * 4));
         attr_set[slot] = true;
     }
     int64_t g = p.nq;
