@@ -378,7 +378,10 @@ load_rows_kernel(const void* __restrict__ rows, int64_t n, int d, int lpr, int64
 // fp32 queries -> operand planes of the tensor path (+ exact fp32 squared norms).
 // One plane in the storage format (fp16 / bf16) or three bf16 split planes (fp32 storage).
 // With norm_cols the 8 columns after d8 of plane 0 receive the norm scales (see above).
-__global__ void prepare_queries_kernel(const float* __restrict__ q, int64_t nq, int d, int storage,
+// A warp takes a row, or (WIDE) a whole CTA: a warp's chain of loads and conversions over a row of 770 took 18 us
+// for 24 queries, whose launch every search waits for (now under 5).
+template <bool WIDE>
+__global__ void __launch_bounds__(ROW_THREADS) prepare_queries_kernel(const float* __restrict__ q, int64_t nq, int d, int storage,
                                        uint16_t* __restrict__ a, int64_t a_pitch,
                                        int64_t a_plane_stride, float* __restrict__ qnorm,
                                        int norm_cols, int plane_format, int x_scale_log2,
@@ -387,17 +390,18 @@ __global__ void prepare_queries_kernel(const float* __restrict__ q, int64_t nq, 
         if (init.status && threadIdx.x < 4) init.status[threadIdx.x] = 0;
         if (init.count && threadIdx.x < 2) init.count[16 * threadIdx.x] = 0;
     }
-    const int lane = threadIdx.x & 31;
+    __shared__ float s_part[2][ROW_THREADS / 32];
+    const int lane = WIDE ? threadIdx.x : threadIdx.x & 31;   // position among the threads of a row
+    constexpr int LANES = WIDE ? ROW_THREADS : 32;
     const int d8 = (d + 7) & ~7;
     const int fmt = storage == B200F_STORAGE_F16 ? B200F_STORAGE_F16 : B200F_STORAGE_BF16;
     const bool fp16x2 = storage == B200F_STORAGE_F32 && plane_format == kPlanesFp16x2;
-    const int64_t warps_total = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t r = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < nq;
-         r += warps_total) {
+    const int64_t teams = (int64_t)gridDim.x * (ROW_THREADS / LANES);
+    for (int64_t r = (int64_t)blockIdx.x * (ROW_THREADS / LANES) + (WIDE ? 0 : threadIdx.x >> 5); r < nq; r += teams) {
         const float* row = q + r * (int64_t)d;
         if (init.cand_cnt && lane == 0) init.cand_cnt[r] = 0;
         if (init.gthr)
-            for (int j = lane; j < init.gslots; j += 32) init.gthr[r * init.gslots + j] = 0xffffffffu;
+            for (int j = lane; j < init.gslots; j += LANES) init.gthr[r * init.gslots + j] = 0xffffffffu;
         // fp16x2 planes: every query row gets its own power-of-two scale (largest element near
         // 2^6, as the stored rows), kept at most 2^3 above the rows' scale so that the norm-column
         // scales below stay inside fp16.  The kernel's accumulator is then (sq * sx) * t, and
@@ -405,12 +409,17 @@ __global__ void prepare_queries_kernel(const float* __restrict__ q, int64_t nq, 
         float sq = 1.f, ratio = 1.f;
         if (fp16x2 && a) {
             float amax = 0.f;
-            for (int j = lane; j < d; j += 32) {
+            for (int j = lane; j < d; j += LANES) {
                 const float v = fabsf(row[j]);
                 if (v < CUDART_INF_F) amax = fmaxf(amax, v);
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+            if (WIDE) {
+                if ((threadIdx.x & 31) == 0) s_part[0][threadIdx.x >> 5] = amax;
+                __syncthreads();
+                for (int w = 0; w < ROW_THREADS / 32; w++) amax = fmaxf(amax, s_part[0][w]);
+            }
             int e = 0;
             if (amax > 0.f) (void)frexpf(amax, &e);   // amax = m * 2^e, m in [0.5, 1)
             int lq = amax > 0.f ? 7 - e : x_scale_log2;
@@ -422,7 +431,7 @@ __global__ void prepare_queries_kernel(const float* __restrict__ q, int64_t nq, 
             if (rowscale && lane == 0) rowscale[r] = ldexpf(1.f, -(lq + x_scale_log2));
         }
         float s = 0.f;
-        for (int j = lane; j < a_pitch || j < d; j += 32) {
+        for (int j = lane; j < a_pitch || j < d; j += LANES) {
             float v = (j < d) ? row[j] : 0.f;
             s = fmaf(v, v, s);
             if (a && j < a_pitch) {
@@ -454,8 +463,15 @@ __global__ void prepare_queries_kernel(const float* __restrict__ q, int64_t nq, 
         }
         if (qnorm) {
             s = warp_sum(s);
+            if (WIDE) {
+                if ((threadIdx.x & 31) == 0) s_part[1][threadIdx.x >> 5] = s;
+                __syncthreads();
+                s = 0.f;
+                for (int w = 0; w < ROW_THREADS / 32; w++) s += s_part[1][w];
+            }
             if (lane == 0) qnorm[r] = s;
         }
+        if (WIDE) __syncthreads();   // the shared partials are rewritten by the next row
     }
 }
 
@@ -558,7 +574,10 @@ int launch_prepare_queries(const float* q, int64_t nq, int d, int storage, uint1
                            int plane_format, int x_scale_log2, float* rowscale, const SearchInit& init,
                            cudaStream_t stream) {
     if (nq <= 0) return B200F_OK;
-    prepare_queries_kernel<<<grid_for_rows(nq), ROW_THREADS, 0, stream>>>(
+    // a CTA per row while that leaves no SM with more than a few
+    const bool wide = d >= 128 && nq <= 8 * (int64_t)cached_sm_count();
+    auto* kernel = wide ? prepare_queries_kernel<true> : prepare_queries_kernel<false>;
+    kernel<<<wide ? (int)nq : grid_for_rows(nq), ROW_THREADS, 0, stream>>>(
             q, nq, d, storage, a_planes, a_pitch, a_plane_stride, qnorm, norm_cols, plane_format, x_scale_log2,
             rowscale, init);
     count_launch();
