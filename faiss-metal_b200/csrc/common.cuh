@@ -161,6 +161,7 @@ struct GemmOperands {
     int d_pad;                 // K extent (multiple of 8), norm columns included
     int d_data;                // K extent without them
     const int* nq_dev;         // optional: live rows of A (<= nq) left in device memory by a kernel
+    bool overlap;              // launch while the previous kernel of the stream drains (programmatic launch)
 };
 // Fused top-k (k <= 32): partial lists part_key/part_idx [nq][2 * P][k] (two per column range).
 // gthr holds nq * gslots words (gthr_ready: all ones already); with gslots = s the shared filter bounds the (32 * s)-th best
@@ -201,10 +202,10 @@ int launch_merge_partials(const float* part_key, const int32_t* part_idx, int P,
 // Merged raw keys only: out_key[q][k], best first, +INF where fewer than k entries exist.
 int launch_merge_keys(const float* part_key, const int32_t* part_idx, int P, int64_t nq, int k,
                       float* out_key, cudaStream_t stream);
-// nq_dev (optional): number of live rows, read on the device.
+// nq_dev (optional): number of live rows, read on the device.  overlap: programmatic launch.
 int launch_select_chunk(const float* keys, int64_t nq, int64_t ncols, int64_t ld, int64_t col0,
                         int k, int has_prev, float* run_key, int32_t* run_idx, const int* nq_dev,
-                        cudaStream_t stream);
+                        bool overlap, cudaStream_t stream);
 // row_map (optional): list j belongs to query row_map[j] (output row and query norm).
 int launch_finalize_lists(const float* run_key, const int32_t* run_idx, int64_t nq, int k,
                           int metric, const float* qnorm, int64_t label_base, float* out_dist,

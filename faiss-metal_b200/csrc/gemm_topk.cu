@@ -281,6 +281,12 @@ __device__ __forceinline__ void tc_ld64(uint32_t taddr, uint32_t (&r)[64]) {
             : "r"(taddr)
             : "memory");
 }
+// one 32-byte sector of a row
+__device__ __forceinline__ void st_global_v8(float* dst, const float (&v)[8]) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "f"(v[0]), "f"(v[1]), "f"(v[2]),
+                 "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+                 : "memory");
+}
 __device__ __forceinline__ void tc_wait_ld() {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
@@ -380,6 +386,9 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
     const uint32_t bar_tfull = bar_empty + STAGES * 8;
     const uint32_t bar_tempty = bar_tfull + 2 * 8;
 
+    // (programmatic launches: the next kernel may be set up now, this one starts when its predecessor is done)
+    pdl_trigger();
+    pdl_wait();
     // A launch that redoes rows counted on the device usually finds none: leave before any
     // barrier or TMEM allocation (the value is the same for every thread of every CTA).
     if (p.nq_dev && *p.nq_dev <= 0) return;
@@ -747,14 +756,27 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
                     scan(std::integral_constant<int, 32>{});
                 }
                 } else {
+                const bool whole = !partial && (p.ld & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
 #pragma unroll 1
                 for (int ch = eh * CH_PER_HALF; ch < (eh + 1) * CH_PER_HALF; ch++) {
                     uint32_t r[32];
                     tc_ld32(taddr + ch * 32, r);
                     tc_wait_ld();
                     const int64_t cbase = c_tile + ch * 32;
-                    {
-                        // Store mode: thread t holds 32 consecutive columns of ITS row; writing
+                    if (whole) {
+                        // 32 consecutive columns of the thread's row: four whole sectors
+                        if (row_live) {
+                            float* o = p.out + grow * p.ld + (t * TILE_N + ch * 32);
+#pragma unroll
+                            for (int c = 0; c < 32; c += 8) {
+                                float v[8];
+#pragma unroll
+                                for (int e = 0; e < 8; e++) v[e] = fmaf(p.sign, -ksc * __uint_as_float(r[c + e]), radd);
+                                st_global_v8(o + c, v);
+                            }
+                        }
+                    } else {
+                        // Ragged or unaligned output: thread t holds 32 consecutive columns of ITS row; writing
                         // them directly would touch 32 different rows per instruction.  The warp
                         // transposes the 32 x 32 block through shared memory (the list area is
                         // idle in this mode) and writes one 128-byte row segment per instruction.
@@ -944,19 +966,26 @@ int launch_common(const GemmOperands& op, const GemmPlan& plan, GemmParams& p, i
     if (p.mode < 0 || p.mode > 2) return B200F_ERR_BAD_ARG;
     const KernelFn kernel = kernels[plan.pair ? 1 : 0][p.mode];
     main_kernel_begin(stream);
-    if (plan.pair) {
+    if (plan.pair || op.overlap) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)plan.grid, 1, 1);
         cfg.blockDim = dim3(NUM_THREADS, 1, 1);
-        cfg.dynamicSmemBytes = Cfg<true>::SMEM_BYTES;
+        cfg.dynamicSmemBytes = plan.pair ? Cfg<true>::SMEM_BYTES : Cfg<false>::SMEM_BYTES;
         cfg.stream = stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
+        cudaLaunchAttribute attr[2];
         cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        if (plan.pair) {
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = 2;
+            attr[0].val.clusterDim.y = 1;
+            attr[0].val.clusterDim.z = 1;
+            cfg.numAttrs = 1;
+        }
+        if (op.overlap) {
+            attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+            cfg.numAttrs++;
+        }
         cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, ma, mb, p);
         if (e != cudaSuccess) {
             (void)cudaGetLastError();
@@ -1057,6 +1086,28 @@ GemmPlan plan_gemm(int64_t nq, int64_t ncols, int sm_count) {
     return g;
 }
 
+// Filter and store launches carry nothing from one tile of a range to the next: ranges as short as even
+// out the last wave (1,000 queries, 100,000 rows: 784 tiles on 74 CTA pairs, 12 tile times with ranges of
+// six, 11 with ranges of one), a tenth of a tile being what a range costs by itself.
+static GemmPlan spread_plan(GemmPlan g) {
+    double best = 0.0;
+    const int64_t longest = g.tiles_per_range;
+    for (int64_t tpr = 1; tpr <= longest; tpr = tpr < 8 ? tpr + 1 : tpr + tpr / 4) {
+        const int64_t P = ceil_div64(g.ntiles, tpr);
+        const double cost = (double)ceil_div64(P * g.nqb, g.units) * ((double)tpr + 0.1);
+        if (tpr == 1 || cost < best) {
+            best = cost;
+            g.tiles_per_range = tpr;
+            g.P = (int)P;
+        }
+    }
+    if (longest > 0) {
+        const int64_t items = (int64_t)g.nqb * g.P, u = items < g.units ? items : g.units;
+        g.grid = (int)(g.pair ? 2 * u : u);
+    }
+    return g;
+}
+
 int launch_gemm_topk(const GemmOperands& op, const GemmPlan& plan, int64_t col0, int64_t ncols,
                      int64_t tile_stride, float kscale, int k, int gslots, float* part_key,
                      int32_t* part_idx, uint32_t* gthr, bool gthr_ready, int32_t* status,
@@ -1100,7 +1151,7 @@ int launch_gemm_filter(const GemmOperands& op, const GemmPlan& plan, float kscal
     p.cand_cap = cand_cap;
     p.wide = few_hits ? 1 : 0;
     p.status = status;
-    return launch_common(op, plan, p, 0, op.nb, stream);
+    return launch_common(op, spread_plan(plan), p, 0, op.nb, stream);
 }
 
 int launch_gemm_store(const GemmOperands& op, const GemmPlan& plan, int64_t col0, int64_t ncols,
@@ -1118,7 +1169,7 @@ int launch_gemm_store(const GemmOperands& op, const GemmPlan& plan, int64_t col0
     p.out = out;
     p.ld = ld;
     p.status = status;
-    return launch_common(op, plan, p, col0, ncols, stream);
+    return launch_common(op, spread_plan(plan), p, col0, ncols, stream);
 }
 
 }  // namespace b200f

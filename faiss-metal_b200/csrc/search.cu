@@ -949,6 +949,11 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
     float* run_key = reinterpret_cast<float*>(scratch + pl.off_run_key);
     int32_t* run_idx = reinterpret_cast<int32_t*>(scratch + pl.off_run_idx);
     int has_prev = 0;
+    // Rows to redo are usually none: dozens of launches that leave at once, 4 us each with the gap.  Launched
+    // while their predecessor drains they take half; not while the stream is being captured.
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    op.overlap = nq_dev && pl.path == B200F_PATH_TENSOR && a->nb > pl.chunk_cols &&
+                 cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
     for (int64_t c0 = 0; c0 < a->nb; c0 += pl.chunk_cols) {
         const int64_t nc = (a->nb - c0) < pl.chunk_cols ? (a->nb - c0) : pl.chunk_cols;
         if (pl.path == B200F_PATH_TENSOR) {
@@ -968,7 +973,7 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
             return launch_matrix_select(matrix, a->nq, nc, pl.chunk_cols, a->k, a->metric, qnorm, a->label_base,
                                         a->out_dist, a->out_labels, nq_dev, row_map, st);
         rc = launch_select_chunk(matrix, a->nq, nc, pl.chunk_cols, c0, a->k, has_prev, run_key,
-                                 run_idx, nq_dev, st);
+                                 run_idx, nq_dev, op.overlap, st);
         if (rc != B200F_OK) return rc;
         has_prev = 1;
     }

@@ -20,6 +20,7 @@
 // Keys are "smaller is better" everywhere: L2 key = distance, inner product key = -dot.
 // Ties go to the lower id.
 #include "common.cuh"
+#include "ptx.cuh"
 
 namespace b200f {
 
@@ -245,6 +246,8 @@ __global__ void __launch_bounds__(SS_THREADS) sort_select_kernel(const SortSelec
         s_pending[0] = 0;
         s_pending[1] = 0;
     }
+    pdl_trigger();
+    pdl_wait();
 
     const int64_t nq_live = p.nq_dev ? min((int64_t)*p.nq_dev, p.nq) : p.nq;
     for (int64_t q = blockIdx.x; q < nq_live; q += gridDim.x) {
@@ -559,7 +562,7 @@ __global__ void gather_rows_kernel(const uint16_t* __restrict__ a, int npl, int6
 }
 
 template <int SRC>
-int launch_sort_select(const SortSelectParams& p, cudaStream_t stream) {
+int launch_sort_select(const SortSelectParams& p, cudaStream_t stream, bool overlap = false) {
     if (p.nq <= 0) return B200F_OK;
     if (p.k < 1 || p.k > B200F_MAX_K) return B200F_ERR_UNSUPPORTED;
     const int smem = SS_CAP * 8;
@@ -575,7 +578,17 @@ int launch_sort_select(const SortSelectParams& p, cudaStream_t stream) {
     if (g > cap) g = cap;
     // rows counted on the device are usually few or none: idle CTAs leave at once
     if (p.nq_dev && g > cached_sm_count()) g = cached_sm_count();
-    sort_select_kernel<SRC><<<(int)g, SS_THREADS, smem, stream>>>(p);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)g, 1, 1);
+    cfg.blockDim = dim3(SS_THREADS, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = overlap ? 1 : 0;
+    B200F_CUDA_TRY(cudaLaunchKernelEx(&cfg, sort_select_kernel<SRC>, p));
     count_launch();
     B200F_LAUNCH_CHECK();
     return B200F_OK;
@@ -638,7 +651,7 @@ int launch_merge_keys(const float* part_key, const int32_t* part_idx, int P, int
 
 int launch_select_chunk(const float* keys, int64_t nq, int64_t ncols, int64_t ld, int64_t col0,
                         int k, int has_prev, float* run_key, int32_t* run_idx, const int* nq_dev,
-                        cudaStream_t stream) {
+                        bool overlap, cudaStream_t stream) {
     SortSelectParams p{};
     p.nq_dev = nq_dev;
     p.keys = keys;
@@ -652,7 +665,7 @@ int launch_select_chunk(const float* keys, int64_t nq, int64_t ncols, int64_t ld
     p.run_key = run_key;
     p.run_idx = run_idx;
     p.out_dist = nullptr;
-    return launch_sort_select<SRC_MATRIX>(p, stream);
+    return launch_sort_select<SRC_MATRIX>(p, stream, overlap);
 }
 
 int launch_select_parts(const float* part_key, const int32_t* part_idx, int nlists, int64_t nq,
