@@ -386,9 +386,8 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
     const uint32_t bar_tfull = bar_empty + STAGES * 8;
     const uint32_t bar_tempty = bar_tfull + 2 * 8;
 
-    // (programmatic launches: the next kernel may be set up now, this one starts when its predecessor is done)
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();
     // A launch that redoes rows counted on the device usually finds none: leave before any
     // barrier or TMEM allocation (the value is the same for every thread of every CTA).
     if (p.nq_dev && *p.nq_dev <= 0) return;

@@ -15,7 +15,8 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 // Programmatic dependent launch.  pdl_trigger: the next kernel of the stream, launched with the attribute, may
 // take its place on the SMs; pdl_wait: everything earlier in the stream has completed and is visible
 // (no effect in a kernel launched without the attribute).  A kernel that may be launched that way waits
-// before its first access to memory.
+// before its first access to memory, and triggers after it: its successor then overlaps with no
+// other kernel than itself.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -246,8 +246,8 @@ __global__ void __launch_bounds__(SS_THREADS) sort_select_kernel(const SortSelec
         s_pending[0] = 0;
         s_pending[1] = 0;
     }
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();
 
     const int64_t nq_live = p.nq_dev ? min((int64_t)*p.nq_dev, p.nq) : p.nq;
     for (int64_t q = blockIdx.x; q < nq_live; q += gridDim.x) {
