@@ -15,7 +15,8 @@
 //    Sources: a key matrix chunk, sorted lists of other ranks, the fused kernel's 32-entry
 //    lists, or a threshold-filtered candidate buffer; the last two also report rows whose
 //    result is not proven exact.
-//  * compact_rows / gather_rows: the rows to redo, counted and gathered on the device.
+//  * compact_rows / gather_rows: the rows to redo, counted and gathered on the device, after
+//    sort_select (row_select, select_rank.cu, does both itself).
 //
 // Keys are "smaller is better" everywhere: L2 key = distance, inner product key = -dot.
 // Ties go to the lower id.
