@@ -951,9 +951,14 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
     int has_prev = 0;
     // Rows to redo are usually none: dozens of launches that leave at once, 4 us each with the gap.  Launched
     // while their predecessor drains they take half; not while the stream is being captured.
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    op.overlap = nq_dev && pl.path == B200F_PATH_TENSOR && a->nb > pl.chunk_cols &&
-                 cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+    if (nq_dev && pl.path == B200F_PATH_TENSOR && a->nb > pl.chunk_cols) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
+            (void)cudaGetLastError();
+            cap = cudaStreamCaptureStatusActive;
+        }
+        op.overlap = cap == cudaStreamCaptureStatusNone;
+    }
     for (int64_t c0 = 0; c0 < a->nb; c0 += pl.chunk_cols) {
         const int64_t nc = (a->nb - c0) < pl.chunk_cols ? (a->nb - c0) : pl.chunk_cols;
         if (pl.path == B200F_PATH_TENSOR) {
