@@ -148,14 +148,21 @@ __device__ __forceinline__ void norm_pieces(float v, int storage, uint16_t (&out
 //   kPlanesBf16x3  x = b0 + b1 + b2, three bf16 planes (24 bits, fp32's exponent range): six plane
 //                  products reproduce the fp32 product to 2^-24
 //   kPlanesFp16x2  x * s = h0 + h1, two fp16 planes (22 bits) of the row scaled by a power of two s
-//                  chosen for the index (largest element near 2^6): three plane products, half
+//                  chosen for the index (largest element of a sample of its first rows near 2^6): three
+//                  plane products, half
 //                  the tensor work and two thirds of the plane bytes.  fp16 has a narrow exponent
-//                  range, so the format only holds while every stored row fits it: an element
-//                  at or beyond 2^15 after scaling, or a row whose largest element falls below
-//                  2^-4 (1/1024 of the scale target: its low plane would go subnormal and lose
-//                  bits), raises `range_flag`, and the index re-splits itself into bf16x3.
+//                  range, so the format only holds while every stored row fits it.  `range_flag` is
+//                  raised, and the index takes another scale or re-splits itself into bf16x3, by
+//                    an element at or beyond 2^15 after scaling;
+//                    a row whose largest element falls below 2^-4 (1/1024 of the scale target: its
+//                    low plane would go subnormal and lose bits);
+//                    with norm columns, a row whose ||s x||^2 / 2 is beyond what their four pieces
+//                    hold (kNormPiecesMax): the first would be -inf and the row's keys NaN, on no
+//                    result list even for a query equal to it.  Long before the first bound: d = 128
+//                    from elements of 2,100 on.
 constexpr int kPlanesBf16x3 = 0;
 constexpr int kPlanesFp16x2 = 1;
+constexpr float kNormPiecesMax = 4096.f * 65504.f;   // largest scale times the largest fp16 value
 
 // V consecutive elements of a row per lane and access: 4 (or 8, load_rows_kernel) where the row
 // length and every pitch and base allow it, else 2 or 1.
@@ -282,7 +289,9 @@ store_rows_kernel(const float* __restrict__ src, int64_t src_pitch, int64_t n, i
             amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
         }
         if (!live || cl != 0) continue;
-        if (range_flag && planes && plane_format == kPlanesFp16x2 && (amax >= 32768.f || (amax > 0.f && amax < 0.0625f)))
+        if (range_flag && planes && plane_format == kPlanesFp16x2 &&
+            (amax >= 32768.f || (amax > 0.f && amax < 0.0625f) ||
+             (norm_cols && 0.5f * s * plane_scale * plane_scale > kNormPiecesMax)))
             atomicOr(range_flag, 1);
         if (norms) norms[r] = s;
         if (norm_cols) {

@@ -495,9 +495,9 @@ void B200IndexFlat::add(faiss::idx_t n, const float* x) {
             return;
         }
         if (impl_->planeFormat == B200F_PLANES_FP16X2 && !impl_->planeScaleKnown) {
-            // The index's scale: the largest element of the first rows it is given goes to [2^6, 2^7).  A
-            // few thousand rows spread over the block tell it (a pass over all of them costs a quarter of
-            // what storing them does: 242 us of 1.5 GB); rows that do not fit it raise the range flag.
+            // The index's scale: the largest element of a few thousand rows spread over the first block it is
+            // given goes to [2^6, 2^7) (a pass over all of them costs a quarter of what storing them does: 242 us
+            // of 1.5 GB).  A row that does not fit it, an element or its norm, raises the range flag.
             const int64_t stride = std::max<int64_t>(1, nr / kScaleSampleRows);
             if (!setPlaneScale(src, (nr + stride - 1) / stride, (int64_t)d * stride) && stride > 1)
                 (void)setPlaneScale(src, nr, d);   // nothing but zeros in the sample

@@ -56,12 +56,13 @@ extern "C" {
  * half precision, shaders/simdgroup_gemm.metal:62-69, ~1e-2 relative; the contract here is 1e-4):
  *   BF16X3  x = b0 + b1 + b2, three bf16 planes, six plane products, exact to 2^-24.
  *   FP16X2  2^s x = h0 + h1, two fp16 planes of the row scaled by the index's power of two 2^s
- *           (largest element near 2^6), three plane products, exact to 2^-22: half the tensor
- *           work, two thirds of the plane bytes.  Valid while every row fits fp16's range
- *           (elements below 2^15 after scaling, no non-zero row whose largest element is below
- *           2^-4); b200f_store_rows_fp32 reports rows that do not through range_flag, and the
- *           index then re-splits itself into BF16X3.  Queries are scaled per row inside
- *           b200f_search, so their magnitude does not matter. */
+ *           (largest element of a sample of its first rows near 2^6), three plane products, exact
+ *           to 2^-22: half the tensor work, two thirds of the plane bytes.  Valid while every row
+ *           fits fp16's range (elements below 2^15 after scaling, no non-zero row whose largest
+ *           element is below 2^-4, with norm columns ||2^s x||^2 / 2 at most 2^12 * 65504);
+ *           b200f_store_rows_fp32 reports rows that do not through range_flag, and the index
+ *           then takes its scale from all rows or re-splits itself into BF16X3.  Queries are
+ *           scaled per row inside b200f_search, so their magnitude does not matter. */
 #define B200F_PLANES_BF16X3 0
 #define B200F_PLANES_FP16X2 1
 

@@ -90,3 +90,40 @@ def test_plane_scale_from_a_sample(fm, res, n):
     D, I = idx.search(xq, 10)
     H.check_against_oracle(O.METRIC_L2, 0, True, xb, xq, 10, D, I)
     idx.close()
+
+
+@pytest.mark.parametrize("where", ["device", "host", "second_add"])
+@pytest.mark.parametrize("d", [48, 128, 1536])
+@pytest.mark.parametrize("factor", [20, 50, 100, 250])
+def test_a_row_far_longer_than_the_sample(fm, res, where, d, factor):
+    # one row the sample does not take (it takes every third), its elements inside fp16's range at a scale made for
+    # the others but its norm beyond what the norm columns hold: found on the tensor path all the same
+    n, nq, k, row = 30_000, 12, 5, 20_000
+    xb = H.uniform_pm1(n, d, 13)
+    xb[row] *= np.float32(factor)
+    xq = H.uniform_pm1(nq, d, 14)
+    xq[3] = xb[row]
+    idx = fm.B200IndexFlat(res, d, O.METRIC_L2, 0)
+    if where == "host":
+        idx.add(xb)
+    elif where == "device":
+        idx.add(torch.from_numpy(xb).to("cuda:0"))
+        # at the scale made for the long row the others keep 0.9 * 64 / 250 > 2^-4
+        assert idx.fp32_planes == fm.abi.PLANES_FP16X2
+    else:
+        idx.add(torch.from_numpy(xb[:row]).to("cuda:0"))
+        idx.add(torch.from_numpy(xb[row:]).to("cuda:0"))
+    D, I = idx.search(xq, k)
+    assert I[3, 0] == row
+    x64, q64 = xb.astype(np.float64), xq.astype(np.float64)
+    length = np.sqrt((x64 ** 2).sum(1))
+    for q in range(nq):
+        true = ((x64 - q64[q]) ** 2).sum(1)
+        want = np.sort(np.partition(true, k - 1)[:k])
+        # 22-bit products: 2^-21 (||q|| + ||x||)^2 of a distance.  Their fp32 sum grows 16 columns at a time, d / 16 + 1
+        # steps, each dropping up to 2^-23 of a sum of at most ||q|| ||x||, of which a distance takes twice: another
+        # (d / 16 + 1) 2^-24 (||q|| + ||x||)^2, 5.8e-6 for d = 1536, where the distance of the long row to itself came
+        # out as 6.5e-6 ||x||^2
+        tol = (2.0 ** -21 + (d / 16 + 1) * 2.0 ** -24) * (np.sqrt((q64[q] ** 2).sum()) + length[I[q]].max()) ** 2
+        assert np.abs(D[q] - want).max() <= tol and np.abs(true[I[q]] - D[q]).max() <= tol
+    idx.close()
