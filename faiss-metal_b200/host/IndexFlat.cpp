@@ -316,6 +316,16 @@ struct B200IndexFlat::Impl {
         capacity = want;
     }
 
+    // Scratch for n queries taken `batch` at a time.  Fewer queries may need more of it (the paths change with the
+    // number of queries: up to 2^24 pairs the whole key matrix is kept, beyond only lists), so the last,
+    // shorter batch is asked for too.  0: the shape cannot be planned.
+    size_t searchScratch(int64_t n, int64_t batch, int64_t ntotal, int64_t k) const {
+        size_t bytes = b200f_search_scratch_bytes(batch, ntotal, d, (int)k, storageCode(), forcePath);
+        if (bytes > 0 && n % batch != 0)
+            bytes = std::max(bytes, b200f_search_scratch_bytes(n % batch, ntotal, d, (int)k, storageCode(), forcePath));
+        return bytes;
+    }
+
     void fillArgs(B200FSearchArgs& a, int64_t ntotal) const {
         std::memset(&a, 0, sizeof(a));
         a.d = d;
@@ -784,8 +794,7 @@ void B200IndexFlat::search(faiss::idx_t n, const float* x, faiss::idx_t k, float
         searchFromGraph(n, x, k, distances, labels))
         return;
     const int64_t batch = std::min<int64_t>(n, k <= B200F_LIST_MAX_K ? kFusedBatch : kSelectBatch);
-    const size_t scratchBytes =
-            b200f_search_scratch_bytes(batch, ntotal, d, (int)k, impl_->storageCode(), impl_->forcePath);
+    const size_t scratchBytes = impl_->searchScratch(n, batch, ntotal, k);
     B200_THROW_ARG_IF_NOT(B200F_ERR_BAD_ARG, scratchBytes > 0, "search: cannot plan this shape");
     CallLayout L = makeLayout(batch, batch, d, k, !qOnDevice, batch, true, scratchBytes);
     uint8_t* region = static_cast<uint8_t*>(impl_->res->getScratch(L.total));
@@ -1098,8 +1107,7 @@ B200SearchToken B200IndexFlat::searchAsync(faiss::idx_t n, const float* x, faiss
     const bool qOnDevice = isDevicePointer(x);
     const int64_t batch = std::min<int64_t>(n, k <= B200F_LIST_MAX_K ? kFusedBatch : kSelectBatch);
     t->nbatches = (int)((n + batch - 1) / batch);
-    const size_t scratchBytes =
-            b200f_search_scratch_bytes(batch, ntotal, d, (int)k, impl_->storageCode(), impl_->forcePath);
+    const size_t scratchBytes = impl_->searchScratch(n, batch, ntotal, k);
     B200_THROW_ARG_IF_NOT(B200F_ERR_BAD_ARG, scratchBytes > 0, "searchAsync: cannot plan this shape");
     // per-call buffers: the token owns them (src/MetalIndexFlat.mm:441-476)
     CallLayout L = makeLayout(n, batch, d, k, !qOnDevice, n, true, scratchBytes);

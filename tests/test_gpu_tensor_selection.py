@@ -43,3 +43,24 @@ def test_rows_the_sample_misjudges(fm, res, storage, k):
     D, I = idx.search(xq, k)
     H.check_against_oracle(O.METRIC_L2, storage, True, xb, xq[:8], k, D[:8], I[:8], loose=False)
     idx.close()
+
+
+@pytest.mark.parametrize("how", ["search", "search_async"])
+@pytest.mark.parametrize("nb,tail,k", [(2000, 2000, 10), (2000, 8000, 32), (5000, 900, 3), (32_768, 14_000, 10)])
+def test_last_batch_that_needs_more_scratch(fm, res, how, nb, tail, k):
+    # a search takes 16,384 queries at a time; the shorter rest needs more scratch than a full batch does
+    size = fm.lib().b200f_search_scratch_bytes
+    d, n = 32, 16_384 + tail
+    assert size(tail, nb, d, k, 0, 0) > size(16_384, nb, d, k, 0, 0)
+    xb = H.gaussian(nb, d, 1)
+    xq = H.gaussian(n, d, 2)
+    idx = fm.B200IndexFlat(res, d, O.METRIC_L2, 0)
+    idx.add(xb)
+    if how == "search":
+        D, I = idx.search(xq, k)
+    else:
+        D, I = np.empty((n, k), np.float32), np.empty((n, k), np.int64)
+        idx.search_async(xq, k, D, I).wait()
+    idx.close()
+    for q in (slice(0, 8), slice(16_380, 16_390), slice(n - 8, n)):
+        H.check_against_oracle(O.METRIC_L2, 0, True, xb, xq[q], k, D[q], I[q], loose=False)
