@@ -202,10 +202,11 @@ int launch_merge_partials(const float* part_key, const int32_t* part_idx, int P,
 // Merged raw keys only: out_key[q][k], best first, +INF where fewer than k entries exist.
 int launch_merge_keys(const float* part_key, const int32_t* part_idx, int P, int64_t nq, int k,
                       float* out_key, cudaStream_t stream);
-// nq_dev (optional): number of live rows, read on the device.  overlap: programmatic launch.
+// nq_dev (optional): number of live rows, read on the device.  inf_empty: a +INF key is no result, as in the
+// tensor path's lists and filter.  overlap: programmatic launch.
 int launch_select_chunk(const float* keys, int64_t nq, int64_t ncols, int64_t ld, int64_t col0,
                         int k, int has_prev, float* run_key, int32_t* run_idx, const int* nq_dev,
-                        bool overlap, cudaStream_t stream);
+                        bool inf_empty, bool overlap, cudaStream_t stream);
 // row_map (optional): list j belongs to query row_map[j] (output row and query norm).
 int launch_finalize_lists(const float* run_key, const int32_t* run_idx, int64_t nq, int k,
                           int metric, const float* qnorm, int64_t label_base, float* out_dist,
@@ -233,10 +234,11 @@ int launch_rank_select(const float* cand_key, const int32_t* cand_idx, const int
                        int64_t nb, int64_t nq, int k, int metric, const float* qnorm, int64_t label_base,
                        float* out_dist, int64_t* out_labels, int32_t* dirty, const float* thr,
                        const RedoRows& redo, cudaStream_t stream);
-// The k best of every row of a key matrix (n columns, column c is row c of the shard), finalised.
-int launch_matrix_select(const float* keys, int64_t nq, int64_t n, int64_t ld, int k, int metric, const float* qnorm,
-                         int64_t label_base, float* out_dist, int64_t* out_labels, const int* nq_dev,
-                         const int32_t* row_map, cudaStream_t stream);
+// The k best of every row of a key matrix (n columns, column c is row c of the shard), finalised.  inf_empty
+// as above.
+int launch_matrix_select(const float* keys, int64_t nq, int64_t n, int64_t ld, int k, bool inf_empty, int metric,
+                         const float* qnorm, int64_t label_base, float* out_dist, int64_t* out_labels,
+                         const int* nq_dev, const int32_t* row_map, cudaStream_t stream);
 // out[q]: an upper bound, close to it, of the r-th smallest (r <= 512) of the n keys of row q; +INF when
 // there are too few.  NaN keys are skipped.  bad (optional): one more for every row with more than about
 // `most` keys up to its bound + margin * qnorm[q], or with qnorm[q] >= qnorm_max.

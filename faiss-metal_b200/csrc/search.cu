@@ -949,6 +949,9 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
     float* run_key = reinterpret_cast<float*>(scratch + pl.off_run_key);
     int32_t* run_idx = reinterpret_cast<int32_t*>(scratch + pl.off_run_idx);
     int has_prev = 0;
+    // Lists and filter leave out rows whose key is +INF (an overflowed product).  So does the key matrix where
+    // they may serve the same k: which of them runs depends on the number of rows and queries.
+    const bool inf_empty = pl.path == B200F_PATH_TENSOR && a->k <= B200F_LIST_MAX_K;
     // Rows to redo are usually none: dozens of launches that leave at once, 4 us each with the gap.  Launched
     // while their predecessor drains they take half; not while the stream is being captured.
     if (nq_dev && pl.path == B200F_PATH_TENSOR && a->nb > pl.chunk_cols) {
@@ -975,10 +978,10 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
         }
         // the whole shard in one chunk: select from it at once (a few passes over a row that stays in L2)
         if (nc == a->nb && nc <= MATRIX_SELECT_MAX_COLS && rank_select_enabled())
-            return launch_matrix_select(matrix, a->nq, nc, pl.chunk_cols, a->k, a->metric, qnorm, a->label_base,
-                                        a->out_dist, a->out_labels, nq_dev, row_map, st);
+            return launch_matrix_select(matrix, a->nq, nc, pl.chunk_cols, a->k, inf_empty, a->metric, qnorm,
+                                        a->label_base, a->out_dist, a->out_labels, nq_dev, row_map, st);
         rc = launch_select_chunk(matrix, a->nq, nc, pl.chunk_cols, c0, a->k, has_prev, run_key,
-                                 run_idx, nq_dev, op.overlap, st);
+                                 run_idx, nq_dev, inf_empty, op.overlap, st);
         if (rc != B200F_OK) return rc;
         has_prev = 1;
     }

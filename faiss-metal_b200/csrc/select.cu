@@ -193,6 +193,7 @@ struct SortSelectParams {
     int P;
     int64_t nq;
     const int* nq_dev;    // optional: live rows (<= nq), read on the device
+    int inf_empty;        // SRC_MATRIX: columns with a +INF key are no candidates
     const int32_t* part_idx;  // SRC_PARTS
     const int32_t* cand_cnt;  // SRC_PARTS: candidates counted per row (may exceed ld: overflow)
     int64_t nb_total;     // SRC_PARTS with cand_cnt: rows in the shard
@@ -250,6 +251,8 @@ __global__ void __launch_bounds__(SS_THREADS) sort_select_kernel(const SortSelec
     pdl_wait();
     pdl_trigger();
 
+    // in front of every word of a +INF key, or behind all words
+    const uint64_t thr_first = p.inf_empty ? pack(CUDART_INF_F, 0u) : SS_EMPTY;
     const int64_t nq_live = p.nq_dev ? min((int64_t)*p.nq_dev, p.nq) : p.nq;
     for (int64_t q = blockIdx.x; q < nq_live; q += gridDim.x) {
         __syncthreads();
@@ -257,7 +260,7 @@ __global__ void __launch_bounds__(SS_THREADS) sort_select_kernel(const SortSelec
         // right before each sort that would read them
         if (tid == 0) {
             s_count = 0;
-            s_thr = SS_EMPTY;
+            s_thr = thr_first;
             s_pending[0] = 0;
             s_pending[1] = 0;
         }
@@ -279,7 +282,7 @@ __global__ void __launch_bounds__(SS_THREADS) sort_select_kernel(const SortSelec
                 }
                 c = lo;
                 s_count = c;
-                s_thr = (c >= p.k) ? buf[p.k - 1] : SS_EMPTY;
+                s_thr = (c >= p.k) ? buf[p.k - 1] : thr_first;
             }
             __syncthreads();
         }
@@ -652,8 +655,9 @@ int launch_merge_keys(const float* part_key, const int32_t* part_idx, int P, int
 
 int launch_select_chunk(const float* keys, int64_t nq, int64_t ncols, int64_t ld, int64_t col0,
                         int k, int has_prev, float* run_key, int32_t* run_idx, const int* nq_dev,
-                        bool overlap, cudaStream_t stream) {
+                        bool inf_empty, bool overlap, cudaStream_t stream) {
     SortSelectParams p{};
+    p.inf_empty = inf_empty ? 1 : 0;
     p.nq_dev = nq_dev;
     p.keys = keys;
     p.ld = ld;

@@ -16,6 +16,7 @@
 // Both write exactly what sort_select_kernel writes for the same input: ascending key, ties to the
 // lower id / label.
 #include <atomic>
+#include <cfloat>
 #include <cmath>
 
 #include "common.cuh"
@@ -73,6 +74,7 @@ __device__ __forceinline__ void warp_sort(uint64_t (&v)[R], int lane) {
 struct RowSelectParams {
     const float* keys;        // [nq][ld] keys, smaller is better
     const int32_t* ids;       // [nq][ld] row ids (-1 = empty); null: the id is the column, NaN keys are empty
+    float last_key;           // ids null: keys beyond this one are empty too (+INF, or the largest finite one)
     const int32_t* cnt;       // candidates counted per row (may exceed ld: overflow); null: n
     int64_t ld;
     int64_t n;
@@ -320,7 +322,7 @@ __global__ void __launch_bounds__(1024) row_select_kernel(const RowSelectParams 
         // (ordered key, live) of column c; both loads are issued before either is used
         auto load = [&](int c, uint32_t& key, int32_t& id) {
             const float f = __ldg(keys + c) + 0.f;   // -0 becomes +0: the two tie
-            id = ids ? __ldg(ids + c) : (f == f ? c : -1);
+            id = ids ? __ldg(ids + c) : (f <= p.last_key ? c : -1);
             key = float_to_ordered(f);
         };
         int live = 0;
@@ -835,14 +837,15 @@ int launch_merge_partials(const float* part_key, const int32_t* part_idx, int P,
     return launch_row_select(p, p.n, stream);
 }
 
-int launch_matrix_select(const float* keys, int64_t nq, int64_t n, int64_t ld, int k, int metric, const float* qnorm,
-                         int64_t label_base, float* out_dist, int64_t* out_labels, const int* nq_dev,
-                         const int32_t* row_map, cudaStream_t stream) {
+int launch_matrix_select(const float* keys, int64_t nq, int64_t n, int64_t ld, int k, bool inf_empty, int metric,
+                         const float* qnorm, int64_t label_base, float* out_dist, int64_t* out_labels,
+                         const int* nq_dev, const int32_t* row_map, cudaStream_t stream) {
     if (n < 0 || n > 0x7fffffffLL || ld < n) return B200F_ERR_BAD_ARG;
     RowSelectParams p{};
     p.keys = keys;
     p.ld = ld;
     p.n = n;
+    p.last_key = inf_empty ? FLT_MAX : kHostInf;
     p.nq = nq;
     p.nq_dev = nq_dev;
     p.row_map = row_map;

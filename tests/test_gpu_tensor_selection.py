@@ -45,6 +45,30 @@ def test_rows_the_sample_misjudges(fm, res, storage, k):
     idx.close()
 
 
+@pytest.mark.parametrize("storage,metric", [(2, O.METRIC_INNER_PRODUCT), (2, O.METRIC_L2)])
+@pytest.mark.parametrize("nb", [3000, 32_768, 32_769, 140_000, 600_000])
+@pytest.mark.parametrize("k", [2, 10, 32, 100, 1000])
+def test_infinite_keys_are_no_results(fm, res, storage, metric, nb, k):
+    # products (or norms) of all rows but a few overflow fp32: as in the oracle, such rows fill no slot, whichever
+    # way their number selects
+    nq, d, few = 20, 16, 7
+    xb = np.full((nb, d), 2.0 ** 126, np.float32)
+    rows = np.linspace(0, nb - 1, few).astype(int)
+    xb[rows] = H.gaussian(few, d, 3)
+    xq = -1.0 - np.abs(H.gaussian(nq, d, 4))
+    if metric == O.METRIC_INNER_PRODUCT:
+        xq *= np.float32(1024.0)
+    idx = fm.B200IndexFlat(res, d, metric, storage)
+    idx.add(xb)
+    D, I = idx.search(xq, k)
+    live = min(k, few)
+    assert (np.sort(I[:, :live], axis=1) >= 0).all() and np.isin(I[:, :live], rows).all()
+    assert (I[:, live:] == -1).all()
+    assert (np.isposinf(D[:, live:]) if metric == O.METRIC_L2 else np.isneginf(D[:, live:])).all()
+    H.check_against_oracle(metric, storage, True, xb[rows], xq, live, D[:, :live], np.searchsorted(rows, I[:, :live]))
+    idx.close()
+
+
 @pytest.mark.parametrize("how", ["search", "search_async"])
 @pytest.mark.parametrize("nb,tail,k", [(2000, 2000, 10), (2000, 8000, 32), (5000, 900, 3), (32_768, 14_000, 10)])
 def test_last_batch_that_needs_more_scratch(fm, res, how, nb, tail, k):
