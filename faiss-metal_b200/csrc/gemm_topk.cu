@@ -622,7 +622,8 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
             // slot of the row's bound array this list publishes to
             uint32_t* const gslot = p.gthr ? p.gthr + grow * p.gslots + (int)((2 * xr + eh) % p.gslots) : nullptr;
             float ksc = p.kscale;          // this row's key scale
-            if (p.rowscale && row_live) ksc *= __ldg(p.rowscale + (p.rowscale_map ? (int64_t)__ldg(p.rowscale_map + grow) : grow));
+            // coherent loads: the kernel before a programmatic launch wrote the map
+            if (p.rowscale && row_live) ksc *= __ldcg(p.rowscale + (p.rowscale_map ? (int64_t)__ldcg(p.rowscale_map + grow) : grow));
             float thr = CUDART_INF_F;      // worst key of this thread's list (k-th best of the range)
             float thr_eff = CUDART_INF_F;  // filter: min(thr, bound shared by all ranges of the row)
             float thr_pub = CUDART_INF_F;  // last value published to gthr

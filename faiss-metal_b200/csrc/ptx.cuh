@@ -16,7 +16,8 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 // take its place on the SMs; pdl_wait: everything earlier in the stream has completed and is visible
 // (no effect in a kernel launched without the attribute).  A kernel that may be launched that way waits
 // before its first access to memory, and triggers after it: its successor then overlaps with no
-// other kernel than itself.
+// other kernel than itself.  What its predecessor wrote it reads with coherent loads (no __ldg, no
+// const __restrict__): the read-only path wants data that nobody writes while the kernel is resident.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

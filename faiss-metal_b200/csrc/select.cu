@@ -248,6 +248,8 @@ __global__ void __launch_bounds__(SS_THREADS) sort_select_kernel(const SortSelec
         s_pending[0] = 0;
         s_pending[1] = 0;
     }
+    // SRC_MATRIX may be resident while the kernel before it still writes the matrix: its keys are read with
+    // coherent loads only (__ldcg), since the wait orders those and not the read-only path
     pdl_wait();
     pdl_trigger();
 
@@ -322,11 +324,11 @@ __global__ void __launch_bounds__(SS_THREADS) sort_select_kernel(const SortSelec
                 for (int i = 0; i < WV; i++) {
                     const int64_t c = w0 + ((int64_t)i * SS_THREADS + tid) * 4;
                     if (c + 4 <= total) {
-                        v[i] = __ldg(reinterpret_cast<const float4*>(rowp + c));
+                        v[i] = __ldcg(reinterpret_cast<const float4*>(rowp + c));
                     } else {
                         float t4[4];
 #pragma unroll
-                        for (int e = 0; e < 4; e++) t4[e] = (c + e < total) ? __ldg(rowp + c + e) : CUDART_NAN_F;
+                        for (int e = 0; e < 4; e++) t4[e] = (c + e < total) ? __ldcg(rowp + c + e) : CUDART_NAN_F;
                         v[i] = make_float4(t4[0], t4[1], t4[2], t4[3]);
                     }
                 }
@@ -435,7 +437,7 @@ __global__ void __launch_bounds__(SS_THREADS) sort_select_kernel(const SortSelec
                     uint32_t payload;
                     bool live = true;
                     if (SRC == SRC_MATRIX) {
-                        key = p.key_sign * __ldg(p.keys + q * p.ld + c);
+                        key = p.key_sign * __ldcg(p.keys + q * p.ld + c);
                         payload = (uint32_t)(p.col0 + c);
                     } else if (SRC == SRC_PARTS) {
                         const int64_t off = q * p.ld + c;

@@ -69,6 +69,26 @@ def test_infinite_keys_are_no_results(fm, res, storage, metric, nb, k):
     idx.close()
 
 
+@pytest.mark.parametrize("storage", [0, 2])
+def test_rows_redone_over_several_column_chunks(fm, res, storage):
+    # 300 of 9,000 queries find one row 30,000 times, more than a candidate buffer holds; their key matrix has
+    # 2^30 / 4 / 9,000 columns a chunk, so five stores and selections follow one another
+    nb, nq, d, k = 120_000, 9_000, 24, 100
+    xb = H.gaussian(nb, d, 3)
+    xb[80_000:110_000] = xb[80_000]
+    xq = H.gaussian(nq, d, 5)
+    xq[::30] = xb[80_000] + np.float32(0.1) * H.gaussian(len(xq[::30]), d, 6)
+    idx = fm.B200IndexFlat(res, d, O.METRIC_L2, storage)
+    idx.add(xb)
+    for _ in range(3):
+        D, I = idx.search(xq, k)
+        # ||q||^2 + ||x||^2 - 2 q.x in 22 bits leaves 2^-22 (||q|| + ||x||)^2 of a distance: up to 1e-4 of the 0.24
+        # between such a query and its rows, within the 2e-4 of the comparison
+        pick = np.r_[0:1800:30, 8970, 1:30, nq - 3:nq]
+        H.check_against_oracle(O.METRIC_L2, storage, True, xb, xq[pick], k, D[pick], I[pick], loose=False)
+    idx.close()
+
+
 @pytest.mark.parametrize("how", ["search", "search_async"])
 @pytest.mark.parametrize("nb,tail,k", [(2000, 2000, 10), (2000, 8000, 32), (5000, 900, 3), (32_768, 14_000, 10)])
 def test_last_batch_that_needs_more_scratch(fm, res, how, nb, tail, k):
