@@ -242,6 +242,9 @@ int launch_matrix_select(const float* keys, int64_t nq, int64_t n, int64_t ld, i
 // out[q]: an upper bound, close to it, of the r-th smallest (r <= 512) of the n keys of row q; +INF when
 // there are too few.  NaN keys are skipped.  bad (optional): one more for every row with more than about
 // `most` keys up to its bound + margin * qnorm[q], or with qnorm[q] >= qnorm_max.
+// Threads it gives a row, and what `most` keys in random columns amount to among that many minima.
+int row_bound_threads(int64_t nq, int64_t n, int r);
+int row_bound_most(int64_t nq, int64_t n, int r, double most);
 int launch_row_bound(const float* keys, int64_t nq, int64_t n, int64_t ld, int r, float* out, int32_t* bad,
                      const float* qnorm, float margin, float qnorm_max, double most, cudaStream_t stream);
 bool rank_merge_fits(int P, int k);

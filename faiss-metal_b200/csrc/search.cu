@@ -143,28 +143,40 @@ static int64_t matrix_chunk_cols(int64_t nq, int64_t nb) {
     return cols;
 }
 
-// Sample of every stride-th row of a shard, from which a threshold for a query's k best is taken: the
-// sample holds on average e = k / stride of them, and its r-th best key, r = e + 4.5 sqrt(e) + 3, has
-// fewer than k rows of the shard under it only if the sample caught r of the k best (about one query in a
-// million).  About r * stride rows do lie under it; more than stride (r + 6 sqrt(r) + 12), what the
-// candidate buffers hold, for one query in 10^8.  Of about `target` rows, fewer where r would be beyond
-// 400.  buffers: more where that admits thousands of candidates beyond 2 k (lists spread what the
-// threshold admits over every warp of the GPU and keep the sample small: it has to fit the scratch of
-// the search without allocation at any shard size).  False: shard too small.
+// A threshold for a query's k best from a sample of one row (or column tile) in `stride`: the sample holds on
+// average e = k / stride of them, and its r-th best key, r = e + 4.5 sqrt(e) + 3, has fewer than k rows of the
+// shard under it only if the sample caught r of the k best (about one query in a million).
+int sample_rank(int k, int stride) {
+    const double e = (double)k / stride;
+    return (int)(e + 4.5 * std::sqrt(e) + 3.0 + 0.999);
+}
+
+// Candidates that threshold admits, and six deviations more: what a query's buffer holds.  row_bound does not
+// give the r-th best key but the r-th smallest of T thread minima, up to which the sample has R = T ln(T / (T - r))
+// keys on average (T >= 8 r up to r = 128: R <= 1.07 r; T = 1024 and r = 381: R = 477), their number and that of the
+// shard's rows per sampled one varying by T r / (T - r) together.  Simulated with r = 381, stride 8: 3,750 +- 180 of
+// 5,120 candidates; room for r + 6 sqrt(r) + 12 of the sample was exceeded by one query in forty, and one query redoes
+// all of a scan.
+int sample_capacity(int stride, int r) {
+    const double T = row_bound_threads(1ll << 40, 0, r);
+    const double R = T * std::log(T / (T - r)), var = T * r / (T - r);
+    return (int)round_up64((int64_t)(stride * (R + 6.0 * std::sqrt(var) + 12.0)), 256);
+}
+
+// The scans' sample: of about `target` rows, fewer where r would be beyond 400.  buffers: more where that
+// admits thousands of candidates beyond 2 k (lists spread what the threshold admits over every warp of the
+// GPU and keep the sample small: it has to fit the scratch of the search without allocation at any shard
+// size).  False: shard too small.
 bool choose_sample(int64_t nb, int k, int64_t target, bool buffers, int* stride_out, int* rank_out, int* cap_out) {
-    auto rank_of = [k](int stride) {
-        const double e = (double)k / stride;
-        return (int)(e + 4.5 * std::sqrt(e) + 3.0 + 0.999);
-    };
     int stride = 1;
     while (nb / (2 * stride) >= target) stride *= 2;
-    while (buffers && stride > 2 && (int64_t)rank_of(stride) * stride > 2 * (int64_t)k + 2048) stride /= 2;
-    while (rank_of(stride) > 400) stride *= 2;
-    const int r = rank_of(stride);
+    while (buffers && stride > 2 && (int64_t)sample_rank(k, stride) * stride > 2 * (int64_t)k + 2048) stride /= 2;
+    while (sample_rank(k, stride) > 400) stride *= 2;
+    const int r = sample_rank(k, stride);
     if (stride < 2 || nb / stride < 8 * (int64_t)r) return false;
     *stride_out = stride;
     *rank_out = r;
-    *cap_out = (int)round_up64((int64_t)(stride * (r + 6.0 * std::sqrt((double)r) + 12.0)), 256);
+    *cap_out = sample_capacity(stride, r);
     return true;
 }
 
@@ -222,14 +234,6 @@ bool make_plan(int64_t nq, int64_t nb, int d, int k, int storage, int path, bool
         pl.direct = true;
     }
     if (!pl.direct && !pairwise && pl.path == B200F_PATH_TENSOR && !filter_disabled()) {
-        // The pilot sample holds nb / stride rows and, on average, e = k / stride of a query's k
-        // best.  The threshold is the sample's r-th best key with r = e + 4.5 sqrt(e) + 3: fewer
-        // than k rows of the shard lie under it only if the sample caught r of the k best, which
-        // is about one row in a million; about r * stride rows do lie under it.
-        auto rank_of = [k](int stride) {
-            const double e = (double)k / stride;
-            return (int)(e + 4.5 * std::sqrt(e) + 3.0 + 0.999);
-        };
         const GemmPlan g0 = plan_gemm(nq, nb, sm);
         const int64_t n1 = nq > 0 ? nq : 1;
         // A list starts empty and takes every key of its first tile: ~0.1 ms per work item, and a small
@@ -240,6 +244,9 @@ bool make_plan(int64_t nq, int64_t nb, int d, int k, int storage, int path, bool
             return rank_select_enabled() && (k <= B200F_FUSED_MAX_K ? n1 * pcols * 4 <= PILOT_MATRIX_BYTES
                                                                     : pcols <= matrix_chunk_cols(nq, nb));
         };
+        auto can_halve = [&](int stride) {
+            return !filter_forced() && stride > 8 && as_matrix(stride / 2) && sample_rank(k, stride / 2) <= PILOT_MAX_RANK;
+        };
         int stride = k <= 128 ? 64 : 128;
         const bool matrix = as_matrix(stride);
         if (matrix) {
@@ -247,19 +254,20 @@ bool make_plan(int64_t nq, int64_t nb, int d, int k, int storage, int path, bool
             // well be larger: a closer threshold, fewer candidates (1,000 queries, 100,000 rows: one
             // row in 16 instead of 64, 128 candidates instead of 320).  Forced, the filter keeps its sparse
             // sample, which misjudges more rows.
-            while (!filter_forced() && stride > 8 && (k > SHORT_LIST || nb >= 65536) && ceil_div64(g0.ntiles, stride / 2) * g0.nqb <= g0.units && as_matrix(stride / 2) &&
-                   rank_of(stride / 2) <= PILOT_MAX_RANK)
+            while (can_halve(stride) && (k > SHORT_LIST || nb >= 65536) &&
+                   ceil_div64(g0.ntiles, stride / 2) * g0.nqb <= g0.units)
                 stride /= 2;
         }
         // rows of a sample worth having
-        auto least = [&](int stride) { return std::max<int64_t>(1024, 8 * (int64_t)rank_of(stride)); };
-        while (!filter_forced() && k > SHORT_LIST && matrix && stride > 8 && nb < stride * least(stride) && as_matrix(stride / 2) &&
-               rank_of(stride / 2) <= PILOT_MAX_RANK)
-            stride /= 2;
-        const int r = rank_of(stride);
-        const int64_t min_pairs = !matrix ? FILTER_MIN_PAIRS : k > SHORT_LIST ? FILTER_MIN_PAIRS_MATRIX : 16 * FILTER_MIN_PAIRS_MATRIX;
-        if ((r <= B200F_FUSED_MAX_K || matrix) && nb >= stride * least(stride) && (nq * nb >= min_pairs || filter_forced())) {
-            const int bound = (int)round_up64((int64_t)(stride * (r + 6.0 * std::sqrt((double)r) + 12.0)), 256);
+        auto least = [&](int stride) { return std::max<int64_t>(1024, 8 * (int64_t)sample_rank(k, stride)); };
+        while (matrix && can_halve(stride) && k > SHORT_LIST && nb < stride * least(stride)) stride /= 2;
+        const int r = sample_rank(k, stride);
+        const int64_t min_pairs = !matrix          ? FILTER_MIN_PAIRS
+                                  : k > SHORT_LIST ? FILTER_MIN_PAIRS_MATRIX
+                                                   : 16 * FILTER_MIN_PAIRS_MATRIX;
+        if ((r <= B200F_FUSED_MAX_K || matrix) && nb >= stride * least(stride) &&
+            (nq * nb >= min_pairs || filter_forced())) {
+            const int bound = sample_capacity(stride, r);
             int cap = 1024;
             while (cap < 4 * r * stride && cap < 8192) cap <<= 1;
             pl.filter = true;
@@ -721,18 +729,20 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
     const int qnc = l2 ? 1 : 0;
 
     // scans with k > 32: filter with keys that are bounds (see BoundFilter) where it pays
+    // what a query's sample may hold under its widened threshold: 0.7 of what its buffer takes.  Where even the
+    // threshold itself has more under it, no query could pass.
+    const double most = pl.sample ? 0.7 * pl.fcap / pl.fstride : 0.0;
     BoundFilter bf;
     if (pl.sample && !pl.fused && l2 && a->nq >= 2 && a->d <= BOUND_MAX_D &&
-        a->nb * a->row_pitch >= BOUND_MIN_ELEMS && scan_bound_filter_fits(*a)) {
+        a->nb * a->row_pitch >= BOUND_MIN_ELEMS && row_bound_most(a->nq, pl.nsample, pl.frank, most) >= pl.frank &&
+        scan_bound_filter_fits(*a)) {
         bf.eps = scan_bound_eps(a->storage);
         bf.qnorm = qnorm;
         if (a->storage == B200F_STORAGE_F16) bf.thr_abs = std::ldexp((float)a->d, -38);
         bf.bad = reinterpret_cast<const int32_t*>(scratch + pl.off_count) + 16;
     }
     int32_t* const bad = const_cast<int32_t*>(bf.bad);
-    // what a query's sample may hold under its widened threshold: 0.7 of what its buffer takes; the
-    // margin there is that of a row as long as the query.  fp16 queries: elements below 2^15.
-    const double most = pl.sample ? 0.7 * pl.fcap / pl.fstride : 0.0;
+    // the margin there is that of a row as long as the query.  fp16 queries: elements below 2^15.
     const float margin = 2.5f * bf.eps, qnorm_max = a->storage == B200F_STORAGE_F16 ? 1073741824.f : kHostInf;
 
     SearchInit init;

@@ -777,18 +777,28 @@ void set_output(RowSelectParams& p, int metric, const float* qnorm, int64_t labe
 
 }  // namespace
 
+int row_bound_threads(int64_t nq, int64_t n, int r) {
+    const int64_t sm = cached_sm_count();
+    int T = 128;
+    while (T < 1024 && (T < 8 * r || (nq < sm * 512 / T && T * 8 < n))) T <<= 1;
+    return T;
+}
+
+int row_bound_most(int64_t nq, int64_t n, int r, double most) {
+    const int T = row_bound_threads(nq, n, r);
+    return (int)(T * (1.0 - std::exp(-most / T)));
+}
+
 int launch_row_bound(const float* keys, int64_t nq, int64_t n, int64_t ld, int r, float* out, int32_t* bad,
                      const float* qnorm, float margin, float qnorm_max, double most, cudaStream_t stream) {
     if (r < 1 || r > 512 || n < 0 || ld < n || !keys || !out) return B200F_ERR_BAD_ARG;
     if (nq <= 0) return B200F_OK;
     const int64_t sm = cached_sm_count();
-    int T = 128;
-    while (T < 1024 && (T < 8 * r || (nq * T < sm * 512 && T * 8 < n))) T <<= 1;
+    const int T = row_bound_threads(nq, n, r);
     int64_t g = nq;
     const int64_t gcap = sm * (2048 / T);
     if (g > gcap) g = gcap;
-    // `most` keys in random columns are the minima of this many threads
-    const int most_minima = (int)(T * (1.0 - std::exp(-most / T)));
+    const int most_minima = row_bound_most(nq, n, r, most);
     row_bound_kernel<<<(int)g, T, 0, stream>>>(keys, ld, n, nq, r, out, bad, qnorm, margin, qnorm_max, most_minima);
     count_launch();
     B200F_LAUNCH_CHECK();

@@ -1,5 +1,7 @@
 """Streaming scans whose thresholds come from a sample of the rows: candidate buffers (k > 32) and lists
 cut at a threshold (k <= 32), at the row counts where they begin, on rows the sample misjudges and on ties."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -7,6 +9,19 @@ import helpers as H
 from oracle import flat_oracle as O
 
 pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+def redone(fm, stored, xq, metric, k, path=1):
+    """Queries whose result had to be found again without the sample's threshold (status word 1), and the result."""
+    q = torch.from_numpy(xq).to("cuda:0")
+    D = torch.empty((len(xq), k), dtype=torch.float32, device="cuda:0")
+    I = torch.empty((len(xq), k), dtype=torch.int64, device="cuda:0")
+    a = stored.args(fm, q, metric, k, path, D, I)
+    fm.abi.check_op(fm.lib().b200f_search(ctypes.byref(a)), "search")
+    torch.cuda.synchronize()
+    return int(stored.status[1]), D.cpu().numpy(), I.cpu().numpy()
 
 
 @pytest.mark.parametrize("storage,metric", [(0, O.METRIC_L2), (1, O.METRIC_INNER_PRODUCT), (2, O.METRIC_L2)])
@@ -47,3 +62,13 @@ def test_rows_the_sample_misjudges(fm, res, storage, nq, k):
         tensor = storage != 0 and k <= 32    # the streaming kernel rounds the query like the tensor path
         H.check_against_oracle(O.METRIC_L2, storage, tensor, xb, xq, k, D, I, loose=False)
         idx.close()
+
+
+@pytest.mark.parametrize("nb,k", [(66_000, 2400), (100_000, 2400), (100_000, 4096), (100_000, 100)])
+def test_candidate_buffers_hold_what_the_threshold_admits(fm, res, nb, k):
+    # independent rows: of 24 x 8 queries none may overflow (six deviations), whatever the rank of the threshold
+    from test_gpu_ops import Stored
+    d = 16
+    st = Stored(fm, H.gaussian(nb, d, 1), 2)
+    for seed in range(24):
+        assert redone(fm, st, H.gaussian(8, d, 100 + seed), O.METRIC_L2, k)[0] == 0
