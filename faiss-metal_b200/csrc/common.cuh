@@ -119,7 +119,7 @@ int launch_scan_topk(const B200FSearchArgs& a, const ScanPlan& plan, float* part
                      int32_t* part_idx, int* out_P, bool stream_f32, const float* thr, const int* guard,
                      cudaStream_t stream);
 // Scan that stores keys (smaller = better) to a matrix [nq][ld] for columns [col0, col0+ncols); with
-// stride > 1 column c is row (col0 + c) * stride of the shard.
+// stride > 1 column c is one of rows [(col0 + c) * stride, (col0 + c + 1) * stride) of the shard.
 int launch_scan_store(const B200FSearchArgs& a, int64_t col0, int64_t ncols, int64_t stride, float* out,
                       int64_t ld, int sm_count, const int* guard, cudaStream_t stream);
 // Scan that appends every row whose key is <= thr[q] to the query's candidate buffer

@@ -143,7 +143,7 @@ static int64_t matrix_chunk_cols(int64_t nq, int64_t nb) {
     return cols;
 }
 
-// A threshold for a query's k best from a sample of one row (or column tile) in `stride`: the sample holds on
+// A threshold for a query's k best from a sample of one row (tensor path: column tile) in `stride`: the sample holds on
 // average e = k / stride of them, and its r-th best key, r = e + 4.5 sqrt(e) + 3, has fewer than k rows of the
 // shard under it only if the sample caught r of the k best (about one query in a million).
 int sample_rank(int k, int stride) {

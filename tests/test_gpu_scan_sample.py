@@ -42,8 +42,7 @@ def test_candidates(fm, res, storage, metric, nb, nq, k):
 @pytest.mark.parametrize("storage", [0, 2])
 @pytest.mark.parametrize("nq,k", [(1, 24), (1, 100), (5, 32), (8, 100)])
 def test_rows_the_sample_misjudges(fm, res, storage, nq, k):
-    # every row the sample takes (row numbers that are multiples of its stride) is nearer to the first query
-    # than any other: its threshold admits far fewer than k rows; for the second query one row is repeated
+    # rows in groups of four and of 64 that begin with near ones, and, for the second query, one row repeated
     # 40,000 times, more than its candidate buffer holds.  Both must come out exactly.
     nb, d = 600_000, 16
     xb = H.gaussian(nb, d, 3)
@@ -72,3 +71,49 @@ def test_candidate_buffers_hold_what_the_threshold_admits(fm, res, nb, k):
     st = Stored(fm, H.gaussian(nb, d, 1), 2)
     for seed in range(24):
         assert redone(fm, st, H.gaussian(8, d, 100 + seed), O.METRIC_L2, k)[0] == 0
+
+
+def sampled_rows(nb, stride, pieces):
+    """The rows a scan takes its thresholds from: one in every `stride`, as in the scan kernel.  A row of `pieces` 16-byte
+    pieces belongs to up to eight lanes; eight columns of the sample share an offset."""
+    per_step = 32 // min(8, 1 << (pieces - 1).bit_length())
+    c = np.arange(nb // stride, dtype=np.uint64)
+    j = c // (8 * per_step) * per_step + c % per_step
+    return (c * stride + ((j * 2654435769 & 0xffffffff) * stride >> 32)).astype(np.int64)
+
+
+@pytest.mark.parametrize("storage", [0, 2])
+@pytest.mark.parametrize("nq,k", [(1, 24), (1, 100), (5, 32), (8, 100)])
+def test_sampled_rows_nearer_than_all_others(fm, res, storage, nq, k):
+    # 600,000 rows: the sample takes one in 64.  All it takes are nearer to the first query than any other row, so
+    # that its threshold admits the 7 to 11 rows of its rank and no more: redone, and exact
+    from test_gpu_ops import Stored
+    nb, d = 600_000, 16
+    xb = 6.0 + 0.1 * H.gaussian(nb, d, 3)
+    near = sampled_rows(nb, 64, d // (8 if storage else 4))
+    xb[near] = 3.0 + 0.1 * H.gaussian(len(near), d, 5)
+    xq = H.gaussian(nq, d, 6)
+    xq[0] = 2.5
+    count, D, I = redone(fm, Stored(fm, xb, storage), xq, O.METRIC_L2, k)
+    assert count == nq
+    tensor = storage != 0 and k <= 32    # the streaming kernel rounds the query like the tensor path
+    H.check_against_oracle(O.METRIC_L2, storage, tensor, xb, xq, k, D, I, loose=False)
+
+
+@pytest.mark.parametrize("storage", [0, 2])
+@pytest.mark.parametrize("period,k", [(8, 200), (16, 200), (64, 32), (64, 200)])
+@pytest.mark.parametrize("first", ["nearest", "farthest"])
+def test_rows_that_repeat_with_a_period(fm, res, storage, period, k, first):
+    # an original and its augmentations, one after the other: the sample sees all of them alike, nothing is redone
+    from test_gpu_ops import Stored
+    nb, d, nq = 600_000, 32, 4
+    xb = np.repeat(H.gaussian(nb // period, d, 7), period, axis=0)
+    noise = H.gaussian(nb, d, 8, scale=0.7)
+    own = np.arange(nb) % period == 0
+    noise[own if first == "nearest" else ~own] = 0
+    xb += noise
+    xq = H.gaussian(nq, d, 9)
+    count, D, I = redone(fm, Stored(fm, xb, storage), xq, O.METRIC_L2, k)
+    assert count == 0
+    tensor = storage != 0 and k <= 32
+    H.check_against_oracle(O.METRIC_L2, storage, tensor, xb, xq, k, D, I, loose=False)
