@@ -93,6 +93,7 @@ SIGNATURES = {
     "b200f_resources_stream": (c_vp, [c_vp]),
     "b200f_resources_wait_stream": (c_int, [c_vp, c_vp]),
     "b200f_resources_scratch_bytes": (c_sz, [c_vp]),
+    "b200f_resources_release_retained": (c_sz, [c_vp]),
     "b200f_index_create": (c_int, [c_vp, c_int, c_int, c_int, ctypes.POINTER(c_vp)]),
     "b200f_index_destroy": (None, [c_vp]),
     "b200f_index_add": (c_int, [c_vp, c_i64, c_vp]),

@@ -187,6 +187,7 @@ Registry& registry() {
 void retainStorage(const void* owner, std::unique_ptr<IndexArrays> arrays) {
     if (!arrays) return;
     const int device = arrays->device;
+    if (arrays->backedBytes() > kRetainBytes) return;   // unmapped here; others keep theirs
     std::vector<std::unique_ptr<IndexArrays>> drop;   // unmapped outside the lock
     {
         Registry& r = registry();

@@ -63,7 +63,9 @@ class GrowableDeviceArray {
 /// takes), and reset() is usually followed by add() on the same index.  At most kRetainBytes per
 /// device are kept, the oldest go first; an index takes its own storage back with take(), its
 /// destructor drops it, and every allocation of this library that runs out of memory calls
-/// trimRetainedStorage() and tries again.  All calls are safe from any thread: what is in the
+/// trimRetainedStorage() and tries again.  Other users of the device cannot: for them the program has
+/// StandardB200Resources::releaseRetainedStorage().  (Asking what the device has free, to keep less on a
+/// full one, costs 75 us a reset().)  All calls are safe from any thread: what is in the
 /// registry belongs to no stream (reset() has synchronised) and to no other owner.
 struct IndexArrays {
     GrowableDeviceArray rows, planes, norms;

@@ -214,10 +214,8 @@ struct B200IndexFlat::Impl {
 
     // keep: the mapped memory stays reachable for this index's next add() (see retainStorage)
     void freeStorage(bool keep = false) {
-        if (arrays) {
-            if (keep) retainStorage(this, std::move(arrays));
-            arrays.reset();
-        } else {
+        std::unique_ptr<IndexArrays> a = std::move(arrays);
+        if (!a) {
             if (rows) res->deallocBuffer(rows);
             if (planes) res->deallocBuffer(planes);
             if (norms) res->deallocBuffer(norms);
@@ -226,6 +224,7 @@ struct B200IndexFlat::Impl {
         planes = nullptr;
         norms = nullptr;
         capacity = 0;
+        if (keep) retainStorage(this, std::move(a));
     }
 
     // First allocation of an empty index: reserve the address ranges, or take back what reset()

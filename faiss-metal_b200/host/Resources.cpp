@@ -304,6 +304,11 @@ void StandardB200Resources::deallocBuffer(void* buf) {
     (void)cudaFree(buf);
 }
 
+size_t StandardB200Resources::releaseRetainedStorage() {
+    DeviceGuard g(impl_->device);
+    return trimRetainedStorage(impl_->device);
+}
+
 void* StandardB200Resources::acquireDeviceTemp(size_t size) {
     DeviceGuard g(impl_->device);
     const int device = impl_->device;

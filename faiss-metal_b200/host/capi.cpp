@@ -118,6 +118,15 @@ size_t b200f_resources_scratch_bytes(const B200FResources* res) {
     return res ? res->res->getScratchSize() : 0;
 }
 
+size_t b200f_resources_release_retained(B200FResources* res) {
+    if (!res) return 0;
+    try {
+        return res->res->releaseRetainedStorage();
+    } catch (...) {
+        return 0;
+    }
+}
+
 int b200f_index_create(B200FResources* res, int d, int metric, int storage, B200FIndex** out) {
     if (!out) return fail(B200F_ERR_BAD_ARG, "null output pointer");
     *out = nullptr;

@@ -61,6 +61,8 @@ class B200IndexFlat : public faiss::Index {
     void search(faiss::idx_t n, const float* x, faiss::idx_t k, float* distances,
                 faiss::idx_t* labels,
                 const faiss::SearchParameters* params = nullptr) const override;
+    /// Removes all rows.  The device memory behind them stays mapped for the next add() of this index, up to 8 GiB a
+    /// device, until the index is destroyed, an allocation of this library needs it or StandardB200Resources::releaseRetainedStorage() is called.
     void reset() override;
     void reconstruct(faiss::idx_t key, float* recons) const override;
 

@@ -34,6 +34,11 @@ class StandardB200Resources : public B200Resources {
     void releaseDeviceTemp(void* buf) override;
     void* acquirePinnedTemp(size_t size) override;
     void releasePinnedTemp(void* buf) override;
+    /// Gives back the device memory that reset() indexes keep for their next add() (B200IndexFlat::reset), of every
+    /// index on this device; returns its bytes.  Allocations of this library do so by themselves before they fail;
+    /// a program calls it before it needs the memory elsewhere.
+    size_t releaseRetainedStorage();
+
     /// Requests served from idle blocks / by a fresh allocation since construction.
     size_t tempPoolHits() const;
     size_t tempPoolMisses() const;

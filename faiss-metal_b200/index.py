@@ -75,6 +75,11 @@ class StandardB200Resources:
     def scratch_bytes(self) -> int:
         return abi.lib().b200f_resources_scratch_bytes(self._h)
 
+    def release_retained(self) -> int:
+        """Gives back the device memory that reset() indexes keep for their next add(), of every index on
+        this device; returns its bytes."""
+        return abi.lib().b200f_resources_release_retained(self._h)
+
     def wait_stream(self, producer_stream: int = 0):
         """Orders the resources' stream after everything queued so far on `producer_stream`
         (a cudaStream_t as an integer; 0 = the legacy default stream)."""
@@ -216,6 +221,8 @@ class B200IndexFlat:
         return SearchToken(t, (distances, labels))
 
     def reset(self):
+        """Removes all rows.  Their device memory stays mapped for the next add(), up to 8 GiB a device;
+        StandardB200Resources.release_retained() gives it back."""
         abi.check(abi.lib().b200f_index_reset(self._h), "reset")
 
     def reconstruct(self, key: int) -> np.ndarray:

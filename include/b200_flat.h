@@ -367,6 +367,9 @@ void* b200f_resources_stream(const B200FResources* res);
 int b200f_resources_wait_stream(B200FResources* res, void* producer_stream);
 /* bytes currently held by the grow-only scratch arena (src/MetalIndexFlat.mm:102-142) */
 size_t b200f_resources_scratch_bytes(const B200FResources* res);
+/* Gives back the device memory that reset indexes keep for their next add (b200f_index_reset), of
+ * every index on the resources' device; returns its bytes. */
+size_t b200f_resources_release_retained(B200FResources* res);
 
 /* MetalIndexFlat(resources, d, metric, storage) (src/MetalIndexFlat.mm:162-183). */
 int b200f_index_create(B200FResources* res, int d, int metric, int storage, B200FIndex** out);
@@ -395,7 +398,9 @@ int b200f_index_search_async(const B200FIndex* index, int64_t n, const float* x,
 int b200f_token_wait(B200FToken* token);
 int b200f_token_is_ready(const B200FToken* token, int* ready);
 void b200f_token_destroy(B200FToken* token);
-/* reset() (src/MetalIndexFlat.mm:492-506), reconstruct(key, out) (:508-527). */
+/* reset() (src/MetalIndexFlat.mm:492-506), reconstruct(key, out) (:508-527).  The device memory of a
+ * reset index stays mapped for its next add, up to 8 GiB a device, until the index is destroyed, an
+ * allocation of this library needs it or b200f_resources_release_retained() is called. */
 int b200f_index_reset(B200FIndex* index);
 int b200f_index_reconstruct(const B200FIndex* index, int64_t key, float* recons);
 /* Bulk form used by index_metal_to_cpu (src/MetalIndexFlat.mm:565-587):

@@ -76,6 +76,30 @@ def test_reset_gives_back_what_exceeds_the_bound(fm, res):
     idx.close()
 
 
+def test_what_reset_keeps_is_given_back(fm, res):
+    # 4.3 GB of an empty index, on request
+    idx = fm.B200IndexFlat(res, 768, O.METRIC_INNER_PRODUCT, 1)
+    res.release_retained()
+    torch.cuda.empty_cache()
+    free0 = torch.cuda.mem_get_info()[0]
+    xb = H.uniform_pm1(500, 768, 5)
+
+    def used():
+        return free0 - torch.cuda.mem_get_info()[0]
+
+    for _ in range(2):
+        idx.reserve(2_800_000)
+        idx.add(xb)
+        assert used() > 4 << 30
+        idx.reset()
+        assert used() > 4 << 30
+        assert res.release_retained() > 4 << 30
+        assert used() < 1 << 28 and res.release_retained() == 0
+    idx.add(xb)
+    assert np.array_equal(idx.reconstruct_n(0, 500), O.round_storage(xb, 1))
+    idx.close()
+
+
 @pytest.mark.parametrize("n", [8192, 30_000])
 def test_plane_scale_from_a_sample(fm, res, n):
     # one row 600 times larger than the others: over fp16's range at a scale made for them (2^7), while they
