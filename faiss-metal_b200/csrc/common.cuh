@@ -227,8 +227,8 @@ int launch_select_candidates(const float* cand_key, const int32_t* cand_idx, con
                              int cap, int64_t nb, int64_t nq, int k, int metric, const float* qnorm,
                              int64_t label_base, float* out_dist, int64_t* out_labels, int32_t* dirty,
                              const float* thr, const RedoRows& redo, cudaStream_t stream);
-// select_rank.cu: the same selection / merge for inputs of at most 8192 entries per row, sorted in
-// registers and placed by binary search; results identical to the kernels of select.cu.
+// select_rank.cu: the same selection from a row of any length (row_select: candidates, lists, a key matrix) and
+// the merge of up to 8192 / k shards' lists (rank_merge); results identical to the kernels of select.cu.
 bool rank_select_enabled();
 int launch_rank_select(const float* cand_key, const int32_t* cand_idx, const int32_t* cand_cnt, int cap,
                        int64_t nb, int64_t nq, int k, int metric, const float* qnorm, int64_t label_base,

@@ -2,21 +2,23 @@
 //
 // Replaces the encode sequence of MetalIndexFlat::search (src/MetalIndexFlat.mm:358-378)
 // and the path selection of MetalDistance / MetalSelect (src/MetalDistance.mm:107-128,
-// 327-363; src/MetalSelect.mm:34-89).  Paths here depend on (nq, k) only:
-//   nq <= 4 (8 on 16-bit rows)   streaming scan (scan.cu)
-//   more queries                 tensor-core GEMM (gemm_topk.cu)
-//   k  <= 32           top-k fused into the distance kernel, partial lists merged after
-//   k  <= 1024         (tensor path, shard of >= 64k / 128k rows) threshold filter: a pilot pass
-//                      over every 64th / 128th column tile gives each query a key threshold
-//                      that admits a few times k rows; the full pass appends every column under
-//                      the threshold to the query's candidate buffer (no lists, no matrix);
-//                      the k best candidates are selected.  A row whose buffer overflowed or
-//                      holds fewer than k candidates is redone by the paths below.
-//   32 < k <= 1024     (tensor path, enough column ranges) the fused kernel keeps 32 entries
-//                      per list, the k best of all lists are selected, and a row is redone
-//                      through the key matrix only when a full list could have dropped one of
-//                      its k results (rows counted and compacted on the device, no host sync)
-//   k   > 32 otherwise distance keys written per column chunk, running sort-select
+// 327-363; src/MetalSelect.mm:34-89).  make_plan chooses by the numbers of queries and rows, k and
+// storage; each rule's reason stands at its constants:
+//   nq <= 8 (4 on small or wide fp32 shards)   streaming scan (scan.cu)
+//     k <= 32          lists fused into the scan, on larger shards started from thresholds that a sample of
+//                      the rows gives (choose_sample), merged by row_select
+//     k  > 32          from 32 Ki rows: the rows under such a threshold go to candidate buffers (on large L2
+//                      shards found by keys that are bounds, and scored again), row_select takes the k
+//                      best; below: keys of all rows, selected from
+//   more queries                               tensor-core GEMM (gemm_topk.cu)
+//     few pairs        (direct) the keys of all rows as one matrix, row_select
+//     else             (filter) a pilot pass over one column tile in 8 to 128 gives each query a threshold; the
+//                      full pass appends every column under it to the query's candidate buffer, row_select
+//     else k <= 32     top-k lists fused into the distance kernel, merged
+//     else k <= 1024   (lists) the fused kernel's 32-entry lists, the k best of all of them
+//     else             keys per column chunk, running sort_select
+// Thresholds and short lists are optimistic: a query whose buffer overflowed, or that found fewer than k rows, is
+// redone by the last rule that fits it, counted and gathered on the device, no host synchronisation.
 #include <algorithm>
 #include <atomic>
 #include <cstdio>

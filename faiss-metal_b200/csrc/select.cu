@@ -5,7 +5,7 @@
 // final list merge inside the fused kernels (shaders/fused_l2_topk.metal:88-131).
 //
 // Building blocks:
-//  * merge_small: k <= 32.  One CTA per query; each warp folds a subset of sorted input
+//  * merge_small: k <= 32 (lists of other ranks, list pilots).  One CTA per query; each warp folds a subset of sorted input
 //    lists into a sorted warp list (lane j = rank j) by ballot + shuffle insertion with
 //    early exit, then warp 0 folds the warp lists.
 //  * sort_select: any k <= 4096.  One CTA per query streams candidates, keeps those under

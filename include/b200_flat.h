@@ -91,7 +91,9 @@ const char* b200f_status_string(int status);
  * Until the setter is called the default comes from the environment variable
  * B200F_SELECT_MODE (auto | filter | no_filter | matrix), which is read once, at the first
  * search; nothing else in the search path reads the environment. */
-#define B200F_SELECT_AUTO 0       /* threshold filter from 2^27 (query, row) pairs (2^22 where the pilot sample fits a key matrix), 32-entry lists below */
+#define B200F_SELECT_AUTO 0       /* by size: key matrix of all rows (k > 2, up to 32,768 rows and 2^24 (query, row) pairs), threshold filter
+                                    (from 2^18 pairs, 2^22 for k <= 2, where the pilot sample fits a key matrix, else
+                                    from 2^27), 32-entry lists otherwise */
 #define B200F_SELECT_FILTER 1     /* threshold filter wherever the shard allows a pilot sample */
 #define B200F_SELECT_NO_FILTER 2  /* never the threshold filter                                */
 #define B200F_SELECT_MATRIX 3     /* neither filter nor lists: fused lists (k <= 32), key matrix beyond */
@@ -103,13 +105,13 @@ int b200f_get_selection_mode(void);
 #define B200F_GEMM_SHAPE_SINGLE 0
 #define B200F_GEMM_SHAPE_PAIR 1
 int b200f_set_gemm_shape(int shape);
-/* Selection of more than 32 results from at most 8192 entries per row (a row's threshold-filtered
- * candidates; the sorted lists of up to 8192 / k shards): with on != 0 (the default) the kernels
- * that sort in registers and place every entry by binary search, else the shared-memory sorting
- * kernel that also serves larger inputs.  The same switch decides how the threshold filter takes
- * its pilot sample: on, as a key matrix picked over by a selection kernel wherever it fits (and the
- * filter is then used from 2^22 pairs); off, always as 32-entry lists.  Results are identical
- * either way; a testing aid.  No counterpart in the reference (its block_select,
+/* Selection from a row's threshold-filtered candidates or its key matrix (up to 2^19 columns), and the
+ * merge of more than 32 results from the sorted lists of up to 8192 / k shards: with on != 0 (the
+ * default) the kernels that bound the k-th key first and place every entry by its rank, else the
+ * shared-memory sorting kernel that also serves larger inputs.  The same switch decides how the
+ * threshold filter takes its pilot sample: on, as a key matrix wherever it fits; off, always as
+ * 32-entry lists, and neither the key matrix of small searches nor the scans' candidate buffers are
+ * used.  Results are identical either way; a testing aid.  No counterpart in the reference (its block_select,
  * shaders/block_select.metal:111-274, is the one kernel). */
 int b200f_set_rank_select(int on);
 /* Debug canaries, the stand-in for a memory checker on the scratch arena: with on != 0 every
