@@ -289,10 +289,11 @@ store_rows_kernel(const float* __restrict__ src, int64_t src_pitch, int64_t n, i
             amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
         }
         if (!live || cl != 0) continue;
-        if (range_flag && planes && plane_format == kPlanesFp16x2 &&
-            (amax >= 32768.f || (amax > 0.f && amax < 0.0625f) ||
-             (norm_cols && 0.5f * s * plane_scale * plane_scale > kNormPiecesMax)))
-            atomicOr(range_flag, 1);
+        if (range_flag && planes && plane_format == kPlanesFp16x2) {
+            if (amax > 0.f && amax < 0.0625f) atomicOr(range_flag, 3);
+            else if (amax >= 32768.f || (norm_cols && 0.5f * s * plane_scale * plane_scale > kNormPiecesMax))
+                atomicOr(range_flag, 1);
+        }
         if (norms) norms[r] = s;
         if (norm_cols) {
             uint16_t pc[8];

@@ -593,8 +593,9 @@ void B200IndexFlat::add(faiss::idx_t n, const float* x) {
     ntotal = newTotal;
     impl_->mirrorValid = false;
     auto flagged = [&] { return fp32 && impl_->planeFormat == B200F_PLANES_FP16X2 && impl_->hostStatus[9] != 0; };
-    if (flagged() && scaleFromSample) {
-        // the sample missed the largest rows: the scale of all of them, if there is one
+    if (flagged() && scaleFromSample && impl_->hostStatus[9] == 1) {
+        // the sample missed the largest rows: the scale of all of them, if there is one (it can only be smaller, so
+        // not where a row is too small already)
         cudaCheck(cudaMemsetAsync(impl_->rangeFlag(), 0, 4, st), "add: clear range flag");
         (void)setPlaneScale(static_cast<const float*>(impl_->rows), ntotal, impl_->pitch);
         resplit(ntotal);

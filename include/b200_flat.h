@@ -178,7 +178,8 @@ int b200f_store_rows(const float* src, int64_t n, int d, int storage, void* dst_
 /* The same for FP32 storage with a choice of plane format (B200F_PLANES_*) and, for FP16X2, the
  * index's scale 2^plane_scale_log2.  src rows are src_pitch elements apart; src == dst_rows
  * (with src_pitch == dst_pitch) re-splits rows that are stored already.  range_flag (device
- * int32, may be NULL): bit 1 is OR-ed in when a row does not fit the FP16X2 format. */
+ * int32, may be NULL): 1 is OR-ed in when a row does not fit the FP16X2 format, 3 when it is too small
+ * for it (a smaller scale, made for larger rows, would not help). */
 int b200f_store_rows_fp32(const float* src, int64_t src_pitch, int64_t n, int d, float* dst_rows,
                           int64_t dst_pitch, uint16_t* planes, int64_t plane_pitch, int64_t plane_stride,
                           int plane_format, int plane_scale_log2, int32_t* range_flag, float* norms_or_null,

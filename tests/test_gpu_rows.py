@@ -116,6 +116,22 @@ def test_plane_scale_from_a_sample(fm, res, n):
     idx.close()
 
 
+@pytest.mark.parametrize("row", [2, 20_000])
+def test_a_row_far_shorter_than_the_others(fm, res, row):
+    # below 2^-4 at any scale that fits the others (sampled or not): three bf16 planes
+    n, d = 30_000, 48
+    xb = H.uniform_pm1(n, d, 13)
+    xb[row] *= np.float32(2.0 ** -12)
+    xb[row + 2] *= np.float32(600.0)
+    idx = fm.B200IndexFlat(res, d, O.METRIC_INNER_PRODUCT, 0)
+    idx.add(xb)
+    assert idx.fp32_planes == fm.abi.PLANES_BF16X3
+    xq = H.uniform_pm1(40, d, 12)
+    D, I = idx.search(xq, 10)
+    H.check_against_oracle(O.METRIC_INNER_PRODUCT, 0, True, xb, xq, 10, D, I)
+    idx.close()
+
+
 @pytest.mark.parametrize("where", ["device", "host", "second_add"])
 @pytest.mark.parametrize("d", [48, 128, 1536])
 @pytest.mark.parametrize("factor", [20, 50, 100, 250])
