@@ -141,16 +141,15 @@ __device__ __forceinline__ void norm_pieces(float v, int storage, uint16_t (&out
 }
 
 // ---- append-time conversion -----------------------------------------------------------
-// One warp per row.  Writes the stored row (pad columns zeroed), the squared norm of
-// the stored values, for fp32 storage the three bf16 split planes, and (norm_cols) the
+// Writes the stored row (pad columns zeroed), the squared norm of
+// the stored values, for fp32 storage the split planes, and (norm_cols) the
 // 8 norm columns after the d8 = round_up(d, 8) data columns of the 16-bit row / plane 0.
 // FP32 storage keeps, beside the fp32 rows, split planes for the tensor path, in one of two formats:
 //   kPlanesBf16x3  x = b0 + b1 + b2, three bf16 planes (24 bits, fp32's exponent range): six plane
 //                  products reproduce the fp32 product to 2^-24
 //   kPlanesFp16x2  x * s = h0 + h1, two fp16 planes (22 bits) of the row scaled by a power of two s
 //                  chosen for the index (largest element of a sample of its first rows near 2^6): three
-//                  plane products, half
-//                  the tensor work and two thirds of the plane bytes.  fp16 has a narrow exponent
+//                  plane products, half the tensor work and two thirds of the plane bytes.  fp16 has a narrow exponent
 //                  range, so the format only holds while every stored row fits it.  `range_flag` is
 //                  raised, and the index takes another scale or re-splits itself into bf16x3, by
 //                    an element at or beyond 2^15 after scaling;

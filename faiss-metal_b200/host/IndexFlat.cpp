@@ -165,7 +165,7 @@ struct B200IndexFlat::Impl {
 
     // FP32 storage: format of the split planes (B200F_PLANES_*).  An index starts with two fp16
     // planes (half the tensor work of three bf16 planes) unless told otherwise, takes its
-    // power-of-two scale from the first rows it sees, and re-splits itself into three bf16 planes
+    // power-of-two scale from a sample of its first rows, and re-splits itself into three bf16 planes
     // the moment a row does not fit fp16's range (the conversion kernel raises a flag).
     int planeFormat = B200F_PLANES_FP16X2;
     int planeFormatWanted = B200F_PLANES_FP16X2;

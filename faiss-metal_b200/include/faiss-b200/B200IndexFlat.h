@@ -91,7 +91,7 @@ class B200IndexFlat : public faiss::Index {
     void setGrowthMode(int mode);
     /// FP32 storage only: which split planes the tensor path multiplies (B200F_PLANES_BF16X3: three
     /// bf16 planes, six products; B200F_PLANES_FP16X2: two fp16 planes of the rows scaled by a power of
-    /// two the index picks from its first rows, three products).  The default is FP16X2; an index
+    /// two the index picks from a sample of its first rows, three products).  The default is FP16X2; an index
     /// whose rows stop fitting fp16's range re-splits itself into BF16X3 during that add().  Both
     /// hold the 1e-4 contract.  Only on an empty index.
     void setFp32PlaneFormat(int format);
@@ -108,7 +108,7 @@ class B200IndexFlat : public faiss::Index {
     /// The resources this index was built on.
     std::shared_ptr<B200Resources> getResources() const;
     /// Enqueue a search whose queries and outputs are all DEVICE pointers on the resources'
-    /// stream and return without synchronising (single batch: n <= 16384 for k <= 32,
+    /// stream and return without synchronising (single batch: n <= 16384 for k <= 1024,
     /// n <= 1024 otherwise).  The multi-GPU layer chains the candidate exchange and the merge
     /// behind it on the same stream; call synchronize() before reading results on the host.
     /// `scratch` (device, searchScratchBytes(n, k) bytes): used instead of the resources' shared

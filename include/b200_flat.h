@@ -387,7 +387,7 @@ int b200f_index_search(const B200FIndex* index, int64_t n, const float* x, int64
 /* Device-only, enqueue-only form of search: x / distances / labels are DEVICE pointers, the
  * work is queued on the resources' stream (b200f_resources_stream) and the call returns
  * without synchronising, so a caller can chain its own work (the multi-GPU exchange and
- * merge) on that stream.  One launch batch only (n <= 16384 for k <= 32, else n <= 1024).
+ * merge) on that stream.  One launch batch only (n <= 16384 for k <= 1024, else n <= 1024).
  * b200f_index_synchronize waits for the stream and reports a device-side error, if any.
  * The reference's closest relative is the encode-without-wait half of searchAsync
  * (src/MetalIndexFlat.mm:478-486). */
