@@ -42,29 +42,20 @@
 // Every wait on an mbarrier is bounded: after ~1 s of clock the waiting thread
 // records kDevErrBarrierWait in the status word, raises the CTA abort flag and
 // all roles drain out, TMEM is released and the kernel returns.
-#include <cuda.h>
-
 #include <atomic>
 #include <cstdlib>
 #include <type_traits>
 
-#include "common.cuh"
-#include "ptx.cuh"
+#include "gemm_common.cuh"
 
 namespace b200f {
 
 namespace {
 
-constexpr int BM = 128;
-constexpr int BN = 256;
-constexpr int BK = 64;  // 16-bit elements: 128 bytes = one swizzle row
-constexpr int UMMA_K = 16;
 constexpr int A_STAGE_BYTES = BM * BK * 2;  // 16 KiB
 constexpr int KMAX = B200F_FUSED_MAX_K;
-constexpr int NUM_EPI_WARPS = 8;   // two per TMEM lane quarter: each takes half of the tile's columns
 constexpr int MMA2_WARP = 2 + NUM_EPI_WARPS;   // second MMA issuer (pair shape): one thread per accumulator chain
 constexpr int NUM_THREADS = 32 * (3 + NUM_EPI_WARPS);
-constexpr int TMEM_COLS = 512;
 
 // Two shapes of the same kernel:
 //  PAIR = false  one CTA per tile: M = 128 queries, N = 256 rows of X, cta_group::1
@@ -100,208 +91,6 @@ struct Cfg {
     static constexpr int SMEM_BYTES = SM_ABORT + 4 + 8;
 };
 
-enum { MODE_TOPK = 0, MODE_STORE = 1, MODE_FILTER = 2 };
-
-struct GemmParams {
-    int64_t nq;
-    int64_t col0;        // first global column (row of X) of this launch
-    int64_t ncols_end;   // one past the last valid global column of this launch
-    int64_t ntiles;      // column tiles in this launch
-    int64_t tiles_per_range;
-    int nqb;
-    int P;
-    // single CTA: rows of a query box, the live ones rounded up to 8.  Rows beyond the queries are never
-    // fetched: zero-filling 104 of 128 rows held the ring back to one k-block per 1,900 cycles whatever
-    // it cost to read X (24 queries, 1,000,003 fp16 rows of d = 770: 354 us a launch, 242 without).  What the
-    // tile holds there instead reaches only accumulator rows that nobody reads.
-    int a_rows;
-    // k-blocks of 64 and valid K elements (multiple of 8) of a plane product.  The norm columns are zero in
-    // every plane but the first, so only the last product, of the two first planes, takes them (d = 128,
-    // three products: 25 MMAs a tile instead of 27, 7 k-blocks instead of 9).
-    int kb_per_pass, kb_last_pass;
-    int k_extent, k_extent_last;
-    int npass;
-    uint32_t pass_a;     // 4 bits per pass: plane index of A
-    uint32_t pass_b;
-    uint32_t idesc;
-    int mode;
-    int k;
-    float kscale;        // key = -kscale * t  (2 for L2, 1 for inner product)
-    // optional per-row factor on kscale (operands scaled per query row: fp16x2 planes); row j of
-    // this launch is row rowscale_map[j] of the array when the map is set (redone rows)
-    const float* rowscale;
-    const int32_t* rowscale_map;
-    float sign;
-    const float* rowadd; // per query row, may be null (0)
-    float* part_key;
-    int32_t* part_idx;
-    uint32_t* gthr;      // [nq][gslots] ordered-float 32nd-best keys published by the lists of a row
-    int gslots;          // lists publish to slot (list number % gslots); the row's bound is the
-                         // largest slot: gslots full lists hold 32 * gslots distinct candidates
-    const int* nq_dev;   // when set: the number of live query rows is read from device memory
-    int64_t tile_stride; // tile t of the launch is tile t * tile_stride of X (sampling passes)
-    // MODE_FILTER: every column whose key is <= the row's threshold is appended to the row's
-    // candidate buffer (position from an atomic counter; entries past cand_cap are only counted)
-    const float* fthr;   // threshold of row q in scaled key units: fthr[q * fthr_stride + fthr_pos]
-    int fthr_stride, fthr_pos;
-    float* cand_key;     // [nq][cand_cap]
-    int32_t* cand_idx;
-    int32_t* cand_cnt;   // [nq]
-    int cand_cap;
-    int wide;            // MODE_FILTER: 64 columns per TMEM load (few hits expected), else 32
-    float* out;
-    int64_t ld;
-    int32_t* status;
-};
-
-// ---- PTX wrappers (mbarrier and bounded-wait helpers come from ptx.cuh) -----------------
-
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                          int32_t* status) {
-    return mbar_wait_bounded(bar, parity, abort_flag, status, kDevErrBarrierWait);
-}
-
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar,
-                                            int c0, int c1, int c2) {
-    asm volatile(
-            "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-            " [%0], [%1, {%3, %4, %5}], [%2];"
-            ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
-            : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() {
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_after() {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-
-// shared::cluster address of `addr` (a shared::cta address of this CTA) in CTA `rank`
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-// arrive on an mbarrier given by a shared::cluster address (own or peer CTA)
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-
-// TMA load issued inside a CTA pair: the mbarrier may live in the peer CTA
-__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar,
-                                                 int c0, int c1, int c2) {
-    asm volatile(
-            "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-            " [%0], [%1, {%3, %4, %5}], [%2];"
-            ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
-            : "memory");
-}
-
-__device__ __forceinline__ void tc_commit_pair(uint32_t cluster_bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_bar)
-                 : "memory");
-}
-
-__device__ __forceinline__ void tc_mma_f16_pair(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b,
-                                                uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-            "{\n\t"
-            ".reg .pred p;\n\t"
-            "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
-            "}\n" ::"r"(d_tmem),
-            "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-            : "memory");
-}
-
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-                 : "memory");
-}
-
-__device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b,
-                                           uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-            "{\n\t"
-            ".reg .pred p;\n\t"
-            "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-            "}\n" ::"r"(d_tmem),
-            "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-            : "memory");
-}
-
-// 32 lanes x 32 consecutive fp32 columns -> 32 registers per thread
-__device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-            "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-              "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
-              "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
-              "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-              "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]),
-              "=r"(r[31])
-            : "r"(taddr)
-            : "memory");
-}
-// 32 lanes x 64 consecutive fp32 columns -> 64 registers per thread
-__device__ __forceinline__ void tc_ld64(uint32_t taddr, uint32_t (&r)[64]) {
-    asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x64.b32 "
-            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-            "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, "
-            "%32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, "
-            "%48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%64];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-              "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
-              "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
-              "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-              "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]),
-              "=r"(r[31]), "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]),
-              "=r"(r[37]), "=r"(r[38]), "=r"(r[39]), "=r"(r[40]), "=r"(r[41]), "=r"(r[42]),
-              "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47]), "=r"(r[48]),
-              "=r"(r[49]), "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]),
-              "=r"(r[55]), "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]), "=r"(r[60]),
-              "=r"(r[61]), "=r"(r[62]), "=r"(r[63])
-            : "r"(taddr)
-            : "memory");
-}
-// one 32-byte sector of a row
-__device__ __forceinline__ void st_global_v8(float* dst, const float (&v)[8]) {
-    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "f"(v[0]), "f"(v[1]), "f"(v[2]),
-                 "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
-                 : "memory");
-}
-__device__ __forceinline__ void tc_wait_ld() {
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// K-major operand tile, 128-byte swizzle: rows of 128 bytes, 8-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {
-    uint64_t desc = 0;
-    desc |= (uint64_t)((saddr & 0x3FFFFu) >> 4);  // start address
-    desc |= (uint64_t)1 << 16;                    // leading byte offset (unused with swizzle)
-    desc |= (uint64_t)(1024 >> 4) << 32;          // stride byte offset between 8-row groups
-    desc |= (uint64_t)1 << 46;                    // descriptor version (sm_100)
-    desc |= (uint64_t)2 << 61;                    // SWIZZLE_128B
-    return desc;
-}
-
 // Per-row candidate list held in REGISTERS by the thread that owns the row: 32 (key, id)
 // pairs sorted ascending by key, every index static so nothing spills.  Inserting s drops
 // the largest element: slot j takes the old slot j-1 if that is greater than s, keeps its
@@ -325,14 +114,6 @@ __device__ __forceinline__ void reglist_insert(float (&lk)[KMAX], int32_t (&li)[
     }
 }
 
-// Hits of the tile in flight are staged per thread in shared memory (entry i of a thread at
-// [i * STAGE_LD]: raw key s = -t and column) and worked off AFTER the accumulator has been handed
-// back to the MMA issuers, so that list insertion and buffer appends run beside the next
-// tile's MMAs instead of in front of them.  Only a thread whose stage fills up inside one
-// tile (list warm-up, massive ties) drains it on the spot.
-constexpr int STAGE_N = 16;
-constexpr int STAGE_LD = 32 * NUM_EPI_WARPS;
-
 __device__ __forceinline__ void drain_to_list(float (&lk)[KMAX], int32_t (&li)[KMAX], const float* sk,
                                               const int32_t* si, int n, float& thr, float& thr_eff) {
     for (int i = 0; i < n; i++) {
@@ -341,20 +122,6 @@ __device__ __forceinline__ void drain_to_list(float (&lk)[KMAX], int32_t (&li)[K
             reglist_insert(lk, li, sc, si[i * STAGE_LD]);
             thr = lk[KMAX - 1];
             thr_eff = fminf(thr_eff, thr);
-        }
-    }
-}
-
-// MODE_FILTER: one atomic takes n slots of the row's candidate buffer; the counter also counts
-// entries that no longer fit.
-__device__ __forceinline__ void drain_to_buffer(int32_t* cnt, float* ck, int32_t* ci, int cap,
-                                                float kscale, const float* sk, const int32_t* si, int n) {
-    if (n <= 0) return;
-    const int base = atomicAdd(cnt, n);
-    for (int i = 0; i < n; i++) {
-        if (base + i < cap) {
-            ck[base + i] = kscale * sk[i * STAGE_LD];
-            ci[base + i] = si[i * STAGE_LD];
         }
     }
 }
@@ -635,14 +402,7 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
                     li[j] = -1;
                 }
             } else if (MODE == MODE_FILTER) {
-                // keys <= threshold pass: the filter below is exclusive, so take the next float up
-                // (+INF, the threshold of a row whose sample was too small, stays; -INF passes nothing)
-                thr_eff = -CUDART_INF_F;
-                if (row_live) {
-                    const float t = p.fthr[grow * p.fthr_stride + p.fthr_pos] / ksc;
-                    const uint32_t o = float_to_ordered(t);
-                    thr_eff = (o >= 0xff800000u) ? t : ordered_to_float(o + 1u);
-                }
+                thr_eff = row_live ? filter_threshold(p.fthr[grow * p.fthr_stride + p.fthr_pos] / ksc) : -CUDART_INF_F;   // -INF passes nothing
             } else if (row_live && p.rowadd) {
                 radd = p.rowadd[grow];
             }
@@ -763,40 +523,9 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
                     tc_ld32(taddr + ch * 32, r);
                     tc_wait_ld();
                     const int64_t cbase = c_tile + ch * 32;
-                    if (whole) {
-                        // 32 consecutive columns of the thread's row: four whole sectors
-                        if (row_live) {
-                            float* o = p.out + grow * p.ld + (t * TILE_N + ch * 32);
-#pragma unroll
-                            for (int c = 0; c < 32; c += 8) {
-                                float v[8];
-#pragma unroll
-                                for (int e = 0; e < 8; e++) v[e] = fmaf(p.sign, -ksc * __uint_as_float(r[c + e]), radd);
-                                st_global_v8(o + c, v);
-                            }
-                        }
-                    } else {
-                        // Ragged or unaligned output: thread t holds 32 consecutive columns of ITS row; writing
-                        // them directly would touch 32 different rows per instruction.  The warp
-                        // transposes the 32 x 32 block through shared memory (the list area is
-                        // idle in this mode) and writes one 128-byte row segment per instruction.
-                        float* tbuf = reinterpret_cast<float*>(smem + SM_LKEY) + (warp - 2) * (32 * 33);
-#pragma unroll
-                        for (int c = 0; c < 32; c++) {
-                            const float key = -ksc * __uint_as_float(r[c]);
-                            tbuf[lane * 33 + c] = fmaf(p.sign, key, radd);
-                        }
-                        __syncwarp();
-                        const int64_t grow0 = grow - lane;  // first row of this warp's 32 rows
-                        const bool col_ok = cbase + lane < p.ncols_end;
-                        float* obase = p.out + (t * TILE_N + ch * 32) + lane;   // tiles lie side by side, whatever the stride
-#pragma unroll 8
-                        for (int rr = 0; rr < 32; rr++) {
-                            const float v = tbuf[rr * 33 + lane];
-                            if (col_ok && grow0 + rr < nq_live) obase[(grow0 + rr) * p.ld] = v;
-                        }
-                        __syncwarp();
-                    }
+                    // tiles lie side by side in the output, whatever the stride; the list area is idle in this mode
+                    store_keys(p, r, whole, grow, lane, nq_live, row_live, cbase, t * TILE_N + ch * 32, ksc, radd,
+                               reinterpret_cast<float*>(smem + SM_LKEY) + (warp - 2) * (32 * 33));
                 }
                 }
                 tc_fence_before();
@@ -856,48 +585,6 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
 }
 
 // ---- host side -------------------------------------------------------------------------
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
-                                  const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn get_encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
-        void* ptr = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) ==
-                    cudaSuccess &&
-            qres == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(ptr);
-        else
-            (void)cudaGetLastError();
-    }
-    return fn;
-}
-
-// 3-D map {k, row, plane} over a [planes][rows][pitch] 16-bit array; box {64, box_rows, 1}.
-int make_operand_map(CUtensorMap* map, const uint16_t* base, int is_bf16, int64_t k_extent,
-                     int64_t rows, int64_t pitch, int planes, int64_t plane_stride, int box_rows) {
-    EncodeTiledFn fn = get_encode_fn();
-    if (!fn) return B200F_ERR_CUDA;
-    if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || (pitch % 8) != 0 ||
-        (planes > 1 && (plane_stride % 8) != 0))
-        return B200F_ERR_BAD_ARG;
-    cuuint64_t dims[3] = {(cuuint64_t)k_extent, (cuuint64_t)rows, (cuuint64_t)planes};
-    cuuint64_t pstride = (planes > 1) ? (cuuint64_t)plane_stride * 2 : (cuuint64_t)pitch * 2 * (cuuint64_t)(rows > 0 ? rows : 1);
-    cuuint64_t strides[2] = {(cuuint64_t)pitch * 2, pstride};
-    cuuint32_t box[3] = {(cuuint32_t)BK, (cuuint32_t)box_rows, 1};
-    cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = fn(map, is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
-                    3, const_cast<uint16_t*>(base), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? B200F_OK : B200F_ERR_CUDA;
-}
 
 int launch_common(const GemmOperands& op, const GemmPlan& plan, GemmParams& p, int64_t col0,
                   int64_t ncols, cudaStream_t stream) {
@@ -966,6 +653,13 @@ int launch_common(const GemmOperands& op, const GemmPlan& plan, GemmParams& p, i
     if (p.mode < 0 || p.mode > 2) return B200F_ERR_BAD_ARG;
     const KernelFn kernel = kernels[plan.pair ? 1 : 0][p.mode];
     main_kernel_begin(stream);
+    if (p.mode != MODE_TOPK && resident_fits(op, plan)) {
+        rc = launch_resident(op, plan, p, ma, mb, stream);
+        main_kernel_end(stream);
+        if (rc != B200F_OK) return rc;
+        count_launch();
+        return B200F_OK;
+    }
     if (plan.pair || op.overlap) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)plan.grid, 1, 1);

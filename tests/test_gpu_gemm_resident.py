@@ -1,0 +1,62 @@
+"""The distance GEMM that keeps the query block in shared memory (more than 128 queries, narrow rows): edges of its
+k-blocks (64 columns, norm columns in a block of their own), of its tiles (256 rows of X, halves of 512) and of
+its query blocks, the widths where the general kernel takes over, and ranges that change their query block."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+import helpers as H
+from oracle import flat_oracle as O
+from test_gpu_ops import Stored, cur_stream, vp
+
+pytestmark = pytest.mark.gpu
+
+# fp32 rows: two planes of up to three blocks, 16-bit rows: up to six; L2 adds eight norm columns
+WIDTHS = {0: (8, 56, 64, 65, 128, 184, 185, 192, 193), 1: (63, 128, 376, 384, 385), 2: (16, 64, 320, 376, 377)}
+
+
+@pytest.mark.parametrize("storage,d", [(s, d) for s, ds in WIDTHS.items() for d in ds])
+@pytest.mark.parametrize("metric", [O.METRIC_L2, O.METRIC_INNER_PRODUCT])
+@pytest.mark.parametrize("nq,nb", [(129, 1), (256, 256), (257, 769), (600, 40_001)])
+def test_matrix(fm, res, storage, metric, d, nq, nb):
+    xb = H.uniform_pm1(nb, d, 99)
+    xq = H.uniform_pm1(nq, d, 77)
+    st = Stored(fm, xb, storage)
+    xq_dev = torch.from_numpy(xq).cuda()
+    out = torch.full((nq, nb), float("nan"), dtype=torch.float32, device="cuda:0")
+    a = st.args(fm, xq_dev, metric, 1, 2)
+    if storage == 0:   # two fp16 planes of 2^6 x
+        fm.abi.check_op(fm.lib().b200f_store_rows_fp32(vp(st.rows), st.pitch, nb, d, vp(st.rows), st.pitch, vp(st.planes),
+                                                       st.ppitch, nb * st.ppitch, 1, 6, None, None, 1, cur_stream()), "planes")
+        a.plane_format, a.plane_scale_log2 = 1, 6
+    fm.abi.check_op(fm.lib().b200f_pairwise(ctypes.byref(a), vp(out), nb), "pairwise")
+    torch.cuda.synchronize()
+    assert int(st.status[0]) == 0
+    xb_eff, xq_eff = H.effective_operands(storage, True, xb, xq)
+    want = torch.from_numpy(xq_eff).cuda().double() @ torch.from_numpy(xb_eff).cuda().double().T
+    if metric == O.METRIC_L2:
+        want = ((xq.astype(np.float64) ** 2).sum(1)[:, None] + (xb_eff.astype(np.float64) ** 2).sum(1)[None]) - 2 * want.cpu().numpy()
+        want = torch.from_numpy(want).cuda()
+    # fp32 sums of at most 400 products and (fp32 rows) 2^-22 left out of each
+    scale = float(want.abs().max())
+    assert float((out.double() - want).abs().max()) <= 2e-5 * scale
+
+
+@pytest.mark.parametrize("storage,metric,d,nq,nb,k", [
+    (0, O.METRIC_L2, 96, 300, 140_001, 100), (0, O.METRIC_INNER_PRODUCT, 192, 129, 131_328, 10),
+    (0, O.METRIC_L2, 128, 1000, 70_000, 5), (1, O.METRIC_L2, 40, 513, 131_329, 1024),
+    (2, O.METRIC_INNER_PRODUCT, 384, 257, 100_100, 32), (2, O.METRIC_L2, 64, 16_000, 33_000, 3),
+    (0, O.METRIC_L2, 64, 6000, 40_000, 20)])
+def test_filter(fm, res, storage, metric, d, nq, nb, k):
+    xb = H.gaussian(nb, d, 1)
+    xq = H.gaussian(nq, d, 2)
+    idx = fm.B200IndexFlat(res, d, metric, storage)
+    idx.add(xb)
+    D, I = idx.search(xq, k)
+    D2, I2 = idx.search(xq, k)   # candidates come in any order, results do not
+    assert np.array_equal(D, D2) and np.array_equal(I, I2)
+    for q in (slice(0, 8), slice(nq // 2, nq // 2 + 8), slice(nq - 8, nq)):
+        H.check_against_oracle(metric, storage, True, xb, xq[q], k, D[q], I[q], loose=False)
+    idx.close()
