@@ -54,6 +54,29 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
+// Where a kernel goes: a stream and, overlap, whether it may take its place on the SMs while the kernel before it
+// drains (programmatic launch; only for kernels that call pdl_wait, ptx.cuh).
+struct Launch {
+    cudaStream_t stream;
+    bool overlap;
+    Launch(cudaStream_t s, bool o = false) : stream(s), overlap(o) {}
+    operator cudaStream_t() const { return stream; }
+};
+template <typename... P, typename... A>
+inline cudaError_t launch_kernel(void (*kernel)(P...), dim3 grid, int block, size_t smem, const Launch& ln, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)block, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ln.stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = ln.overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Launchers implemented in the other translation units ------------------------
 
 // rows.cu: queries fp32 [nq][d] -> A planes (16-bit, [npl][nq][d_pad]) + squared norms.
@@ -117,24 +140,24 @@ ScanPlan plan_scan(int64_t nq, int64_t nb, int d, int storage, int sm_count);
 // device memory the kernel does nothing.
 int launch_scan_topk(const B200FSearchArgs& a, const ScanPlan& plan, float* part_key,
                      int32_t* part_idx, int* out_P, bool stream_f32, const float* thr, const int* guard,
-                     cudaStream_t stream);
+                     const Launch& ln);
 // Scan that stores keys (smaller = better) to a matrix [nq][ld] for columns [col0, col0+ncols); with
 // stride > 1 column c is one of rows [(col0 + c) * stride, (col0 + c + 1) * stride) of the shard.
 int launch_scan_store(const B200FSearchArgs& a, int64_t col0, int64_t ncols, int64_t stride, float* out,
-                      int64_t ld, int sm_count, const int* guard, cudaStream_t stream);
+                      int64_t ld, int sm_count, const int* guard, const Launch& ln);
 // Scan that appends every row whose key is <= thr[q] to the query's candidate buffer
 // cand_key / cand_idx [nq][cap]; cand_cnt[q] (zeroed by the caller) counts every hit.
 int launch_scan_filter(const B200FSearchArgs& a, const float* thr, float* cand_key, int32_t* cand_idx,
-                       int32_t* cand_cnt, int cap, int sm_count, const BoundFilter& bf, cudaStream_t stream);
+                       int32_t* cand_cnt, int cap, int sm_count, const BoundFilter& bf, const Launch& ln);
 // The same by the streaming kernels (up to 8 queries, L2, keys that are bounds); false: no such kernel for this shape.
 bool scan_bound_filter_fits(const B200FSearchArgs& a);
 // eps of those kernels for a storage type
 float scan_bound_eps(int storage);
 int launch_scan_bound_filter(const B200FSearchArgs& a, const float* thr, float* cand_key, int32_t* cand_idx,
-                             int32_t* cand_cnt, int cap, const BoundFilter& bf, cudaStream_t stream);
+                             int32_t* cand_cnt, int cap, const BoundFilter& bf, const Launch& ln);
 // ckey[q][c] = ||x||^2 - 2 q.x in fp32 for every candidate of a query whose buffer did not overflow.
 int launch_rescore(const B200FSearchArgs& a, const int32_t* cand_idx, const int32_t* cand_cnt, int cap,
-                   float* cand_key, const BoundFilter& bf, cudaStream_t stream);
+                   float* cand_key, const BoundFilter& bf, const Launch& ln);
 
 // gemm_topk.cu
 struct GemmPlan {
@@ -161,7 +184,6 @@ struct GemmOperands {
     int d_pad;                 // K extent (multiple of 8), norm columns included
     int d_data;                // K extent without them
     const int* nq_dev;         // optional: live rows of A (<= nq) left in device memory by a kernel
-    bool overlap;              // launch while the previous kernel of the stream drains (programmatic launch)
 };
 // Fused top-k (k <= 32): partial lists part_key/part_idx [nq][2 * P][k] (two per column range).
 // gthr holds nq * gslots words (gthr_ready: all ones already); with gslots = s the shared filter bounds the (32 * s)-th best
@@ -170,7 +192,7 @@ struct GemmOperands {
 int launch_gemm_topk(const GemmOperands& op, const GemmPlan& plan, int64_t col0, int64_t ncols,
                      int64_t tile_stride, float kscale, int k, int gslots, float* part_key,
                      int32_t* part_idx, uint32_t* gthr, bool gthr_ready, int32_t* status,
-                     cudaStream_t stream);
+                     const Launch& ln);
 // Threshold filter over the whole shard: column c of row q with scaled key <= thr[q * thr_stride +
 // thr_pos] is appended to the row's candidate buffer cand_key/cand_idx [nq][cand_cap] in any
 // order; cand_cnt[q] (zeroed by the caller) counts every hit, also those beyond cand_cap, which are
@@ -179,13 +201,13 @@ int launch_gemm_topk(const GemmOperands& op, const GemmPlan& plan, int64_t col0,
 int launch_gemm_filter(const GemmOperands& op, const GemmPlan& plan, float kscale, const float* thr,
                        int thr_stride, int thr_pos, float* cand_key, int32_t* cand_idx,
                        int32_t* cand_cnt, int cand_cap, int few_hits, int32_t* status,
-                       cudaStream_t stream);
+                       const Launch& ln);
 // Store mode: out[row*ld + (col-col0)] = sign*(-kscale*t) + rowadd[row], t = q.x (- ||x||^2/2).
 // tile_stride > 1 visits only every tile_stride-th column tile (plan made for that many tiles);
 // the visited tiles lie side by side in out.
 int launch_gemm_store(const GemmOperands& op, const GemmPlan& plan, int64_t col0, int64_t ncols,
                       int64_t tile_stride, float kscale, float sign, const float* rowadd, float* out,
-                      int64_t ld, int32_t* status, cudaStream_t stream);
+                      int64_t ld, int32_t* status, const Launch& ln);
 
 // select.cu
 // Merge P sorted partial lists (key smaller=better, int32 local ids; -1 = empty) per
@@ -196,29 +218,29 @@ int launch_gemm_store(const GemmOperands& op, const GemmPlan& plan, int64_t col0
 int launch_merge_partials(const float* part_key, const int32_t* part_idx, int P, int64_t nq, int k,
                           int metric, const float* qnorm, int64_t label_base, float* out_dist,
                           int64_t* out_labels, const int* nq_dev, const int32_t* row_map,
-                          int64_t nb, int32_t* dirty, const RedoRows& redo, cudaStream_t stream);
+                          int64_t nb, int32_t* dirty, const RedoRows& redo, const Launch& ln);
 // Running top-k over a key matrix chunk: run lists [nq][k] (key, int32 id) are read
 // (if has_prev) and rewritten with the best k of (previous list U chunk columns).
 // Merged raw keys only: out_key[q][k], best first, +INF where fewer than k entries exist.
 int launch_merge_keys(const float* part_key, const int32_t* part_idx, int P, int64_t nq, int k,
-                      float* out_key, cudaStream_t stream);
+                      float* out_key, const Launch& ln);
 // nq_dev (optional): number of live rows, read on the device.  inf_empty: a +INF key is no result, as in the
-// tensor path's lists and filter.  overlap: programmatic launch.
+// tensor path's lists and filter.
 int launch_select_chunk(const float* keys, int64_t nq, int64_t ncols, int64_t ld, int64_t col0,
                         int k, int has_prev, float* run_key, int32_t* run_idx, const int* nq_dev,
-                        bool inf_empty, bool overlap, cudaStream_t stream);
+                        bool inf_empty, const Launch& ln);
 // row_map (optional): list j belongs to query row_map[j] (output row and query norm).
 int launch_finalize_lists(const float* run_key, const int32_t* run_idx, int64_t nq, int k,
                           int metric, const float* qnorm, int64_t label_base, float* out_dist,
                           int64_t* out_labels, const int* nq_dev, const int32_t* row_map,
-                          cudaStream_t stream);
+                          const Launch& ln);
 // Selection of k > 32 results from nlists sorted 32-entry lists per query (the fused kernel's
 // output).  A list that is full may have dropped candidates; when its worst entry is not
 // behind the k-th selected one the row's result is not proven exact and dirty[q] is set to 1
 // (else 0).  Results are written for every row.
 int launch_select_parts(const float* part_key, const int32_t* part_idx, int nlists, int64_t nq,
                         int k, int metric, const float* qnorm, int64_t label_base, float* out_dist,
-                        int64_t* out_labels, int32_t* dirty, cudaStream_t stream);
+                        int64_t* out_labels, int32_t* dirty, const Launch& ln);
 // Selection of the k best of a row's threshold-filtered candidates (unordered buffer of
 // min(cand_cnt[q], cap) entries).  dirty[q] = 1 when entries were lost to overflow or fewer than
 // k candidates were found although the shard has more rows.
@@ -226,19 +248,19 @@ int launch_select_parts(const float* part_key, const int32_t* part_idx, int nlis
 int launch_select_candidates(const float* cand_key, const int32_t* cand_idx, const int32_t* cand_cnt,
                              int cap, int64_t nb, int64_t nq, int k, int metric, const float* qnorm,
                              int64_t label_base, float* out_dist, int64_t* out_labels, int32_t* dirty,
-                             const float* thr, const RedoRows& redo, cudaStream_t stream);
+                             const float* thr, const RedoRows& redo, const Launch& ln);
 // select_rank.cu: the same selection from a row of any length (row_select: candidates, lists, a key matrix) and
 // the merge of up to 8192 / k shards' lists (rank_merge); results identical to the kernels of select.cu.
 bool rank_select_enabled();
 int launch_rank_select(const float* cand_key, const int32_t* cand_idx, const int32_t* cand_cnt, int cap,
                        int64_t nb, int64_t nq, int k, int metric, const float* qnorm, int64_t label_base,
                        float* out_dist, int64_t* out_labels, int32_t* dirty, const float* thr,
-                       const RedoRows& redo, cudaStream_t stream);
+                       const RedoRows& redo, const Launch& ln);
 // The k best of every row of a key matrix (n columns, column c is row c of the shard), finalised.  inf_empty
 // as above.
 int launch_matrix_select(const float* keys, int64_t nq, int64_t n, int64_t ld, int k, bool inf_empty, int metric,
                          const float* qnorm, int64_t label_base, float* out_dist, int64_t* out_labels,
-                         const int* nq_dev, const int32_t* row_map, cudaStream_t stream);
+                         const int* nq_dev, const int32_t* row_map, const Launch& ln);
 // out[q]: an upper bound, close to it, of the r-th smallest (r <= 512) of the n keys of row q; +INF when
 // there are too few.  NaN keys are skipped.  bad (optional): one more for every row with more than about
 // `most` keys up to its bound + margin * qnorm[q], or with qnorm[q] >= qnorm_max.
@@ -246,7 +268,7 @@ int launch_matrix_select(const float* keys, int64_t nq, int64_t n, int64_t ld, i
 int row_bound_threads(int64_t nq, int64_t n, int r);
 int row_bound_most(int64_t nq, int64_t n, int r, double most);
 int launch_row_bound(const float* keys, int64_t nq, int64_t n, int64_t ld, int r, float* out, int32_t* bad,
-                     const float* qnorm, float margin, float qnorm_max, double most, cudaStream_t stream);
+                     const float* qnorm, float margin, float qnorm_max, double most, const Launch& ln);
 bool rank_merge_fits(int P, int k);
 int launch_rank_merge(const float* dist, const int64_t* labels, int64_t stride_d, int64_t stride_l, int P,
                       int64_t nq, int k, int metric, float* out_dist, int64_t* out_labels,

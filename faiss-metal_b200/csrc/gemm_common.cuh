@@ -351,6 +351,6 @@ inline int make_operand_map(CUtensorMap* map, const uint16_t* base, int is_bf16,
 // general kernel; its ranges are chosen anew.
 bool resident_fits(const GemmOperands& op, const GemmPlan& plan);
 int launch_resident(const GemmOperands& op, const GemmPlan& plan, GemmParams& g, const CUtensorMap& ma,
-                    const CUtensorMap& mb, cudaStream_t stream);
+                    const CUtensorMap& mb, const Launch& ln);
 
 }  // namespace b200f

@@ -113,6 +113,7 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     if (warp == 0) {
         // ------------------------------ producer ------------------------------
         if (elect_one()) {
+            fence_proxy_async_global();   // the query operand
             const uint32_t sb = sbase + nb * RES_BLOCK_BYTES;   // the ring
             const uint32_t full0 = map_to_cta(bar_full, 0), qfull0 = map_to_cta(bar_qfull, 0);
             int slot = 0, have_qb = -1;
@@ -272,7 +273,7 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
             if (p.rowscale && row_live) ksc *= __ldcg(p.rowscale + (p.rowscale_map ? (int64_t)__ldcg(p.rowscale_map + grow) : grow));
             float thr = -CUDART_INF_F, radd = 0.f;
             if (MODE == MODE_FILTER) {
-                if (row_live) thr = filter_threshold(p.fthr[grow * p.fthr_stride + p.fthr_pos] / ksc);
+                if (row_live) thr = filter_threshold(__ldcg(p.fthr + grow * p.fthr_stride + p.fthr_pos) / ksc);
             } else if (row_live && p.rowadd) {
                 radd = p.rowadd[grow];
             }
@@ -404,7 +405,7 @@ int resident_blocks(const GemmOperands& op) {
 bool resident_fits(const GemmOperands& op, const GemmPlan& plan) { return plan.pair && resident_blocks(op) > 0; }
 
 int launch_resident(const GemmOperands& op, const GemmPlan& plan, GemmParams& g, const CUtensorMap& ma,
-                    const CUtensorMap& mb, cudaStream_t stream) {
+                    const CUtensorMap& mb, const Launch& ln) {
     ResidentParams p{};
     p.n_blocks = resident_blocks(op);
     p.nkd = (int)ceil_div64(op.d_data, BK);
@@ -444,14 +445,14 @@ int launch_resident(const GemmOperands& op, const GemmPlan& plan, GemmParams& g,
     cfg.gridDim = dim3((unsigned)grid, 1, 1);
     cfg.blockDim = dim3(RES_THREADS, 1, 1);
     cfg.dynamicSmemBytes = RES_SMEM_BYTES;
-    cfg.stream = stream;
+    cfg.stream = ln.stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.numAttrs = 1;
-    if (op.overlap) {
+    if (ln.overlap) {
         attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.numAttrs = 2;

@@ -208,6 +208,7 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
     if (warp == 0) {
         // ------------------------------ TMA producer ------------------------------
         if (lane == 0) {
+            fence_proxy_async_global();   // the query operand
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -402,7 +403,7 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
                     li[j] = -1;
                 }
             } else if (MODE == MODE_FILTER) {
-                thr_eff = row_live ? filter_threshold(p.fthr[grow * p.fthr_stride + p.fthr_pos] / ksc) : -CUDART_INF_F;   // -INF passes nothing
+                thr_eff = row_live ? filter_threshold(__ldcg(p.fthr + grow * p.fthr_stride + p.fthr_pos) / ksc) : -CUDART_INF_F;   // -INF passes nothing
             } else if (row_live && p.rowadd) {
                 radd = p.rowadd[grow];
             }
@@ -587,7 +588,7 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
 // ---- host side -------------------------------------------------------------------------
 
 int launch_common(const GemmOperands& op, const GemmPlan& plan, GemmParams& p, int64_t col0,
-                  int64_t ncols, cudaStream_t stream) {
+                  int64_t ncols, const Launch& ln) {
     if (op.nq <= 0 || ncols <= 0) return B200F_OK;
     if (col0 + ncols > op.nb || op.nb > 0x7fffffffLL) return B200F_ERR_BAD_ARG;
     CUtensorMap ma, mb;
@@ -652,20 +653,20 @@ int launch_common(const GemmOperands& op, const GemmPlan& plan, GemmParams& p, i
     }
     if (p.mode < 0 || p.mode > 2) return B200F_ERR_BAD_ARG;
     const KernelFn kernel = kernels[plan.pair ? 1 : 0][p.mode];
-    main_kernel_begin(stream);
+    main_kernel_begin(ln);
     if (p.mode != MODE_TOPK && resident_fits(op, plan)) {
-        rc = launch_resident(op, plan, p, ma, mb, stream);
-        main_kernel_end(stream);
+        rc = launch_resident(op, plan, p, ma, mb, ln);
+        main_kernel_end(ln);
         if (rc != B200F_OK) return rc;
         count_launch();
         return B200F_OK;
     }
-    if (plan.pair || op.overlap) {
+    if (plan.pair || ln.overlap) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)plan.grid, 1, 1);
         cfg.blockDim = dim3(NUM_THREADS, 1, 1);
         cfg.dynamicSmemBytes = plan.pair ? Cfg<true>::SMEM_BYTES : Cfg<false>::SMEM_BYTES;
-        cfg.stream = stream;
+        cfg.stream = ln.stream;
         cudaLaunchAttribute attr[2];
         cfg.attrs = attr;
         if (plan.pair) {
@@ -675,7 +676,7 @@ int launch_common(const GemmOperands& op, const GemmPlan& plan, GemmParams& p, i
             attr[0].val.clusterDim.z = 1;
             cfg.numAttrs = 1;
         }
-        if (op.overlap) {
+        if (ln.overlap) {
             attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
             attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
             cfg.numAttrs++;
@@ -683,13 +684,13 @@ int launch_common(const GemmOperands& op, const GemmPlan& plan, GemmParams& p, i
         cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, ma, mb, p);
         if (e != cudaSuccess) {
             (void)cudaGetLastError();
-            main_kernel_end(stream);
+            main_kernel_end(ln);
             return B200F_ERR_CUDA;
         }
     } else {
-        kernel<<<plan.grid, NUM_THREADS, Cfg<false>::SMEM_BYTES, stream>>>(ma, mb, p);
+        kernel<<<plan.grid, NUM_THREADS, Cfg<false>::SMEM_BYTES, ln.stream>>>(ma, mb, p);
     }
-    main_kernel_end(stream);
+    main_kernel_end(ln);
     count_launch();
     B200F_LAUNCH_CHECK();
     return B200F_OK;
@@ -805,11 +806,11 @@ static GemmPlan spread_plan(GemmPlan g) {
 int launch_gemm_topk(const GemmOperands& op, const GemmPlan& plan, int64_t col0, int64_t ncols,
                      int64_t tile_stride, float kscale, int k, int gslots, float* part_key,
                      int32_t* part_idx, uint32_t* gthr, bool gthr_ready, int32_t* status,
-                     cudaStream_t stream) {
+                     const Launch& ln) {
     if (k <= 0 || k > KMAX || gslots < 1) return B200F_ERR_UNSUPPORTED;
     if (!gthr) return B200F_ERR_BAD_ARG;
     // all-ones is above every ordered float: no bound yet
-    if (!gthr_ready) B200F_CUDA_TRY(cudaMemsetAsync(gthr, 0xff, (size_t)op.nq * gslots * sizeof(uint32_t), stream));
+    if (!gthr_ready) B200F_CUDA_TRY(cudaMemsetAsync(gthr, 0xff, (size_t)op.nq * gslots * sizeof(uint32_t), ln.stream));
     GemmParams p{};
     p.mode = MODE_TOPK;
     p.tile_stride = tile_stride;
@@ -824,13 +825,13 @@ int launch_gemm_topk(const GemmOperands& op, const GemmPlan& plan, int64_t col0,
     p.out = nullptr;
     p.ld = 0;
     p.status = status;
-    return launch_common(op, plan, p, col0, ncols, stream);
+    return launch_common(op, plan, p, col0, ncols, ln);
 }
 
 int launch_gemm_filter(const GemmOperands& op, const GemmPlan& plan, float kscale, const float* thr,
                        int thr_stride, int thr_pos, float* cand_key, int32_t* cand_idx,
                        int32_t* cand_cnt, int cand_cap, int few_hits, int32_t* status,
-                       cudaStream_t stream) {
+                       const Launch& ln) {
     if (!thr || !cand_key || !cand_idx || !cand_cnt || cand_cap < 1) return B200F_ERR_BAD_ARG;
     GemmParams p{};
     p.mode = MODE_FILTER;
@@ -845,12 +846,12 @@ int launch_gemm_filter(const GemmOperands& op, const GemmPlan& plan, float kscal
     p.cand_cap = cand_cap;
     p.wide = few_hits ? 1 : 0;
     p.status = status;
-    return launch_common(op, spread_plan(plan), p, 0, op.nb, stream);
+    return launch_common(op, spread_plan(plan), p, 0, op.nb, ln);
 }
 
 int launch_gemm_store(const GemmOperands& op, const GemmPlan& plan, int64_t col0, int64_t ncols,
                       int64_t tile_stride, float kscale, float sign, const float* rowadd, float* out,
-                      int64_t ld, int32_t* status, cudaStream_t stream) {
+                      int64_t ld, int32_t* status, const Launch& ln) {
     GemmParams p{};
     p.mode = MODE_STORE;
     p.tile_stride = tile_stride;
@@ -863,7 +864,7 @@ int launch_gemm_store(const GemmOperands& op, const GemmPlan& plan, int64_t col0
     p.out = out;
     p.ld = ld;
     p.status = status;
-    return launch_common(op, spread_plan(plan), p, col0, ncols, stream);
+    return launch_common(op, spread_plan(plan), p, col0, ncols, ln);
 }
 
 }  // namespace b200f

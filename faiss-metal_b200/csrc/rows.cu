@@ -11,6 +11,7 @@
 #include <cmath>
 
 #include "common.cuh"
+#include "ptx.cuh"
 
 namespace b200f {
 
@@ -395,6 +396,7 @@ __global__ void __launch_bounds__(ROW_THREADS) prepare_queries_kernel(const floa
                                        int64_t a_plane_stride, float* __restrict__ qnorm,
                                        int norm_cols, int plane_format, int x_scale_log2,
                                        float* __restrict__ rowscale, const SearchInit init) {
+    pdl_trigger();   // never launched programmatically itself: everything before it has completed
     if (blockIdx.x == 0) {
         if (init.status && threadIdx.x < 4) init.status[threadIdx.x] = 0;
         if (init.count && threadIdx.x < 2) init.count[16 * threadIdx.x] = 0;

@@ -67,11 +67,11 @@ struct ScanParams {
 };
 
 __device__ __forceinline__ bool filter_leaves(const BoundFilter& bf) {
-    return bf.bad && (*bf.bad > bf.bad_limit) != (bf.run_if_bad != 0);
+    return bf.bad && (__ldcg(bf.bad) > bf.bad_limit) != (bf.run_if_bad != 0);
 }
 // threshold of query qi for keys that are bounds
 __device__ __forceinline__ float filter_thr(const ScanParams& p, int qi) {
-    return fmaf(p.bf.eps, __ldg(p.bf.qnorm + qi), p.thr[qi] + p.bf.thr_abs);
+    return fmaf(p.bf.eps, __ldg(p.bf.qnorm + qi), __ldcg(p.thr + qi) + p.bf.thr_abs);
 }
 
 template <int STORAGE>
@@ -184,7 +184,9 @@ template <int STORAGE, int NQ, int MODE>
 __global__ void __launch_bounds__(SCAN_THREADS, (NQ == 4 || (NQ == 2 && STORAGE == B200F_STORAGE_F32 && MODE == SCAN_TOPK)) ? 2 : 3)
 scan_kernel(const ScanParams p) {
     constexpr bool STORE = MODE == SCAN_STORE;
-    if (p.guard && *p.guard == 0) return;
+    pdl_wait();   // thresholds, counts and candidates of the kernel before: coherent loads
+    pdl_trigger();
+    if (p.guard && __ldcg(p.guard) == 0) return;
     if (MODE == SCAN_FILTER && filter_leaves(p.bf)) return;
     constexpr int E = Piece<STORAGE>::E;
     // rows per lane and block; fp32 rows keep two partial sums per (row, query), so fewer rows fit the registers
@@ -227,7 +229,7 @@ scan_kernel(const ScanParams p) {
     for (int qi = 0; qi < NQ; qi++) {
         lk[qi] = CUDART_INF_F;
         li[qi] = -1;
-        thr[qi] = (MODE != SCAN_STORE && p.thr && qi < p.nq) ? p.thr[qi] : CUDART_INF_F;
+        thr[qi] = (MODE != SCAN_STORE && p.thr && qi < p.nq) ? __ldcg(p.thr + qi) : CUDART_INF_F;
         thr_id[qi] = -1;
     }
 
@@ -472,7 +474,9 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
 template <bool BF16, int NW, bool FILTER>
 __global__ void __launch_bounds__(32 * (1 + NW), 1) scan_mma_kernel(const ScanParams p) {
     extern __shared__ __align__(128) uint8_t sm[];
-    if (p.guard && *p.guard == 0) return;
+    pdl_wait();   // thresholds, counts and candidates of the kernel before: coherent loads
+    pdl_trigger();
+    if (p.guard && __ldcg(p.guard) == 0) return;
     if (FILTER && filter_leaves(p.bf)) return;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -524,7 +528,7 @@ __global__ void __launch_bounds__(32 * (1 + NW), 1) scan_mma_kernel(const ScanPa
     for (int qi = 0; qi < SM_NQ; qi++) {
         lk[qi] = CUDART_INF_F;
         li[qi] = -1;
-        thr[qi] = (p.thr && qi < p.nq) ? (FILTER ? filter_thr(p, qi) : p.thr[qi]) : CUDART_INF_F;
+        thr[qi] = (p.thr && qi < p.nq) ? (FILTER ? filter_thr(p, qi) : __ldcg(p.thr + qi)) : CUDART_INF_F;
         thr_id[qi] = -1;
     }
 
@@ -755,7 +759,9 @@ constexpr int ST_THREADS = 32 * (1 + ST_NW);
 template <bool FILTER>
 __global__ void __launch_bounds__(ST_THREADS, 1) scan_tf32_kernel(const ScanParams p) {
     extern __shared__ __align__(128) uint8_t sm[];
-    if (p.guard && *p.guard == 0) return;
+    pdl_wait();   // thresholds, counts and candidates of the kernel before: coherent loads
+    pdl_trigger();
+    if (p.guard && __ldcg(p.guard) == 0) return;
     if (FILTER && filter_leaves(p.bf)) return;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -806,7 +812,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tf32_kernel(const ScanPara
     for (int qi = 0; qi < SM_NQ; qi++) {
         lk[qi] = CUDART_INF_F;
         li[qi] = -1;
-        thr[qi] = (p.thr && qi < p.nq) ? (FILTER ? filter_thr(p, qi) : p.thr[qi]) : CUDART_INF_F;
+        thr[qi] = (p.thr && qi < p.nq) ? (FILTER ? filter_thr(p, qi) : __ldcg(p.thr + qi)) : CUDART_INF_F;
         thr_id[qi] = -1;
     }
 
@@ -1035,9 +1041,11 @@ template <int STORAGE>
 __global__ void __launch_bounds__(RC_THREADS) rescore_kernel(const ScanParams p) {
     constexpr int E = Piece<STORAGE>::E;
     constexpr int LPR = 8, U = 2, PER_CTA = RC_THREADS / LPR;
+    pdl_wait();   // thresholds, counts and candidates of the kernel before: coherent loads
+    pdl_trigger();
     if (filter_leaves(p.bf)) return;
     const int q = blockIdx.x;
-    const int n = p.cand_cnt[q];
+    const int n = __ldcg(p.cand_cnt + q);
     if (n > p.cand_cap || (int)blockIdx.y * PER_CTA * U >= n) return;   // overflow: the query is redone
     extern __shared__ __align__(16) float sq[];   // the query, zero padded to whole pieces
     for (int j = threadIdx.x; j < p.qstride; j += RC_THREADS) sq[j] = j < p.d ? p.queries[(int64_t)q * p.d + j] : 0.f;
@@ -1052,7 +1060,7 @@ __global__ void __launch_bounds__(RC_THREADS) rescore_kernel(const ScanParams p)
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const int c = c0 + u * PER_CTA + grp;
-            row[u] = c < n ? __ldg(idx + c) : -1;
+            row[u] = c < n ? __ldcg(idx + c) : -1;
             nrm[u] = row[u] >= 0 ? __ldg(p.norms + row[u]) : 0.f;
             acc[u] = 0.f;
         }
@@ -1133,16 +1141,16 @@ void fill_geometry(ScanParams& p, int storage, int d, int64_t row_pitch, int nor
 }
 
 template <int STORAGE, int MODE>
-int launch_nq(const ScanParams& p, int grid, size_t smem, cudaStream_t stream) {
+int launch_nq(const ScanParams& p, int grid, size_t smem, const Launch& ln) {
 #define B200F_SCAN_CASE(NQ)                                                                      \
     {                                                                                            \
         if (smem > 48 * 1024)                                                                    \
             B200F_CUDA_TRY(cudaFuncSetAttribute(scan_kernel<STORAGE, NQ, MODE>,                 \
                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,     \
                                                 (int)smem));                                     \
-        main_kernel_begin(stream);                                                               \
-        scan_kernel<STORAGE, NQ, MODE><<<grid, SCAN_THREADS, smem, stream>>>(p);                \
-        main_kernel_end(stream);                                                                 \
+        main_kernel_begin(ln);                                                               \
+        B200F_CUDA_TRY(launch_kernel(scan_kernel<STORAGE, NQ, MODE>, dim3((unsigned)grid), SCAN_THREADS, smem, ln, p)); \
+        main_kernel_end(ln);                                                                 \
         count_launch();                                                                          \
     }
     if (p.nq == 1) B200F_SCAN_CASE(1)
@@ -1154,14 +1162,14 @@ int launch_nq(const ScanParams& p, int grid, size_t smem, cudaStream_t stream) {
 }
 
 template <int MODE>
-int launch_storage(const ScanParams& p, int storage, int grid, cudaStream_t stream) {
+int launch_storage(const ScanParams& p, int storage, int grid, const Launch& ln) {
     const int nq_t = p.nq == 1 ? 1 : (p.nq == 2 ? 2 : 4);
     const size_t smem = scan_smem_bytes(nq_t, p.qstride);
     if (smem > 200 * 1024) return B200F_ERR_UNSUPPORTED;
     switch (storage) {
-        case B200F_STORAGE_F32: return launch_nq<B200F_STORAGE_F32, MODE>(p, grid, smem, stream);
-        case B200F_STORAGE_F16: return launch_nq<B200F_STORAGE_F16, MODE>(p, grid, smem, stream);
-        case B200F_STORAGE_BF16: return launch_nq<B200F_STORAGE_BF16, MODE>(p, grid, smem, stream);
+        case B200F_STORAGE_F32: return launch_nq<B200F_STORAGE_F32, MODE>(p, grid, smem, ln);
+        case B200F_STORAGE_F16: return launch_nq<B200F_STORAGE_F16, MODE>(p, grid, smem, ln);
+        case B200F_STORAGE_BF16: return launch_nq<B200F_STORAGE_BF16, MODE>(p, grid, smem, ln);
     }
     return B200F_ERR_BAD_ARG;
 }
@@ -1224,7 +1232,7 @@ ScanPlan plan_scan(int64_t nq, int64_t nb, int d, int storage, int sm_count) {
 
 int launch_scan_topk(const B200FSearchArgs& a, const ScanPlan& plan, float* part_key,
                      int32_t* part_idx, int* out_P, bool stream_f32, const float* thr, const int* guard,
-                     cudaStream_t stream) {
+                     const Launch& ln) {
     if (a.nq < 1 || a.nq > 8 || a.k < 1 || a.k > 32) return B200F_ERR_UNSUPPORTED;
     ScanParams p{};
     fill_geometry(p, a.storage, a.d, a.row_pitch, a.metric == B200F_METRIC_L2 ? a.norm_cols : 0,
@@ -1261,8 +1269,8 @@ int launch_scan_topk(const B200FSearchArgs& a, const ScanPlan& plan, float* part
     {                                                                                                     \
         B200F_CUDA_TRY(cudaFuncSetAttribute(scan_mma_kernel<BF, NW, false>,                               \
                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));     \
-        main_kernel_begin(stream);                                                                        \
-        scan_mma_kernel<BF, NW, false><<<grid, 32 * (1 + NW), smem, stream>>>(ps);                               \
+        main_kernel_begin(ln);                                                                        \
+        B200F_CUDA_TRY(launch_kernel(scan_mma_kernel<BF, NW, false>, dim3((unsigned)grid), 32 * (1 + NW), smem, ln, ps)); \
     }
             const bool bf = a.storage == B200F_STORAGE_BF16;
             if (a.nq <= 2) {
@@ -1271,7 +1279,7 @@ int launch_scan_topk(const B200FSearchArgs& a, const ScanPlan& plan, float* part
                 if (bf) B200F_SCAN_MMA(true, SM_NW_MANY) else B200F_SCAN_MMA(false, SM_NW_MANY)
             }
 #undef B200F_SCAN_MMA
-            main_kernel_end(stream);
+            main_kernel_end(ln);
             count_launch();
             B200F_LAUNCH_CHECK();
             return B200F_OK;
@@ -1289,9 +1297,9 @@ int launch_scan_topk(const B200FSearchArgs& a, const ScanPlan& plan, float* part
             *out_P = grid;
             B200F_CUDA_TRY(cudaFuncSetAttribute(scan_tf32_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                 (int)smem));
-            main_kernel_begin(stream);
-            scan_tf32_kernel<false><<<grid, ST_THREADS, smem, stream>>>(ps);
-            main_kernel_end(stream);
+            main_kernel_begin(ln);
+            B200F_CUDA_TRY(launch_kernel(scan_tf32_kernel<false>, dim3((unsigned)grid), ST_THREADS, smem, ln, ps));
+            main_kernel_end(ln);
             count_launch();
             B200F_LAUNCH_CHECK();
             return B200F_OK;
@@ -1299,11 +1307,11 @@ int launch_scan_topk(const B200FSearchArgs& a, const ScanPlan& plan, float* part
     }
     if (a.nq > 4) return B200F_ERR_UNSUPPORTED;
     *out_P = plan.grid;
-    return launch_storage<SCAN_TOPK>(p, a.storage, plan.grid, stream);
+    return launch_storage<SCAN_TOPK>(p, a.storage, plan.grid, ln);
 }
 
 int launch_scan_store(const B200FSearchArgs& a, int64_t col0, int64_t ncols, int64_t stride, float* out, int64_t ld,
-                      int sm_count, const int* guard, cudaStream_t stream) {
+                      int sm_count, const int* guard, const Launch& ln) {
     if (a.nq < 1 || a.nq > 4 || stride < 1 || stride > 0x7fffffffLL) return B200F_ERR_UNSUPPORTED;
     if (ncols <= 0) return B200F_OK;
     ScanParams p{};
@@ -1327,11 +1335,11 @@ int launch_scan_store(const B200FSearchArgs& a, int64_t col0, int64_t ncols, int
     return launch_storage<SCAN_STORE>(p, a.storage,
                                       scan_grid(ncols, a.d, a.storage, sm_count, lanes_per_row_cap(a.nq),
                                                 resident_ctas(a.nq, a.storage, true)),
-                                      stream);
+                                      ln);
 }
 
 int launch_scan_filter(const B200FSearchArgs& a, const float* thr, float* cand_key, int32_t* cand_idx,
-                       int32_t* cand_cnt, int cap, int sm_count, const BoundFilter& bf, cudaStream_t stream) {
+                       int32_t* cand_cnt, int cap, int sm_count, const BoundFilter& bf, const Launch& ln) {
     if (a.nq < 1 || a.nq > 4 || !thr || !cand_key || !cand_idx || !cand_cnt || cap < 1) return B200F_ERR_BAD_ARG;
     ScanParams p{};
     fill_geometry(p, a.storage, a.d, a.row_pitch, a.metric == B200F_METRIC_L2 ? a.norm_cols : 0,
@@ -1355,7 +1363,7 @@ int launch_scan_filter(const B200FSearchArgs& a, const float* thr, float* cand_k
     return launch_storage<SCAN_FILTER>(p, a.storage,
                                        scan_grid(a.nb, a.d, a.storage, sm_count, lanes_per_row_cap(a.nq),
                                                  resident_ctas(a.nq, a.storage, true)),
-                                       stream);
+                                       ln);
 }
 
 namespace {
@@ -1382,7 +1390,7 @@ float scan_bound_eps(int storage) {
 }
 
 int launch_scan_bound_filter(const B200FSearchArgs& a, const float* thr, float* cand_key, int32_t* cand_idx,
-                             int32_t* cand_cnt, int cap, const BoundFilter& bf, cudaStream_t stream) {
+                             int32_t* cand_cnt, int cap, const BoundFilter& bf, const Launch& ln) {
     if (!thr || !cand_key || !cand_idx || !cand_cnt || cap < 1 || !bf.qnorm) return B200F_ERR_BAD_ARG;
     ScanParams p{};
     if (!plan_bound_filter(a, p)) return B200F_ERR_UNSUPPORTED;
@@ -1413,16 +1421,16 @@ int launch_scan_bound_filter(const B200FSearchArgs& a, const float* thr, float* 
                                                                   : scan_mma_kernel<false, SM_NW_MANY, true>;
     B200F_CUDA_TRY(cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)smem));
-    main_kernel_begin(stream);
-    kernel<<<grid, f32 ? ST_THREADS : 32 * (1 + SM_NW_MANY), smem, stream>>>(p);
-    main_kernel_end(stream);
+    main_kernel_begin(ln);
+    B200F_CUDA_TRY(launch_kernel(kernel, dim3((unsigned)grid), f32 ? ST_THREADS : 32 * (1 + SM_NW_MANY), smem, ln, p));
+    main_kernel_end(ln);
     count_launch();
     B200F_LAUNCH_CHECK();
     return B200F_OK;
 }
 
 int launch_rescore(const B200FSearchArgs& a, const int32_t* cand_idx, const int32_t* cand_cnt, int cap,
-                   float* cand_key, const BoundFilter& bf, cudaStream_t stream) {
+                   float* cand_key, const BoundFilter& bf, const Launch& ln) {
     if (a.metric != B200F_METRIC_L2 || !a.norms || !cand_idx || !cand_cnt || !cand_key) return B200F_ERR_BAD_ARG;
     if (a.nq <= 0) return B200F_OK;
     ScanParams p{};
@@ -1444,9 +1452,9 @@ int launch_rescore(const B200FSearchArgs& a, const int32_t* cand_idx, const int3
     if (split > most) split = most;
     const dim3 grid((unsigned)a.nq, (unsigned)split);
     switch (a.storage) {
-        case B200F_STORAGE_F32: rescore_kernel<B200F_STORAGE_F32><<<grid, RC_THREADS, smem, stream>>>(p); break;
-        case B200F_STORAGE_F16: rescore_kernel<B200F_STORAGE_F16><<<grid, RC_THREADS, smem, stream>>>(p); break;
-        default: rescore_kernel<B200F_STORAGE_BF16><<<grid, RC_THREADS, smem, stream>>>(p); break;
+        case B200F_STORAGE_F32: B200F_CUDA_TRY(launch_kernel(rescore_kernel<B200F_STORAGE_F32>, grid, RC_THREADS, smem, ln, p)); break;
+        case B200F_STORAGE_F16: B200F_CUDA_TRY(launch_kernel(rescore_kernel<B200F_STORAGE_F16>, grid, RC_THREADS, smem, ln, p)); break;
+        default: B200F_CUDA_TRY(launch_kernel(rescore_kernel<B200F_STORAGE_BF16>, grid, RC_THREADS, smem, ln, p)); break;
     }
     count_launch();
     B200F_LAUNCH_CHECK();

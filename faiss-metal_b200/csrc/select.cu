@@ -108,6 +108,8 @@ template <typename IdT>
 __global__ void __launch_bounds__(MS_THREADS) merge_small_kernel(const MergeSmallParams<IdT> p) {
     __shared__ float sk[MS_WARPS][32];
     __shared__ IdT si[MS_WARPS][32];
+    pdl_wait();
+    pdl_trigger();
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int64_t nq_live = p.nq_dev ? min((int64_t)*p.nq_dev, p.nq) : p.nq;
@@ -123,8 +125,8 @@ __global__ void __launch_bounds__(MS_THREADS) merge_small_kernel(const MergeSmal
             float myk = CUDART_INF_F;
             IdT myi = (IdT)-1;
             if (lane < p.k) {
-                myk = p.key_sign * lkey[lane];
-                myi = lid[lane];
+                myk = p.key_sign * __ldcg(lkey + lane);
+                myi = __ldcg(lid + lane);
             }
             for (int j = 0; j < p.k; j++) {
                 const float s = __shfl_sync(FULL, myk, j);
@@ -568,7 +570,7 @@ __global__ void gather_rows_kernel(const uint16_t* __restrict__ a, int npl, int6
 }
 
 template <int SRC>
-int launch_sort_select(const SortSelectParams& p, cudaStream_t stream, bool overlap = false) {
+int launch_sort_select(const SortSelectParams& p, const Launch& ln) {
     if (p.nq <= 0) return B200F_OK;
     if (p.k < 1 || p.k > B200F_MAX_K) return B200F_ERR_UNSUPPORTED;
     const int smem = SS_CAP * 8;
@@ -584,40 +586,31 @@ int launch_sort_select(const SortSelectParams& p, cudaStream_t stream, bool over
     if (g > cap) g = cap;
     // rows counted on the device are usually few or none: idle CTAs leave at once
     if (p.nq_dev && g > cached_sm_count()) g = cached_sm_count();
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)g, 1, 1);
-    cfg.blockDim = dim3(SS_THREADS, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = overlap ? 1 : 0;
-    B200F_CUDA_TRY(cudaLaunchKernelEx(&cfg, sort_select_kernel<SRC>, p));
+    B200F_CUDA_TRY(launch_kernel(sort_select_kernel<SRC>, dim3((unsigned)g), SS_THREADS, smem, ln, p));
     count_launch();
     B200F_LAUNCH_CHECK();
     return B200F_OK;
 }
 
-__global__ void finalize_lists_kernel(const float* __restrict__ run_key,
-                                      const int32_t* __restrict__ run_idx, int64_t nq, int k,
+__global__ void finalize_lists_kernel(const float* run_key, const int32_t* run_idx, int64_t nq, int k,
                                       float out_sign, const float* __restrict__ qnorm, int clamp,
                                       float pad, int64_t label_base, float* __restrict__ out_dist,
                                       int64_t* __restrict__ out_labels,
                                       const int* __restrict__ nq_dev,
                                       const int32_t* __restrict__ row_map) {
+    pdl_wait();
+    pdl_trigger();
     if (nq_dev) nq = min((int64_t)*nq_dev, nq);
     const int64_t total = nq * k;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t q = i / k;
         const int64_t qo = row_map ? (int64_t)row_map[q] : q;  // output row
-        const int32_t id = run_idx[i];
+        const int32_t id = __ldcg(run_idx + i);
         float dist = pad;
         int64_t label = -1;
         if (id >= 0) {
-            dist = out_sign * run_key[i] + (qnorm ? qnorm[qo] : 0.f);
+            dist = out_sign * __ldcg(run_key + i) + (qnorm ? qnorm[qo] : 0.f);
             if (clamp && dist < 0.f) dist = 0.f;
             label = (int64_t)id + label_base;
         }
@@ -629,7 +622,7 @@ __global__ void finalize_lists_kernel(const float* __restrict__ run_key,
 }  // namespace
 
 int launch_merge_keys(const float* part_key, const int32_t* part_idx, int P, int64_t nq, int k,
-                      float* out_key, cudaStream_t stream) {
+                      float* out_key, const Launch& ln) {
     if (nq <= 0) return B200F_OK;
     if (k < 1 || k > 32 || P < 1) return B200F_ERR_UNSUPPORTED;
     MergeSmallParams<int32_t> p{};
@@ -649,7 +642,7 @@ int launch_merge_keys(const float* part_key, const int32_t* part_idx, int P, int
     int64_t g = nq;
     const int64_t cap = (int64_t)cached_sm_count() * 32;
     if (g > cap) g = cap;
-    merge_small_kernel<int32_t><<<(int)g, MS_THREADS, 0, stream>>>(p);
+    B200F_CUDA_TRY(launch_kernel(merge_small_kernel<int32_t>, dim3((unsigned)g), MS_THREADS, 0, ln, p));
     count_launch();
     B200F_LAUNCH_CHECK();
     return B200F_OK;
@@ -657,7 +650,7 @@ int launch_merge_keys(const float* part_key, const int32_t* part_idx, int P, int
 
 int launch_select_chunk(const float* keys, int64_t nq, int64_t ncols, int64_t ld, int64_t col0,
                         int k, int has_prev, float* run_key, int32_t* run_idx, const int* nq_dev,
-                        bool inf_empty, bool overlap, cudaStream_t stream) {
+                        bool inf_empty, const Launch& ln) {
     SortSelectParams p{};
     p.inf_empty = inf_empty ? 1 : 0;
     p.nq_dev = nq_dev;
@@ -672,12 +665,12 @@ int launch_select_chunk(const float* keys, int64_t nq, int64_t ncols, int64_t ld
     p.run_key = run_key;
     p.run_idx = run_idx;
     p.out_dist = nullptr;
-    return launch_sort_select<SRC_MATRIX>(p, stream, overlap);
+    return launch_sort_select<SRC_MATRIX>(p, ln);
 }
 
 int launch_select_parts(const float* part_key, const int32_t* part_idx, int nlists, int64_t nq,
                         int k, int metric, const float* qnorm, int64_t label_base, float* out_dist,
-                        int64_t* out_labels, int32_t* dirty, cudaStream_t stream) {
+                        int64_t* out_labels, int32_t* dirty, const Launch& ln) {
     if (nlists < 1 || (int64_t)nlists * 32 > 0x7fffffffLL) return B200F_ERR_UNSUPPORTED;
     const bool l2 = metric == B200F_METRIC_L2;
     SortSelectParams p{};
@@ -697,17 +690,17 @@ int launch_select_parts(const float* part_key, const int32_t* part_idx, int nlis
     p.out_dist = out_dist;
     p.out_labels = out_labels;
     p.dirty = dirty;
-    return launch_sort_select<SRC_PARTS>(p, stream);
+    return launch_sort_select<SRC_PARTS>(p, ln.stream);   // its lists and candidates come through the read-only path
 }
 
 int launch_select_candidates(const float* cand_key, const int32_t* cand_idx, const int32_t* cand_cnt,
                              int cap, int64_t nb, int64_t nq, int k, int metric, const float* qnorm,
                              int64_t label_base, float* out_dist, int64_t* out_labels, int32_t* dirty,
-                             const float* thr, const RedoRows& redo, cudaStream_t stream) {
+                             const float* thr, const RedoRows& redo, const Launch& ln) {
     if (cap < 1 || !cand_cnt) return B200F_ERR_BAD_ARG;
     if (rank_select_enabled() && dirty)
         return launch_rank_select(cand_key, cand_idx, cand_cnt, cap, nb, nq, k, metric, qnorm, label_base,
-                                  out_dist, out_labels, dirty, thr, redo, stream);
+                                  out_dist, out_labels, dirty, thr, redo, ln);
     if (thr || redo.count) return B200F_ERR_BAD_ARG;   // only row_select knows them
     const bool l2 = metric == B200F_METRIC_L2;
     SortSelectParams p{};
@@ -728,7 +721,7 @@ int launch_select_candidates(const float* cand_key, const int32_t* cand_idx, con
     p.out_dist = out_dist;
     p.out_labels = out_labels;
     p.dirty = dirty;
-    return launch_sort_select<SRC_PARTS>(p, stream);
+    return launch_sort_select<SRC_PARTS>(p, ln.stream);   // its lists and candidates come through the read-only path
 }
 
 int launch_compact_rows(const int32_t* dirty, int64_t nq, int32_t* rows, int32_t* count,
@@ -755,16 +748,15 @@ int launch_gather_rows(const uint16_t* a, int npl, int64_t plane_stride, int64_t
 int launch_finalize_lists(const float* run_key, const int32_t* run_idx, int64_t nq, int k,
                           int metric, const float* qnorm, int64_t label_base, float* out_dist,
                           int64_t* out_labels, const int* nq_dev, const int32_t* row_map,
-                          cudaStream_t stream) {
+                          const Launch& ln) {
     if (nq <= 0) return B200F_OK;
     const bool l2 = metric == B200F_METRIC_L2;
     int64_t g = ceil_div64(nq * k, 256);
     const int64_t cap = (int64_t)cached_sm_count() * 16;
     if (g > cap) g = cap;
-    finalize_lists_kernel<<<(int)g, 256, 0, stream>>>(run_key, run_idx, nq, k, l2 ? 1.f : -1.f,
-                                                      l2 ? qnorm : nullptr, l2 ? 1 : 0,
-                                                      l2 ? kHostInf : -kHostInf, label_base,
-                                                      out_dist, out_labels, nq_dev, row_map);
+    B200F_CUDA_TRY(launch_kernel(finalize_lists_kernel, dim3((unsigned)g), 256, 0, ln, run_key, run_idx, nq, k, l2 ? 1.f : -1.f,
+                                 l2 ? qnorm : nullptr, l2 ? 1 : 0, l2 ? kHostInf : -kHostInf, label_base, out_dist,
+                                 out_labels, nq_dev, row_map));
     count_launch();
     B200F_LAUNCH_CHECK();
     return B200F_OK;

@@ -20,6 +20,7 @@
 #include <cmath>
 
 #include "common.cuh"
+#include "ptx.cuh"
 
 namespace b200f {
 
@@ -310,19 +311,21 @@ __global__ void __launch_bounds__(1024) row_select_kernel(const RowSelectParams 
     __shared__ int s_live[32];
     __shared__ int s_sel[2];
     __shared__ int s_count, s_have, s_beyond;
+    pdl_wait();   // what the kernel before wrote is read with coherent loads
+    pdl_trigger();
     const int W = blockDim.x >> 5;
     const int T = blockDim.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t nq_live = p.nq_dev ? min((int64_t)*p.nq_dev, p.nq) : p.nq;
     for (int64_t q = blockIdx.x; q < nq_live; q += gridDim.x) {
-        const int64_t cnt = p.cnt ? (int64_t)__ldg(p.cnt + q) : p.n;
+        const int64_t cnt = p.cnt ? (int64_t)__ldcg(p.cnt + q) : p.n;
         const int n = (int)min(cnt, p.ld);
         const float* keys = p.keys + q * p.ld;
         const int32_t* ids = p.ids ? p.ids + q * p.ld : nullptr;
         // (ordered key, live) of column c; both loads are issued before either is used
         auto load = [&](int c, uint32_t& key, int32_t& id) {
-            const float f = __ldg(keys + c) + 0.f;   // -0 becomes +0: the two tie
-            id = ids ? __ldg(ids + c) : (f <= p.last_key ? c : -1);
+            const float f = __ldca(keys + c) + 0.f;   // -0 becomes +0: the two tie
+            id = ids ? __ldca(ids + c) : (f <= p.last_key ? c : -1);
             key = float_to_ordered(f);
         };
         int live = 0;
@@ -490,7 +493,7 @@ __global__ void __launch_bounds__(1024) row_select_kernel(const RowSelectParams 
 // smallest of the T thread minima (T several times r keeps it close; +INF where fewer than r threads
 // have a key, which lets every row pass).  One CTA per row; out[q] may be exceeded by no key that
 // belongs to the r smallest.
-__global__ void __launch_bounds__(1024) row_bound_kernel(const float* __restrict__ keys, int64_t ld, int64_t n,
+__global__ void __launch_bounds__(1024) row_bound_kernel(const float* keys, int64_t ld, int64_t n,
                                                          int64_t nq, int r, float* __restrict__ out,
                                                          int32_t* __restrict__ bad, const float* __restrict__ qnorm,
                                                          float margin, float qnorm_max, int most) {
@@ -499,6 +502,8 @@ __global__ void __launch_bounds__(1024) row_bound_kernel(const float* __restrict
     __shared__ int s_live[32];
     __shared__ int s_sel[2];
     const int tid = threadIdx.x, T = blockDim.x;
+    pdl_wait();   // the sample's keys are read with coherent loads
+    pdl_trigger();
     const bool vec = (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(keys) & 15) == 0;
     for (int64_t q = blockIdx.x; q < nq; q += gridDim.x) {
         const float* row = keys + q * ld;
@@ -506,13 +511,13 @@ __global__ void __launch_bounds__(1024) row_bound_kernel(const float* __restrict
         if (vec) {
 #pragma unroll 4
             for (int64_t c = (int64_t)tid * 4; c + 4 <= n; c += (int64_t)T * 4) {
-                const float4 f = __ldg(reinterpret_cast<const float4*>(row + c));
+                const float4 f = __ldcg(reinterpret_cast<const float4*>(row + c));
                 best = fminf(best, fminf(fminf(f.x, f.y), fminf(f.z, f.w)));
             }
-            if (tid < (n & 3)) best = fminf(best, __ldg(row + (n & ~(int64_t)3) + tid));
+            if (tid < (n & 3)) best = fminf(best, __ldcg(row + (n & ~(int64_t)3) + tid));
         } else {
 #pragma unroll 4
-            for (int64_t c = tid; c < n; c += T) best = fminf(best, __ldg(row + c));
+            for (int64_t c = tid; c < n; c += T) best = fminf(best, __ldcg(row + c));
         }
         const bool have = best < CUDART_INF_F;
         const uint32_t key = float_to_ordered(best + 0.f);
@@ -726,7 +731,7 @@ namespace {
 
 // Threads per row: few for many rows of few candidates, many for few long rows.  The staging area
 // holds 4 k words and at least 1024, 8192 at most: W warps sort at most RS_RUN words each.
-int launch_row_select(RowSelectParams& p, int64_t n_typical, cudaStream_t stream) {
+int launch_row_select(RowSelectParams& p, int64_t n_typical, const Launch& ln) {
     if (p.nq <= 0) return B200F_OK;
     if (p.k < 1 || p.k > B200F_MAX_K) return B200F_ERR_UNSUPPORTED;
     const int64_t sm = cached_sm_count();
@@ -756,8 +761,7 @@ int launch_row_select(RowSelectParams& p, int64_t n_typical, cudaStream_t stream
     if (g > gcap) g = gcap;
     // rows counted on the device are usually few or none: idle CTAs leave at once
     if (p.nq_dev && g > sm) g = sm;
-    if (four) row_select_kernel<4><<<(int)g, T, smem, stream>>>(p);
-    else row_select_kernel<1><<<(int)g, T, smem, stream>>>(p);
+    B200F_CUDA_TRY(launch_kernel(four ? row_select_kernel<4> : row_select_kernel<1>, dim3((unsigned)g), T, smem, ln, p));
     count_launch();
     B200F_LAUNCH_CHECK();
     return B200F_OK;
@@ -790,7 +794,7 @@ int row_bound_most(int64_t nq, int64_t n, int r, double most) {
 }
 
 int launch_row_bound(const float* keys, int64_t nq, int64_t n, int64_t ld, int r, float* out, int32_t* bad,
-                     const float* qnorm, float margin, float qnorm_max, double most, cudaStream_t stream) {
+                     const float* qnorm, float margin, float qnorm_max, double most, const Launch& ln) {
     if (r < 1 || r > 512 || n < 0 || ld < n || !keys || !out) return B200F_ERR_BAD_ARG;
     if (nq <= 0) return B200F_OK;
     const int64_t sm = cached_sm_count();
@@ -799,7 +803,8 @@ int launch_row_bound(const float* keys, int64_t nq, int64_t n, int64_t ld, int r
     const int64_t gcap = sm * (2048 / T);
     if (g > gcap) g = gcap;
     const int most_minima = row_bound_most(nq, n, r, most);
-    row_bound_kernel<<<(int)g, T, 0, stream>>>(keys, ld, n, nq, r, out, bad, qnorm, margin, qnorm_max, most_minima);
+    B200F_CUDA_TRY(launch_kernel(row_bound_kernel, dim3((unsigned)g), T, 0, ln, keys, ld, n, nq, r, out, bad, qnorm, margin,
+                                 qnorm_max, most_minima));
     count_launch();
     B200F_LAUNCH_CHECK();
     return B200F_OK;
@@ -808,7 +813,7 @@ int launch_row_bound(const float* keys, int64_t nq, int64_t n, int64_t ld, int r
 int launch_rank_select(const float* cand_key, const int32_t* cand_idx, const int32_t* cand_cnt, int cap,
                        int64_t nb, int64_t nq, int k, int metric, const float* qnorm, int64_t label_base,
                        float* out_dist, int64_t* out_labels, int32_t* dirty, const float* thr,
-                       const RedoRows& redo, cudaStream_t stream) {
+                       const RedoRows& redo, const Launch& ln) {
     if (cap < 1 || !cand_cnt || !dirty) return B200F_ERR_BAD_ARG;
     RowSelectParams p{};
     p.keys = cand_key;
@@ -822,13 +827,13 @@ int launch_rank_select(const float* cand_key, const int32_t* cand_idx, const int
     p.thr = thr;
     p.redo = redo;
     set_output(p, metric, qnorm, label_base, out_dist, out_labels);
-    return launch_row_select(p, cap / 4, stream);
+    return launch_row_select(p, cap / 4, ln);
 }
 
 int launch_merge_partials(const float* part_key, const int32_t* part_idx, int P, int64_t nq, int k,
                           int metric, const float* qnorm, int64_t label_base, float* out_dist,
                           int64_t* out_labels, const int* nq_dev, const int32_t* row_map,
-                          int64_t nb, int32_t* dirty, const RedoRows& redo, cudaStream_t stream) {
+                          int64_t nb, int32_t* dirty, const RedoRows& redo, const Launch& ln) {
     if (nq <= 0) return B200F_OK;
     if (k < 1 || k > 32 || P < 1) return B200F_ERR_UNSUPPORTED;
     RowSelectParams p{};
@@ -844,12 +849,12 @@ int launch_merge_partials(const float* part_key, const int32_t* part_idx, int P,
     p.row_map = row_map;
     p.k = k;
     set_output(p, metric, qnorm, label_base, out_dist, out_labels);
-    return launch_row_select(p, p.n, stream);
+    return launch_row_select(p, p.n, ln);
 }
 
 int launch_matrix_select(const float* keys, int64_t nq, int64_t n, int64_t ld, int k, bool inf_empty, int metric,
                          const float* qnorm, int64_t label_base, float* out_dist, int64_t* out_labels,
-                         const int* nq_dev, const int32_t* row_map, cudaStream_t stream) {
+                         const int* nq_dev, const int32_t* row_map, const Launch& ln) {
     if (n < 0 || n > 0x7fffffffLL || ld < n) return B200F_ERR_BAD_ARG;
     RowSelectParams p{};
     p.keys = keys;
@@ -861,7 +866,7 @@ int launch_matrix_select(const float* keys, int64_t nq, int64_t n, int64_t ld, i
     p.row_map = row_map;
     p.k = k;
     set_output(p, metric, qnorm, label_base, out_dist, out_labels);
-    return launch_row_select(p, n, stream);
+    return launch_row_select(p, n, ln);
 }
 
 bool rank_merge_fits(int P, int k) { return k > 32 && P >= 1 && (int64_t)P * k <= 8192; }
