@@ -392,7 +392,8 @@ bool make_plan(int64_t nq, int64_t nb, int d, int k, int storage, int path, bool
     return true;
 }
 
-__global__ void fill_pad_kernel(float* dist, int64_t* labels, int64_t n, float pad) {
+__global__ void fill_pad_kernel(float* dist, int64_t* labels, int64_t n, float pad, int32_t* status) {
+    if (status && blockIdx.x == 0 && threadIdx.x < 4) status[threadIdx.x] = 0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
         dist[i] = pad;
@@ -698,10 +699,9 @@ extern "C" int b200f_search(const B200FSearchArgs* a) {
     if (a->nq == 0) return B200F_OK;
     const bool l2 = a->metric == B200F_METRIC_L2;
     if (a->nb == 0) {
-        if (a->status) B200F_CUDA_TRY(cudaMemsetAsync(a->status, 0, 4 * sizeof(int32_t), st));
         const int64_t n = a->nq * a->k;
         fill_pad_kernel<<<(int)(ceil_div64(n, 256) < 1024 ? ceil_div64(n, 256) : 1024), 256, 0, st>>>(
-                a->out_dist, a->out_labels, n, l2 ? kHostInf : -kHostInf);
+                a->out_dist, a->out_labels, n, l2 ? kHostInf : -kHostInf, a->status);
         count_launch();
         B200F_LAUNCH_CHECK();
         return B200F_OK;

@@ -32,6 +32,7 @@ constexpr size_t kStageBytes = 32ull << 20;   // fp32 staging chunk of add / rec
 constexpr int64_t kScaleSampleRows = 8192;    // rows an fp32 index takes its plane scale from
 constexpr int64_t kGraphMaxQueries = 8;        // searches this small are replayed from a CUDA graph
 constexpr int64_t kGraphDirectResults = 512;   // results of a captured search written to host memory by the kernel
+constexpr size_t kGraphFetchBytes = 64 << 10;  // queries of a captured search fetched by a kernel
 constexpr size_t kMaxGraphs = 8;               // graphs kept per index (least recently used goes)
 constexpr int64_t kFusedBatch = 16384;        // queries per launch, k <= 1024 (fused kernel, lists)
 constexpr int64_t kSelectBatch = 1024;        // queries per launch beyond: few rows, wide column chunks
@@ -62,6 +63,9 @@ void abiCheck(int rc, const char* what) {
     throw B200RuntimeError(code, std::string("faiss-b200: ") + what + " reported device status " +
                                          std::to_string(word) + " (" + b200f_status_string(code) + ")");
 }
+
+// Status words are written by kernels, straight to pinned memory; read once the stream has been waited for.
+int32_t statusWord(const int32_t* words) { return *static_cast<const volatile int32_t*>(words); }
 
 struct DeviceGuard {
     int prev = -1;
@@ -142,9 +146,11 @@ struct B200IndexFlat::Impl {
     uint16_t* planes = nullptr;
     float* norms = nullptr;
     int64_t capacity = 0;
-    int32_t* status = nullptr;    // device int32[4]
+    int32_t* deviceWords = nullptr;   // device int32[64]: range flag and largest element of add()
     float* oneRow = nullptr;      // device fp32[d] for reconstruct
-    int32_t* hostStatus = nullptr;  // pinned int32[4]
+    // Pinned int32[16].  First four, a search's status words: the kernels write them, when they start and where something
+    // is wrong.  Copied down from the device they cost every search 8 us behind its last kernel.
+    int32_t* status = nullptr;
     int forcePath = B200F_PATH_AUTO;
     int64_t labelBase = 0;
     mutable std::vector<float> mirror;
@@ -172,11 +178,11 @@ struct B200IndexFlat::Impl {
     int planeScaleLog2 = 0;
     bool planeScaleKnown = false;
     int planesBacked() const { return planeFormat == B200F_PLANES_FP16X2 ? 2 : 3; }
-    int32_t* rangeFlag() const { return status + 8; }   // device word beside the status words
+    int32_t* rangeFlag() const { return deviceWords + 8; }
 
     // Small searches (n <= kGraphMaxQueries, host buffers) replayed from CUDA graphs.  A graph
     // holds the whole call: host-to-device copy of the queries out of its pinned slot, the
-    // search, and the copies of distances, labels and status word back into the slot.  It is
+    // search (which leaves its status words in the slot), and the results on their way back into it.  It is
     // tied to the addresses and sizes it was captured with: `generation` changes whenever the
     // stored rows, the label base or the forced path change, and stale graphs are dropped.
     struct SearchGraph {
@@ -394,11 +400,12 @@ B200IndexFlat::B200IndexFlat(std::shared_ptr<B200Resources> resources, int d_,
     impl_->pitch = storage == StorageType::Float32 ? roundUp(d_, 4) : roundUp(d_, 8) + normCols;
     impl_->planePitch = roundUp(d_, 8) + normCols;
     DeviceGuard g(impl_->res->getDevice());
-    impl_->status = static_cast<int32_t*>(impl_->res->allocBuffer(256));
+    impl_->deviceWords = static_cast<int32_t*>(impl_->res->allocBuffer(256));
     impl_->oneRow = static_cast<float*>(impl_->res->allocBuffer((size_t)d_ * 4));
-    impl_->hostStatus = static_cast<int32_t*>(alloc_pinned(64));
-    if (!impl_->hostStatus) throw B200RuntimeError(B200F_ERR_OOM, "faiss-b200: pinned allocation failed");
-    cudaCheck(cudaMemsetAsync(impl_->status, 0, 256, impl_->stream()), "memset status");
+    impl_->status = static_cast<int32_t*>(alloc_pinned(64));
+    if (!impl_->status) throw B200RuntimeError(B200F_ERR_OOM, "faiss-b200: pinned allocation failed");
+    std::memset(impl_->status, 0, 64);
+    cudaCheck(cudaMemsetAsync(impl_->deviceWords, 0, 256, impl_->stream()), "memset status");
     is_trained = true;
     ntotal = 0;
 }
@@ -411,9 +418,9 @@ B200IndexFlat::~B200IndexFlat() {
         impl_->invalidateGraphs();
         impl_->freeStorage();
         (void)takeRetainedStorage(impl_.get());   // unmapped here
-        impl_->res->deallocBuffer(impl_->status);
+        impl_->res->deallocBuffer(impl_->deviceWords);
         impl_->res->deallocBuffer(impl_->oneRow);
-        free_pinned(impl_->hostStatus);
+        free_pinned(impl_->status);
     } catch (...) {
     }
 }
@@ -474,10 +481,10 @@ void B200IndexFlat::add(faiss::idx_t n, const float* x) {
     auto setPlaneScale = [&](const float* src, int64_t nr, int64_t pitch) {
         uint32_t* bits = reinterpret_cast<uint32_t*>(impl_->rangeFlag() + 1);
         abiCheck(b200f_rows_absmax(src, nr, d, pitch, bits, st), "add: rows absmax");
-        cudaCheck(cudaMemcpyAsync(impl_->hostStatus + 8, bits, 4, cudaMemcpyDeviceToHost, st), "add: absmax copy");
+        cudaCheck(cudaMemcpyAsync(impl_->status + 8, bits, 4, cudaMemcpyDeviceToHost, st), "add: absmax copy");
         cudaCheck(cudaStreamSynchronize(st), "add: synchronize");
         float amax;
-        std::memcpy(&amax, impl_->hostStatus + 8, 4);
+        std::memcpy(&amax, impl_->status + 8, 4);
         int e = 0;
         if (amax > 0.f) (void)std::frexp(amax, &e);
         impl_->planeScaleLog2 = amax > 0.f ? std::max(-120, std::min(120, 7 - e)) : 0;
@@ -587,19 +594,19 @@ void B200IndexFlat::add(faiss::idx_t n, const float* x) {
     }
     // the caller may free x as soon as add returns
     if (fp32 && impl_->planeFormat == B200F_PLANES_FP16X2)
-        cudaCheck(cudaMemcpyAsync(impl_->hostStatus + 9, impl_->rangeFlag(), 4, cudaMemcpyDeviceToHost, st),
+        cudaCheck(cudaMemcpyAsync(impl_->status + 9, impl_->rangeFlag(), 4, cudaMemcpyDeviceToHost, st),
                   "add: range flag copy");
     cudaCheck(cudaStreamSynchronize(st), "add: synchronize");
     ntotal = newTotal;
     impl_->mirrorValid = false;
-    auto flagged = [&] { return fp32 && impl_->planeFormat == B200F_PLANES_FP16X2 && impl_->hostStatus[9] != 0; };
-    if (flagged() && scaleFromSample && impl_->hostStatus[9] == 1) {
+    auto flagged = [&] { return fp32 && impl_->planeFormat == B200F_PLANES_FP16X2 && impl_->status[9] != 0; };
+    if (flagged() && scaleFromSample && impl_->status[9] == 1) {
         // the sample missed the largest rows: the scale of all of them, if there is one (it can only be smaller, so
         // not where a row is too small already)
         cudaCheck(cudaMemsetAsync(impl_->rangeFlag(), 0, 4, st), "add: clear range flag");
         (void)setPlaneScale(static_cast<const float*>(impl_->rows), ntotal, impl_->pitch);
         resplit(ntotal);
-        cudaCheck(cudaMemcpyAsync(impl_->hostStatus + 9, impl_->rangeFlag(), 4, cudaMemcpyDeviceToHost, st),
+        cudaCheck(cudaMemcpyAsync(impl_->status + 9, impl_->rangeFlag(), 4, cudaMemcpyDeviceToHost, st),
                   "add: range flag copy");
         cudaCheck(cudaStreamSynchronize(st), "add: synchronize");
     }
@@ -830,12 +837,10 @@ void B200IndexFlat::search(faiss::idx_t n, const float* x, faiss::idx_t k, float
             cudaCheck(cudaMemcpyAsync(labels + (size_t)q0 * k, dLab, (size_t)nq * k * 8,
                                       cudaMemcpyDeviceToHost, st),
                       "search: device to host copy of labels");
-        cudaCheck(cudaMemcpyAsync(impl_->hostStatus, impl_->status, 16, cudaMemcpyDeviceToHost, st),
-                  "search: status copy");
         cudaCheck(cudaStreamSynchronize(st), "search: synchronize");
-        if (impl_->hostStatus[0] != 0) {
-            impl_->lastStatus = impl_->hostStatus[0];
-            throwDeviceStatus(impl_->hostStatus[0], "search");
+        if (const int32_t word = statusWord(impl_->status)) {
+            impl_->lastStatus = word;
+            throwDeviceStatus(word, "search");
         }
     }
 }
@@ -889,6 +894,7 @@ bool B200IndexFlat::searchFromGraph(faiss::idx_t n, const float* x, faiss::idx_t
             uint8_t* region = static_cast<uint8_t*>(e.region);
             B200FSearchArgs a;
             im.fillArgs(a, ntotal);
+            a.status = reinterpret_cast<int32_t*>(e.host + e.hostStatusOff);
             a.queries = reinterpret_cast<const float*>(region + L.offQueries);
             a.nq = n;
             a.k = (int)k;
@@ -900,15 +906,21 @@ bool B200IndexFlat::searchFromGraph(faiss::idx_t n, const float* x, faiss::idx_t
             a.scratch = region + L.offScratch;
             a.scratch_bytes = L.scratchBytes;
             cudaCheck(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "search: begin capture");
-            cudaError_t ce = cudaMemcpyAsync(region + L.offQueries, e.host, (size_t)n * d * 4, cudaMemcpyHostToDevice, st);
-            int rc = ce == cudaSuccess ? b200f_search(&a) : B200F_ERR_CUDA;
+            // a few KB of queries are fetched by a kernel: a graph's next node starts 10 us after a copy from the host
+            // (single query of d = 128 on 100,000 rows), at once after a kernel
+            cudaError_t ce = cudaSuccess;
+            int rc = B200F_OK;
+            if ((size_t)n * d * 4 <= kGraphFetchBytes)
+                rc = b200f_load_rows(e.host, B200F_STORAGE_F32, n, d, d, reinterpret_cast<float*>(region + L.offQueries), st);
+            else
+                ce = cudaMemcpyAsync(region + L.offQueries, e.host, (size_t)n * d * 4, cudaMemcpyHostToDevice, st);
+            if (ce != cudaSuccess) rc = B200F_ERR_CUDA;
+            if (rc == B200F_OK) rc = b200f_search(&a);
             if (rc == B200F_OK) {
                 if (!direct)
                     ce = cudaMemcpyAsync(e.host + e.hostDistOff, a.out_dist, (size_t)n * k * 4, cudaMemcpyDeviceToHost, st);
                 if (!direct && ce == cudaSuccess)
                     ce = cudaMemcpyAsync(e.host + e.hostLabOff, a.out_labels, (size_t)n * k * 8, cudaMemcpyDeviceToHost, st);
-                if (ce == cudaSuccess)
-                    ce = cudaMemcpyAsync(e.host + e.hostStatusOff, im.status, 16, cudaMemcpyDeviceToHost, st);
                 if (ce != cudaSuccess) rc = B200F_ERR_CUDA;
             }
             cudaError_t ee = cudaStreamEndCapture(st, &e.graph);   // always ends the capture
@@ -932,7 +944,7 @@ bool B200IndexFlat::searchFromGraph(faiss::idx_t n, const float* x, faiss::idx_t
     cudaCheck(cudaStreamSynchronize(st), "search: synchronize");
     std::memcpy(distances, g->host + g->hostDistOff, (size_t)n * k * 4);
     std::memcpy(labels, g->host + g->hostLabOff, (size_t)n * k * 8);
-    const int32_t word = *reinterpret_cast<const int32_t*>(g->host + g->hostStatusOff);
+    const int32_t word = statusWord(reinterpret_cast<const int32_t*>(g->host + g->hostStatusOff));
     im.lastStatus = word;
     if (word != 0) throwDeviceStatus(word, "search");
     return true;
@@ -974,12 +986,10 @@ void B200IndexFlat::searchDeviceEnqueue(faiss::idx_t n, const float* x, faiss::i
 void B200IndexFlat::synchronize() const {
     DeviceGuard g(impl_->res->getDevice());
     cudaStream_t st = impl_->stream();
-    cudaCheck(cudaMemcpyAsync(impl_->hostStatus, impl_->status, 16, cudaMemcpyDeviceToHost, st),
-              "synchronize: status copy");
     cudaCheck(cudaStreamSynchronize(st), "synchronize");
-    if (impl_->hostStatus[0] != 0) {
-        impl_->lastStatus = impl_->hostStatus[0];
-        throwDeviceStatus(impl_->hostStatus[0], "search");
+    if (const int32_t word = statusWord(impl_->status)) {
+        impl_->lastStatus = word;
+        throwDeviceStatus(word, "search");
     }
 }
 
@@ -989,8 +999,7 @@ void B200IndexFlat::synchronize() const {
 struct B200SearchToken::Impl {
     std::shared_ptr<B200Resources> res;
     void* region = nullptr;       // device: queries, outputs, scratch
-    int32_t* status = nullptr;    // device int32[4 * nbatches]
-    uint8_t* host = nullptr;      // pinned: staged queries, result staging, status
+    uint8_t* host = nullptr;      // pinned: staged queries, result staging, status words (written by the kernels)
     size_t hostDistOff = 0, hostLabOff = 0, hostStatusOff = 0;
     int64_t n = 0, k = 0;
     int nbatches = 0;
@@ -1008,7 +1017,7 @@ struct B200SearchToken::Impl {
             int prev = -1;
             (void)cudaGetDevice(&prev);
             (void)cudaSetDevice(res->getDevice());
-            if (!finished && (region || status || host)) {
+            if (!finished && (region || host)) {
                 // dropped before its work was waited for: everything of this token is in front of `done`
                 if (!done || cudaEventSynchronize(done) != cudaSuccess) {
                     (void)cudaGetLastError();
@@ -1019,7 +1028,6 @@ struct B200SearchToken::Impl {
             }
             if (done) res->releaseEvent(reinterpret_cast<EventHandle>(done));
             if (region) res->releaseDeviceTemp(region);
-            if (status) res->releaseDeviceTemp(status);
             if (host) res->releasePinnedTemp(host);
             if (prev >= 0) (void)cudaSetDevice(prev);
         } else {
@@ -1027,7 +1035,6 @@ struct B200SearchToken::Impl {
         }
         done = nullptr;
         region = nullptr;
-        status = nullptr;
         host = nullptr;
     }
     ~Impl() { release(); }
@@ -1066,7 +1073,7 @@ void B200SearchToken::wait() {
             std::memcpy(impl_->userLabels, impl_->host + impl_->hostLabOff, (size_t)impl_->n * impl_->k * 8);
         const int32_t* hs = reinterpret_cast<const int32_t*>(impl_->host + impl_->hostStatusOff);
         int bad = 0;
-        for (int b = 0; b < impl_->nbatches; b++) bad |= hs[4 * b];
+        for (int b = 0; b < impl_->nbatches; b++) bad |= statusWord(hs + 4 * b);
         impl_->release();
         if (bad)
             throwDeviceStatus(bad, "async search");
@@ -1112,7 +1119,6 @@ B200SearchToken B200IndexFlat::searchAsync(faiss::idx_t n, const float* x, faiss
     // per-call buffers: the token owns them (src/MetalIndexFlat.mm:441-476)
     CallLayout L = makeLayout(n, batch, d, k, !qOnDevice, n, true, scratchBytes);
     t->region = impl_->res->acquireDeviceTemp(L.total);
-    t->status = static_cast<int32_t*>(impl_->res->acquireDeviceTemp(align256((size_t)t->nbatches * 16)));
     size_t hoff = 0;
     const size_t hostQOff = hoff;
     if (!qOnDevice) hoff += align256((size_t)n * d * 4);
@@ -1162,7 +1168,7 @@ B200SearchToken B200IndexFlat::searchAsync(faiss::idx_t n, const float* x, faiss
         a.out_labels = dLabAll + (size_t)q0 * k;
         a.scratch = region + L.offScratch;
         a.scratch_bytes = L.scratchBytes;
-        a.status = t->status + 4 * b;
+        a.status = reinterpret_cast<int32_t*>(t->host + t->hostStatusOff) + 4 * b;
         abiCheck(b200f_search(&a), "searchAsync");
     }
     if (down != st) {
@@ -1177,9 +1183,6 @@ B200SearchToken B200IndexFlat::searchAsync(faiss::idx_t n, const float* x, faiss
         cudaCheck(cudaMemcpyAsync(t->host + t->hostLabOff, dLabAll, (size_t)n * k * 8,
                                   cudaMemcpyDeviceToHost, down),
                   "searchAsync: labels copy");
-    cudaCheck(cudaMemcpyAsync(t->host + t->hostStatusOff, t->status, (size_t)t->nbatches * 16,
-                              cudaMemcpyDeviceToHost, down),
-              "searchAsync: status copy");
     cudaCheck(cudaEventRecord(t->done, down), "event record");
     return B200SearchToken(std::move(t));
 }

@@ -214,7 +214,7 @@ typedef struct B200FSearchArgs {
     int64_t* out_labels;     /* device [nq][k]; tail -1                                     */
     void* scratch;           /* device, >= b200f_search_scratch_bytes(), 256-byte aligned   */
     size_t scratch_bytes;
-    int32_t* status;         /* device int32[4], zeroed by the call; [0] != 0 after the
+    int32_t* status;         /* int32[4] in device or pinned host memory, zeroed by the call; [0] != 0 after the
                                 stream drains means a bounded device wait ran out          */
     void* stream;
     int32_t path;            /* B200F_PATH_*                                                */
