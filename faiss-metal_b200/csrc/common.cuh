@@ -141,10 +141,12 @@ ScanPlan plan_scan(int64_t nq, int64_t nb, int d, int storage, int sm_count);
 int launch_scan_topk(const B200FSearchArgs& a, const ScanPlan& plan, float* part_key,
                      int32_t* part_idx, int* out_P, bool stream_f32, const float* thr, const int* guard,
                      const Launch& ln);
-// Scan that stores keys (smaller = better) to a matrix [nq][ld] for columns [col0, col0+ncols); with
-// stride > 1 column c is one of rows [(col0 + c) * stride, (col0 + c + 1) * stride) of the shard.
-int launch_scan_store(const B200FSearchArgs& a, int64_t col0, int64_t ncols, int64_t stride, float* out,
-                      int64_t ld, int sm_count, const int* guard, const Launch& ln);
+// Scan that stores keys (smaller = better) to a matrix [nq][ld] for columns [col0, col0+ncols).
+int launch_scan_store(const B200FSearchArgs& a, int64_t col0, int64_t ncols, float* out, int64_t ld, int sm_count,
+                      const int* guard, const Launch& ln);
+// Keys of a sample: column c < ncols is one of rows [c * stride, (c + 1) * stride) of the shard.  Only for the launch
+// that follows prepare_queries (see sample_kernel).
+int launch_scan_sample(const B200FSearchArgs& a, int64_t ncols, int64_t stride, float* out, int64_t ld, const Launch& ln);
 // Scan that appends every row whose key is <= thr[q] to the query's candidate buffer
 // cand_key / cand_idx [nq][cap]; cand_cnt[q] (zeroed by the caller) counts every hit.
 int launch_scan_filter(const B200FSearchArgs& a, const float* thr, float* cand_key, int32_t* cand_idx,

@@ -51,8 +51,7 @@ struct ScanParams {
     const int* guard;       // optional: *guard == 0 in device memory leaves at once
     float* out;             // store mode: [nq][ld]
     int64_t ld;
-    int row_stride;         // store mode: 1, or one row in row_stride (see sample_offset): pitch_bytes then spans such a step
-    int64_t row_bytes;      // store mode: from one row to the next
+    int row_stride;         // sample_kernel: one row in row_stride
     float* cand_key;        // filter mode: [nq][cand_cap]
     int32_t* cand_idx;
     int32_t* cand_cnt;      // [nq]
@@ -212,16 +211,6 @@ __device__ __forceinline__ void filter_append(const ScanParams& p, int qi, float
     }
 }
 
-// Store mode over a sample of one row in `stride`: column c is row c stride + sample_offset(j, stride), j the eight
-// columns of a lane group's turn that share it (a column by itself: 16 integer operations a row, 3 us of a
-// sample's 16).  Moving by the golden ratio it takes every place of the stride equally often.  Every
-// stride-th row would always be the same of rows that repeat with a period (chunks of a document, augmentations of
-// an image): their thresholds admitted too few rows or too many, and the scan was done twice (eight queries, k = 1000,
-// 1.5 M fp32 rows of d = 64 in groups of 8: 911 us, 183 for the same rows shuffled; now 185).
-__device__ __forceinline__ int64_t sample_offset(int64_t j, int stride) {
-    return __umulhi((uint32_t)j * 2654435769u, (uint32_t)stride);
-}
-
 enum { SCAN_TOPK = 0, SCAN_STORE = 1, SCAN_FILTER = 2 };
 
 template <int STORAGE, int NQ, int MODE>
@@ -283,8 +272,6 @@ scan_kernel(const ScanParams p) {
 
     for (int64_t blk = gw; blk < nblocks; blk += total_warps) {
         const int64_t row_base = p.col0 + blk * rows_per_block;
-        const int64_t offset = STORE ? sample_offset(blk * rps + sub, p.row_stride) : 0;
-        const uint8_t* const rows = base + (STORE ? offset * p.row_bytes : 0);
         float acc[U][NQ];
 #pragma unroll
         for (int u = 0; u < U; u++)
@@ -309,7 +296,7 @@ scan_kernel(const ScanParams p) {
             for (int u = 0; u < U; u++) {
                 const int64_t row = row_base + u * rps + sub;
                 if (pv && row < p.col1)
-                    v[u] = ldg_stream(rows + row * p.pitch_bytes + (int64_t)piece * 16);
+                    v[u] = ldg_stream(base + row * p.pitch_bytes + (int64_t)piece * 16);
                 else
                     v[u] = make_uint4(0, 0, 0, 0);
             }
@@ -432,7 +419,7 @@ scan_kernel(const ScanParams p) {
             const int64_t row = row_base + u * rps + sub;
             const bool owner = (cl == 0) && row < p.col1;
             float nrm = 0.f;
-            if (!PREVOTE && owner && l2) nrm = __ldg(p.norms + (STORE ? row * p.row_stride + offset : row));
+            if (!PREVOTE && owner && l2) nrm = __ldg(p.norms + row);
 #pragma unroll
             for (int qi = 0; qi < NQ; qi++) {
                 const float key = PREVOTE ? acc[u][qi] : (l2 ? fmaf(-2.f, acc[u][qi], nrm) : -acc[u][qi]);
@@ -1050,6 +1037,88 @@ __global__ void __launch_bounds__(ST_THREADS, 1) scan_tf32_kernel(const ScanPara
     }
 }
 
+// Keys of a sample of one row in `stride` for up to NQ queries: column c of the output is row c stride + a
+// place in its stride that moves by the golden ratio and takes every one equally often: every stride-th row
+// would always be the same of rows that repeat with a period (chunks of a document, augmentations of an image), their
+// thresholds admitted too few rows or too many, and the scan was done twice (eight queries, k = 1000, 1.5 M fp32
+// rows of d = 64 in groups of 8: 911 us, 183 for the same rows shuffled).
+// A few thousand scattered rows: bound by latency, so eight lanes share a row, every row has lanes of its own, and its
+// pieces, up to eight a lane, are on their way before the queries are staged.  Nothing of that was written by the kernel
+// before (prepare_queries, which itself starts behind whatever wrote rows or queries), so only the stores wait for it.
+// Six queries, 9,766 rows of d = 100: two launches of the scan took 20 us; the search (k = 32, 2.5 M fp32 rows)
+// 241 -> 228.5 us with this one.
+constexpr int SAMPLE_THREADS = 256;
+constexpr int SAMPLE_LPR = 8;
+
+__device__ __forceinline__ int64_t sample_offset(int64_t j, int stride) {
+    return __umulhi((uint32_t)j * 2654435769u, (uint32_t)stride);
+}
+
+template <int STORAGE, int NQ>
+__global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(const ScanParams p) {
+    constexpr int E = Piece<STORAGE>::E, U = 8;
+    extern __shared__ __align__(16) float sq[];   // [NQ][qstride] queries, zero padded to whole pieces
+    const int cl = threadIdx.x & (SAMPLE_LPR - 1);
+    const int64_t c = ((int64_t)blockIdx.x * SAMPLE_THREADS + threadIdx.x) / SAMPLE_LPR;
+    const bool live = c < p.col1;
+    // eight columns, one after the other among the rows a warp of scan_kernel takes at a time, share a place
+    const int step = 32 / p.lpr;
+    const int64_t row = live ? c * p.row_stride + sample_offset(c / (8 * step) * step + c % step, p.row_stride) : 0;
+    const uint8_t* src = reinterpret_cast<const uint8_t*>(p.rows) + row * p.pitch_bytes;
+    uint4 v[U];
+    auto load = [&](int piece0) {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int piece = piece0 + u * SAMPLE_LPR + cl;
+            v[u] = live && piece < p.C ? ldg_stream(src + (int64_t)piece * 16) : make_uint4(0, 0, 0, 0);
+        }
+    };
+    load(0);
+    const float nrm = live && p.norms ? __ldg(p.norms + row) : 0.f;
+    for (int i = threadIdx.x; i < NQ * p.qstride; i += SAMPLE_THREADS) {
+        const int qi = i / p.qstride;
+        const int j = i - qi * p.qstride;
+        sq[i] = qi < p.nq && j < p.d ? p.queries[(int64_t)qi * p.d + j] : 0.f;
+    }
+    __syncthreads();
+    float acc[NQ];
+#pragma unroll
+    for (int qi = 0; qi < NQ; qi++) acc[qi] = 0.f;
+    for (int piece0 = 0;;) {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int piece = piece0 + u * SAMPLE_LPR + cl;
+            if (piece >= p.C) break;
+            float x[E];
+            unpack<STORAGE>(v[u], x);
+#pragma unroll
+            for (int qi = 0; qi < NQ; qi++) {
+                const float4* q4 = reinterpret_cast<const float4*>(sq + qi * p.qstride + piece * E);
+#pragma unroll
+                for (int e = 0; e < E; e += 4) {
+                    const float4 f = q4[e / 4];
+                    acc[qi] = fmaf(f.x, x[e], acc[qi]);
+                    acc[qi] = fmaf(f.y, x[e + 1], acc[qi]);
+                    acc[qi] = fmaf(f.z, x[e + 2], acc[qi]);
+                    acc[qi] = fmaf(f.w, x[e + 3], acc[qi]);
+                }
+            }
+        }
+        piece0 += U * SAMPLE_LPR;
+        if (piece0 >= p.C) break;
+        load(piece0);
+    }
+    pdl_wait();
+    pdl_trigger();
+#pragma unroll
+    for (int qi = 0; qi < NQ; qi++) {
+#pragma unroll
+        for (int o = SAMPLE_LPR / 2; o > 0; o >>= 1) acc[qi] += __shfl_xor_sync(FULL, acc[qi], o);
+        if (cl == (qi & (SAMPLE_LPR - 1)) && live && qi < p.nq)
+            p.out[(int64_t)qi * p.ld + c] = p.norms ? fmaf(-2.f, acc[qi], nrm) : -acc[qi];
+    }
+}
+
 // Candidates of a filter whose keys are bounds, scored again in fp32 (L2): eight lanes share a candidate's row
 // and two rows are in flight per lane group; a few us, bound by latency.  blockIdx.x is the query, blockIdx.y its share of the candidates.
 constexpr int RC_THREADS = 256;
@@ -1326,18 +1395,16 @@ int launch_scan_topk(const B200FSearchArgs& a, const ScanPlan& plan, float* part
     return launch_storage<SCAN_TOPK>(p, a.storage, plan.grid, ln);
 }
 
-int launch_scan_store(const B200FSearchArgs& a, int64_t col0, int64_t ncols, int64_t stride, float* out, int64_t ld,
-                      int sm_count, const int* guard, const Launch& ln) {
-    if (a.nq < 1 || a.nq > 4 || stride < 1 || stride > 0x7fffffffLL) return B200F_ERR_UNSUPPORTED;
+int launch_scan_store(const B200FSearchArgs& a, int64_t col0, int64_t ncols, float* out, int64_t ld, int sm_count,
+                      const int* guard, const Launch& ln) {
+    if (a.nq < 1 || a.nq > 4) return B200F_ERR_UNSUPPORTED;
     if (ncols <= 0) return B200F_OK;
     ScanParams p{};
-    fill_geometry(p, a.storage, a.d, a.row_pitch * stride, a.metric == B200F_METRIC_L2 ? a.norm_cols : 0,
+    fill_geometry(p, a.storage, a.d, a.row_pitch, a.metric == B200F_METRIC_L2 ? a.norm_cols : 0,
                   lanes_per_row_cap(a.nq));
     p.queries = a.queries;
     p.rows = a.rows;
     p.norms = a.norms;
-    p.row_stride = (int)stride;
-    p.row_bytes = p.pitch_bytes / stride;
     p.nb = a.nb;
     p.col0 = col0;
     p.col1 = col0 + ncols;
@@ -1352,6 +1419,43 @@ int launch_scan_store(const B200FSearchArgs& a, int64_t col0, int64_t ncols, int
                                       scan_grid(ncols, a.d, a.storage, sm_count, lanes_per_row_cap(a.nq),
                                                 resident_ctas(a.nq, a.storage, true)),
                                       ln);
+}
+
+int launch_scan_sample(const B200FSearchArgs& a, int64_t ncols, int64_t stride, float* out, int64_t ld, const Launch& ln) {
+    if (a.nq < 1 || stride < 1 || stride > 0x7fffffffLL || ncols * stride > a.nb) return B200F_ERR_BAD_ARG;
+    if (ncols <= 0) return B200F_OK;
+    ScanParams p{};
+    fill_geometry(p, a.storage, a.d, a.row_pitch, 0, SAMPLE_LPR);
+    p.rows = a.rows;
+    p.norms = a.metric == B200F_METRIC_L2 ? a.norms : nullptr;
+    p.d = a.d;
+    p.row_stride = (int)stride;
+    p.col1 = ncols;
+    p.ld = ld;
+    const dim3 grid((unsigned)ceil_div64(ncols * SAMPLE_LPR, SAMPLE_THREADS));
+    // eight queries a launch, fewer where they are long (64 KB of them)
+    const int64_t query_bytes = (int64_t)p.qstride * 4;
+    int group = 8;
+    while (group > 1 && (group / 2 >= a.nq || group * query_bytes > 64 * 1024)) group /= 2;
+    if (group * query_bytes > 200 * 1024) return B200F_ERR_UNSUPPORTED;
+    const size_t smem = (size_t)(group * query_bytes);
+    typedef void (*KernelFn)(const ScanParams);
+#define B200F_SAMPLE(ST) {sample_kernel<ST, 1>, sample_kernel<ST, 2>, sample_kernel<ST, 4>, sample_kernel<ST, 8>}
+    static const KernelFn kernels[3][4] = {B200F_SAMPLE(B200F_STORAGE_F32), B200F_SAMPLE(B200F_STORAGE_F16),
+                                           B200F_SAMPLE(B200F_STORAGE_BF16)};
+#undef B200F_SAMPLE
+    const KernelFn kernel = kernels[a.storage][group == 1 ? 0 : group == 2 ? 1 : group == 4 ? 2 : 3];
+    if (smem > 48 * 1024)
+        B200F_CUDA_TRY(cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
+                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    for (int64_t q0 = 0; q0 < a.nq; q0 += group) {
+        p.queries = a.queries + q0 * (int64_t)a.d;
+        p.nq = (int)(a.nq - q0 < group ? a.nq - q0 : group);
+        p.out = out + q0 * ld;
+        B200F_CUDA_TRY(launch_kernel(kernel, grid, SAMPLE_THREADS, smem, ln, p));
+        count_launch();
+    }
+    return B200F_OK;
 }
 
 int launch_scan_filter(const B200FSearchArgs& a, const float* thr, float* cand_key, int32_t* cand_idx,

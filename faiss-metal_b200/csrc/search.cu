@@ -865,11 +865,8 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
     };
     if (pl.sample) {
         float* keys = reinterpret_cast<float*>(scratch + pl.off_sample);
-        for (int64_t q0 = 0; q0 < a->nq; q0 += SCAN_GROUP) {
-            rc = launch_scan_store(query_group(q0, SCAN_GROUP), 0, pl.nsample, pl.fstride, keys + q0 * pl.nsample,
-                                   pl.nsample, sm, nullptr, ln);
-            if (rc != B200F_OK) return rc;
-        }
+        rc = launch_scan_sample(*a, pl.nsample, pl.fstride, keys, pl.nsample, ln);
+        if (rc != B200F_OK) return rc;
         rc = launch_row_bound(keys, a->nq, pl.nsample, pl.nsample, pl.frank, thr, bad, qnorm, margin, qnorm_max, most, ln);
         if (rc != B200F_OK) return rc;
     }
@@ -982,7 +979,7 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
             if (rc != B200F_OK) return rc;
         } else {
             for (int64_t q0 = 0; q0 < a->nq; q0 += SCAN_GROUP) {
-                rc = launch_scan_store(query_group(q0, SCAN_GROUP), c0, nc, 1, matrix + q0 * pl.chunk_cols,
+                rc = launch_scan_store(query_group(q0, SCAN_GROUP), c0, nc, matrix + q0 * pl.chunk_cols,
                                        pl.chunk_cols, sm, nq_dev, ln);
                 if (rc != B200F_OK) return rc;
             }
@@ -1054,7 +1051,7 @@ extern "C" int b200f_pairwise(const B200FSearchArgs* a, float* out_matrix, int64
         B200FSearchArgs sub = *a;
         sub.queries = a->queries + g * SCAN_GROUP * (int64_t)a->d;
         sub.nq = (a->nq - g * SCAN_GROUP) < SCAN_GROUP ? (a->nq - g * SCAN_GROUP) : SCAN_GROUP;
-        rc = launch_scan_store(sub, 0, a->nb, 1, out_matrix + g * SCAN_GROUP * ld_out, ld_out, sm, nullptr, st);
+        rc = launch_scan_store(sub, 0, a->nb, out_matrix + g * SCAN_GROUP * ld_out, ld_out, sm, nullptr, st);
         if (rc != B200F_OK) return rc;
     }
     const int64_t total = a->nq * a->nb;

@@ -42,3 +42,17 @@ def test_keys_that_are_no_numbers_or_infinite(fm, res):
     assert I[0, 20:30].tolist() == list(range(10, 20)) and np.isposinf(D[0, 20:30]).all()
     assert (I[0, 30:] == -1).all()
     idx.close()
+
+
+@pytest.mark.parametrize("storage,d,nq", [(0, 2100, 8), (0, 257, 5), (2, 1000, 8), (1, 24, 7)])
+def test_sample_of_wide_and_narrow_rows(fm, res, storage, d, nq):
+    # more pieces than the sample's lanes hold at a time, and more queries than share a launch
+    nb, k = 40_000, 40
+    xb = H.gaussian(nb, d, 5)
+    xq = H.gaussian(nq, d, 6)
+    idx = fm.B200IndexFlat(res, d, O.METRIC_L2, storage)
+    idx.set_path(1)
+    idx.add(xb)
+    D, I = idx.search(xq, k)
+    H.check_against_oracle(O.METRIC_L2, storage, False, xb, xq, k, D, I, strict=storage == 0)
+    idx.close()
