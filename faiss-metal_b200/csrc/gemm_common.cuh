@@ -197,6 +197,16 @@ __device__ __forceinline__ void tc_ld64(uint32_t taddr, uint32_t (&r)[64]) {
             : "r"(taddr)
             : "memory");
 }
+// The same wait, tied to the registers of one load: nothing that reads them moves in front of it.
+__device__ __forceinline__ void tc_wait_ld32(uint32_t (&r)[32]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]),
+                   "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]),
+                   "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
+                 :
+                 : "memory");
+}
 // one 32-byte sector of a row
 __device__ __forceinline__ void st_global_v8(float* dst, const float (&v)[8]) {
     asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "f"(v[0]), "f"(v[1]), "f"(v[2]),
@@ -257,6 +267,64 @@ __device__ __forceinline__ void drain_to_buffer(int32_t* cnt, float* ck, int32_t
             ck[base + i] = kscale * sk[i * STAGE_LD];
             ci[base + i] = si[i * STAGE_LD];
         }
+    }
+}
+
+// MODE_FILTER: 32 accumulator columns of a thread's row, hits (-r < thr) to the thread's stage.  All lanes of the warp call
+// it.  The largest of every group of eight columns, then of all; the groups that hold a hit of any row are gone through
+// column by column.
+template <typename Drain>
+__device__ __forceinline__ void filter_columns(uint32_t (&r)[32], int64_t cbase, int64_t ncols_end, bool partial, const float& thr,
+                                               float* stage_key, int32_t* stage_idx, int& nstaged, Drain drain) {
+    if (partial) {   // columns beyond the end were zero-filled
+#pragma unroll
+        for (int c = 0; c < 32; c++)
+            if (cbase + c >= ncols_end) r[c] = 0xff800000u;   // -INF
+    }
+    float gm[4];
+#pragma unroll
+    for (int g = 0; g < 4; g++) {
+        const float a = max3(__uint_as_float(r[8 * g]), __uint_as_float(r[8 * g + 1]), __uint_as_float(r[8 * g + 2]));
+        const float b = max3(__uint_as_float(r[8 * g + 3]), __uint_as_float(r[8 * g + 4]), __uint_as_float(r[8 * g + 5]));
+        gm[g] = max3(fmaxf(__uint_as_float(r[8 * g + 6]), __uint_as_float(r[8 * g + 7])), a, b);
+    }
+    if (!__any_sync(0xffffffffu, -fmaxf(max3(gm[0], gm[1], gm[2]), gm[3]) < thr)) return;
+#pragma unroll
+    for (int g = 0; g < 4; g++) {
+        const bool hit = -gm[g] < thr;
+        if (!__any_sync(0xffffffffu, hit)) continue;
+        if (hit) {
+            if (nstaged > STAGE_N - 8) drain();   // rare: massive ties
+#pragma unroll
+            for (int c = 0; c < 8; c++) {
+                const float sc = -__uint_as_float(r[8 * g + c]);
+                if (sc < thr) {
+                    stage_key[nstaged * STAGE_LD] = sc;
+                    stage_idx[nstaged * STAGE_LD] = (int32_t)cbase + 8 * g + c;
+                    nstaged++;
+                }
+            }
+        }
+    }
+    __syncwarp();
+}
+
+// NCH x 32 accumulator columns from taddr on, through `use(registers, chunk)`: a chunk is used while the next one is on
+// its way, and `release` is called once the last one has arrived.
+template <int NCH, typename Use, typename Release>
+__device__ __forceinline__ void scan_columns(uint32_t taddr, Use use, Release release) {
+    static_assert(NCH % 2 == 0, "chunks are taken in pairs");
+    uint32_t a[32], b[32];
+    tc_ld32(taddr, a);
+#pragma unroll 1
+    for (int ch = 0; ch < NCH; ch += 2) {
+        tc_wait_ld32(a);
+        tc_ld32(taddr + (ch + 1) * 32, b);
+        use(a, ch);
+        tc_wait_ld32(b);
+        if (ch + 2 < NCH) tc_ld32(taddr + (ch + 2) * 32, a);
+        else release();
+        use(b, ch + 1);
     }
 }
 

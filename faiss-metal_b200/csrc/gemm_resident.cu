@@ -19,8 +19,6 @@
 // Against the pair shape of gemm_topk.cu: 2,048 queries, k = 1024, 5 M fp32 rows of d = 96: 8.15 -> 6.08 ms a search;
 // 1,000 queries, k = 10, 100,000 fp32 rows of d = 128: 189 -> 156 us.  Bound by the epilogue (tensor pipe 50 % busy where
 // one column in 400 is a hit).
-#include <type_traits>
-
 #include "gemm_common.cuh"
 
 namespace b200f {
@@ -277,6 +275,11 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
             } else if (row_live && p.rowadd) {
                 radd = p.rowadd[grow];
             }
+            auto drain = [&]() {
+                drain_to_buffer(p.cand_cnt + grow, p.cand_key + grow * p.cand_cap, p.cand_idx + grow * p.cand_cap,
+                                p.cand_cap, ksc, stage_key, stage_idx, nstaged);
+                nstaged = 0;
+            };
             for (int64_t t = t0; t < t1; t++) {
                 const int64_t c_tile = tile_col(t);
                 {
@@ -288,96 +291,42 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                 }
                 tc_fence_after();
                 const bool partial = c_tile + RES_TILE_N > p.ncols_end;
-                const uint32_t taddr = tmem_base + ((uint32_t)(ew * 32) << 16) + acc * RES_TILE_N;
+                const uint32_t taddr = tmem_base + ((uint32_t)(ew * 32) << 16) + acc * RES_TILE_N + eh * (RES_TILE_N / 2);
+                const int64_t cbase = c_tile + eh * (RES_TILE_N / 2);
+                auto release = [&]() {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(tempty0 + acc * 8);
+                };
                 if constexpr (MODE == MODE_FILTER) {
-                    auto scan = [&](auto cw_tag) {
-                        constexpr int CW = decltype(cw_tag)::value;
-#pragma unroll 1
-                        for (int ch = 0; ch < RES_TILE_N / 2 / CW; ch++) {
-                            uint32_t r[CW];
-                            const int col = eh * (RES_TILE_N / 2) + ch * CW;
-                            if constexpr (CW == 64) tc_ld64(taddr + col, r);
-                            else tc_ld32(taddr + col, r);
-                            tc_wait_ld();
-                            const int64_t cbase = c_tile + col;
-                            if (partial) {
-#pragma unroll
-                                for (int c = 0; c < CW; c++)
-                                    if (cbase + c >= p.ncols_end) r[c] = 0xff800000u;   // -INF
-                            }
-                            // the largest of every group of eight columns, then of all
-                            constexpr int NG = CW / 8;
-                            float gm[NG];
-#pragma unroll
-                            for (int g = 0; g < NG; g++) {
-                                const float a = max3(__uint_as_float(r[8 * g]), __uint_as_float(r[8 * g + 1]), __uint_as_float(r[8 * g + 2]));
-                                const float b = max3(__uint_as_float(r[8 * g + 3]), __uint_as_float(r[8 * g + 4]), __uint_as_float(r[8 * g + 5]));
-                                gm[g] = max3(fmaxf(__uint_as_float(r[8 * g + 6]), __uint_as_float(r[8 * g + 7])), a, b);
-                            }
-                            float m = gm[0];
-#pragma unroll
-                            for (int g = 1; g + 1 < NG; g += 2) m = max3(m, gm[g], gm[g + 1]);
-                            m = fmaxf(m, gm[NG - 1]);
-                            // Entered by the whole warp when any row has a candidate: the groups that hold
-                            // one, column by column, each hit to its thread's stage.
-                            if (__any_sync(0xffffffffu, -m < thr)) {
-#pragma unroll
-                                for (int g = 0; g < NG; g++) {
-                                    const bool hit = -gm[g] < thr;
-                                    if (!__any_sync(0xffffffffu, hit)) continue;
-                                    if (hit) {
-                                        if (nstaged > STAGE_N - 8) {
-                                            drain_to_buffer(p.cand_cnt + grow, p.cand_key + grow * p.cand_cap,
-                                                            p.cand_idx + grow * p.cand_cap, p.cand_cap, ksc, stage_key,
-                                                            stage_idx, nstaged);
-                                            nstaged = 0;
-                                        }
-#pragma unroll
-                                        for (int c = 0; c < 8; c++) {
-                                            const float sc = -__uint_as_float(r[8 * g + c]);
-                                            if (sc < thr) {
-                                                stage_key[nstaged * STAGE_LD] = sc;
-                                                stage_idx[nstaged * STAGE_LD] = (int32_t)cbase + 8 * g + c;
-                                                nstaged++;
-                                            }
-                                        }
-                                    }
-                                }
-                                __syncwarp();
-                            }
-                        }
-                    };
-                    if (p.wide) scan(std::integral_constant<int, 64>{});
-                    else scan(std::integral_constant<int, 32>{});
+                    scan_columns<RES_TILE_N / 64>(
+                            taddr,
+                            [&](uint32_t(&r)[32], int ch) {
+                                filter_columns(r, cbase + ch * 32, p.ncols_end, partial, thr, stage_key, stage_idx, nstaged, drain);
+                            },
+                            release);
                 } else {
                     const bool whole = !partial && (p.ld & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
-#pragma unroll 1
-                    for (int ch = eh * 4; ch < eh * 4 + 4; ch++) {
-                        uint32_t r[32];
-                        tc_ld32(taddr + ch * 32, r);
-                        tc_wait_ld();
-                        store_keys(p, r, whole, grow, lane, nq_live, row_live, c_tile + ch * 32, t * RES_TILE_N + ch * 32, ksc,
-                                   radd, reinterpret_cast<float*>(smem + RES_SM_STAGE) + (warp - 2) * (32 * 33));
-                    }
+                    float* const tbuf = reinterpret_cast<float*>(smem + RES_SM_STAGE) + (warp - 2) * (32 * 33);
+                    const int64_t ocol = t * RES_TILE_N + eh * (RES_TILE_N / 2);
+                    scan_columns<RES_TILE_N / 64>(
+                            taddr,
+                            [&](uint32_t(&r)[32], int ch) {
+                                store_keys(p, r, whole, grow, lane, nq_live, row_live, cbase + ch * 32, ocol + ch * 32, ksc, radd, tbuf);
+                            },
+                            release);
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(tempty0 + acc * 8);
                 // Staged hits wait for company: an atomic's round trip each tile is a third of what a tile of 19
                 // MMAs leaves its epilogue.
                 if (MODE == MODE_FILTER && __any_sync(0xffffffffu, nstaged > STAGE_N / 2)) {
-                    drain_to_buffer(p.cand_cnt + grow, p.cand_key + grow * p.cand_cap, p.cand_idx + grow * p.cand_cap,
-                                    p.cand_cap, ksc, stage_key, stage_idx, nstaged);
-                    nstaged = 0;
+                    drain();
                     __syncwarp();
                 }
                 acc ^= 1;
                 if (acc == 0) acc_phase ^= 1;
             }
             if (MODE == MODE_FILTER) {
-                drain_to_buffer(p.cand_cnt + grow, p.cand_key + grow * p.cand_cap, p.cand_idx + grow * p.cand_cap,
-                                p.cand_cap, ksc, stage_key, stage_idx, nstaged);
-                nstaged = 0;
+                drain();
                 __syncwarp();
             }
         }

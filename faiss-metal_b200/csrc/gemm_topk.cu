@@ -407,6 +407,15 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
             } else if (row_live && p.rowadd) {
                 radd = p.rowadd[grow];
             }
+            if (MODE == MODE_TOPK && !row_live) thr_eff = -CUDART_INF_F;   // takes nothing
+            auto drain = [&]() {
+                if (MODE == MODE_TOPK)
+                    drain_to_list(lk, li, stage_key, stage_idx, nstaged, thr, thr_eff);
+                else
+                    drain_to_buffer(p.cand_cnt + grow, p.cand_key + grow * p.cand_cap, p.cand_idx + grow * p.cand_cap,
+                                    p.cand_cap, ksc, stage_key, stage_idx, nstaged);
+                nstaged = 0;
+            };
             for (int64_t t = t0; t < t1 && ok; t++) {
                 const int64_t c_tile = p.col0 + t * p.tile_stride * TILE_N;
                 {
@@ -437,114 +446,46 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
                 // column are zero-filled by TMA (t = 0) and must be masked out.
                 const bool partial = c_tile + TILE_N > p.ncols_end;
                 const uint32_t taddr = tmem_base + ((uint32_t)(ew * 32) << 16) + acc * TILE_N;
-                if constexpr (MODE != MODE_STORE) {
-                // CW columns per TMEM load.  64 saves ~3 % of the tile time when hits are rare
-                // (filter mode has the registers for it: no lists to keep); with a hit in most
-                // chunks the 64-column masks cost more than the wider load saves.
-                auto scan = [&](auto cw_tag) {
-                constexpr int CW = decltype(cw_tag)::value;
-#pragma unroll 1
-                for (int ch = 0; ch < CH_PER_HALF * 32 / CW; ch++) {
-                    uint32_t r[CW];
-                    const int col = eh * CH_PER_HALF * 32 + ch * CW;  // first column inside the tile
-                    if constexpr (CW == 64) tc_ld64(taddr + col, r);
-                    else tc_ld32(taddr + col, r);
-                    tc_wait_ld();
-                    const int64_t cbase = c_tile + col;
-                    {
-                        if (partial) {
-#pragma unroll
-                            for (int c = 0; c < CW; c++)
-                                if (cbase + c >= p.ncols_end) r[c] = 0xff800000u;  // -INF
-                        }
-                        // one max per column: of every group of eight columns, then of all
-                        constexpr int NG = CW / 8;
-                        float gm[NG];
-#pragma unroll
-                        for (int g = 0; g < NG; g++) {
-                            float m4[4];
-#pragma unroll
-                            for (int c = 0; c < 4; c++)
-                                m4[c] = fmaxf(__uint_as_float(r[8 * g + c]), __uint_as_float(r[8 * g + 4 + c]));
-                            gm[g] = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
-                        }
-                        float m[NG];
-#pragma unroll
-                        for (int g = 0; g < NG; g++) m[g] = gm[g];
-#pragma unroll
-                        for (int w2 = NG / 2; w2 > 0; w2 >>= 1)
-#pragma unroll
-                            for (int g = 0; g < w2; g++) m[g] = fmaxf(m[g], m[g + w2]);
-                        // Slow path, entered by the whole warp when any row has a candidate in this chunk:
-                        // the groups that hold one, column by column, each hit to its thread's stage (1,000
-                        // queries, 100,000 fp32 rows of d = 128, 320 candidates a query: 243 us a search with a
-                        // mask over all columns and a select chain per hit, 222 with this).
-                        if (__any_sync(0xffffffffu, row_live && -m[0] < thr_eff)) {
-#pragma unroll
-                            for (int g = 0; g < NG; g++) {
-                                const bool hit = row_live && -gm[g] < thr_eff;
-                                if (!__any_sync(0xffffffffu, hit)) continue;
-                                if (hit) {
-                                    if (nstaged > STAGE_N - 8) {  // rare: list warm-up, massive ties
-                                        if (MODE == MODE_TOPK)
-                                            drain_to_list(lk, li, stage_key, stage_idx, nstaged, thr, thr_eff);
-                                        else
-                                            drain_to_buffer(p.cand_cnt + grow, p.cand_key + grow * p.cand_cap,
-                                                            p.cand_idx + grow * p.cand_cap, p.cand_cap,
-                                                            ksc, stage_key, stage_idx, nstaged);
-                                        nstaged = 0;
-                                    }
-#pragma unroll
-                                    for (int c = 0; c < 8; c++) {
-                                        const float sc = -__uint_as_float(r[8 * g + c]);
-                                        if (sc < thr_eff) {
-                                            stage_key[nstaged * STAGE_LD] = sc;
-                                            stage_idx[nstaged * STAGE_LD] = (int32_t)cbase + 8 * g + c;
-                                            nstaged++;
-                                        }
-                                    }
-                                }
-                            }
-                            __syncwarp();
-                        }
+                auto release = [&]() {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (PAIR) mbar_arrive_cluster(map_to_cta(bar_tempty + eh * 8, 0));
+                        else mbar_arrive(bar_tempty + acc * 8);
                     }
-                }
                 };
-                if constexpr (MODE == MODE_FILTER) {
-                    if (p.wide) scan(std::integral_constant<int, 64>{});
-                    else scan(std::integral_constant<int, 32>{});
-                } else {
-                    scan(std::integral_constant<int, 32>{});
-                }
-                } else {
-                const bool whole = !partial && (p.ld & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
+                const int64_t chalf = c_tile + eh * CH_PER_HALF * 32;   // this warp's half of the columns
+                const uint32_t thalf = taddr + eh * CH_PER_HALF * 32;
+                if constexpr (MODE == MODE_TOPK) {
 #pragma unroll 1
-                for (int ch = eh * CH_PER_HALF; ch < (eh + 1) * CH_PER_HALF; ch++) {
+                for (int ch = 0; ch < CH_PER_HALF; ch++) {
                     uint32_t r[32];
-                    tc_ld32(taddr + ch * 32, r);
+                    tc_ld32(thalf + ch * 32, r);
                     tc_wait_ld();
-                    const int64_t cbase = c_tile + ch * 32;
-                    // tiles lie side by side in the output, whatever the stride; the list area is idle in this mode
-                    store_keys(p, r, whole, grow, lane, nq_live, row_live, cbase, t * TILE_N + ch * 32, ksc, radd,
-                               reinterpret_cast<float*>(smem + SM_LKEY) + (warp - 2) * (32 * 33));
+                    filter_columns(r, chalf + ch * 32, p.ncols_end, partial, thr_eff, stage_key, stage_idx, nstaged, drain);
                 }
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) {
-                    if (PAIR) mbar_arrive_cluster(map_to_cta(bar_tempty + eh * 8, 0));
-                    else mbar_arrive(bar_tempty + acc * 8);
+                release();
+                } else if constexpr (MODE == MODE_FILTER) {
+                    scan_columns<CH_PER_HALF>(
+                            thalf,
+                            [&](uint32_t(&r)[32], int ch) {
+                                filter_columns(r, chalf + ch * 32, p.ncols_end, partial, thr_eff, stage_key, stage_idx, nstaged, drain);
+                            },
+                            release);
+                } else {
+                    const bool whole = !partial && (p.ld & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
+                    // the list area is idle in this mode; tiles lie side by side in the output, whatever the stride
+                    float* const tbuf = reinterpret_cast<float*>(smem + SM_LKEY) + (warp - 2) * (32 * 33);
+                    const int64_t ohalf = t * TILE_N + eh * CH_PER_HALF * 32;
+                    scan_columns<CH_PER_HALF>(
+                            thalf,
+                            [&](uint32_t(&r)[32], int ch) {
+                                store_keys(p, r, whole, grow, lane, nq_live, row_live, chalf + ch * 32, ohalf + ch * 32, ksc, radd, tbuf);
+                            },
+                            release);
                 }
                 // the accumulator is back with the MMA issuers: now work off the staged hits
-                if (nstaged > 0) {
-                    if (MODE == MODE_TOPK)
-                        drain_to_list(lk, li, stage_key, stage_idx, nstaged, thr, thr_eff);
-                    else
-                        drain_to_buffer(p.cand_cnt + grow, p.cand_key + grow * p.cand_cap,
-                                        p.cand_idx + grow * p.cand_cap, p.cand_cap, ksc, stage_key,
-                                        stage_idx, nstaged);
-                    nstaged = 0;
-                }
+                if (nstaged > 0) drain();
                 __syncwarp();
                 if (C::ACC_BUFS == 2) {
                     acc ^= 1;
