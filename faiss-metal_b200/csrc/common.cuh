@@ -210,6 +210,10 @@ int launch_gemm_filter(const GemmOperands& op, const GemmPlan& plan, float kscal
 int launch_gemm_store(const GemmOperands& op, const GemmPlan& plan, int64_t col0, int64_t ncols,
                       int64_t tile_stride, float kscale, float sign, const float* rowadd, float* out,
                       int64_t ld, int32_t* status, const Launch& ln);
+// Minima: out[row * ld + g] = the smallest key of columns [32 g, 32 g + 32) of the visited tiles side by side, +INF
+// where all of them lie beyond the end (ld a multiple of 8, out on a 32-byte boundary).
+int launch_gemm_minima(const GemmOperands& op, const GemmPlan& plan, int64_t ncols, int64_t tile_stride, float kscale,
+                       float* out, int64_t ld, int32_t* status, const Launch& ln);
 
 // select.cu
 // Merge P sorted partial lists (key smaller=better, int32 local ids; -1 = empty) per

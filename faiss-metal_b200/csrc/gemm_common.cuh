@@ -16,7 +16,7 @@ constexpr int UMMA_K = 16;
 constexpr int NUM_EPI_WARPS = 8;   // two per TMEM lane quarter: each takes half of the tile's columns
 constexpr int TMEM_COLS = 512;
 
-enum { MODE_TOPK = 0, MODE_STORE = 1, MODE_FILTER = 2 };
+enum { MODE_TOPK = 0, MODE_STORE = 1, MODE_FILTER = 2, MODE_MINIMA = 3 };
 
 struct GemmParams {
     int64_t nq;
@@ -270,24 +270,31 @@ __device__ __forceinline__ void drain_to_buffer(int32_t* cnt, float* ck, int32_t
     }
 }
 
-// MODE_FILTER: 32 accumulator columns of a thread's row, hits (-r < thr) to the thread's stage.  All lanes of the warp call
-// it.  The largest of every group of eight columns, then of all; the groups that hold a hit of any row are gone through
-// column by column.
-template <typename Drain>
-__device__ __forceinline__ void filter_columns(uint32_t (&r)[32], int64_t cbase, int64_t ncols_end, bool partial, const float& thr,
-                                               float* stage_key, int32_t* stage_idx, int& nstaged, Drain drain) {
-    if (partial) {   // columns beyond the end were zero-filled
+// Columns beyond the end were zero-filled: out of every comparison.
+__device__ __forceinline__ void mask_columns(uint32_t (&r)[32], int64_t cbase, int64_t ncols_end) {
 #pragma unroll
-        for (int c = 0; c < 32; c++)
-            if (cbase + c >= ncols_end) r[c] = 0xff800000u;   // -INF
-    }
-    float gm[4];
+    for (int c = 0; c < 32; c++)
+        if (cbase + c >= ncols_end) r[c] = 0xff800000u;   // -INF
+}
+// the largest of every group of eight columns
+__device__ __forceinline__ void group_maxima(const uint32_t (&r)[32], float (&gm)[4]) {
 #pragma unroll
     for (int g = 0; g < 4; g++) {
         const float a = max3(__uint_as_float(r[8 * g]), __uint_as_float(r[8 * g + 1]), __uint_as_float(r[8 * g + 2]));
         const float b = max3(__uint_as_float(r[8 * g + 3]), __uint_as_float(r[8 * g + 4]), __uint_as_float(r[8 * g + 5]));
         gm[g] = max3(fmaxf(__uint_as_float(r[8 * g + 6]), __uint_as_float(r[8 * g + 7])), a, b);
     }
+}
+
+// MODE_FILTER: 32 accumulator columns of a thread's row, hits (-r < thr) to the thread's stage.  All lanes of the warp call
+// it.  The largest of every group of eight columns, then of all; the groups that hold a hit of any row are gone through
+// column by column.
+template <typename Drain>
+__device__ __forceinline__ void filter_columns(uint32_t (&r)[32], int64_t cbase, int64_t ncols_end, bool partial, const float& thr,
+                                               float* stage_key, int32_t* stage_idx, int& nstaged, Drain drain) {
+    if (partial) mask_columns(r, cbase, ncols_end);
+    float gm[4];
+    group_maxima(r, gm);
     if (!__any_sync(0xffffffffu, -fmaxf(max3(gm[0], gm[1], gm[2]), gm[3]) < thr)) return;
 #pragma unroll
     for (int g = 0; g < 4; g++) {
@@ -311,12 +318,12 @@ __device__ __forceinline__ void filter_columns(uint32_t (&r)[32], int64_t cbase,
 
 // NCH x 32 accumulator columns from taddr on, through `use(registers, chunk)`: a chunk is used while the next one is on
 // its way, and `release` is called once the last one has arrived.
-template <int NCH, typename Use, typename Release>
+template <int NCH, int UNROLL = 1, typename Use, typename Release>
 __device__ __forceinline__ void scan_columns(uint32_t taddr, Use use, Release release) {
     static_assert(NCH % 2 == 0, "chunks are taken in pairs");
     uint32_t a[32], b[32];
     tc_ld32(taddr, a);
-#pragma unroll 1
+#pragma unroll UNROLL
     for (int ch = 0; ch < NCH; ch += 2) {
         tc_wait_ld32(a);
         tc_ld32(taddr + (ch + 1) * 32, b);
@@ -326,6 +333,15 @@ __device__ __forceinline__ void scan_columns(uint32_t taddr, Use use, Release re
         else release();
         use(b, ch + 1);
     }
+}
+
+// MODE_MINIMA: the smallest key of every MIN_GROUP columns of a thread's row; N consecutive ones to out.
+constexpr int MIN_GROUP = 32;
+template <int N>
+__device__ __forceinline__ void store_minima(const float (&v)[N], float* out) {
+    static_assert(N == 4 || N == 8, "");
+    if constexpr (N == 8) st_global_v8(out, v);
+    else *reinterpret_cast<float4*>(out) = make_float4(v[0], v[1], v[2], v[3]);
 }
 
 // Keys up to the threshold pass a filter whose comparison excludes its bound: the next float up (+INF, the

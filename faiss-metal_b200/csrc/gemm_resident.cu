@@ -305,6 +305,18 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                                 filter_columns(r, cbase + ch * 32, p.ncols_end, partial, thr, stage_key, stage_idx, nstaged, drain);
                             },
                             release);
+                } else if constexpr (MODE == MODE_MINIMA) {
+                    float v[RES_TILE_N / 64];
+                    scan_columns<RES_TILE_N / 64, RES_TILE_N / 64>(
+                            taddr,
+                            [&](uint32_t(&r)[32], int ch) {
+                                if (partial) mask_columns(r, cbase + ch * 32, p.ncols_end);
+                                float gm[4];
+                                group_maxima(r, gm);
+                                v[ch] = -ksc * fmaxf(max3(gm[0], gm[1], gm[2]), gm[3]);
+                            },
+                            release);
+                    if (row_live) store_minima(v, p.out + grow * p.ld + t * (RES_TILE_N / MIN_GROUP) + eh * (RES_TILE_N / 64));
                 } else {
                     const bool whole = !partial && (p.ld & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
                     float* const tbuf = reinterpret_cast<float*>(smem + RES_SM_STAGE) + (warp - 2) * (32 * 33);
@@ -382,11 +394,13 @@ int launch_resident(const GemmOperands& op, const GemmPlan& plan, GemmParams& g,
     const int grid = (int)(2 * (items < plan.units ? items : plan.units));
 
     typedef void (*KernelFn)(const CUtensorMap, const CUtensorMap, const ResidentParams);
-    const KernelFn kernel = g.mode == MODE_FILTER ? gemm_resident_kernel<MODE_FILTER> : gemm_resident_kernel<MODE_STORE>;
+    const KernelFn kernel = g.mode == MODE_FILTER   ? gemm_resident_kernel<MODE_FILTER>
+                            : g.mode == MODE_STORE ? gemm_resident_kernel<MODE_STORE>
+                                                   : gemm_resident_kernel<MODE_MINIMA>;
     static bool attr_set[kMaxDevices] = {false};
     const int slot = device_slot();
     if (!attr_set[slot]) {
-        for (KernelFn fn : {gemm_resident_kernel<MODE_FILTER>, gemm_resident_kernel<MODE_STORE>})
+        for (KernelFn fn : {gemm_resident_kernel<MODE_FILTER>, gemm_resident_kernel<MODE_STORE>, gemm_resident_kernel<MODE_MINIMA>})
             B200F_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, RES_SMEM_BYTES));
         attr_set[slot] = true;
     }

@@ -30,7 +30,8 @@
 //   filter  a fixed per-row threshold; every column under it is appended to the row's
 //           candidate buffer in global memory
 //   store   the keys are written out as a matrix (k beyond the list paths, pairwise distances)
-// The mode is a template parameter (six instantiations with the two shapes): the filter and
+//   minima  the smallest key of every 32 columns is (samples that thresholds are taken from)
+// The mode is a template parameter (eight instantiations with the two shapes): the filter and
 // store kernels carry no list registers, which lets the filter kernel read 64 accumulator
 // columns per TMEM load.  A work item is (query block, column range).
 //
@@ -472,6 +473,18 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
                                 filter_columns(r, chalf + ch * 32, p.ncols_end, partial, thr_eff, stage_key, stage_idx, nstaged, drain);
                             },
                             release);
+                } else if constexpr (MODE == MODE_MINIMA) {
+                    float v[CH_PER_HALF];
+                    scan_columns<CH_PER_HALF, CH_PER_HALF>(
+                            thalf,
+                            [&](uint32_t(&r)[32], int ch) {
+                                if (partial) mask_columns(r, chalf + ch * 32, p.ncols_end);
+                                float gm[4];
+                                group_maxima(r, gm);
+                                v[ch] = -ksc * fmaxf(max3(gm[0], gm[1], gm[2]), gm[3]);
+                            },
+                            release);
+                    if (row_live) store_minima(v, p.out + grow * p.ld + t * (TILE_N / MIN_GROUP) + eh * CH_PER_HALF);
                 } else {
                     const bool whole = !partial && (p.ld & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
                     // the list area is idle in this mode; tiles lie side by side in the output, whatever the stride
@@ -577,22 +590,22 @@ int launch_common(const GemmOperands& op, const GemmPlan& plan, GemmParams& p, i
               ((uint32_t)((plan.pair ? 2 * BM : BM) >> 4) << 24);
 
     typedef void (*KernelFn)(const CUtensorMap, const CUtensorMap, const GemmParams);
-    static const KernelFn kernels[2][3] = {
+    static const KernelFn kernels[2][4] = {
             {gemm_topk_kernel<false, MODE_TOPK>, gemm_topk_kernel<false, MODE_STORE>,
-             gemm_topk_kernel<false, MODE_FILTER>},
+             gemm_topk_kernel<false, MODE_FILTER>, gemm_topk_kernel<false, MODE_MINIMA>},
             {gemm_topk_kernel<true, MODE_TOPK>, gemm_topk_kernel<true, MODE_STORE>,
-             gemm_topk_kernel<true, MODE_FILTER>}};
+             gemm_topk_kernel<true, MODE_FILTER>, gemm_topk_kernel<true, MODE_MINIMA>}};
     static bool attr_set[kMaxDevices] = {false};   // the shared-memory opt-in is per device
     const int slot = device_slot();
     if (!attr_set[slot]) {
         for (int pr = 0; pr < 2; pr++)
-            for (int m = 0; m < 3; m++)
+            for (int m = 0; m < 4; m++)
                 B200F_CUDA_TRY(cudaFuncSetAttribute(reinterpret_cast<const void*>(kernels[pr][m]),
                                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                     pr ? Cfg<true>::SMEM_BYTES : Cfg<false>::SMEM_BYTES));
         attr_set[slot] = true;
     }
-    if (p.mode < 0 || p.mode > 2) return B200F_ERR_BAD_ARG;
+    if (p.mode < 0 || p.mode > 3) return B200F_ERR_BAD_ARG;
     const KernelFn kernel = kernels[plan.pair ? 1 : 0][p.mode];
     main_kernel_begin(ln);
     if (p.mode != MODE_TOPK && resident_fits(op, plan)) {
@@ -806,6 +819,20 @@ int launch_gemm_store(const GemmOperands& op, const GemmPlan& plan, int64_t col0
     p.ld = ld;
     p.status = status;
     return launch_common(op, spread_plan(plan), p, col0, ncols, ln);
+}
+
+int launch_gemm_minima(const GemmOperands& op, const GemmPlan& plan, int64_t ncols, int64_t tile_stride, float kscale,
+                       float* out, int64_t ld, int32_t* status, const Launch& ln) {
+    if (!out || ld % 8 != 0 || (reinterpret_cast<uintptr_t>(out) & 31) != 0) return B200F_ERR_BAD_ARG;
+    GemmParams p{};
+    p.mode = MODE_MINIMA;
+    p.tile_stride = tile_stride;
+    p.kscale = kscale;
+    p.sign = 1.f;
+    p.out = out;
+    p.ld = ld;
+    p.status = status;
+    return launch_common(op, spread_plan(plan), p, 0, ncols, ln);
 }
 
 }  // namespace b200f

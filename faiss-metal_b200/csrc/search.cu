@@ -70,6 +70,7 @@ struct SearchPlan {
     int fcap;         // candidate buffer entries per query
     GemmPlan pilot;
     bool pilot_matrix; // pilot sample as a key matrix (store mode + key selection) instead of lists
+    bool pilot_minima; // of which only the smallest key of every 32 columns is kept
     int npl;
     int64_t a_pitch, a_plane_stride;
     GemmPlan gemm;    // tensor path (fused: whole shard; chunked: per chunk)
@@ -196,6 +197,14 @@ constexpr int64_t SCAN_FILTER_MIN_ROWS = 1 << 15;
 constexpr int64_t BOUND_MIN_ELEMS = 32ll << 20;    // stored elements
 constexpr int BOUND_MAX_D = 8192;                  // a query in a rescoring CTA's shared memory
 
+// What a query's pilot sample of pcols columns leaves behind: row_bound takes the r-th smallest of T thread minima, so where
+// it would have a group of 32 columns and more for every thread the distance kernel keeps their smallest keys only
+// (10,000 queries, 1,000,000 rows: 20 MB instead of 640 written and read).
+constexpr int SAMPLE_GROUP = 32;
+int64_t sample_floats(int64_t pcols, int r) {
+    return pcols / SAMPLE_GROUP >= row_bound_threads(1ll << 40, 0, r) ? pcols / SAMPLE_GROUP : pcols;
+}
+
 bool make_plan(int64_t nq, int64_t nb, int d, int k, int storage, int path, bool pairwise,
                SearchPlan& pl) {
     // the query operand always reserves the 8 norm columns (used for L2 only)
@@ -242,9 +251,9 @@ bool make_plan(int64_t nq, int64_t nb, int d, int k, int storage, int path, bool
         // shard's pilot is all first tiles.  Where the sample's keys fit the matrix slice they are
         // written out instead and a selection kernel bounds the r-th best.
         auto as_matrix = [&](int stride) {
-            const int64_t pcols = ceil_div64(g0.ntiles, stride) * g0.tile_n;
-            return rank_select_enabled() && (k <= B200F_FUSED_MAX_K ? n1 * pcols * 4 <= PILOT_MATRIX_BYTES
-                                                                    : pcols <= matrix_chunk_cols(nq, nb));
+            const int64_t floats = sample_floats(ceil_div64(g0.ntiles, stride) * g0.tile_n, sample_rank(k, stride));
+            return rank_select_enabled() && (k <= B200F_FUSED_MAX_K ? n1 * floats * 4 <= PILOT_MATRIX_BYTES
+                                                                    : floats <= matrix_chunk_cols(nq, nb));
         };
         auto can_halve = [&](int stride) {
             return !filter_forced() && stride > 8 && as_matrix(stride / 2) && sample_rank(k, stride / 2) <= PILOT_MAX_RANK;
@@ -346,6 +355,8 @@ bool make_plan(int64_t nq, int64_t nb, int d, int k, int storage, int path, bool
         const int64_t n1 = nq > 0 ? nq : 1;
         if (!pl.fused) pl.gemm = plan_gemm(nq, nb, sm);
         pl.pilot = plan_gemm(nq, ceil_div64(pl.gemm.ntiles, pl.fstride) * pl.gemm.tile_n, sm);
+        const int64_t pcols = pl.pilot.ntiles * pl.pilot.tile_n;
+        pl.pilot_minima = pl.pilot_matrix && sample_floats(pcols, pl.frank) < pcols;
         if (!pl.pilot_matrix) {
             pl.off_pilot_key = off;
             adv((size_t)n1 * 2 * (pl.pilot.P > 0 ? pl.pilot.P : 1) * pl.frank * 4);
@@ -365,7 +376,7 @@ bool make_plan(int64_t nq, int64_t nb, int d, int k, int storage, int path, bool
         // k <= 32 has no matrix slice of its own: a small one for the pilot sample alone (the lists'
         // first-tile cost, ~0.1 ms per work item, is most of a small search)
         pl.off_matrix = off;
-        adv((size_t)(nq > 0 ? nq : 1) * pl.pilot.ntiles * pl.pilot.tile_n * 4);
+        adv((size_t)(nq > 0 ? nq : 1) * sample_floats(pl.pilot.ntiles * pl.pilot.tile_n, pl.frank) * 4);
     }
     if (pl.lists || pl.filter) {
         pl.off_dirty = off;
@@ -824,10 +835,12 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
             int64_t last_valid = a->nb - last0;
             if (last_valid > pl.pilot.tile_n) last_valid = pl.pilot.tile_n;
             const int64_t valid = (pl.pilot.ntiles - 1) * pl.pilot.tile_n + last_valid;
-            rc = launch_gemm_store(op, pl.pilot, 0, a->nb, pl.fstride, kscale, 1.f, nullptr, matrix, pcols,
-                                   a->status, ln);
+            const int64_t group = pl.pilot_minima ? SAMPLE_GROUP : 1;
+            rc = pl.pilot_minima ? launch_gemm_minima(op, pl.pilot, a->nb, pl.fstride, kscale, matrix, pcols / group, a->status, ln)
+                                 : launch_gemm_store(op, pl.pilot, 0, a->nb, pl.fstride, kscale, 1.f, nullptr, matrix, pcols,
+                                                     a->status, ln);
             if (rc != B200F_OK) return rc;
-            rc = launch_row_bound(matrix, a->nq, valid, pcols, pl.frank, thr, nullptr, nullptr, 0.f, 0.f, 0.0, ln);
+            rc = launch_row_bound(matrix, a->nq, ceil_div64(valid, group), pcols / group, pl.frank, thr, nullptr, nullptr, 0.f, 0.f, 0.0, ln);
             if (rc != B200F_OK) return rc;
         } else {
             rc = launch_gemm_topk(op, pl.pilot, 0, a->nb, pl.fstride, kscale, pl.frank, 1, pkey, pidx, gthr, true,

@@ -504,7 +504,8 @@ __global__ void __launch_bounds__(1024) row_bound_kernel(const float* keys, int6
     const int tid = threadIdx.x, T = blockDim.x;
     pdl_wait();   // the sample's keys are read with coherent loads
     pdl_trigger();
-    const bool vec = (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(keys) & 15) == 0;
+    // four keys a load while that leaves every thread several
+    const bool vec = n >= 8 * T && (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(keys) & 15) == 0;
     for (int64_t q = blockIdx.x; q < nq; q += gridDim.x) {
         const float* row = keys + q * ld;
         float best = CUDART_INF_F;   // fminf drops NaN
