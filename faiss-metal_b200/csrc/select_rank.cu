@@ -294,7 +294,128 @@ __device__ bool bucket_place(const RowSelectParams& p, int64_t qo, int c, float 
     return true;
 }
 
-// One CTA per row, latency-bound (a row is a few KB in L1 / L2).  A pass over the keys leaves every
+// The k best of a row that fits the CTA's registers, RS_REGS words a thread: read once, counted in buckets of equal
+// width, and the buckets up to the one that holds the k-th word are scattered and ranked inside themselves.  Five
+// barriers.  The buckets span [lo, hi]: hi is a key that k words are known to be up to (the largest of the warps'
+// smallest keys where there are k warps, of the threads' where there are k threads, else the largest key), lo the second
+// smallest of the warps' smallest keys, so that one row far nearer than the others (a query that is itself
+// stored) does not stretch the buckets.  Four buckets a thread, 2,048 at most: clearing and summing 16 of them took
+// longer than placing 130 candidates.  False, with nothing written, where the keys do not spread (ties, infinities).
+// 50 rows of 3,900 candidates, k = 2048: 18 us with thread minima, radix digits and a second reading of the row;
+// the search 116 -> 102.5 us.
+constexpr int RS_REGS = 10;
+__device__ __forceinline__ bool register_select(const RowSelectParams& p, int64_t qo, const float* keys, const int32_t* ids, int n,
+                                                uint64_t* words, int* end, int* s_live, uint32_t* s_min, uint32_t* s_max,
+                                                uint32_t* s_maxmin, int* s_warp, int* s_cut, int& live, int& c, int* s_beyond) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, T = blockDim.x, W = T >> 5;
+    // consecutive buckets belong to one thread, T words apart
+    const int nbk = min(RS_BUCKETS, 4 * T), per = nbk / T, log_per = 31 - __clz(per);
+    auto at = [&](int b) { return (b & (per - 1)) * T + (b >> log_per); };
+    uint32_t key[RS_REGS];
+    int32_t id[RS_REGS];
+#pragma unroll
+    for (int r = 0; r < RS_REGS; r++) {
+        const int col = r * T + tid;
+        id[r] = -1;
+        key[r] = 0xffffffffu;
+        if (col < n) {
+            const float f = __ldca(keys + col) + 0.f;   // -0 becomes +0: the two tie
+            id[r] = ids ? __ldca(ids + col) : (f <= p.last_key ? col : -1);
+            key[r] = float_to_ordered(f);
+        }
+    }
+    for (int i = tid; i < nbk; i += T) end[i] = 0;
+    uint32_t tmin = 0xffffffffu, tmax = 0;
+    int have = 0;
+#pragma unroll
+    for (int r = 0; r < RS_REGS; r++) {
+        if (id[r] < 0) continue;
+        tmin = min(tmin, key[r]);
+        tmax = max(tmax, key[r]);
+        have++;
+    }
+    {
+        const uint32_t a = __reduce_min_sync(FULL, tmin), b = __reduce_max_sync(FULL, tmax), m = __reduce_max_sync(FULL, tmin);
+        const int l = __reduce_add_sync(FULL, have);
+        if (lane == 0) {
+            s_min[warp] = a;
+            s_max[warp] = b;
+            s_maxmin[warp] = m;
+            s_live[warp] = l;
+        }
+    }
+    __syncthreads();
+    const uint32_t wmin = lane < W ? s_min[lane] : 0xffffffffu;
+    live = __reduce_add_sync(FULL, lane < W ? s_live[lane] : 0);
+    const uint32_t mx = __reduce_max_sync(FULL, lane < W ? s_max[lane] : 0u);
+    const uint32_t mn = __reduce_min_sync(FULL, wmin);
+    const uint32_t mn_of_threads = __reduce_max_sync(FULL, lane < W ? s_maxmin[lane] : 0u);   // 0xffffffff: a thread without a word
+    const uint32_t mn_of_warps = __reduce_max_sync(FULL, lane < W ? wmin : 0u);
+    uint32_t hi_key = mx;
+    if (p.k <= W && mn_of_warps != 0xffffffffu) hi_key = mn_of_warps;
+    else if (p.k <= T && mn_of_threads != 0xffffffffu) hi_key = mn_of_threads;
+    const int first = __ffs(__ballot_sync(FULL, wmin == mn)) - 1;
+    uint32_t lo_key = __reduce_min_sync(FULL, lane == first ? 0xffffffffu : wmin);
+    if (lo_key > hi_key) lo_key = mn;
+    const float lo = ordered_to_float(lo_key), hi = ordered_to_float(hi_key);
+    const float scale = (nbk - 1) / (hi - lo);
+    if (live == 0 || !(scale > 0.f && scale < CUDART_INF_F && hi - lo < CUDART_INF_F)) return false;   // the same for every thread
+    auto bucket = [&](uint32_t k) {   // ascending with the key
+        return max(0, min((int)((ordered_to_float(k) - lo) * scale), nbk - 1));
+    };
+#pragma unroll
+    for (int r = 0; r < RS_REGS; r++)
+        if (id[r] >= 0 && key[r] <= hi_key) atomicAdd(&end[at(bucket(key[r]))], 1);
+    __syncthreads();
+    int sum = 0;
+    for (int i = 0; i < per; i++) sum += end[i * T + tid];
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(FULL, incl, o);
+        if (lane >= o) incl += up;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    if (tid == 0) s_cut[0] = s_cut[1] = -1;
+    __syncthreads();
+    int start = incl - sum;
+    for (int w = 0; w < warp; w++) start += s_warp[w];
+    bool full = false;
+    for (int i = 0; i < per; i++) {
+        const int b = tid * per + i, h = end[i * T + tid];
+        end[i * T + tid] = start;
+        if (start < p.k && h > RS_BUCKET_MAX) full = true;
+        if (start < p.k && start + h >= p.k) {   // one bucket of one thread
+            s_cut[0] = b;
+            s_cut[1] = start + h;
+        }
+        start += h;
+    }
+    if (tid == T - 1) s_cut[2] = start;   // words up to hi
+    if (__syncthreads_or(full)) return false;
+    // fewer than k up to hi: then hi is the largest key, and all of them count
+    const int cut = s_cut[0] < 0 ? nbk - 1 : s_cut[0];
+    c = s_cut[0] < 0 ? s_cut[2] : s_cut[1];
+#pragma unroll
+    for (int r = 0; r < RS_REGS; r++) {
+        if (id[r] < 0 || key[r] > hi_key) continue;
+        const int b = bucket(key[r]);
+        if (b <= cut) words[atomicAdd(&end[at(b)], 1)] = ((uint64_t)key[r] << 32) | (uint32_t)id[r];
+    }
+    __syncthreads();
+    for (int i = tid; i < c; i += T) {
+        const uint64_t w = words[i];
+        const int b = bucket((uint32_t)(w >> 32));
+        const int from = b > 0 ? end[at(b - 1)] : 0, to = end[at(b)];
+        int rank = from;
+        for (int j = from; j < to; j++) rank += words[j] < w ? 1 : 0;
+        if (rank < p.k) rs_write(p, qo, rank, w, s_beyond);
+    }
+    return true;
+}
+
+// One CTA per row, latency-bound (a row is a few KB in L1 / L2).  Rows of up to RS_REGS words a thread: register_select.
+// Longer ones, and those whose keys do not spread: a pass over the keys leaves every
 // thread with the M smallest keys of its share; with k <= M T / 2 the k-th smallest of those M T bounds the
 // row's k-th key from above and admits little more than k keys (2 histogram passes over registers instead
 // of 4 over the row: 10,000 rows of 20,000 keys, k = 1000: 2,415 us with M = 1, which leaves k > T / 2 to
@@ -309,7 +430,7 @@ __global__ void __launch_bounds__(1024) row_select_kernel(const RowSelectParams 
     __shared__ int s_hist[256];
     __shared__ uint32_t s_min[32], s_max[32];
     __shared__ int s_live[32];
-    __shared__ int s_sel[2];
+    __shared__ int s_sel[4];
     __shared__ int s_count, s_have, s_beyond;
     pdl_wait();   // what the kernel before wrote is read with coherent loads
     pdl_trigger();
@@ -322,135 +443,142 @@ __global__ void __launch_bounds__(1024) row_select_kernel(const RowSelectParams 
         const int n = (int)min(cnt, p.ld);
         const float* keys = p.keys + q * p.ld;
         const int32_t* ids = p.ids ? p.ids + q * p.ld : nullptr;
-        // (ordered key, live) of column c; both loads are issued before either is used
-        auto load = [&](int c, uint32_t& key, int32_t& id) {
-            const float f = __ldca(keys + c) + 0.f;   // -0 becomes +0: the two tie
-            id = ids ? __ldca(ids + c) : (f <= p.last_key ? c : -1);
-            key = float_to_ordered(f);
-        };
-        int live = 0;
-        uint32_t mx = 0;
-        uint32_t best[M];   // ascending
+        const int64_t qo = p.row_map ? (int64_t)p.row_map[q] : q;
+        int live = 0, c = 0;
+        if (tid == 0) s_beyond = 0;   // behind several barriers before the first word is written
+        if (n > RS_REGS * T || !register_select(p, qo, keys, ids, n, rs_runs, reinterpret_cast<int*>(rs_runs + p.bound), s_live,
+                                                s_min, s_max, reinterpret_cast<uint32_t*>(s_hist), s_hist + 32, s_sel, live, c,
+                                                &s_beyond)) {
+            __syncthreads();
+            // (ordered key, live) of column c; both loads are issued before either is used
+            auto load = [&](int c, uint32_t& key, int32_t& id) {
+                const float f = __ldca(keys + c) + 0.f;   // -0 becomes +0: the two tie
+                id = ids ? __ldca(ids + c) : (f <= p.last_key ? c : -1);
+                key = float_to_ordered(f);
+            };
+            live = 0;
+            uint32_t mx = 0;
+            uint32_t best[M];   // ascending
 #pragma unroll
-        for (int i = 0; i < M; i++) best[i] = 0xffffffffu;
+            for (int i = 0; i < M; i++) best[i] = 0xffffffffu;
 #pragma unroll 8
-        for (int c = tid; c < n; c += T) {
-            uint32_t key;
-            int32_t id;
-            load(c, key, id);
-            if (id >= 0) {
-                live++;
-                mx = max(mx, key);
-#pragma unroll
-                for (int i = 0; i < M; i++) {
-                    const uint32_t lo = min(best[i], key);
-                    key = max(best[i], key);
-                    best[i] = lo;
-                }
-            }
-        }
-        uint32_t mn = best[0];
-        const int my_have = min(live, M);
-        if (tid == 0) s_count = s_have = s_beyond = 0;
-        const Spread sp = block_spread(live, mn, mx, s_live, s_min, s_max);
-        live = sp.live;
-        mn = sp.mn;
-        auto visit_all = [&](auto f) {
-#pragma unroll 4
-            for (int c = tid; c < n; c += T) {
+            for (int col = tid; col < n; col += T) {
                 uint32_t key;
                 int32_t id;
-                load(c, key, id);
-                if (id >= 0) f(key);
-            }
-        };
-        const int bits = 32 - __clz(sp.mx - mn);   // significant bits of the spread (live > 0)
-        uint32_t thr_x = live > 0 ? sp.mx - mn : 0;
-        uint32_t tie_id = 0x7fffffffu;             // of the keys equal to thr_x: ids up to this one
-        bool loose = false;
-        if (live > p.k) {
-            if (2 * p.k <= M * T) {
-                const int have = __reduce_add_sync(FULL, my_have);   // s_have was cleared before block_spread's barrier
-                if (lane == 0) atomicAdd(&s_have, have);
-                __syncthreads();
-                loose = s_have >= p.k;
-            }
-            if (loose) {
-                int kk = p.k;
-                thr_x = radix_kth(
-                        [&](auto f) {
+                load(col, key, id);
+                if (id >= 0) {
+                    live++;
+                    mx = max(mx, key);
 #pragma unroll
-                            for (int i = 0; i < M; i++)
-                                if (i < my_have) f(best[i]);
-                        },
-                        mn, bits, bits > 16 ? bits - 16 : 0, kk,
-                                  s_hist, s_sel);
-            } else {
-                int kk = p.k;
-                thr_x = radix_kth(visit_all, mn, bits, 0, kk, s_hist, s_sel);
+                    for (int i = 0; i < M; i++) {
+                        const uint32_t lo = min(best[i], key);
+                        key = max(best[i], key);
+                        best[i] = lo;
+                    }
+                }
             }
-        }
-        // compaction of the candidates up to the threshold (k of them plus a few, or all)
-        int c = 0;
-        for (int pass = 0; pass < 2; pass++) {
-            for (int c0 = warp * 32; c0 < n; c0 += T) {
-                const int cc = c0 + lane;
-                bool keep = false;
-                uint64_t word = 0;
-                if (cc < n) {
+            uint32_t mn = best[0];
+            const int my_have = min(live, M);
+            if (tid == 0) s_count = s_have = 0;
+            const Spread sp = block_spread(live, mn, mx, s_live, s_min, s_max);
+            live = sp.live;
+            mn = sp.mn;
+            auto visit_all = [&](auto f) {
+#pragma unroll 4
+                for (int col = tid; col < n; col += T) {
                     uint32_t key;
                     int32_t id;
-                    load(cc, key, id);
-                    const uint32_t x = key - mn;           // live keys are >= mn
-                    keep = id >= 0 && (x < thr_x || (x == thr_x && (uint32_t)id <= tie_id));
-                    word = ((uint64_t)key << 32) | (uint32_t)id;
+                    load(col, key, id);
+                    if (id >= 0) f(key);
                 }
-                const unsigned b = __ballot_sync(FULL, keep);
-                int base = 0;
-                if (lane == 0 && b) base = atomicAdd(&s_count, __popc(b));
-                base = __shfl_sync(FULL, base, 0);
-                const int pos = base + __popc(b & ((1u << lane) - 1u));
-                if (keep && pos < p.bound) rs_runs[pos] = word;
+            };
+            const int bits = 32 - __clz(sp.mx - mn);   // significant bits of the spread (live > 0)
+            uint32_t thr_x = live > 0 ? sp.mx - mn : 0;
+            uint32_t tie_id = 0x7fffffffu;             // of the keys equal to thr_x: ids up to this one
+            bool loose = false;
+            if (live > p.k) {
+                if (2 * p.k <= M * T) {
+                    const int have = __reduce_add_sync(FULL, my_have);   // s_have was cleared before block_spread's barrier
+                    if (lane == 0) atomicAdd(&s_have, have);
+                    __syncthreads();
+                    loose = s_have >= p.k;
+                }
+                if (loose) {
+                    int kk = p.k;
+                    thr_x = radix_kth(
+                            [&](auto f) {
+#pragma unroll
+                                for (int i = 0; i < M; i++)
+                                    if (i < my_have) f(best[i]);
+                            },
+                            mn, bits, bits > 16 ? bits - 16 : 0, kk,
+                                      s_hist, s_sel);
+                } else {
+                    int kk = p.k;
+                    thr_x = radix_kth(visit_all, mn, bits, 0, kk, s_hist, s_sel);
+                }
             }
-            __syncthreads();
-            c = s_count;
-            if (c <= p.bound || pass == 1) break;
-            // more than fit: the exact k-th key, and of the keys equal to it the ids that are wanted
-            // (exactly k words are kept the second time)
-            __syncthreads();   // everybody has read the count
-            if (tid == 0) s_count = 0;
-            int kk = p.k;
-            thr_x = radix_kth(visit_all, mn, bits, 0, kk, s_hist, s_sel);
-            tie_id = radix_kth(
-                    [&](auto f) {
-                        for (int cc = tid; cc < n; cc += T) {
-                            uint32_t key;
-                            int32_t id;
-                            load(cc, key, id);
-                            if (id >= 0 && key - mn == thr_x) f((uint32_t)id);
-                        }
-                    },
-                    0u, 31, 0, kk, s_hist, s_sel);
-        }
-        c = min(c, p.bound);   // ids are distinct: the second pass keeps k words
-        const int64_t qo = p.row_map ? (int64_t)p.row_map[q] : q;
-        if (c <= RS_COUNT_MAX) {
-            for (int i = tid; i < c; i += T) {
-                const uint64_t w = rs_runs[i];
-                int rank = 0;
+            // compaction of the candidates up to the threshold (k of them plus a few, or all)
+            c = 0;
+            for (int pass = 0; pass < 2; pass++) {
+                for (int c0 = warp * 32; c0 < n; c0 += T) {
+                    const int cc = c0 + lane;
+                    bool keep = false;
+                    uint64_t word = 0;
+                    if (cc < n) {
+                        uint32_t key;
+                        int32_t id;
+                        load(cc, key, id);
+                        const uint32_t x = key - mn;           // live keys are >= mn
+                        keep = id >= 0 && (x < thr_x || (x == thr_x && (uint32_t)id <= tie_id));
+                        word = ((uint64_t)key << 32) | (uint32_t)id;
+                    }
+                    const unsigned b = __ballot_sync(FULL, keep);
+                    int base = 0;
+                    if (lane == 0 && b) base = atomicAdd(&s_count, __popc(b));
+                    base = __shfl_sync(FULL, base, 0);
+                    const int pos = base + __popc(b & ((1u << lane) - 1u));
+                    if (keep && pos < p.bound) rs_runs[pos] = word;
+                }
+                __syncthreads();
+                c = s_count;
+                if (c <= p.bound || pass == 1) break;
+                // more than fit: the exact k-th key, and of the keys equal to it the ids that are wanted
+                // (exactly k words are kept the second time)
+                __syncthreads();   // everybody has read the count
+                if (tid == 0) s_count = 0;
+                int kk = p.k;
+                thr_x = radix_kth(visit_all, mn, bits, 0, kk, s_hist, s_sel);
+                tie_id = radix_kth(
+                        [&](auto f) {
+                            for (int cc = tid; cc < n; cc += T) {
+                                uint32_t key;
+                                int32_t id;
+                                load(cc, key, id);
+                                if (id >= 0 && key - mn == thr_x) f((uint32_t)id);
+                            }
+                        },
+                        0u, 31, 0, kk, s_hist, s_sel);
+            }
+            c = min(c, p.bound);   // ids are distinct: the second pass keeps k words
+            if (c <= RS_COUNT_MAX) {
+                for (int i = tid; i < c; i += T) {
+                    const uint64_t w = rs_runs[i];
+                    int rank = 0;
 #pragma unroll 8
-                for (int j = 0; j < c; j++) rank += rs_runs[j] < w ? 1 : 0;
-                if (rank < p.k) rs_write(p, qo, rank, w, &s_beyond);
+                    for (int j = 0; j < c; j++) rank += rs_runs[j] < w ? 1 : 0;
+                    if (rank < p.k) rs_write(p, qo, rank, w, &s_beyond);
+                }
+            } else if (!bucket_place(p, qo, c, ordered_to_float(mn), ordered_to_float(mn + min(thr_x, sp.mx - mn)), rs_runs,
+                                     reinterpret_cast<int*>(rs_runs + p.bound),
+                                     reinterpret_cast<uint16_t*>(rs_runs + p.bound) + 2 * RS_BUCKETS, s_live, &s_beyond)) {
+                const int m = (c + W - 1) / W;    // <= RS_RUN
+                if (m <= 32) rank_place<1>(p, qo, c, m, rs_runs, W, &s_beyond);
+                else if (m <= 64) rank_place<2>(p, qo, c, m, rs_runs, W, &s_beyond);
+                else if (m <= 128) rank_place<4>(p, qo, c, m, rs_runs, W, &s_beyond);
+                else if (m <= 256) rank_place<8>(p, qo, c, m, rs_runs, W, &s_beyond);
+                else rank_place<16>(p, qo, c, m, rs_runs, W, &s_beyond);
             }
-        } else if (!bucket_place(p, qo, c, ordered_to_float(mn), ordered_to_float(mn + min(thr_x, sp.mx - mn)), rs_runs,
-                                 reinterpret_cast<int*>(rs_runs + p.bound),
-                                 reinterpret_cast<uint16_t*>(rs_runs + p.bound) + 2 * RS_BUCKETS, s_live, &s_beyond)) {
-            const int m = (c + W - 1) / W;    // <= RS_RUN
-            if (m <= 32) rank_place<1>(p, qo, c, m, rs_runs, W, &s_beyond);
-            else if (m <= 64) rank_place<2>(p, qo, c, m, rs_runs, W, &s_beyond);
-            else if (m <= 128) rank_place<4>(p, qo, c, m, rs_runs, W, &s_beyond);
-            else if (m <= 256) rank_place<8>(p, qo, c, m, rs_runs, W, &s_beyond);
-            else rank_place<16>(p, qo, c, m, rs_runs, W, &s_beyond);
         }
         for (int j = c + tid; j < p.k; j += T) {
             p.out_dist[qo * p.k + j] = p.pad;
