@@ -965,8 +965,10 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
             exact.run_if_bad = 1;
         }
         for (int64_t q0 = 0; q0 < a->nq; q0 += SCAN_GROUP) {
+            // not in the wake of the streaming filter: launched before the SMs were idle this kernel would keep that one's
+            // partition of shared memory and L1 (eight queries, k = 1024, 1 M bf16 rows of d = 1024, all bounds too wide: 1,489 us, 1,235)
             rc = launch_scan_filter(query_group(q0, SCAN_GROUP), thr + q0, ckey + q0 * pl.fcap, cidx + q0 * pl.fcap,
-                                    ccnt + q0, pl.fcap, sm, exact, ln);
+                                    ccnt + q0, pl.fcap, sm, exact, bad ? Launch(st) : ln);
             if (rc != B200F_OK) return rc;
         }
         rc = launch_select_candidates(ckey, cidx, ccnt, pl.fcap, a->nb, a->nq, a->k, a->metric, qnorm,
