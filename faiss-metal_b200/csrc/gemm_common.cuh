@@ -131,6 +131,31 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t cluster_bar) {
                  : "memory");
 }
 
+// The same two for a whole converged warp, of which the lane with `leader` issues: control flow and operands stay uniform.
+__device__ __forceinline__ void tc_mma_f16_pair_by(bool leader, uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+                                                   uint32_t accumulate) {
+    asm volatile(
+            "{\n\t"
+            ".reg .pred p, q;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "setp.ne.b32 q, %5, 0;\n\t"
+            "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
+            "}\n" ::"r"(d_tmem),
+            "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"((uint32_t)leader)
+            : "memory");
+}
+// arrives on the barrier at `bar` (an address of this CTA) in both CTAs of the pair
+__device__ __forceinline__ void tc_commit_both_by(bool leader, uint32_t bar) {
+    asm volatile(
+            "{\n\t"
+            ".reg .pred q;\n\t"
+            "setp.ne.b32 q, %1, 0;\n\t"
+            "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %2;\n\t"
+            "}\n" ::"r"(bar),
+            "r"((uint32_t)leader), "h"((uint16_t)3)
+            : "memory");
+}
+
 __device__ __forceinline__ void tc_mma_f16_pair(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b,
                                                 uint32_t idesc, uint32_t accumulate) {
     asm volatile(

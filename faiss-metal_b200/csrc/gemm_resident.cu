@@ -10,7 +10,9 @@
 // (query block, range of X tiles):
 //   warp 0     producer: the CTA's half of the query block once per item, then its half (128 rows) of the X k-blocks,
 //              16 KiB each, through a ring of barriers per block
-//   warp 1     of the even CTA: MMAs of one tile after another into two accumulators of 256 columns
+//   warp 1     of the even CTA: MMAs of one tile after another into two accumulators of 256 columns.  The whole warp walks through
+//              the tiles and one lane issues: by a lane alone an MMA took 190 cycles with the waits and commits around it, the
+//              tensor pipe 128 (tile of 19 MMAs: 3,689 -> 2,920 cycles)
 //   warps 2-9  epilogue: a warp reads 32 rows and half the columns of one accumulator while the MMAs of the
 //              next tile fill the other
 // X blocks that two plane products share (fp32 rows: plane 0 meets both query planes) are loaded once and used
@@ -164,12 +166,12 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------ MMA issuer ------------------------------
-        if (cta_rank == 0 && elect_one()) {
+        // The whole warp walks through the tiles and one lane issues.
+        if (cta_rank == 0) {
+            const bool leader = elect_one();
             const uint64_t da0 = make_smem_desc(sbase);
             const uint64_t db0 = make_smem_desc(sbase + nb * RES_BLOCK_BYTES);
-            const uint32_t empty0 = map_to_cta(bar_empty, 0), empty1 = map_to_cta(bar_empty, 1);
-            const uint32_t qempty0 = map_to_cta(bar_qempty, 0), qempty1 = map_to_cta(bar_qempty, 1);
-            const uint32_t tfull0 = map_to_cta(bar_tfull, 0), tfull1 = map_to_cta(bar_tfull, 1);
+            constexpr uint64_t BLOCK = RES_BLOCK_BYTES >> 4;
             // the last k-block of a product may hold fewer than 64 valid K elements (the rest is zero): skip those
             const int nk4_data = (p.k_extent - (nkd - 1) * BK + UMMA_K - 1) / UMMA_K;
             const int nk4_end = (p.k_extent_last - (nkl - 1) * BK + UMMA_K - 1) / UMMA_K;
@@ -177,74 +179,82 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
             uint32_t phase = 0, qphase = 0, acc_phase = 0;
             int acc = 0, have_qb = -1;
             bool ok = true;
+            uint32_t accumulate = 0;
+            uint32_t d_tmem = 0;
+            auto block = [&](uint64_t da, int s, int nk4) {   // a k-block of the query block and X block s of the ring
+                const uint64_t db = db0 + (uint64_t)s * BLOCK;
+                tc_mma_f16_pair_by(leader, d_tmem, da, db, p.idesc, accumulate);
+                accumulate = 1;
+                if (nk4 > 1) tc_mma_f16_pair_by(leader, d_tmem, da + 2, db + 2, p.idesc, 1);
+                if (nk4 > 2) tc_mma_f16_pair_by(leader, d_tmem, da + 4, db + 4, p.idesc, 1);
+                if (nk4 > 3) tc_mma_f16_pair_by(leader, d_tmem, da + 6, db + 6, p.idesc, 1);
+            };
+            auto full = [&](int s, uint32_t ph) {
+                return mbar_try_wait(bar_full + s * 8, ph) || mbar_wait(bar_full + s * 8, ph, abort_flag, p.status);
+            };
             for (int64_t item = unit; item < nitems && ok; item += nunits) {
                 const int qb = (int)(item % nqb);
                 const int64_t t0 = item / nqb * p.tiles_per_range, t1 = min(t0 + p.tiles_per_range, p.ntiles);
                 if (qb != have_qb) {
-                    if (!mbar_wait(bar_qfull, qphase, abort_flag, p.status)) break;
+                    ok = __all_sync(0xffffffffu, mbar_wait(bar_qfull, qphase, abort_flag, p.status));
+                    if (!ok) break;
                     qphase ^= 1;
                     have_qb = qb;
                 }
-                for (int64_t t = t0; t < t1; t++) {
-                    if (!mbar_wait(bar_tempty + acc * 8, acc_phase ^ 1, abort_flag, p.status)) {
-                        ok = false;
-                        break;
-                    }
+                for (int64_t t = t0; t < t1 && ok; t++) {
+                    ok = mbar_wait(bar_tempty + acc * 8, acc_phase ^ 1, abort_flag, p.status);
                     tc_fence_after();
-                    const uint32_t d_tmem = tmem_base + acc * RES_TILE_N;
-                    uint32_t accumulate = 0;
-                    for (int pass = 0; pass < p.npass && ok; pass++) {
-                        const bool last = pass == p.npass - 1;
-                        const int n = last ? nkl : nkd;
-                        const int a_first = two && pass > 0 ? nkd : 0;           // query plane 1, then plane 0
-                        const int b_first = two && pass == 1 ? nkd : 0;          // X planes 0, 1, 0
-                        for (int kb = 0; kb < n; kb++) {
-                            const int i = last && two && kb == nkd ? 2 * nkd : b_first + kb;
-                            int s = base + i;
-                            uint32_t ph = phase;
-                            if (s >= ring) {
-                                s -= ring;
-                                ph ^= 1;
-                            }
-                            // plane 0's blocks of the last product are there since the first
-                            if (!(last && two && kb < nkd) && !mbar_try_wait(bar_full + s * 8, ph) &&
-                                !mbar_wait(bar_full + s * 8, ph, abort_flag, p.status)) {
-                                ok = false;
-                                break;
-                            }
-                            const uint64_t da = da0 + (uint64_t)((a_first + kb) * (RES_BLOCK_BYTES >> 4));
-                            const uint64_t db = db0 + (uint64_t)(s * (RES_BLOCK_BYTES >> 4));
-                            const int nk4 = kb < n - 1 ? BK / UMMA_K : last ? nk4_end : nk4_data;
-#pragma unroll
-                            for (int k4 = 0; k4 < BK / UMMA_K; k4++) {
-                                if (k4 < nk4) {
-                                    tc_mma_f16_pair(d_tmem, da + (uint64_t)(k4 * 2), db + (uint64_t)(k4 * 2), p.idesc,
-                                                    accumulate);
-                                    accumulate = 1;
-                                }
-                            }
-                            // the block's last use: free in both CTAs when the MMAs retire
-                            if (!two || pass > 0) {
-                                tc_commit_pair(empty0 + s * 8);
-                                tc_commit_pair(empty1 + s * 8);
-                            }
+                    d_tmem = tmem_base + acc * RES_TILE_N;
+                    accumulate = 0;
+                    int s = base;            // block by block through the ring
+                    uint32_t ph = phase;
+                    auto step = [&]() {
+                        if (++s == ring) {
+                            s = 0;
+                            ph ^= 1;
+                        }
+                    };
+                    uint64_t da = da0;
+                    if (two) {
+                        // query plane 1 with X plane 0, whose blocks stay
+                        for (int kb = 0; kb < nkd; kb++, da += BLOCK, step()) {
+                            ok = ok && full(s, ph);
+                            block(da, s, kb < nkd - 1 ? 4 : nk4_data);
+                        }
+                        // query plane 0 with X plane 1
+                        uint64_t da_low = da;
+                        for (int kb = 0; kb < nkd; kb++, da_low += BLOCK, step()) {
+                            ok = ok && full(s, ph);
+                            block(da_low, s, kb < nkd - 1 ? 4 : nk4_data);
+                            tc_commit_both_by(leader, bar_empty + s * 8);   // its last use
+                        }
+                        // query plane 0 with X plane 0
+                        int s0 = base;
+                        for (int kb = 0; kb < nkd; kb++, da += BLOCK) {
+                            block(da, s0, kb < nkl - 1 ? 4 : nk4_end);
+                            tc_commit_both_by(leader, bar_empty + s0 * 8);
+                            if (++s0 == ring) s0 = 0;
                         }
                     }
-                    if (!ok) break;
-                    tc_commit_pair(tfull0 + acc * 8);
-                    tc_commit_pair(tfull1 + acc * 8);
-                    base += nb;
-                    if (base >= ring) {
-                        base -= ring;
-                        phase ^= 1;
+                    // one plane: all its blocks; two: the norm columns' block, where they have one
+                    for (int kb = two ? nkd : 0; kb < nkl; kb++, da += BLOCK, step()) {
+                        ok = ok && full(s, ph);
+                        block(da, s, kb < nkl - 1 ? 4 : nk4_end);
+                        tc_commit_both_by(leader, bar_empty + s * 8);
                     }
+                    tc_commit_both_by(leader, bar_tfull + acc * 8);
+                    base = s;
+                    phase = ph;
                     acc ^= 1;
                     if (acc == 0) acc_phase ^= 1;
+                    ok = __all_sync(0xffffffffu, ok);   // a wait that ran out: the epilogues give up by themselves
                 }
                 const int64_t next = item + nunits;
-                if (ok && next < nitems && (int)(next % nqb) != qb) {
-                    tc_commit_pair(qempty0);
-                    tc_commit_pair(qempty1);
+                if (ok && next < nitems && (int)(next % nqb) != qb) tc_commit_both_by(leader, bar_qempty);
+            }
+            if (!ok) {   // let the MMAs in flight retire before tensor memory goes away
+                const long long t0 = clock64();
+                while (clock64() - t0 < 200000LL) {
                 }
             }
         }
