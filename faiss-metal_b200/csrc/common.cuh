@@ -198,11 +198,10 @@ int launch_gemm_topk(const GemmOperands& op, const GemmPlan& plan, int64_t col0,
 // Threshold filter over the whole shard: column c of row q with scaled key <= thr[q * thr_stride +
 // thr_pos] is appended to the row's candidate buffer cand_key/cand_idx [nq][cand_cap] in any
 // order; cand_cnt[q] (zeroed by the caller) counts every hit, also those beyond cand_cap, which are
-// not stored.
-// few_hits: the threshold admits well under one column in a thousand (tunes the scan width).
+// not stored.  dense: many hits (see the caller's rule).
 int launch_gemm_filter(const GemmOperands& op, const GemmPlan& plan, float kscale, const float* thr,
                        int thr_stride, int thr_pos, float* cand_key, int32_t* cand_idx,
-                       int32_t* cand_cnt, int cand_cap, int few_hits, int32_t* status,
+                       int32_t* cand_cnt, int cand_cap, int dense, int32_t* status,
                        const Launch& ln);
 // Store mode: out[row*ld + (col-col0)] = sign*(-kscale*t) + rowadd[row], t = q.x (- ||x||^2/2).
 // tile_stride > 1 visits only every tile_stride-th column tile (plan made for that many tiles);

@@ -1,5 +1,5 @@
-// What the two distance GEMM kernels share: launch parameters, tcgen05 and TMA wrappers, the staging of filter
-// hits, operand tensor maps.
+// What the two distance GEMM kernels share: launch parameters, tcgen05 and TMA wrappers, the epilogue's work on
+// accumulator columns, operand tensor maps.
 #pragma once
 
 #include <cuda.h>
@@ -16,7 +16,7 @@ constexpr int UMMA_K = 16;
 constexpr int NUM_EPI_WARPS = 8;   // two per TMEM lane quarter: each takes half of the tile's columns
 constexpr int TMEM_COLS = 512;
 
-enum { MODE_TOPK = 0, MODE_STORE = 1, MODE_FILTER = 2, MODE_MINIMA = 3 };
+enum { MODE_TOPK = 0, MODE_STORE = 1, MODE_FILTER = 2, MODE_MINIMA = 3, MODE_DENSE = 4 };
 
 struct GemmParams {
     int64_t nq;
@@ -64,7 +64,7 @@ struct GemmParams {
     int32_t* cand_idx;
     int32_t* cand_cnt;   // [nq]
     int cand_cap;
-    int wide;            // MODE_FILTER: 64 columns per TMEM load (few hits expected), else 32
+    int dense;           // MODE_FILTER: many hits expected
     float* out;
     int64_t ld;
     int32_t* status;
@@ -131,6 +131,18 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t cluster_bar) {
                  : "memory");
 }
 
+__device__ __forceinline__ void tc_mma_f16_pair(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b,
+                                                uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+            "{\n\t"
+            ".reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
+            "}\n" ::"r"(d_tmem),
+            "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+            : "memory");
+}
+
 // The same two for a whole converged warp, of which the lane with `leader` issues: control flow and operands stay uniform.
 __device__ __forceinline__ void tc_mma_f16_pair_by(bool leader, uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
                                                    uint32_t accumulate) {
@@ -153,18 +165,6 @@ __device__ __forceinline__ void tc_commit_both_by(bool leader, uint32_t bar) {
             "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %2;\n\t"
             "}\n" ::"r"(bar),
             "r"((uint32_t)leader), "h"((uint16_t)3)
-            : "memory");
-}
-
-__device__ __forceinline__ void tc_mma_f16_pair(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b,
-                                                uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-            "{\n\t"
-            ".reg .pred p;\n\t"
-            "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
-            "}\n" ::"r"(d_tmem),
-            "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
             : "memory");
 }
 
@@ -197,28 +197,6 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&r)[32]) {
               "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
               "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]),
               "=r"(r[31])
-            : "r"(taddr)
-            : "memory");
-}
-// 32 lanes x 64 consecutive fp32 columns -> 64 registers per thread
-__device__ __forceinline__ void tc_ld64(uint32_t taddr, uint32_t (&r)[64]) {
-    asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x64.b32 "
-            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-            "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, "
-            "%32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, "
-            "%48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%64];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-              "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
-              "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
-              "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-              "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]),
-              "=r"(r[31]), "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]),
-              "=r"(r[37]), "=r"(r[38]), "=r"(r[39]), "=r"(r[40]), "=r"(r[41]), "=r"(r[42]),
-              "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47]), "=r"(r[48]),
-              "=r"(r[49]), "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]),
-              "=r"(r[55]), "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]), "=r"(r[60]),
-              "=r"(r[61]), "=r"(r[62]), "=r"(r[63])
             : "r"(taddr)
             : "memory");
 }
@@ -273,28 +251,6 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {
     return desc;
 }
 
-// Hits of the tile in flight are staged per thread in shared memory (entry i of a thread at
-// [i * STAGE_LD]: raw key s = -t and column) and worked off AFTER the accumulator has been handed
-// back to the MMA issuers, so that list insertion and buffer appends run beside the next
-// tile's MMAs instead of in front of them.  Only a thread whose stage fills up inside one
-// tile (list warm-up, massive ties) drains it on the spot.
-constexpr int STAGE_N = 16;
-constexpr int STAGE_LD = 32 * NUM_EPI_WARPS;
-
-// MODE_FILTER: one atomic takes n slots of the row's candidate buffer; the counter also counts
-// entries that no longer fit.
-__device__ __forceinline__ void drain_to_buffer(int32_t* cnt, float* ck, int32_t* ci, int cap,
-                                                float kscale, const float* sk, const int32_t* si, int n) {
-    if (n <= 0) return;
-    const int base = atomicAdd(cnt, n);
-    for (int i = 0; i < n; i++) {
-        if (base + i < cap) {
-            ck[base + i] = kscale * sk[i * STAGE_LD];
-            ci[base + i] = si[i * STAGE_LD];
-        }
-    }
-}
-
 // Columns beyond the end were zero-filled: out of every comparison.
 __device__ __forceinline__ void mask_columns(uint32_t (&r)[32], int64_t cbase, int64_t ncols_end) {
 #pragma unroll
@@ -311,12 +267,106 @@ __device__ __forceinline__ void group_maxima(const uint32_t (&r)[32], float (&gm
     }
 }
 
-// MODE_FILTER: 32 accumulator columns of a thread's row, hits (-r < thr) to the thread's stage.  All lanes of the warp call
-// it.  The largest of every group of eight columns, then of all; the groups that hold a hit of any row are gone through
-// column by column.
+// MODE_FILTER of the resident kernel, few hits.  The epilogue's code has to stay small: the hits' part runs for every second
+// chunk of 32 columns at the usual thresholds, and unrolled comparisons of eight columns after the other cost 700 cycles a visit
+// there.  So a row with a hit goes to shared memory whole, a loop looks at one such row at a time, a column per lane, and hits
+// queue up there from tile to tile (2,048 queries, k = 1024, 5 M fp32 rows: 5,733 -> 5,256 us).
+constexpr int HIT_ROWS = 8;     // rows of a chunk looked at together
+constexpr int HIT_LD = 36;      // floats from one to the next
+constexpr int QUEUE_N = 96;
+constexpr int QUEUE_DRAIN = 64; // worked off between tiles from here on
+constexpr int HITS_BYTES = HIT_ROWS * HIT_LD * 4 + HIT_ROWS * 4 + QUEUE_N * 12;
+struct WarpHits {
+    float* rows;      // [HIT_ROWS][HIT_LD]
+    int* src;         // [HIT_ROWS] lanes they belong to
+    float* key;       // [QUEUE_N] -accumulator
+    int* col;
+    int* lane;
+};
+__device__ __forceinline__ WarpHits warp_hits(uint8_t* area) {   // HITS_BYTES, 16-byte aligned
+    WarpHits h;
+    h.rows = reinterpret_cast<float*>(area);
+    h.src = reinterpret_cast<int*>(h.rows + HIT_ROWS * HIT_LD);
+    h.key = reinterpret_cast<float*>(h.src + HIT_ROWS);
+    h.col = reinterpret_cast<int*>(h.key + QUEUE_N);
+    h.lane = h.col + QUEUE_N;
+    return h;
+}
+
+// n queued hits to the candidate buffers of the warp's 32 rows (cnt, ck, ci: those of its first).  One atomic takes the slots
+// of a row's hits among 32; the counter also counts hits that no longer fit.  All lanes call it, ksc is the lane's.
+static __device__ __noinline__ void drain_hits(int32_t* cnt, float* ck, int32_t* ci, int cap, float ksc, const float* key, const int* col,
+                                        const int* lanes, int n) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+    for (int i0 = 0; i0 < n; i0 += 32) {
+        const bool live = i0 + lane < n;
+        const int row = live ? lanes[i0 + lane] : lane;
+        const float k = __shfl_sync(0xffffffffu, ksc, row);
+        const unsigned same = __match_any_sync(0xffffffffu, live ? row : 32);
+        const int leader = __ffs(same) - 1;
+        int base = 0;
+        if (live && lane == leader) base = atomicAdd(cnt + row, __popc(same));
+        const int pos = __shfl_sync(0xffffffffu, base, leader) + __popc(same & ((1u << lane) - 1u));
+        if (live && pos < cap) {
+            ck[(int64_t)row * cap + pos] = k * key[i0 + lane];
+            ci[(int64_t)row * cap + pos] = col[i0 + lane];
+        }
+    }
+    __syncwarp();
+}
+
+// 32 accumulator columns of the warp's rows: hits (-r < thr) to the queue, which holds n.  All lanes call it.
 template <typename Drain>
-__device__ __forceinline__ void filter_columns(uint32_t (&r)[32], int64_t cbase, int64_t ncols_end, bool partial, const float& thr,
-                                               float* stage_key, int32_t* stage_idx, int& nstaged, Drain drain) {
+__device__ __forceinline__ void filter_columns(uint32_t (&r)[32], int64_t cbase, int64_t ncols_end, bool partial, float thr,
+                                               const WarpHits& h, int& n, Drain drain) {
+    if (partial) mask_columns(r, cbase, ncols_end);
+    float gm[4];
+    group_maxima(r, gm);
+    unsigned rows = __ballot_sync(0xffffffffu, -fmaxf(max3(gm[0], gm[1], gm[2]), gm[3]) < thr);
+    if (!rows) return;
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    do {
+        const int rank = __popc(rows & below);
+        const bool mine = ((rows >> lane) & 1u) && rank < HIT_ROWS;
+        if (mine) {
+            float4* dst = reinterpret_cast<float4*>(h.rows + rank * HIT_LD);
+#pragma unroll
+            for (int c = 0; c < 8; c++)
+                dst[c] = make_float4(__uint_as_float(r[4 * c]), __uint_as_float(r[4 * c + 1]), __uint_as_float(r[4 * c + 2]),
+                                     __uint_as_float(r[4 * c + 3]));
+            h.src[rank] = lane;
+        }
+        const int take = min(__popc(rows), HIT_ROWS);
+        rows &= ~__ballot_sync(0xffffffffu, mine);
+        __syncwarp();
+#pragma unroll 1
+        for (int j = 0; j < take; j++) {
+            const float key = -h.rows[j * HIT_LD + lane];
+            const int src = h.src[j];
+            const bool hit = key < __shfl_sync(0xffffffffu, thr, src);
+            const unsigned b = __ballot_sync(0xffffffffu, hit);
+            if (n > QUEUE_N - 32) drain();
+            if (hit) {
+                const int pos = n + __popc(b & below);
+                h.key[pos] = key;
+                h.col[pos] = (int)cbase + lane;
+                h.lane[pos] = src;
+            }
+            n += __popc(b);
+        }
+        __syncwarp();
+    } while (rows);
+}
+
+// Hits of gemm_topk.cu, and many of the resident kernel's, wait per thread in shared memory (entry i of a thread at [i * STAGE_LD]: raw key s = -t and column), found by groups of
+// eight columns that hold one.  All lanes of the warp call it.
+constexpr int STAGE_N = 16;
+constexpr int STAGE_LD = 32 * NUM_EPI_WARPS;
+template <typename Drain>
+__device__ __forceinline__ void stage_columns(uint32_t (&r)[32], int64_t cbase, int64_t ncols_end, bool partial, float thr,
+                                              float* stage_key, int32_t* stage_idx, int& nstaged, Drain drain) {
     if (partial) mask_columns(r, cbase, ncols_end);
     float gm[4];
     group_maxima(r, gm);
@@ -340,15 +390,28 @@ __device__ __forceinline__ void filter_columns(uint32_t (&r)[32], int64_t cbase,
     }
     __syncwarp();
 }
+// A thread's n staged hits to its row's candidate buffer: one atomic takes their slots; the counter also counts entries
+// that no longer fit.
+__device__ __forceinline__ void drain_stage(int32_t* cnt, float* ck, int32_t* ci, int cap, float ksc, const float* sk,
+                                            const int32_t* si, int n) {
+    if (n <= 0) return;
+    const int base = atomicAdd(cnt, n);
+    for (int i = 0; i < n; i++) {
+        if (base + i < cap) {
+            ck[base + i] = ksc * sk[i * STAGE_LD];
+            ci[base + i] = si[i * STAGE_LD];
+        }
+    }
+}
 
-// NCH x 32 accumulator columns from taddr on, through `use(registers, chunk)`: a chunk is used while the next one is on
-// its way, and `release` is called once the last one has arrived.
-template <int NCH, int UNROLL = 1, typename Use, typename Release>
-__device__ __forceinline__ void scan_columns(uint32_t taddr, Use use, Release release) {
+// NCH x 32 accumulator columns from taddr on, through `use(registers, chunk)`, a chunk while the next one is on its way;
+// `release` is called once the last one has arrived.  For many hits, which hold a chunk up.
+template <int NCH, typename Use, typename Release>
+__device__ __forceinline__ void scan_columns_ahead(uint32_t taddr, Use use, Release release) {
     static_assert(NCH % 2 == 0, "chunks are taken in pairs");
     uint32_t a[32], b[32];
     tc_ld32(taddr, a);
-#pragma unroll UNROLL
+#pragma unroll 1
     for (int ch = 0; ch < NCH; ch += 2) {
         tc_wait_ld32(a);
         tc_ld32(taddr + (ch + 1) * 32, b);
@@ -357,6 +420,21 @@ __device__ __forceinline__ void scan_columns(uint32_t taddr, Use use, Release re
         if (ch + 2 < NCH) tc_ld32(taddr + (ch + 2) * 32, a);
         else release();
         use(b, ch + 1);
+    }
+}
+
+// nch x 32 accumulator columns from taddr on, through `use(registers, chunk)`; `release` is called once the last ones have
+// arrived.  Reading 32 columns takes 40 cycles beside the other warps of the scheduler and MMAs, too few to read ahead.
+template <int UNROLL = 1, typename Use, typename Release>
+__device__ __forceinline__ void scan_columns(uint32_t taddr, int nch, Use use, Release release) {
+    if (nch == 0) release();
+#pragma unroll UNROLL
+    for (int ch = 0; ch < nch; ch++) {
+        uint32_t r[32];
+        tc_ld32(taddr + ch * 32, r);
+        tc_wait_ld32(r);
+        if (ch == nch - 1) release();
+        use(r, ch);
     }
 }
 

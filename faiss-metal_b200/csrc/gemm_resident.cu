@@ -6,28 +6,33 @@
 // tile has so few MMAs there (7 to 30) that reading its accumulator takes as long, and the pair shape of
 // gemm_topk.cu, whose two accumulators fill the tensor memory, cannot do both at once.
 //
-// 320 threads, a cluster of two CTAs per 256 x 256 tile (cta_group::2, M = N = 256), persistent over work items
-// (query block, range of X tiles):
+// A cluster of two CTAs per 256 x 256 tile (cta_group::2, M = N = 256), persistent over work items (query block, range of
+// X tiles):
 //   warp 0     producer: the CTA's half of the query block once per item, then its half (128 rows) of the X k-blocks,
 //              16 KiB each, through a ring of barriers per block
 //   warp 1     of the even CTA: MMAs of one tile after another into two accumulators of 256 columns.  The whole warp walks through
 //              the tiles and one lane issues: by a lane alone an MMA took 190 cycles with the waits and commits around it, the
 //              tensor pipe 128 (tile of 19 MMAs: 3,689 -> 2,920 cycles)
-//   warps 2-9  epilogue: a warp reads 32 rows and half the columns of one accumulator while the MMAs of the
-//              next tile fill the other
+//   warps 2..  epilogue: a warp reads 32 rows and a part of the columns of one accumulator while the MMAs of the
+//              next tile fill the other; twelve warps where hits are few, else eight
 // X blocks that two plane products share (fp32 rows: plane 0 meets both query planes) are loaded once and used
 // twice: 64 KiB a CTA and tile of d = 96 instead of 144 with the query blocks.
 //
-// Against the pair shape of gemm_topk.cu: 2,048 queries, k = 1024, 5 M fp32 rows of d = 96: 8.15 -> 6.08 ms a search;
-// 1,000 queries, k = 10, 100,000 fp32 rows of d = 128: 189 -> 156 us.  Bound by the epilogue (tensor pipe 50 % busy where
-// one column in 400 is a hit).
+// Against the pair shape of gemm_topk.cu, at its introduction: 2,048 queries, k = 1024, 5 M fp32 rows of d = 96: 8.15 -> 6.08 ms a
+// search; 1,000 queries, k = 10, 100,000 fp32 rows of d = 128: 189 -> 156 us; with twelve warps and the hits' queue the first takes
+// 5.2 ms and draws the power cap (1.52 GHz).
 #include "gemm_common.cuh"
 
 namespace b200f {
 
 namespace {
 
-constexpr int RES_THREADS = 32 * (2 + NUM_EPI_WARPS);
+// Epilogue warps: three per TMEM lane quarter where hits are few (5,345 -> 5,170 us for the first search above), which their
+// registers allow; else two.
+template <int MODE>
+constexpr int RES_EPI_WARPS = MODE == MODE_FILTER ? 12 : NUM_EPI_WARPS;
+template <int MODE>
+constexpr int RES_THREADS = 32 * (2 + RES_EPI_WARPS<MODE>);
 constexpr int RES_BLOCK_BYTES = 128 * BK * 2;   // a k-block of 128 query rows or 128 rows of X
 constexpr int RES_BLOCKS = 12;                  // query block and ring together
 constexpr int RES_MAX_RING = 11;
@@ -38,6 +43,7 @@ constexpr int RES_SM_TMEMPTR = RES_SM_BAR + (2 * RES_MAX_RING + 6) * 8;
 constexpr int RES_SM_ABORT = RES_SM_TMEMPTR + 4;
 constexpr int RES_SMEM_BYTES = RES_SM_ABORT + 4 + 8;
 constexpr int RES_TILE_N = 256;
+static_assert(RES_EPI_WARPS<MODE_FILTER> * HITS_BYTES <= RES_SM_BAR - RES_SM_STAGE && HITS_BYTES % 16 == 0, "hits share the transposes' area");
 
 struct ResidentParams {
     GemmParams g;        // ntiles, tiles_per_range and P count tiles of 256 columns
@@ -47,10 +53,11 @@ struct ResidentParams {
 };
 
 template <int MODE>
-__global__ void __launch_bounds__(RES_THREADS, 1)
+__global__ void __launch_bounds__(RES_THREADS<MODE>, 1)
 gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                      const ResidentParams rp) {
     const GemmParams& p = rp.g;
+    constexpr bool FILTER = MODE == MODE_FILTER || MODE == MODE_DENSE;
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t sbase = smem_u32(smem);
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);   // uniform
@@ -86,7 +93,7 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         mbar_init(bar_qempty, 1);
         for (int s = 0; s < 2; s++) {
             mbar_init(bar_tfull + s * 8, 1);
-            mbar_init(bar_tempty + s * 8, 2 * NUM_EPI_WARPS);   // the epilogue warps of both CTAs
+            mbar_init(bar_tempty + s * 8, 2 * RES_EPI_WARPS<MODE>);   // the epilogue warps of both CTAs
         }
         mbar_fence_init();
     }
@@ -262,13 +269,17 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     } else {
         // ------------------------------ epilogue ------------------------------
         const int ew = warp & 3;            // TMEM lane quarter this warp may read
-        const int eh = (warp - 2) >> 2;     // which half of the columns
+        // which chunks of 32 columns: three, three and two, or four and four
+        const int part = (warp - 2) >> 2;
+        constexpr int PER_WARP = MODE == MODE_FILTER ? 3 : 4;
+        const int ch0 = part * PER_WARP, nch = min(PER_WARP, RES_TILE_N / 32 - ch0);
         const int row = ew * 32 + lane;
         float* const stage_key = reinterpret_cast<float*>(smem + RES_SM_STAGE) + (threadIdx.x - 64);
         int32_t* const stage_idx =
                 reinterpret_cast<int32_t*>(smem + RES_SM_STAGE) + STAGE_N * STAGE_LD + (threadIdx.x - 64);
+        const WarpHits hits = warp_hits(smem + RES_SM_STAGE + (warp - 2) * HITS_BYTES);
         const uint32_t tempty0 = map_to_cta(bar_tempty, 0);
-        int acc = 0, nstaged = 0;
+        int acc = 0, nhits = 0, nstaged = 0;
         uint32_t acc_phase = 0;
         bool ok = true;
         for (int64_t item = unit; item < nitems && ok; item += nunits) {
@@ -280,15 +291,21 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
             // coherent loads: the kernel before a programmatic launch wrote the map
             if (p.rowscale && row_live) ksc *= __ldcg(p.rowscale + (p.rowscale_map ? (int64_t)__ldcg(p.rowscale_map + grow) : grow));
             float thr = -CUDART_INF_F, radd = 0.f;
-            if (MODE == MODE_FILTER) {
+            if (FILTER) {
                 if (row_live) thr = filter_threshold(__ldcg(p.fthr + grow * p.fthr_stride + p.fthr_pos) / ksc);
             } else if (row_live && p.rowadd) {
                 radd = p.rowadd[grow];
             }
-            auto drain = [&]() {
-                drain_to_buffer(p.cand_cnt + grow, p.cand_key + grow * p.cand_cap, p.cand_idx + grow * p.cand_cap,
-                                p.cand_cap, ksc, stage_key, stage_idx, nstaged);
+            auto drain = [&]() {   // the stage
+                drain_stage(p.cand_cnt + grow, p.cand_key + grow * p.cand_cap, p.cand_idx + grow * p.cand_cap, p.cand_cap,
+                                          ksc, stage_key, stage_idx, nstaged);
                 nstaged = 0;
+            };
+            auto drain_queue = [&]() {
+                const int64_t row0 = grow - lane;
+                drain_hits(p.cand_cnt + row0, p.cand_key + row0 * p.cand_cap, p.cand_idx + row0 * p.cand_cap, p.cand_cap, ksc, hits.key,
+                           hits.col, hits.lane, nhits);
+                nhits = 0;
             };
             for (int64_t t = t0; t < t1; t++) {
                 const int64_t c_tile = tile_col(t);
@@ -301,24 +318,31 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                 }
                 tc_fence_after();
                 const bool partial = c_tile + RES_TILE_N > p.ncols_end;
-                const uint32_t taddr = tmem_base + ((uint32_t)(ew * 32) << 16) + acc * RES_TILE_N + eh * (RES_TILE_N / 2);
-                const int64_t cbase = c_tile + eh * (RES_TILE_N / 2);
+                const uint32_t taddr = tmem_base + ((uint32_t)(ew * 32) << 16) + acc * RES_TILE_N + ch0 * 32;
+                const int64_t cbase = c_tile + ch0 * 32;
                 auto release = [&]() {
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive_cluster(tempty0 + acc * 8);
                 };
                 if constexpr (MODE == MODE_FILTER) {
-                    scan_columns<RES_TILE_N / 64>(
+                    scan_columns(
+                            taddr, nch,
+                            [&](uint32_t(&r)[32], int ch) {
+                                filter_columns(r, cbase + ch * 32, p.ncols_end, partial, thr, hits, nhits, drain_queue);
+                            },
+                            release);
+                } else if constexpr (MODE == MODE_DENSE) {
+                    scan_columns_ahead<PER_WARP>(
                             taddr,
                             [&](uint32_t(&r)[32], int ch) {
-                                filter_columns(r, cbase + ch * 32, p.ncols_end, partial, thr, stage_key, stage_idx, nstaged, drain);
+                                stage_columns(r, cbase + ch * 32, p.ncols_end, partial, thr, stage_key, stage_idx, nstaged, drain);
                             },
                             release);
                 } else if constexpr (MODE == MODE_MINIMA) {
-                    float v[RES_TILE_N / 64];
-                    scan_columns<RES_TILE_N / 64, RES_TILE_N / 64>(
-                            taddr,
+                    float v[PER_WARP];
+                    scan_columns<PER_WARP>(
+                            taddr, PER_WARP,
                             [&](uint32_t(&r)[32], int ch) {
                                 if (partial) mask_columns(r, cbase + ch * 32, p.ncols_end);
                                 float gm[4];
@@ -326,31 +350,25 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                                 v[ch] = -ksc * fmaxf(max3(gm[0], gm[1], gm[2]), gm[3]);
                             },
                             release);
-                    if (row_live) store_minima(v, p.out + grow * p.ld + t * (RES_TILE_N / MIN_GROUP) + eh * (RES_TILE_N / 64));
+                    if (row_live) store_minima(v, p.out + grow * p.ld + t * (RES_TILE_N / MIN_GROUP) + ch0);
                 } else {
                     const bool whole = !partial && (p.ld & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
                     float* const tbuf = reinterpret_cast<float*>(smem + RES_SM_STAGE) + (warp - 2) * (32 * 33);
-                    const int64_t ocol = t * RES_TILE_N + eh * (RES_TILE_N / 2);
-                    scan_columns<RES_TILE_N / 64>(
-                            taddr,
+                    const int64_t ocol = t * RES_TILE_N + ch0 * 32;
+                    scan_columns(
+                            taddr, nch,
                             [&](uint32_t(&r)[32], int ch) {
                                 store_keys(p, r, whole, grow, lane, nq_live, row_live, cbase + ch * 32, ocol + ch * 32, ksc, radd, tbuf);
                             },
                             release);
                 }
-                // Staged hits wait for company: an atomic's round trip each tile is a third of what a tile of 19
-                // MMAs leaves its epilogue.
-                if (MODE == MODE_FILTER && __any_sync(0xffffffffu, nstaged > STAGE_N / 2)) {
-                    drain();
-                    __syncwarp();
-                }
+                if (MODE == MODE_FILTER && nhits >= QUEUE_DRAIN) drain_queue();
+                if (MODE == MODE_DENSE && __any_sync(0xffffffffu, nstaged > STAGE_N / 2)) drain();
                 acc ^= 1;
                 if (acc == 0) acc_phase ^= 1;
             }
-            if (MODE == MODE_FILTER) {
-                drain();
-                __syncwarp();
-            }
+            if (MODE == MODE_FILTER && ok) drain_queue();   // the next range may have other rows
+            if (MODE == MODE_DENSE && ok) drain();
         }
     }
 
@@ -404,19 +422,21 @@ int launch_resident(const GemmOperands& op, const GemmPlan& plan, GemmParams& g,
     const int grid = (int)(2 * (items < plan.units ? items : plan.units));
 
     typedef void (*KernelFn)(const CUtensorMap, const CUtensorMap, const ResidentParams);
-    const KernelFn kernel = g.mode == MODE_FILTER   ? gemm_resident_kernel<MODE_FILTER>
+    const KernelFn kernel = g.mode == MODE_FILTER   ? (g.dense ? gemm_resident_kernel<MODE_DENSE> : gemm_resident_kernel<MODE_FILTER>)
                             : g.mode == MODE_STORE ? gemm_resident_kernel<MODE_STORE>
                                                    : gemm_resident_kernel<MODE_MINIMA>;
     static bool attr_set[kMaxDevices] = {false};
     const int slot = device_slot();
     if (!attr_set[slot]) {
-        for (KernelFn fn : {gemm_resident_kernel<MODE_FILTER>, gemm_resident_kernel<MODE_STORE>, gemm_resident_kernel<MODE_MINIMA>})
+        for (KernelFn fn : {gemm_resident_kernel<MODE_FILTER>, gemm_resident_kernel<MODE_STORE>, gemm_resident_kernel<MODE_MINIMA>,
+                            gemm_resident_kernel<MODE_DENSE>})
             B200F_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, RES_SMEM_BYTES));
         attr_set[slot] = true;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid, 1, 1);
-    cfg.blockDim = dim3(RES_THREADS, 1, 1);
+    const int threads = g.mode == MODE_FILTER && !g.dense ? RES_THREADS<MODE_FILTER> : RES_THREADS<MODE_STORE>;
+    cfg.blockDim = dim3((unsigned)threads, 1, 1);
     cfg.dynamicSmemBytes = RES_SMEM_BYTES;
     cfg.stream = ln.stream;
     cudaLaunchAttribute attr[2];

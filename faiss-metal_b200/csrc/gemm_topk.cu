@@ -16,9 +16,8 @@
 //   warp 0      TMA producer: Q tile (128 x 64) and X tile per k-block, 128-byte swizzle,
 //               4-stage mbarrier ring
 //   warps 1,10  MMA issuers: tcgen05.mma kind::f16, N = 256, K = 16, fp32 accumulators in
-//               TMEM.  A chain of MMAs on one accumulator runs at about half the tensor rate,
-//               so the pair shape runs two chains (columns 0-255 and 256-511 of the tile),
-//               one issuing thread each.
+//               TMEM; the pair shape has two chains of them (columns 0-255 and 256-511 of the
+//               tile), one issuing thread each.
 //   warps 2-9   epilogue: tcgen05.ld (thread t owns query row t of the tile, two warps per
 //               TMEM lane quarter, half of the tile's columns each), one max per column (the
 //               L2 bias -||x||^2/2 is part of the dot product: 8 extra K columns, see
@@ -31,9 +30,12 @@
 //           candidate buffer in global memory
 //   store   the keys are written out as a matrix (k beyond the list paths, pairwise distances)
 //   minima  the smallest key of every 32 columns is (samples that thresholds are taken from)
-// The mode is a template parameter (eight instantiations with the two shapes): the filter and
-// store kernels carry no list registers, which lets the filter kernel read 64 accumulator
-// columns per TMEM load.  A work item is (query block, column range).
+// The mode is a template parameter (eight instantiations with the two shapes): only the top-k
+// kernels carry list registers.  A work item is (query block, column range).
+//
+// Large launches draw the 1 kW power cap: 10,000 queries, 1 M fp16 rows of d = 768, run at 1.54 GHz, the
+// tensor pipe busy for 12,300 of a tile's 16,000 cycles; 4,096 queries, 10 M bf16 rows of d = 1536, at 1.1 - 1.3 GHz, 25,100
+// of 29,000.
 //
 // FP32 storage: both operands are split into three bf16 planes
 // (x = x0 + x1 + x2 exactly to 24 bits) and six plane products
@@ -67,13 +69,12 @@ template <bool PAIR>
 struct Cfg {
     static constexpr int STAGES = 4;
     static constexpr int B_ROWS = PAIR ? 128 : 256;        // rows of X this CTA stages per sub-tile
-    // A dependent chain of MMAs on ONE accumulator runs at about half the tensor rate (each
-    // MMA waits out the read-modify-write turnaround of the one before it); two chains on two
-    // accumulators, one issuing thread each, come close to the full rate.  The pair shape
-    // therefore computes two 256-column sub-tiles at once (same query k-block, two X k-blocks,
-    // both TMEM halves); the price is that a chain's epilogue no longer overlaps its next MMAs.
-    // Each chain has its own accumulator-full / accumulator-free barriers and its own four
-    // epilogue warps per CTA, so one chain's MMAs do run beside the other chain's epilogue.
+    // The pair shape computes two 256-column sub-tiles at once (same query k-block, two X k-blocks,
+    // both TMEM halves): 48 KiB of shared-memory fill a CTA and 1,024 cycles of MMAs, where a 256 x 256 tile takes 64
+    // (with two such accumulators in turn and 32 KiB stages 1 M fp16 rows of d = 768 took 15,983 us, 14,484 this way).  The price
+    // is that a chain's epilogue does not overlap its own next MMAs.  One thread and one chain of
+    // MMAs fill the tensor pipe (128.5 cycles per 256 x 256 x 16), so one chain's MMAs cover the other's epilogue:
+    // each has its own accumulator-full / accumulator-free barriers and its own four epilogue warps per CTA.
     static constexpr int NSUB = PAIR ? 2 : 1;              // 256-column sub-tiles per tile
     static constexpr int TILE_N = NSUB * BN;               // columns of X per tile: 512 / 256
     static constexpr int ACC_BUFS = PAIR ? 1 : 2;          // TMEM accumulator buffers of TILE_N columns
@@ -115,6 +116,9 @@ __device__ __forceinline__ void reglist_insert(float (&lk)[KMAX], int32_t (&li)[
     }
 }
 
+// Hits of the tile in flight are staged per thread (stage_columns) and worked off AFTER the accumulator has been handed
+// back to the MMA issuers, so that list insertion runs beside the next tile's MMAs instead of in front of them.  Only a
+// thread whose stage fills up inside one tile (list warm-up, massive ties) drains it on the spot.
 __device__ __forceinline__ void drain_to_list(float (&lk)[KMAX], int32_t (&li)[KMAX], const float* sk,
                                               const int32_t* si, int n, float& thr, float& thr_eff) {
     for (int i = 0; i < n; i++) {
@@ -173,7 +177,7 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
         }
         for (int s = 0; s < 2; s++) {
             // single CTA: barrier s = accumulator buffer s, all epilogue warps;
-            // pair: barrier s = chain s, the warps of that column half in both CTAs
+            // pair: barrier s = chain s, the warps of that chain in both CTAs
             mbar_init(bar_tfull + s * 8, 1);
             mbar_init(bar_tempty + s * 8, NUM_EPI_WARPS);
         }
@@ -269,9 +273,8 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
         // The tensor pipe idles whenever this thread is not issuing, so the loop carries
         // nothing but the barrier wait, four MMAs and the commit(s) per k-block:
         // descriptors, barrier addresses and the shape of the last k-block are set up once.
-        // One thread sustains about one MMA per 190 cycles, and a chain of MMAs on one
-        // accumulator about one per 290; in the pair shape the two accumulator chains of a tile
-        // are therefore issued by two threads (warp 1: columns 0-255, warp MMA2_WARP: 256-511).
+        // In the pair shape the two accumulator chains of a tile are issued by a thread each (warp 1: columns 0-255, warp
+        // MMA2_WARP: 256-511), so that neither waits for the other's accumulator.
         const int chain = (warp == 1) ? 0 : 1;
         if (lane == 0 && cta_rank == 0 && (chain == 0 || PAIR)) {
             int stage = 0;
@@ -408,19 +411,16 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
             } else if (row_live && p.rowadd) {
                 radd = p.rowadd[grow];
             }
-            if (MODE == MODE_TOPK && !row_live) thr_eff = -CUDART_INF_F;   // takes nothing
             auto drain = [&]() {
-                if (MODE == MODE_TOPK)
-                    drain_to_list(lk, li, stage_key, stage_idx, nstaged, thr, thr_eff);
-                else
-                    drain_to_buffer(p.cand_cnt + grow, p.cand_key + grow * p.cand_cap, p.cand_idx + grow * p.cand_cap,
-                                    p.cand_cap, ksc, stage_key, stage_idx, nstaged);
+                drain_stage(p.cand_cnt + grow, p.cand_key + grow * p.cand_cap, p.cand_idx + grow * p.cand_cap, p.cand_cap, ksc,
+                            stage_key, stage_idx, nstaged);
                 nstaged = 0;
             };
             for (int64_t t = t0; t < t1 && ok; t++) {
+                const int buf = PAIR ? eh : acc;
                 const int64_t c_tile = p.col0 + t * p.tile_stride * TILE_N;
                 {
-                    const bool w = mbar_wait(bar_tfull + (PAIR ? eh : acc) * 8, acc_phase, abort_flag, p.status);
+                    const bool w = mbar_wait(bar_tfull + buf * 8, acc_phase, abort_flag, p.status);
                     if (!__all_sync(0xffffffffu, w)) {  // keep the warp converged for tcgen05.ld
                         ok = false;
                         break;
@@ -451,8 +451,8 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) {
-                        if (PAIR) mbar_arrive_cluster(map_to_cta(bar_tempty + eh * 8, 0));
-                        else mbar_arrive(bar_tempty + acc * 8);
+                        if (PAIR) mbar_arrive_cluster(map_to_cta(bar_tempty + buf * 8, 0));
+                        else mbar_arrive(bar_tempty + buf * 8);
                     }
                 };
                 const int64_t chalf = c_tile + eh * CH_PER_HALF * 32;   // this warp's half of the columns
@@ -463,20 +463,48 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
                     uint32_t r[32];
                     tc_ld32(thalf + ch * 32, r);
                     tc_wait_ld();
-                    filter_columns(r, chalf + ch * 32, p.ncols_end, partial, thr_eff, stage_key, stage_idx, nstaged, drain);
+                    const int64_t cbase = chalf + ch * 32;
+                    if (partial) mask_columns(r, cbase, p.ncols_end);
+                    float gm[4];
+                    group_maxima(r, gm);
+                    // entered by the whole warp when any row has a candidate in this chunk
+                    if (__any_sync(0xffffffffu, row_live && -fmaxf(max3(gm[0], gm[1], gm[2]), gm[3]) < thr_eff)) {
+#pragma unroll
+                        for (int g = 0; g < 4; g++) {
+                            const bool hit = row_live && -gm[g] < thr_eff;
+                            if (!__any_sync(0xffffffffu, hit)) continue;
+                            if (hit) {
+                                if (nstaged > STAGE_N - 8) {   // rare: list warm-up, massive ties
+                                    drain_to_list(lk, li, stage_key, stage_idx, nstaged, thr, thr_eff);
+                                    nstaged = 0;
+                                }
+#pragma unroll
+                                for (int c = 0; c < 8; c++) {
+                                    const float sc = -__uint_as_float(r[8 * g + c]);
+                                    if (sc < thr_eff) {
+                                        stage_key[nstaged * STAGE_LD] = sc;
+                                        stage_idx[nstaged * STAGE_LD] = (int32_t)cbase + 8 * g + c;
+                                        nstaged++;
+                                    }
+                                }
+                            }
+                        }
+                        __syncwarp();
+                    }
                 }
                 release();
                 } else if constexpr (MODE == MODE_FILTER) {
-                    scan_columns<CH_PER_HALF>(
-                            thalf,
-                            [&](uint32_t(&r)[32], int ch) {
-                                filter_columns(r, chalf + ch * 32, p.ncols_end, partial, thr_eff, stage_key, stage_idx, nstaged, drain);
-                            },
-                            release);
+                    auto stage = [&](uint32_t(&r)[32], int ch) {
+                        stage_columns(r, chalf + ch * 32, p.ncols_end, partial, thr_eff, stage_key, stage_idx, nstaged, drain);
+                    };
+                    // reading ahead pays where hits hold most chunks up (300 queries, k = 1024, 1 M bf16 rows of d = 1024: 1,073 ->
+                    // 965 us), not beside full query blocks with few (1,000 queries, k = 100: 1,760 against 1,888)
+                    if (p.dense) scan_columns_ahead<CH_PER_HALF>(thalf, stage, release);
+                    else scan_columns(thalf, CH_PER_HALF, stage, release);
                 } else if constexpr (MODE == MODE_MINIMA) {
                     float v[CH_PER_HALF];
-                    scan_columns<CH_PER_HALF, CH_PER_HALF>(
-                            thalf,
+                    scan_columns<CH_PER_HALF>(
+                            thalf, CH_PER_HALF,
                             [&](uint32_t(&r)[32], int ch) {
                                 if (partial) mask_columns(r, chalf + ch * 32, p.ncols_end);
                                 float gm[4];
@@ -484,21 +512,26 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
                                 v[ch] = -ksc * fmaxf(max3(gm[0], gm[1], gm[2]), gm[3]);
                             },
                             release);
-                    if (row_live) store_minima(v, p.out + grow * p.ld + t * (TILE_N / MIN_GROUP) + eh * CH_PER_HALF);
+                    if (row_live)
+                        store_minima(v, p.out + grow * p.ld + t * (TILE_N / MIN_GROUP) + eh * CH_PER_HALF);
                 } else {
                     const bool whole = !partial && (p.ld & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
                     // the list area is idle in this mode; tiles lie side by side in the output, whatever the stride
                     float* const tbuf = reinterpret_cast<float*>(smem + SM_LKEY) + (warp - 2) * (32 * 33);
                     const int64_t ohalf = t * TILE_N + eh * CH_PER_HALF * 32;
-                    scan_columns<CH_PER_HALF>(
-                            thalf,
+                    scan_columns(
+                            thalf, CH_PER_HALF,
                             [&](uint32_t(&r)[32], int ch) {
                                 store_keys(p, r, whole, grow, lane, nq_live, row_live, chalf + ch * 32, ohalf + ch * 32, ksc, radd, tbuf);
                             },
                             release);
                 }
                 // the accumulator is back with the MMA issuers: now work off the staged hits
-                if (nstaged > 0) drain();
+                if (MODE == MODE_TOPK && nstaged > 0) {
+                    drain_to_list(lk, li, stage_key, stage_idx, nstaged, thr, thr_eff);
+                    nstaged = 0;
+                }
+                if (MODE == MODE_FILTER && __any_sync(0xffffffffu, nstaged > STAGE_N / 2)) drain();
                 __syncwarp();
                 if (C::ACC_BUFS == 2) {
                     acc ^= 1;
@@ -507,6 +540,7 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
                     acc_phase ^= 1;
                 }
             }
+            if (MODE == MODE_FILTER && ok) drain();   // the next item has other rows
             if (MODE == MODE_TOPK && row_live && ok) {
                 if (thr < thr_pub) atomicMin(gslot, float_to_ordered(thr));
                 // two lists per (row, column range): one per column half
@@ -784,7 +818,7 @@ int launch_gemm_topk(const GemmOperands& op, const GemmPlan& plan, int64_t col0,
 
 int launch_gemm_filter(const GemmOperands& op, const GemmPlan& plan, float kscale, const float* thr,
                        int thr_stride, int thr_pos, float* cand_key, int32_t* cand_idx,
-                       int32_t* cand_cnt, int cand_cap, int few_hits, int32_t* status,
+                       int32_t* cand_cnt, int cand_cap, int dense, int32_t* status,
                        const Launch& ln) {
     if (!thr || !cand_key || !cand_idx || !cand_cnt || cand_cap < 1) return B200F_ERR_BAD_ARG;
     GemmParams p{};
@@ -798,7 +832,7 @@ int launch_gemm_filter(const GemmOperands& op, const GemmPlan& plan, float kscal
     p.cand_idx = cand_idx;
     p.cand_cnt = cand_cnt;
     p.cand_cap = cand_cap;
-    p.wide = few_hits ? 1 : 0;
+    p.dense = dense;
     p.status = status;
     return launch_common(op, spread_plan(plan), p, 0, op.nb, ln);
 }

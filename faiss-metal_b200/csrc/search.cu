@@ -849,10 +849,12 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
             rc = launch_merge_keys(pkey, pidx, 2 * pl.pilot.P, a->nq, pl.frank, thr, ln);
             if (rc != B200F_OK) return rc;
         }
-        // about frank * fstride candidates per row; wide TMEM loads where fewer than one row in 1024 is one
-        const int wide = (int64_t)pl.frank * pl.fstride * 1024 < a->nb ? 1 : 0;
+        // About frank * fstride candidates a query.  Of the GEMMs' two ways with hits that for many pays from one column in 500
+        // to 800 on: 1,000 queries, 1 M fp32 rows of d = 100, k = 100 (704 candidates) 541 us with the one for few, 586 with the
+        // other, k = 200 (1,408) 707 and 632; 100,000 rows of d = 128, k = 32 (136) 109 and 111, k = 100 (264) 118 and 115.
+        const int dense = (int64_t)pl.frank * pl.fstride * 768 > a->nb ? 1 : 0;
         rc = launch_gemm_filter(op, pl.gemm, kscale, thr, pl.pilot_matrix ? 1 : pl.frank,
-                                pl.pilot_matrix ? 0 : pl.frank - 1, ckey, cidx, ccnt, pl.fcap, wide, a->status, ln);
+                                pl.pilot_matrix ? 0 : pl.frank - 1, ckey, cidx, ccnt, pl.fcap, dense, a->status, ln);
         if (rc != B200F_OK) return rc;
         rc = launch_select_candidates(ckey, cidx, ccnt, pl.fcap, a->nb, a->nq, a->k, a->metric, qnorm,
                                       a->label_base, a->out_dist, a->out_labels, dirty, nullptr,
