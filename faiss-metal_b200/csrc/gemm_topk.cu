@@ -19,7 +19,7 @@
 //               TMEM; the pair shape has two chains of them (columns 0-255 and 256-511 of the
 //               tile), one issuing thread each.
 //   warps 2-9   epilogue: tcgen05.ld (thread t owns query row t of the tile, two warps per
-//               TMEM lane quarter, half of the tile's columns each), one max per column (the
+//               TMEM lane quarter, half of an accumulator's columns each), one max per column (the
 //               L2 bias -||x||^2/2 is part of the dot product: 8 extra K columns, see
 //               rows.cu), filter against the row's bound, hits staged in shared memory and
 //               worked off after the accumulator has been released.
@@ -74,7 +74,7 @@ struct Cfg {
     // (with two such accumulators in turn and 32 KiB stages 1 M fp16 rows of d = 768 took 15,983 us, 14,484 this way).  The price
     // is that a chain's epilogue does not overlap its own next MMAs.  One thread and one chain of
     // MMAs fill the tensor pipe (128.5 cycles per 256 x 256 x 16), so one chain's MMAs cover the other's epilogue:
-    // each has its own accumulator-full / accumulator-free barriers and its own four epilogue warps per CTA.
+    // each has its own accumulator-full / accumulator-free barriers, and they are read one after the other.
     static constexpr int NSUB = PAIR ? 2 : 1;              // 256-column sub-tiles per tile
     static constexpr int TILE_N = NSUB * BN;               // columns of X per tile: 512 / 256
     static constexpr int ACC_BUFS = PAIR ? 1 : 2;          // TMEM accumulator buffers of TILE_N columns
@@ -142,6 +142,9 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
     constexpr int TILE_N = C::TILE_N;
     constexpr int SM_A = C::SM_A, SM_B = C::SM_B, SM_LKEY = C::SM_LKEY;
     constexpr int SM_BAR = C::SM_BAR, SM_TMEMPTR = C::SM_TMEMPTR, SM_ABORT = C::SM_ABORT;
+    // pair: all epilogue warps on one accumulator after the other, or half of them on each (lists, whose first tiles insert
+    // nearly every column: 1,000 queries, 12,000 rows, k = 2: 145 us, 201 in turn)
+    constexpr bool IN_TURN = MODE != MODE_TOPK;
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t sbase = smem_u32(smem);
     const int warp = threadIdx.x >> 5;
@@ -177,9 +180,9 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
         }
         for (int s = 0; s < 2; s++) {
             // single CTA: barrier s = accumulator buffer s, all epilogue warps;
-            // pair: barrier s = chain s, the warps of that chain in both CTAs
+            // pair: barrier s = chain s, the epilogue warps of both CTAs
             mbar_init(bar_tfull + s * 8, 1);
-            mbar_init(bar_tempty + s * 8, NUM_EPI_WARPS);
+            mbar_init(bar_tempty + s * 8, (PAIR && IN_TURN ? 2 : 1) * NUM_EPI_WARPS);
         }
         mbar_fence_init();
     }
@@ -370,8 +373,8 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
     } else if (warp >= 2 && warp < 2 + NUM_EPI_WARPS) {
         // ------------------------------ epilogue -----------------------------------
         const int ew = warp & 3;              // TMEM lane quarter this warp may read
-        const int eh = (warp - 2) >> 2;       // which half of the tile's columns this warp scans
-        constexpr int CH_PER_HALF = TILE_N / 64;
+        const int eh = (warp - 2) >> 2;       // which half of an accumulator's columns this warp scans
+        constexpr int CH_PER_HALF = PAIR && !IN_TURN ? BN / 32 : BN / 64;
         const int row = ew * 32 + lane;       // row of the tile owned by this thread
         int acc = 0;
         uint32_t acc_phase = 0;
@@ -417,8 +420,13 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
                 nstaged = 0;
             };
             for (int64_t t = t0; t < t1 && ok; t++) {
-                const int buf = PAIR ? eh : acc;
-                const int64_t c_tile = p.col0 + t * p.tile_stride * TILE_N;
+                // Pair: one accumulator after the other, all eight warps on each, so that the first is back with its
+                // issuer, whose MMAs by themselves fill the pipe, while the second is read.  Half of the warps on each at the same
+                // time left the pipe idle for all of it (10,000 queries, 1 M fp16 rows of d = 768: a fifth of a tile's 17,500 cycles).
+#pragma unroll 1
+                for (int sub = PAIR && !IN_TURN ? eh : 0; sub < (PAIR && !IN_TURN ? eh + 1 : C::NSUB); sub++) {
+                const int buf = PAIR ? sub : acc;
+                const int64_t c_tile = p.col0 + t * p.tile_stride * TILE_N + sub * BN;
                 {
                     const bool w = mbar_wait(bar_tfull + buf * 8, acc_phase, abort_flag, p.status);
                     if (!__all_sync(0xffffffffu, w)) {  // keep the warp converged for tcgen05.ld
@@ -445,8 +453,8 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
                 // The accumulator holds t = q.x (- ||x||^2/2 for L2): larger is better; the
                 // lists keep s = -t (smaller is better).  Rows of X beyond the last valid
                 // column are zero-filled by TMA (t = 0) and must be masked out.
-                const bool partial = c_tile + TILE_N > p.ncols_end;
-                const uint32_t taddr = tmem_base + ((uint32_t)(ew * 32) << 16) + acc * TILE_N;
+                const bool partial = c_tile + BN > p.ncols_end;
+                const uint32_t taddr = tmem_base + ((uint32_t)(ew * 32) << 16) + buf * BN;
                 auto release = [&]() {
                     tc_fence_before();
                     __syncwarp();
@@ -455,8 +463,9 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
                         else mbar_arrive(bar_tempty + buf * 8);
                     }
                 };
-                const int64_t chalf = c_tile + eh * CH_PER_HALF * 32;   // this warp's half of the columns
-                const uint32_t thalf = taddr + eh * CH_PER_HALF * 32;
+                // this warp's columns
+                const int64_t chalf = c_tile + (PAIR && !IN_TURN ? 0 : eh * CH_PER_HALF * 32);
+                const uint32_t thalf = taddr + (PAIR && !IN_TURN ? 0 : eh * CH_PER_HALF * 32);
                 if constexpr (MODE == MODE_TOPK) {
 #pragma unroll 1
                 for (int ch = 0; ch < CH_PER_HALF; ch++) {
@@ -513,12 +522,12 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
                             },
                             release);
                     if (row_live)
-                        store_minima(v, p.out + grow * p.ld + t * (TILE_N / MIN_GROUP) + eh * CH_PER_HALF);
+                        store_minima(v, p.out + grow * p.ld + t * (TILE_N / MIN_GROUP) + sub * (BN / MIN_GROUP) + eh * CH_PER_HALF);
                 } else {
                     const bool whole = !partial && (p.ld & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
                     // the list area is idle in this mode; tiles lie side by side in the output, whatever the stride
                     float* const tbuf = reinterpret_cast<float*>(smem + SM_LKEY) + (warp - 2) * (32 * 33);
-                    const int64_t ohalf = t * TILE_N + eh * CH_PER_HALF * 32;
+                    const int64_t ohalf = t * TILE_N + sub * BN + eh * CH_PER_HALF * 32;
                     scan_columns(
                             thalf, CH_PER_HALF,
                             [&](uint32_t(&r)[32], int ch) {
@@ -526,7 +535,9 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
                             },
                             release);
                 }
-                // the accumulator is back with the MMA issuers: now work off the staged hits
+                }
+                if (!ok) break;
+                // the accumulators are back with the MMA issuers: now work off the staged hits
                 if (MODE == MODE_TOPK && nstaged > 0) {
                     drain_to_list(lk, li, stage_key, stage_idx, nstaged, thr, thr_eff);
                     nstaged = 0;
