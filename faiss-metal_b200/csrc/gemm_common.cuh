@@ -126,63 +126,52 @@ __device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap
             : "memory");
 }
 
-__device__ __forceinline__ void tc_commit_pair(uint32_t cluster_bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_bar)
-                 : "memory");
+// Issued by the lane with `leader` of a whole converged warp: control flow and operands stay uniform.
+template <bool PAIR>
+__device__ __forceinline__ void tc_mma_f16_by(bool leader, uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+                                              uint32_t accumulate) {
+    if (PAIR)
+        asm volatile(
+                "{\n\t"
+                ".reg .pred p, q;\n\t"
+                "setp.ne.b32 p, %4, 0;\n\t"
+                "setp.ne.b32 q, %5, 0;\n\t"
+                "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
+                "}\n" ::"r"(d_tmem),
+                "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"((uint32_t)leader)
+                : "memory");
+    else
+        asm volatile(
+                "{\n\t"
+                ".reg .pred p, q;\n\t"
+                "setp.ne.b32 p, %4, 0;\n\t"
+                "setp.ne.b32 q, %5, 0;\n\t"
+                "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+                "}\n" ::"r"(d_tmem),
+                "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"((uint32_t)leader)
+                : "memory");
 }
-
-__device__ __forceinline__ void tc_mma_f16_pair(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b,
-                                                uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-            "{\n\t"
-            ".reg .pred p;\n\t"
-            "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
-            "}\n" ::"r"(d_tmem),
-            "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-            : "memory");
-}
-
-// The same two for a whole converged warp, of which the lane with `leader` issues: control flow and operands stay uniform.
-__device__ __forceinline__ void tc_mma_f16_pair_by(bool leader, uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                                   uint32_t accumulate) {
-    asm volatile(
-            "{\n\t"
-            ".reg .pred p, q;\n\t"
-            "setp.ne.b32 p, %4, 0;\n\t"
-            "setp.ne.b32 q, %5, 0;\n\t"
-            "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
-            "}\n" ::"r"(d_tmem),
-            "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"((uint32_t)leader)
-            : "memory");
-}
-// arrives on the barrier at `bar` (an address of this CTA) in both CTAs of the pair
-__device__ __forceinline__ void tc_commit_both_by(bool leader, uint32_t bar) {
-    asm volatile(
-            "{\n\t"
-            ".reg .pred q;\n\t"
-            "setp.ne.b32 q, %1, 0;\n\t"
-            "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %2;\n\t"
-            "}\n" ::"r"(bar),
-            "r"((uint32_t)leader), "h"((uint16_t)3)
-            : "memory");
-}
-
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-                 : "memory");
-}
-
-__device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b,
-                                           uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-            "{\n\t"
-            ".reg .pred p;\n\t"
-            "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-            "}\n" ::"r"(d_tmem),
-            "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-            : "memory");
+// Arrives on the barrier at `bar` (an address of this CTA), in a pair on both CTAs', when the MMAs issued so far retire.
+template <bool PAIR>
+__device__ __forceinline__ void tc_commit_by(bool leader, uint32_t bar) {
+    if (PAIR)
+        asm volatile(
+                "{\n\t"
+                ".reg .pred q;\n\t"
+                "setp.ne.b32 q, %1, 0;\n\t"
+                "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %2;\n\t"
+                "}\n" ::"r"(bar),
+                "r"((uint32_t)leader), "h"((uint16_t)3)
+                : "memory");
+    else
+        asm volatile(
+                "{\n\t"
+                ".reg .pred q;\n\t"
+                "setp.ne.b32 q, %1, 0;\n\t"
+                "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
+                "}\n" ::"r"(bar),
+                "r"((uint32_t)leader)
+                : "memory");
 }
 
 // 32 lanes x 32 consecutive fp32 columns -> 32 registers per thread

@@ -190,11 +190,11 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
             uint32_t d_tmem = 0;
             auto block = [&](uint64_t da, int s, int nk4) {   // a k-block of the query block and X block s of the ring
                 const uint64_t db = db0 + (uint64_t)s * BLOCK;
-                tc_mma_f16_pair_by(leader, d_tmem, da, db, p.idesc, accumulate);
+                tc_mma_f16_by<true>(leader, d_tmem, da, db, p.idesc, accumulate);
                 accumulate = 1;
-                if (nk4 > 1) tc_mma_f16_pair_by(leader, d_tmem, da + 2, db + 2, p.idesc, 1);
-                if (nk4 > 2) tc_mma_f16_pair_by(leader, d_tmem, da + 4, db + 4, p.idesc, 1);
-                if (nk4 > 3) tc_mma_f16_pair_by(leader, d_tmem, da + 6, db + 6, p.idesc, 1);
+                if (nk4 > 1) tc_mma_f16_by<true>(leader, d_tmem, da + 2, db + 2, p.idesc, 1);
+                if (nk4 > 2) tc_mma_f16_by<true>(leader, d_tmem, da + 4, db + 4, p.idesc, 1);
+                if (nk4 > 3) tc_mma_f16_by<true>(leader, d_tmem, da + 6, db + 6, p.idesc, 1);
             };
             auto full = [&](int s, uint32_t ph) {
                 return mbar_try_wait(bar_full + s * 8, ph) || mbar_wait(bar_full + s * 8, ph, abort_flag, p.status);
@@ -233,13 +233,13 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                         for (int kb = 0; kb < nkd; kb++, da_low += BLOCK, step()) {
                             ok = ok && full(s, ph);
                             block(da_low, s, kb < nkd - 1 ? 4 : nk4_data);
-                            tc_commit_both_by(leader, bar_empty + s * 8);   // its last use
+                            tc_commit_by<true>(leader, bar_empty + s * 8);   // its last use
                         }
                         // query plane 0 with X plane 0
                         int s0 = base;
                         for (int kb = 0; kb < nkd; kb++, da += BLOCK) {
                             block(da, s0, kb < nkl - 1 ? 4 : nk4_end);
-                            tc_commit_both_by(leader, bar_empty + s0 * 8);
+                            tc_commit_by<true>(leader, bar_empty + s0 * 8);
                             if (++s0 == ring) s0 = 0;
                         }
                     }
@@ -247,9 +247,9 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                     for (int kb = two ? nkd : 0; kb < nkl; kb++, da += BLOCK, step()) {
                         ok = ok && full(s, ph);
                         block(da, s, kb < nkl - 1 ? 4 : nk4_end);
-                        tc_commit_both_by(leader, bar_empty + s * 8);
+                        tc_commit_by<true>(leader, bar_empty + s * 8);
                     }
-                    tc_commit_both_by(leader, bar_tfull + acc * 8);
+                    tc_commit_by<true>(leader, bar_tfull + acc * 8);
                     base = s;
                     phase = ph;
                     acc ^= 1;
@@ -257,7 +257,7 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                     ok = __all_sync(0xffffffffu, ok);   // a wait that ran out: the epilogues give up by themselves
                 }
                 const int64_t next = item + nunits;
-                if (ok && next < nitems && (int)(next % nqb) != qb) tc_commit_both_by(leader, bar_qempty);
+                if (ok && next < nitems && (int)(next % nqb) != qb) tc_commit_by<true>(leader, bar_qempty);
             }
             if (!ok) {   // let the MMAs in flight retire before tensor memory goes away
                 const long long t0 = clock64();

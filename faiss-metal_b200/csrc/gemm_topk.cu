@@ -17,7 +17,7 @@
 //               4-stage mbarrier ring
 //   warps 1,10  MMA issuers: tcgen05.mma kind::f16, N = 256, K = 16, fp32 accumulators in
 //               TMEM; the pair shape has two chains of them (columns 0-255 and 256-511 of the
-//               tile), one issuing thread each.
+//               tile), one issuing warp each.
 //   warps 2-9   epilogue: tcgen05.ld (thread t owns query row t of the tile, two warps per
 //               TMEM lane quarter, half of an accumulator's columns each), one max per column (the
 //               L2 bias -||x||^2/2 is part of the dot product: 8 extra K columns, see
@@ -147,7 +147,7 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
     constexpr bool IN_TURN = MODE != MODE_TOPK;
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t sbase = smem_u32(smem);
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);   // uniform
     const int lane = threadIdx.x & 31;
     const uint32_t cta_rank = PAIR ? cluster_ctarank() : 0u;   // 0 = MMA issuer of the pair
     const int64_t unit = PAIR ? (blockIdx.x >> 1) : blockIdx.x;  // work is dealt to CTAs / CTA pairs
@@ -273,13 +273,12 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
         }
     } else if (warp == 1 || warp == MMA2_WARP) {
         // ------------------------------ MMA issuer --------------------------------
-        // The tensor pipe idles whenever this thread is not issuing, so the loop carries
-        // nothing but the barrier wait, four MMAs and the commit(s) per k-block:
-        // descriptors, barrier addresses and the shape of the last k-block are set up once.
-        // In the pair shape the two accumulator chains of a tile are issued by a thread each (warp 1: columns 0-255, warp
-        // MMA2_WARP: 256-511), so that neither waits for the other's accumulator.
+        // The whole warp walks through the tiles and one lane issues, so that control flow and operands stay uniform: the tensor
+        // pipe idles whenever no MMA is issued.  In the pair shape the two accumulator chains of a tile have a warp each (warp
+        // 1: columns 0-255, warp MMA2_WARP: 256-511), so that neither waits for the other's accumulator.
         const int chain = (warp == 1) ? 0 : 1;
-        if (lane == 0 && cta_rank == 0 && (chain == 0 || PAIR)) {
+        if (cta_rank == 0 && (chain == 0 || PAIR)) {
+            const bool leader = elect_one();
             int stage = 0;
             uint32_t phase = 0;
             int acc = 0;
@@ -287,10 +286,6 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
             bool ok = true;
             const uint64_t da0 = make_smem_desc(sbase + SM_A);
             const uint64_t db0 = make_smem_desc(sbase + SM_B);
-            const uint32_t empty0 = PAIR ? map_to_cta(bar_empty, 0) : bar_empty;
-            const uint32_t empty1 = PAIR ? map_to_cta(bar_empty, 1) : 0;
-            const uint32_t tfull0 = PAIR ? map_to_cta(bar_tfull, 0) : bar_tfull;
-            const uint32_t tfull1 = PAIR ? map_to_cta(bar_tfull, 1) : 0;
             // the last k-block of a plane product may hold fewer than 64 valid K elements
             // (TMA zero-fills the rest): skip the all-zero sub-steps
             const int nk4_pass = (p.k_extent - (p.kb_per_pass - 1) * BK + UMMA_K - 1) / UMMA_K;
@@ -301,23 +296,18 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
                 const int64_t t1 = min(t0 + p.tiles_per_range, p.ntiles);
                 for (int64_t t = t0; t < t1 && ok; t++) {
                     const int bi = PAIR ? chain : acc;  // barrier pair of this chain / buffer
-                    if (!mbar_wait(bar_tempty + bi * 8, acc_phase ^ 1, abort_flag, p.status)) {
-                        ok = false;
-                        break;
-                    }
+                    ok = __all_sync(0xffffffffu, mbar_wait(bar_tempty + bi * 8, acc_phase ^ 1, abort_flag, p.status));
+                    if (!ok) break;
                     tc_fence_after();
-                    const uint32_t d_tmem = tmem_base + acc * TILE_N;
+                    const uint32_t d_tmem = tmem_base + acc * TILE_N + chain * BN;
                     int kin = 0;
                     const int kb_early = kb_total - p.kb_last_pass;   // k-blocks of the products before the last
                     uint32_t accumulate = 0;
                     for (int kb = 0; kb < kb_total; kb++) {
-                        if (!mbar_try_wait(bar_full + stage * 8, phase) &&
-                            !mbar_wait(bar_full + stage * 8, phase, abort_flag, p.status)) {
-                            ok = false;
-                            break;
-                        }
+                        ok = __all_sync(0xffffffffu, mbar_wait(bar_full + stage * 8, phase, abort_flag, p.status));
+                        if (!ok) break;
                         const uint64_t da = da0 + (uint64_t)(stage * (A_STAGE_BYTES >> 4));
-                        const uint64_t db = db0 + (uint64_t)(stage * (B_STAGE_BYTES >> 4));
+                        const uint64_t db = db0 + (uint64_t)(stage * (B_STAGE_BYTES >> 4) + chain * (C::B_SUB_BYTES >> 4));
                         int nk4 = BK / UMMA_K;
                         if (kb < kb_early) {
                             if (++kin == p.kb_per_pass) {
@@ -331,42 +321,30 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
                         for (int k4 = 0; k4 < BK / UMMA_K; k4++) {
                             // advance 32 bytes (16 elements) along K inside the swizzle row
                             if (k4 < nk4) {
-                                if (PAIR) {
-                                    tc_mma_f16_pair(d_tmem + chain * BN, da + (uint64_t)(k4 * 2),
-                                                    db + (uint64_t)(chain * (C::B_SUB_BYTES >> 4) + k4 * 2),
-                                                    p.idesc, accumulate);
-                                } else {
-                                    tc_mma_f16(d_tmem, da + (uint64_t)(k4 * 2), db + (uint64_t)(k4 * 2),
-                                               p.idesc, accumulate);
-                                }
+                                tc_mma_f16_by<PAIR>(leader, d_tmem, da + (uint64_t)(k4 * 2), db + (uint64_t)(k4 * 2), p.idesc,
+                                                    k4 > 0 ? 1 : accumulate);
                                 accumulate = 1;
                             }
                         }
-                        // frees the stage (in both CTAs of a pair) when the MMAs retire
-                        if (PAIR) {
-                            tc_commit_pair(empty0 + stage * 8);
-                            tc_commit_pair(empty1 + stage * 8);
-                        } else {
-                            tc_commit(empty0 + stage * 8);
-                        }
+                        tc_commit_by<PAIR>(leader, bar_empty + stage * 8);   // frees the stage when the MMAs retire
                         if (++stage == STAGES) {
                             stage = 0;
                             phase ^= 1;
                         }
                     }
                     if (!ok) break;
-                    if (PAIR) {  // this chain's accumulator complete, in both CTAs
-                        tc_commit_pair(tfull0 + chain * 8);
-                        tc_commit_pair(tfull1 + chain * 8);
-                    } else {
-                        tc_commit(tfull0 + acc * 8);
-                    }
+                    tc_commit_by<PAIR>(leader, bar_tfull + bi * 8);   // this chain's accumulator complete
                     if (C::ACC_BUFS == 2) {
                         acc ^= 1;
                         if (acc == 0) acc_phase ^= 1;
                     } else {
                         acc_phase ^= 1;
                     }
+                }
+            }
+            if (!ok) {   // let the MMAs in flight retire before tensor memory goes away
+                const long long t0 = clock64();
+                while (clock64() - t0 < 200000LL) {
                 }
             }
         }
