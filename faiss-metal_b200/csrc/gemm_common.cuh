@@ -31,6 +31,7 @@ struct GemmParams {
     // it cost to read X (24 queries, 1,000,003 fp16 rows of d = 770: 354 us a launch, 242 without).  What the
     // tile holds there instead reaches only accumulator rows that nobody reads.
     int a_rows;
+    int warp_rows;       // single CTA: query rows in a TMEM lane quarter, 32 or (at most 64 queries) 16
     // k-blocks of 64 and valid K elements (multiple of 8) of a plane product.  The norm columns are zero in
     // every plane but the first, so only the last product, of the two first planes, takes them (d = 128,
     // three products: 25 MMAs a tile instead of 27, 7 k-blocks instead of 9).
@@ -447,7 +448,7 @@ __device__ __forceinline__ float filter_threshold(float t) {
 // All lanes of a warp call it.  whole: whole sectors, straight from the registers; else (ragged or unaligned output,
 // where that would touch 32 rows per instruction) the warp transposes the 32 x 32 block through tbuf
 // [32][33] and writes one 128-byte row segment per instruction.
-__device__ __forceinline__ void store_keys(const GemmParams& p, const uint32_t (&r)[32], bool whole, int64_t grow, int lane,
+__device__ __forceinline__ void store_keys(const GemmParams& p, const uint32_t (&r)[32], bool whole, int64_t grow, int lane, int warp_rows,
                                            int64_t nq_live, bool row_live, int64_t cbase, int64_t ocol, float ksc,
                                            float radd, float* tbuf) {
     if (whole) {
@@ -468,11 +469,11 @@ __device__ __forceinline__ void store_keys(const GemmParams& p, const uint32_t (
         tbuf[lane * 33 + c] = fmaf(p.sign, key, radd);
     }
     __syncwarp();
-    const int64_t grow0 = grow - lane;   // first row of this warp's 32 rows
+    const int64_t grow0 = grow - lane;   // first of this warp's rows
     const bool col_ok = cbase + lane < p.ncols_end;
     float* obase = p.out + ocol + lane;
 #pragma unroll 8
-    for (int rr = 0; rr < 32; rr++) {
+    for (int rr = 0; rr < warp_rows; rr++) {
         const float v = tbuf[rr * 33 + lane];
         if (col_ok && grow0 + rr < nq_live) obase[(grow0 + rr) * p.ld] = v;
     }

@@ -358,7 +358,7 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                     scan_columns(
                             taddr, nch,
                             [&](uint32_t(&r)[32], int ch) {
-                                store_keys(p, r, whole, grow, lane, nq_live, row_live, cbase + ch * 32, ocol + ch * 32, ksc, radd, tbuf);
+                                store_keys(p, r, whole, grow, lane, 32, nq_live, row_live, cbase + ch * 32, ocol + ch * 32, ksc, radd, tbuf);
                             },
                             release);
                 }

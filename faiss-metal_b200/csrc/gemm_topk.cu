@@ -353,7 +353,8 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
         const int ew = warp & 3;              // TMEM lane quarter this warp may read
         const int eh = (warp - 2) >> 2;       // which half of an accumulator's columns this warp scans
         constexpr int CH_PER_HALF = PAIR && !IN_TURN ? BN / 32 : BN / 64;
-        const int row = ew * 32 + lane;       // row of the tile owned by this thread
+        const int warp_rows = PAIR ? 32 : p.warp_rows;
+        const int row = ew * warp_rows + lane;   // row of the tile owned by this thread, if lane < warp_rows
         int acc = 0;
         uint32_t acc_phase = 0;
         bool ok = true;
@@ -371,7 +372,7 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
             const int64_t t0 = xr * p.tiles_per_range;
             const int64_t t1 = min(t0 + p.tiles_per_range, p.ntiles);
             const int64_t grow = (int64_t)qb * C::QB + (int64_t)cta_rank * BM + row;
-            const bool row_live = grow < nq_live;
+            const bool row_live = grow < nq_live && lane < warp_rows;
             // slot of the row's bound array this list publishes to
             uint32_t* const gslot = p.gthr ? p.gthr + grow * p.gslots + (int)((2 * xr + eh) % p.gslots) : nullptr;
             float ksc = p.kscale;          // this row's key scale
@@ -509,7 +510,7 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
                     scan_columns(
                             thalf, CH_PER_HALF,
                             [&](uint32_t(&r)[32], int ch) {
-                                store_keys(p, r, whole, grow, lane, nq_live, row_live, chalf + ch * 32, ohalf + ch * 32, ksc, radd, tbuf);
+                                store_keys(p, r, whole, grow, lane, warp_rows, nq_live, row_live, chalf + ch * 32, ohalf + ch * 32, ksc, radd, tbuf);
                             },
                             release);
                 }
@@ -607,10 +608,15 @@ int launch_common(const GemmOperands& op, const GemmPlan& plan, GemmParams& p, i
         p.pass_a = 0x010201u;  // nibble i = plane of A in pass i (pass 0 is the lowest nibble)
         p.pass_b = 0x001021u;
     }
+    // At most 64 queries are a tile of M = 64, whose rows lie in all four lane quarters, sixteen in each: half the operand reads
+    // and products on rows that hold no query, and hits that two or four warps share instead of one or two (four batches of 24 queries
+    // in flight, 1,000,003 fp16 rows of d = 770: 1,380 -> 1,290 us; 50 queries, k = 2048, 300,007 rows of d = 256: level).
+    const int m = plan.pair ? 2 * BM : op.nq <= 64 ? 64 : BM;
+    p.warp_rows = m == 64 ? 16 : 32;
     const uint32_t fmt = op.is_bf16 ? 1u : 0u;
-    // fp32 accumulate, K-major operands, N = 256, M = 128 (one CTA) or 256 (CTA pair)
+    // fp32 accumulate, K-major operands, N = 256, M = 64 or 128 (one CTA) or 256 (CTA pair)
     p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(BN >> 3) << 17) |
-              ((uint32_t)((plan.pair ? 2 * BM : BM) >> 4) << 24);
+              ((uint32_t)(m >> 4) << 24);
 
     typedef void (*KernelFn)(const CUtensorMap, const CUtensorMap, const GemmParams);
     static const KernelFn kernels[2][4] = {
