@@ -608,9 +608,10 @@ int launch_common(const GemmOperands& op, const GemmPlan& plan, GemmParams& p, i
         p.pass_a = 0x010201u;  // nibble i = plane of A in pass i (pass 0 is the lowest nibble)
         p.pass_b = 0x001021u;
     }
-    // At most 64 queries are a tile of M = 64, whose rows lie in all four lane quarters, sixteen in each: half the operand reads
-    // and products on rows that hold no query, and hits that two or four warps share instead of one or two (four batches of 24 queries
-    // in flight, 1,000,003 fp16 rows of d = 770: 1,380 -> 1,290 us; 50 queries, k = 2048, 300,007 rows of d = 256: level).
+    // At most 64 queries are a tile of M = 64 (its rows lie in all four lane quarters, sixteen in each): half the operand reads and
+    // products on rows that hold no query, which cost power where the memory is the bound.  Four batches of 24 queries in flight, 1,000,003
+    // fp16 rows of d = 770: 1,380 -> 1,290 us at the power cap, 1.48 -> 1.61 GHz; 50 queries, k = 2048, 300,007 rows of d = 256,
+    // below the cap: level.
     const int m = plan.pair ? 2 * BM : op.nq <= 64 ? 64 : BM;
     p.warp_rows = m == 64 ? 16 : 32;
     const uint32_t fmt = op.is_bf16 ? 1u : 0u;
