@@ -209,7 +209,7 @@ int launch_gemm_filter(const GemmOperands& op, const GemmPlan& plan, float kscal
 int launch_gemm_store(const GemmOperands& op, const GemmPlan& plan, int64_t col0, int64_t ncols,
                       int64_t tile_stride, float kscale, float sign, const float* rowadd, float* out,
                       int64_t ld, int32_t* status, const Launch& ln);
-// Minima: out[row * ld + g] = the smallest key of columns [32 g, 32 g + 32) of the visited tiles side by side, +INF
+// Minima: out[row * ld + g] = the smallest key of columns [4 g, 4 g + 4) of the visited tiles side by side, +INF
 // where all of them lie beyond the end (ld a multiple of 8, out on a 32-byte boundary).
 int launch_gemm_minima(const GemmOperands& op, const GemmPlan& plan, int64_t ncols, int64_t tile_stride, float kscale,
                        float* out, int64_t ld, int32_t* status, const Launch& ln);
@@ -267,12 +267,12 @@ int launch_matrix_select(const float* keys, int64_t nq, int64_t n, int64_t ld, i
                          const float* qnorm, int64_t label_base, float* out_dist, int64_t* out_labels,
                          const int* nq_dev, const int32_t* row_map, const Launch& ln);
 // out[q]: an upper bound, close to it, of the r-th smallest (r <= 512) of the n keys of row q; +INF when
-// there are too few.  NaN keys are skipped.  bad (optional): one more for every row with more than about
+// there are too few.  group: how many keys each of the n stands for (1, or the minima of groups).  NaN keys are skipped.  bad (optional): one more for every row with more than about
 // `most` keys up to its bound + margin * qnorm[q], or with qnorm[q] >= qnorm_max.
 // Threads it gives a row, and what `most` keys in random columns amount to among that many minima.
 int row_bound_threads(int64_t nq, int64_t n, int r);
 int row_bound_most(int64_t nq, int64_t n, int r, double most);
-int launch_row_bound(const float* keys, int64_t nq, int64_t n, int64_t ld, int r, float* out, int32_t* bad,
+int launch_row_bound(const float* keys, int64_t nq, int64_t n, int64_t ld, int group, int r, float* out, int32_t* bad,
                      const float* qnorm, float margin, float qnorm_max, double most, const Launch& ln);
 bool rank_merge_fits(int P, int k);
 int launch_rank_merge(const float* dist, const int64_t* labels, int64_t stride_d, int64_t stride_l, int P,

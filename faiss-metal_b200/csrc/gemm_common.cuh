@@ -415,10 +415,10 @@ __device__ __forceinline__ void scan_columns_ahead(uint32_t taddr, Use use, Rele
 
 // nch x 32 accumulator columns from taddr on, through `use(registers, chunk)`; `release` is called once the last ones have
 // arrived.  Reading 32 columns takes 40 cycles beside the other warps of the scheduler and MMAs, too few to read ahead.
-template <int UNROLL = 1, typename Use, typename Release>
+template <typename Use, typename Release>
 __device__ __forceinline__ void scan_columns(uint32_t taddr, int nch, Use use, Release release) {
     if (nch == 0) release();
-#pragma unroll UNROLL
+#pragma unroll 1
     for (int ch = 0; ch < nch; ch++) {
         uint32_t r[32];
         tc_ld32(taddr + ch * 32, r);
@@ -428,13 +428,17 @@ __device__ __forceinline__ void scan_columns(uint32_t taddr, int nch, Use use, R
     }
 }
 
-// MODE_MINIMA: the smallest key of every MIN_GROUP columns of a thread's row; N consecutive ones to out.
-constexpr int MIN_GROUP = 32;
-template <int N>
-__device__ __forceinline__ void store_minima(const float (&v)[N], float* out) {
-    static_assert(N == 4 || N == 8, "");
-    if constexpr (N == 8) st_global_v8(out, v);
-    else *reinterpret_cast<float4*>(out) = make_float4(v[0], v[1], v[2], v[3]);
+// MODE_MINIMA: of 32 columns of a thread's row the smallest key of every MIN_GROUP, one sector, to out.  Why groups of
+// four: SAMPLE_GROUP (search.cu).
+constexpr int MIN_GROUP = 4;
+__device__ __forceinline__ void store_minima(const uint32_t (&r)[32], float ksc, float* out) {
+    static_assert(32 / MIN_GROUP == 8, "a sector of minima");
+    float v[8];
+#pragma unroll
+    for (int g = 0; g < 8; g++)
+        v[g] = -ksc * fmaxf(max3(__uint_as_float(r[4 * g]), __uint_as_float(r[4 * g + 1]), __uint_as_float(r[4 * g + 2])),
+                            __uint_as_float(r[4 * g + 3]));
+    st_global_v8(out, v);
 }
 
 // Keys up to the threshold pass a filter whose comparison excludes its bound: the next float up (+INF, the

@@ -340,17 +340,14 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                             },
                             release);
                 } else if constexpr (MODE == MODE_MINIMA) {
-                    float v[PER_WARP];
-                    scan_columns<PER_WARP>(
+                    float* const out = p.out + grow * p.ld + (t * RES_TILE_N + ch0 * 32) / MIN_GROUP;
+                    scan_columns(
                             taddr, PER_WARP,
                             [&](uint32_t(&r)[32], int ch) {
                                 if (partial) mask_columns(r, cbase + ch * 32, p.ncols_end);
-                                float gm[4];
-                                group_maxima(r, gm);
-                                v[ch] = -ksc * fmaxf(max3(gm[0], gm[1], gm[2]), gm[3]);
+                                if (row_live) store_minima(r, ksc, out + ch * (32 / MIN_GROUP));
                             },
                             release);
-                    if (row_live) store_minima(v, p.out + grow * p.ld + t * (RES_TILE_N / MIN_GROUP) + ch0);
                 } else {
                     const bool whole = !partial && (p.ld & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
                     float* const tbuf = reinterpret_cast<float*>(smem + RES_SM_STAGE) + (warp - 2) * (32 * 33);

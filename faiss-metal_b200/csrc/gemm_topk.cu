@@ -29,7 +29,7 @@
 //   filter  a fixed per-row threshold; every column under it is appended to the row's
 //           candidate buffer in global memory
 //   store   the keys are written out as a matrix (k beyond the list paths, pairwise distances)
-//   minima  the smallest key of every 32 columns is (samples that thresholds are taken from)
+//   minima  the smallest key of every four columns is (samples that thresholds are taken from)
 // The mode is a template parameter (eight instantiations with the two shapes): only the top-k
 // kernels carry list registers.  A work item is (query block, column range).
 //
@@ -490,18 +490,14 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
                     if (p.dense) scan_columns_ahead<CH_PER_HALF>(thalf, stage, release);
                     else scan_columns(thalf, CH_PER_HALF, stage, release);
                 } else if constexpr (MODE == MODE_MINIMA) {
-                    float v[CH_PER_HALF];
-                    scan_columns<CH_PER_HALF>(
+                    float* const out = p.out + grow * p.ld + (t * TILE_N + sub * BN + eh * CH_PER_HALF * 32) / MIN_GROUP;
+                    scan_columns(
                             thalf, CH_PER_HALF,
                             [&](uint32_t(&r)[32], int ch) {
                                 if (partial) mask_columns(r, chalf + ch * 32, p.ncols_end);
-                                float gm[4];
-                                group_maxima(r, gm);
-                                v[ch] = -ksc * fmaxf(max3(gm[0], gm[1], gm[2]), gm[3]);
+                                if (row_live) store_minima(r, ksc, out + ch * (32 / MIN_GROUP));
                             },
                             release);
-                    if (row_live)
-                        store_minima(v, p.out + grow * p.ld + t * (TILE_N / MIN_GROUP) + sub * (BN / MIN_GROUP) + eh * CH_PER_HALF);
                 } else {
                     const bool whole = !partial && (p.ld & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
                     // the list area is idle in this mode; tiles lie side by side in the output, whatever the stride

@@ -70,7 +70,7 @@ struct SearchPlan {
     int fcap;         // candidate buffer entries per query
     GemmPlan pilot;
     bool pilot_matrix; // pilot sample as a key matrix (store mode + key selection) instead of lists
-    bool pilot_minima; // of which only the smallest key of every 32 columns is kept
+    bool pilot_minima; // of which only the smallest key of every SAMPLE_GROUP columns is kept
     int npl;
     int64_t a_pitch, a_plane_stride;
     GemmPlan gemm;    // tensor path (fused: whole shard; chunked: per chunk)
@@ -198,9 +198,13 @@ constexpr int64_t BOUND_MIN_ELEMS = 32ll << 20;    // stored elements
 constexpr int BOUND_MAX_D = 8192;                  // a query in a rescoring CTA's shared memory
 
 // What a query's pilot sample of pcols columns leaves behind: row_bound takes the r-th smallest of T thread minima, so where
-// it would have a group of 32 columns and more for every thread the distance kernel keeps their smallest keys only
-// (10,000 queries, 1,000,000 rows: 20 MB instead of 640 written and read).
-constexpr int SAMPLE_GROUP = 32;
+// it would have a group of columns and more for every thread the distance kernel keeps their smallest keys only (10,000
+// queries, 1,000,000 rows: 160 MB instead of 640 written and read).  Groups of four, the columns that row_bound takes with
+// one load of the keys themselves: of rows near one another that are stored side by side (chunks of a document,
+// augmentations of an image) a group counts one, and the threshold admits as many times more.  With groups of 32 columns 962
+// of 1,000 queries with k = 100 on 1,000,000 rows in runs of 16 overflowed their buffers and were redone (4.3 ms), with
+// groups of four 126 (1.1 ms), as with the keys themselves.
+constexpr int SAMPLE_GROUP = 4;
 int64_t sample_floats(int64_t pcols, int r) {
     return pcols / SAMPLE_GROUP >= row_bound_threads(1ll << 40, 0, r) ? pcols / SAMPLE_GROUP : pcols;
 }
@@ -840,7 +844,7 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
                                  : launch_gemm_store(op, pl.pilot, 0, a->nb, pl.fstride, kscale, 1.f, nullptr, matrix, pcols,
                                                      a->status, ln);
             if (rc != B200F_OK) return rc;
-            rc = launch_row_bound(matrix, a->nq, ceil_div64(valid, group), pcols / group, pl.frank, thr, nullptr, nullptr, 0.f, 0.f, 0.0, ln);
+            rc = launch_row_bound(matrix, a->nq, ceil_div64(valid, group), pcols / group, (int)group, pl.frank, thr, nullptr, nullptr, 0.f, 0.f, 0.0, ln);
             if (rc != B200F_OK) return rc;
         } else {
             rc = launch_gemm_topk(op, pl.pilot, 0, a->nb, pl.fstride, kscale, pl.frank, 1, pkey, pidx, gthr, true,
@@ -882,7 +886,7 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
         float* keys = reinterpret_cast<float*>(scratch + pl.off_sample);
         rc = launch_scan_sample(*a, pl.nsample, pl.fstride, keys, pl.nsample, ln);
         if (rc != B200F_OK) return rc;
-        rc = launch_row_bound(keys, a->nq, pl.nsample, pl.nsample, pl.frank, thr, bad, qnorm, margin, qnorm_max, most, ln);
+        rc = launch_row_bound(keys, a->nq, pl.nsample, pl.nsample, 1, pl.frank, thr, bad, qnorm, margin, qnorm_max, most, ln);
         if (rc != B200F_OK) return rc;
     }
 

@@ -622,28 +622,53 @@ __global__ void __launch_bounds__(1024) row_select_kernel(const RowSelectParams 
 // have a key, which lets every row pass).  One CTA per row; out[q] may be exceeded by no key that
 // belongs to the r smallest.
 __global__ void __launch_bounds__(1024) row_bound_kernel(const float* keys, int64_t ld, int64_t n,
-                                                         int64_t nq, int r, float* __restrict__ out,
+                                                         int group, int64_t nq, int r, float* __restrict__ out,
                                                          int32_t* __restrict__ bad, const float* __restrict__ qnorm,
                                                          float margin, float qnorm_max, int most) {
     __shared__ int s_hist[256];
     __shared__ uint32_t s_min[32], s_max[32];
     __shared__ int s_live[32];
     __shared__ int s_sel[2];
-    const int tid = threadIdx.x, T = blockDim.x;
+    extern __shared__ float rb_part[];   // [3][T], of minima
+    const int tid = threadIdx.x, T = blockDim.x;   // a power of two
     pdl_wait();   // the sample's keys are read with coherent loads
     pdl_trigger();
-    // four keys a load while that leaves every thread several
-    const bool vec = n >= 8 * T && (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(keys) & 15) == 0;
+    // four values a load: minima always, keys while that leaves every thread several
+    const bool vec = (group > 1 || n >= 8 * T) && (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(keys) & 15) == 0;
     for (int64_t q = blockIdx.x; q < nq; q += gridDim.x) {
         const float* row = keys + q * ld;
         float best = CUDART_INF_F;   // fminf drops NaN
         if (vec) {
-#pragma unroll 4
-            for (int64_t c = (int64_t)tid * 4; c + 4 <= n; c += (int64_t)T * 4) {
-                const float4 f = __ldcg(reinterpret_cast<const float4*>(row + c));
-                best = fminf(best, fminf(fminf(f.x, f.y), fminf(f.z, f.w)));
+            float m[4] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F, CUDART_INF_F};
+            constexpr int U = 4;   // loads on their way together
+            for (int64_t c = (int64_t)tid * 4; c + 4 <= n; c += (int64_t)T * 4 * U) {
+                float4 f[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int64_t cu = c + u * (int64_t)T * 4;
+                    f[u] = cu + 4 <= n ? __ldcg(reinterpret_cast<const float4*>(row + cu))
+                                       : make_float4(CUDART_INF_F, CUDART_INF_F, CUDART_INF_F, CUDART_INF_F);
+                }
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    m[0] = fminf(m[0], f[u].x);
+                    m[1] = fminf(m[1], f[u].y);
+                    m[2] = fminf(m[2], f[u].z);
+                    m[3] = fminf(m[3], f[u].w);
+                }
             }
-            if (tid < (n & 3)) best = fminf(best, __ldcg(row + (n & ~(int64_t)3) + tid));
+            if (tid < (n & 3)) m[0] = fminf(m[0], __ldcg(row + (n & ~(int64_t)3) + tid));
+            if (group > 1) {
+                // Each of a load's four goes to another thread, so that T minima in a row belong to T threads: near rows
+                // side by side are as many of the minima that are ranked as they would be without groups.  One by one,
+                // a coalesced load each, 1,000 rows of 1,664 took the search 3 us longer.
+#pragma unroll
+                for (int j = 1; j < 4; j++) rb_part[(j - 1) * T + tid] = m[j];
+                __syncthreads();
+#pragma unroll
+                for (int j = 1; j < 4; j++) m[j] = rb_part[(j - 1) * T + ((tid + j * (T >> 2)) & (T - 1))];
+            }
+            best = fminf(fminf(m[0], m[1]), fminf(m[2], m[3]));
         } else {
 #pragma unroll 4
             for (int64_t c = tid; c < n; c += T) best = fminf(best, __ldcg(row + c));
@@ -922,18 +947,19 @@ int row_bound_most(int64_t nq, int64_t n, int r, double most) {
     return (int)(T * (1.0 - std::exp(-most / T)));
 }
 
-int launch_row_bound(const float* keys, int64_t nq, int64_t n, int64_t ld, int r, float* out, int32_t* bad,
+int launch_row_bound(const float* keys, int64_t nq, int64_t n, int64_t ld, int group, int r, float* out, int32_t* bad,
                      const float* qnorm, float margin, float qnorm_max, double most, const Launch& ln) {
-    if (r < 1 || r > 512 || n < 0 || ld < n || !keys || !out) return B200F_ERR_BAD_ARG;
+    if (r < 1 || r > 512 || n < 0 || ld < n || group < 1 || !keys || !out) return B200F_ERR_BAD_ARG;
     if (nq <= 0) return B200F_OK;
     const int64_t sm = cached_sm_count();
-    const int T = row_bound_threads(nq, n, r);
+    const int T = row_bound_threads(nq, n * group, r);   // as many as the keys themselves would have
     int64_t g = nq;
     const int64_t gcap = sm * (2048 / T);
     if (g > gcap) g = gcap;
     const int most_minima = row_bound_most(nq, n, r, most);
-    B200F_CUDA_TRY(launch_kernel(row_bound_kernel, dim3((unsigned)g), T, 0, ln, keys, ld, n, nq, r, out, bad, qnorm, margin,
-                                 qnorm_max, most_minima));
+    const size_t smem = group > 1 ? 3 * T * sizeof(float) : 0;
+    B200F_CUDA_TRY(launch_kernel(row_bound_kernel, dim3((unsigned)g), T, smem, ln, keys, ld, n, group, nq, r, out, bad, qnorm,
+                                 margin, qnorm_max, most_minima));
     count_launch();
     B200F_LAUNCH_CHECK();
     return B200F_OK;
