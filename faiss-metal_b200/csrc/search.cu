@@ -795,8 +795,8 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
     const int32_t* row_map = nullptr;
     uint32_t* gthr = reinterpret_cast<uint32_t*>(scratch + pl.off_gthr);
     // the number of redone rows is left in status word 1 for whoever wants to know
+    int32_t* const redone = a->status ? a->status + 1 : nullptr;
     RedoRows redo;
-    redo.count_copy = a->status ? a->status + 1 : nullptr;
     if (pl.lists || pl.filter) {
         redo.rows = reinterpret_cast<int32_t*>(scratch + pl.off_rows);
         redo.count = reinterpret_cast<int32_t*>(scratch + pl.off_count);
@@ -809,7 +809,7 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
     // counted: the selection has listed and gathered the rows itself
     auto redo_setup = [&](int32_t* dirty, bool counted) -> int {
         if (!counted) {
-            int r2 = launch_compact_rows(dirty, a->nq, redo.rows, redo.count, redo.count_copy, st);
+            int r2 = launch_compact_rows(dirty, a->nq, redo.rows, redo.count, st);
             if (r2 != B200F_OK) return r2;
             r2 = launch_gather_rows(op.a_planes, op.npl, op.a_plane_stride, op.a_pitch, redo.rows, redo.count, a->nq,
                                     redo.out, st);
@@ -928,7 +928,7 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
             if (rc != B200F_OK) return rc;
             if (pl.sample) {
                 rc = launch_merge_partials(part_key, part_idx, P, a->nq, a->k, a->metric, qnorm, a->label_base,
-                                           a->out_dist, a->out_labels, nullptr, nullptr, a->nb, dirty, redo_all, ln);
+                                           a->out_dist, a->out_labels, nullptr, nullptr, nullptr, a->nb, dirty, redo_all, ln);
                 if (rc != B200F_OK) return rc;
                 nq_dev = any_count;
                 rc = scan_lists(nullptr, any_count, P);
@@ -936,7 +936,7 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
             }
         }
         return launch_merge_partials(part_key, part_idx, P, a->nq, a->k, a->metric, qnorm,
-                                     a->label_base, a->out_dist, a->out_labels, nq_dev, row_map, 0, nullptr, RedoRows(),
+                                     a->label_base, a->out_dist, a->out_labels, nq_dev, row_map, redone, 0, nullptr, RedoRows(),
                                      ln);
     }
 
@@ -1008,14 +1008,14 @@ static int run_search(const B200FSearchArgs* a, const SearchPlan& pl) {
         // the whole shard in one chunk: select from it at once (a few passes over a row that stays in L2)
         if (nc == a->nb && nc <= MATRIX_SELECT_MAX_COLS && rank_select_enabled())
             return launch_matrix_select(matrix, a->nq, nc, pl.chunk_cols, a->k, inf_empty, a->metric, qnorm,
-                                        a->label_base, a->out_dist, a->out_labels, nq_dev, row_map, ln);
+                                        a->label_base, a->out_dist, a->out_labels, nq_dev, row_map, redone, ln);
         rc = launch_select_chunk(matrix, a->nq, nc, pl.chunk_cols, c0, a->k, has_prev, run_key,
                                  run_idx, nq_dev, inf_empty, ln);
         if (rc != B200F_OK) return rc;
         has_prev = 1;
     }
     return launch_finalize_lists(run_key, run_idx, a->nq, a->k, a->metric, qnorm, a->label_base,
-                                 a->out_dist, a->out_labels, nq_dev, row_map, ln);
+                                 a->out_dist, a->out_labels, nq_dev, row_map, redone, ln);
 }
 
 __global__ void poke_kernel(uint32_t* word) { *word = 0; }

@@ -527,8 +527,7 @@ __global__ void __launch_bounds__(SS_THREADS) sort_select_kernel(const SortSelec
 // rows[0 .. n) = ascending q with flag[q] != 0, n -> *count (one CTA)
 __global__ void __launch_bounds__(1024) compact_rows_kernel(const int32_t* __restrict__ flag, int64_t nq,
                                                             int32_t* __restrict__ rows,
-                                                            int32_t* __restrict__ count,
-                                                            int32_t* __restrict__ count_copy) {
+                                                            int32_t* __restrict__ count) {
     __shared__ int s_warp[32];
     __shared__ int s_base;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -548,10 +547,7 @@ __global__ void __launch_bounds__(1024) compact_rows_kernel(const int32_t* __res
         if (tid == 1023) s_base = base + before + __popc(b);
         __syncthreads();
     }
-    if (tid == 0) {
-        *count = s_base;
-        if (count_copy) *count_copy = s_base;
-    }
+    if (tid == 0) *count = s_base;
 }
 
 __global__ void gather_rows_kernel(const uint16_t* __restrict__ a, int npl, int64_t plane_stride,
@@ -597,9 +593,10 @@ __global__ void finalize_lists_kernel(const float* run_key, const int32_t* run_i
                                       float pad, int64_t label_base, float* __restrict__ out_dist,
                                       int64_t* __restrict__ out_labels,
                                       const int* __restrict__ nq_dev,
-                                      const int32_t* __restrict__ row_map) {
+                                      const int32_t* __restrict__ row_map, int32_t* redone) {
     pdl_wait();
     pdl_trigger();
+    if (redone && nq_dev && *nq_dev > 0 && blockIdx.x == 0 && threadIdx.x == 0) *redone = *nq_dev;
     if (nq_dev) nq = min((int64_t)*nq_dev, nq);
     const int64_t total = nq * k;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -725,9 +722,9 @@ int launch_select_candidates(const float* cand_key, const int32_t* cand_idx, con
 }
 
 int launch_compact_rows(const int32_t* dirty, int64_t nq, int32_t* rows, int32_t* count,
-                        int32_t* count_copy, cudaStream_t stream) {
+                        cudaStream_t stream) {
     if (nq <= 0) return B200F_OK;
-    compact_rows_kernel<<<1, 1024, 0, stream>>>(dirty, nq, rows, count, count_copy);
+    compact_rows_kernel<<<1, 1024, 0, stream>>>(dirty, nq, rows, count);
     count_launch();
     B200F_LAUNCH_CHECK();
     return B200F_OK;
@@ -747,7 +744,7 @@ int launch_gather_rows(const uint16_t* a, int npl, int64_t plane_stride, int64_t
 
 int launch_finalize_lists(const float* run_key, const int32_t* run_idx, int64_t nq, int k,
                           int metric, const float* qnorm, int64_t label_base, float* out_dist,
-                          int64_t* out_labels, const int* nq_dev, const int32_t* row_map,
+                          int64_t* out_labels, const int* nq_dev, const int32_t* row_map, int32_t* redone,
                           const Launch& ln) {
     if (nq <= 0) return B200F_OK;
     const bool l2 = metric == B200F_METRIC_L2;
@@ -756,7 +753,7 @@ int launch_finalize_lists(const float* run_key, const int32_t* run_idx, int64_t 
     if (g > cap) g = cap;
     B200F_CUDA_TRY(launch_kernel(finalize_lists_kernel, dim3((unsigned)g), 256, 0, ln, run_key, run_idx, nq, k, l2 ? 1.f : -1.f,
                                  l2 ? qnorm : nullptr, l2 ? 1 : 0, l2 ? kHostInf : -kHostInf, label_base, out_dist,
-                                 out_labels, nq_dev, row_map));
+                                 out_labels, nq_dev, row_map, redone));
     count_launch();
     B200F_LAUNCH_CHECK();
     return B200F_OK;

@@ -83,6 +83,7 @@ struct RowSelectParams {
     int64_t nq;
     const int* nq_dev;        // optional: live rows (<= nq), read on the device
     const int32_t* row_map;   // optional: row j belongs to query row_map[j]
+    int32_t* redone;          // optional: receives *nq_dev unless that is zero
     int k;
     int bound;                // words of the staging area
     float out_sign;
@@ -438,6 +439,7 @@ __global__ void __launch_bounds__(1024) row_select_kernel(const RowSelectParams 
     const int T = blockDim.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t nq_live = p.nq_dev ? min((int64_t)*p.nq_dev, p.nq) : p.nq;
+    if (p.redone && p.nq_dev && nq_live > 0 && blockIdx.x == 0 && tid == 0) *p.redone = (int32_t)nq_live;
     for (int64_t q = blockIdx.x; q < nq_live; q += gridDim.x) {
         const int64_t cnt = p.cnt ? (int64_t)__ldcg(p.cnt + q) : p.n;
         const int n = (int)min(cnt, p.ld);
@@ -592,10 +594,8 @@ __global__ void __launch_bounds__(1024) row_select_kernel(const RowSelectParams 
             if (bad && p.redo.count) {
                 if (p.redo.all > 0) {
                     *p.redo.count = p.redo.all;
-                    if (p.redo.count_copy) *p.redo.count_copy = p.redo.all;
                 } else {
                     const int j = atomicAdd(p.redo.count, 1);
-                    if (p.redo.count_copy) atomicAdd(p.redo.count_copy, 1);
                     p.redo.rows[j] = (int32_t)q;
                     s_sel[0] = j;
                 }
@@ -987,7 +987,7 @@ int launch_rank_select(const float* cand_key, const int32_t* cand_idx, const int
 
 int launch_merge_partials(const float* part_key, const int32_t* part_idx, int P, int64_t nq, int k,
                           int metric, const float* qnorm, int64_t label_base, float* out_dist,
-                          int64_t* out_labels, const int* nq_dev, const int32_t* row_map,
+                          int64_t* out_labels, const int* nq_dev, const int32_t* row_map, int32_t* redone,
                           int64_t nb, int32_t* dirty, const RedoRows& redo, const Launch& ln) {
     if (nq <= 0) return B200F_OK;
     if (k < 1 || k > 32 || P < 1) return B200F_ERR_UNSUPPORTED;
@@ -1002,6 +1002,7 @@ int launch_merge_partials(const float* part_key, const int32_t* part_idx, int P,
     p.nq = nq;
     p.nq_dev = nq_dev;
     p.row_map = row_map;
+    p.redone = redone;
     p.k = k;
     set_output(p, metric, qnorm, label_base, out_dist, out_labels);
     return launch_row_select(p, p.n, ln);
@@ -1009,7 +1010,7 @@ int launch_merge_partials(const float* part_key, const int32_t* part_idx, int P,
 
 int launch_matrix_select(const float* keys, int64_t nq, int64_t n, int64_t ld, int k, bool inf_empty, int metric,
                          const float* qnorm, int64_t label_base, float* out_dist, int64_t* out_labels,
-                         const int* nq_dev, const int32_t* row_map, const Launch& ln) {
+                         const int* nq_dev, const int32_t* row_map, int32_t* redone, const Launch& ln) {
     if (n < 0 || n > 0x7fffffffLL || ld < n) return B200F_ERR_BAD_ARG;
     RowSelectParams p{};
     p.keys = keys;
@@ -1019,6 +1020,7 @@ int launch_matrix_select(const float* keys, int64_t nq, int64_t n, int64_t ld, i
     p.nq = nq;
     p.nq_dev = nq_dev;
     p.row_map = row_map;
+    p.redone = redone;
     p.k = k;
     set_output(p, metric, qnorm, label_base, out_dist, out_labels);
     return launch_row_select(p, n, ln);
