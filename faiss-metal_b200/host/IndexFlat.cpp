@@ -66,6 +66,13 @@ void abiCheck(int rc, const char* what) {
 
 // Status words are written by kernels, straight to pinned memory; read once the stream has been waited for.
 int32_t statusWord(const int32_t* words) { return *static_cast<const volatile int32_t*>(words); }
+// The same for words that stay: an error is reported once, not again by the next wait (a search replayed from a graph has
+// words of its own and does not clear these).
+int32_t takeStatusWord(int32_t* words) {
+    const int32_t word = statusWord(words);
+    if (word != 0) std::memset(words, 0, 4 * sizeof(int32_t));
+    return word;
+}
 
 struct DeviceGuard {
     int prev = -1;
@@ -838,7 +845,7 @@ void B200IndexFlat::search(faiss::idx_t n, const float* x, faiss::idx_t k, float
                                       cudaMemcpyDeviceToHost, st),
                       "search: device to host copy of labels");
         cudaCheck(cudaStreamSynchronize(st), "search: synchronize");
-        if (const int32_t word = statusWord(impl_->status)) {
+        if (const int32_t word = takeStatusWord(impl_->status)) {
             impl_->lastStatus = word;
             throwDeviceStatus(word, "search");
         }
@@ -987,7 +994,7 @@ void B200IndexFlat::synchronize() const {
     DeviceGuard g(impl_->res->getDevice());
     cudaStream_t st = impl_->stream();
     cudaCheck(cudaStreamSynchronize(st), "synchronize");
-    if (const int32_t word = statusWord(impl_->status)) {
+    if (const int32_t word = takeStatusWord(impl_->status)) {
         impl_->lastStatus = word;
         throwDeviceStatus(word, "search");
     }

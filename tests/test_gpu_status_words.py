@@ -41,3 +41,20 @@ def test_redone_queries(fm, res, storage, nq, nb, k):
     assert (I.cpu().numpy() == np.arange(k)).all()
     # an atomic a redone row across PCIe took 0.9 us each; two writes a search take none that shows
     assert times[1] <= times[0] + 0.2, times
+
+
+def test_an_error_is_reported_once(fm, res):
+    idx = fm.B200IndexFlat(res, 32, O.METRIC_L2, 1)
+    idx.add(H.gaussian(5000, 32, 1))
+    xq = H.gaussian(1, 32, 2)
+    for _ in range(3):   # the third is replayed from a graph
+        D, I = idx.search(xq, 5)
+    fm.abi.check(fm.lib().b200f_index_debug_wait_expiry(idx._h, 2_000_000), "debug_wait_expiry")
+    with pytest.raises(fm.B200Error):
+        idx.synchronize()
+    assert idx.last_device_status == 1
+    idx.synchronize()
+    D2, I2 = idx.search(xq, 5)
+    assert np.array_equal(D, D2) and np.array_equal(I, I2)
+    idx.synchronize()
+    idx.close()
