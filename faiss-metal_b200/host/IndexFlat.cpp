@@ -32,7 +32,8 @@ constexpr size_t kStageBytes = 32ull << 20;   // fp32 staging chunk of add / rec
 constexpr int64_t kScaleSampleRows = 8192;    // rows an fp32 index takes its plane scale from
 constexpr int64_t kGraphMaxQueries = 8;        // searches this small are replayed from a CUDA graph
 constexpr int64_t kGraphDirectResults = 512;   // results of a captured search written to host memory by the kernel
-constexpr size_t kGraphFetchBytes = 64 << 10;  // queries of a captured search fetched by a kernel
+// queries of a captured search fetched by a kernel, not copied (8 x 2,048 elements, which is as many: 169 us a search, 225)
+constexpr size_t kGraphFetchBytes = 64 << 10;
 constexpr size_t kMaxGraphs = 8;               // graphs kept per index (least recently used goes)
 constexpr int64_t kFusedBatch = 16384;        // queries per launch, k <= 1024 (fused kernel, lists)
 constexpr int64_t kSelectBatch = 1024;        // queries per launch beyond: few rows, wide column chunks
@@ -913,12 +914,16 @@ bool B200IndexFlat::searchFromGraph(faiss::idx_t n, const float* x, faiss::idx_t
             a.scratch = region + L.offScratch;
             a.scratch_bytes = L.scratchBytes;
             cudaCheck(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "search: begin capture");
-            // a few KB of queries are fetched by a kernel: a graph's next node starts 10 us after a copy from the host
-            // (single query of d = 128 on 100,000 rows), at once after a kernel
+            // A few KB of queries are fetched by a kernel: a graph's next node starts 10 us after a copy from the host
+            // (single query of d = 128 on 100,000 rows), at once after a kernel.  In pieces of 256 bytes (both slots are whole
+            // ones), not in rows: a row belongs to one warp, which has 2 KB on their way across PCIe at a time.  One query on 20,000
+            // fp16 rows, d = 4,096 / 16,384: 113 / 332 us, in rows 141 / 452, copied 135 / 378.
             cudaError_t ce = cudaSuccess;
             int rc = B200F_OK;
-            if ((size_t)n * d * 4 <= kGraphFetchBytes)
-                rc = b200f_load_rows(e.host, B200F_STORAGE_F32, n, d, d, reinterpret_cast<float*>(region + L.offQueries), st);
+            const size_t queryBytes = align256((size_t)n * d * 4);
+            if (queryBytes <= kGraphFetchBytes)
+                rc = b200f_load_rows(e.host, B200F_STORAGE_F32, (int64_t)(queryBytes / 256), 64, 64,
+                                     reinterpret_cast<float*>(region + L.offQueries), st);
             else
                 ce = cudaMemcpyAsync(region + L.offQueries, e.host, (size_t)n * d * 4, cudaMemcpyHostToDevice, st);
             if (ce != cudaSuccess) rc = B200F_ERR_CUDA;
