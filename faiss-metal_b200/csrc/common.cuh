@@ -196,7 +196,7 @@ int launch_gemm_topk(const GemmOperands& op, const GemmPlan& plan, int64_t col0,
                      const Launch& ln);
 // Threshold filter over the whole shard: column c of row q with scaled key <= thr[q * thr_stride +
 // thr_pos] is appended to the row's candidate buffer cand_key/cand_idx [nq][cand_cap] in any
-// order; cand_cnt[q] (zeroed by the caller) counts every hit, also those beyond cand_cap, which are
+// order; cand_cnt[q] (zeroed by the caller) counts every hit up to cand_cap, and some of those beyond, which are
 // not stored.  dense: many hits (see the caller's rule).
 int launch_gemm_filter(const GemmOperands& op, const GemmPlan& plan, float kscale, const float* thr,
                        int thr_stride, int thr_pos, float* cand_key, int32_t* cand_idx,

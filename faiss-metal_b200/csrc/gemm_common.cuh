@@ -63,7 +63,7 @@ struct GemmParams {
     int fthr_stride, fthr_pos;
     float* cand_key;     // [nq][cand_cap]
     int32_t* cand_idx;
-    int32_t* cand_cnt;   // [nq]
+    int32_t* cand_cnt;   // [nq]; hits of a row are counted until they no longer fit
     int cand_cap;
     int dense;           // MODE_FILTER: many hits expected
     float* out;
@@ -284,10 +284,12 @@ __device__ __forceinline__ WarpHits warp_hits(uint8_t* area) {   // HITS_BYTES, 
 }
 
 // n queued hits to the candidate buffers of the warp's 32 rows (cnt, ck, ci: those of its first).  One atomic takes the slots
-// of a row's hits among 32; the counter also counts hits that no longer fit.  All lanes call it, ksc is the lane's.
-static __device__ __noinline__ void drain_hits(int32_t* cnt, float* ck, int32_t* ci, int cap, float ksc, const float* key, const int* col,
+// of a row's hits among 32; the counter also counts hits that no longer fit.  Returns the rows (a bit each) that have such: they
+// are redone, and need no more of their hits.  All lanes call it, ksc is the lane's.
+static __device__ __noinline__ unsigned drain_hits(int32_t* cnt, float* ck, int32_t* ci, int cap, float ksc, const float* key, const int* col,
                                         const int* lanes, int n) {
     const int lane = threadIdx.x & 31;
+    unsigned over = 0;
     __syncwarp();
     for (int i0 = 0; i0 < n; i0 += 32) {
         const bool live = i0 + lane < n;
@@ -302,13 +304,16 @@ static __device__ __noinline__ void drain_hits(int32_t* cnt, float* ck, int32_t*
             ck[(int64_t)row * cap + pos] = k * key[i0 + lane];
             ci[(int64_t)row * cap + pos] = col[i0 + lane];
         }
+        over |= __reduce_or_sync(0xffffffffu, live && pos >= cap ? 1u << row : 0u);
     }
     __syncwarp();
+    return over;
 }
 
-// 32 accumulator columns of the warp's rows: hits (-r < thr) to the queue, which holds n.  All lanes call it.
+// 32 accumulator columns of the warp's rows: hits (-r < thr) to the queue, which holds n.  All lanes call it.  drain may lower
+// thr.
 template <typename Drain>
-__device__ __forceinline__ void filter_columns(uint32_t (&r)[32], int64_t cbase, int64_t ncols_end, bool partial, float thr,
+__device__ __forceinline__ void filter_columns(uint32_t (&r)[32], int64_t cbase, int64_t ncols_end, bool partial, const float& thr,
                                                const WarpHits& h, int& n, Drain drain) {
     if (partial) mask_columns(r, cbase, ncols_end);
     float gm[4];
@@ -381,10 +386,10 @@ __device__ __forceinline__ void stage_columns(uint32_t (&r)[32], int64_t cbase, 
     __syncwarp();
 }
 // A thread's n staged hits to its row's candidate buffer: one atomic takes their slots; the counter also counts entries
-// that no longer fit.
-__device__ __forceinline__ void drain_stage(int32_t* cnt, float* ck, int32_t* ci, int cap, float ksc, const float* sk,
+// that no longer fit.  True where there were such: the row is redone, and needs no more of its hits.
+__device__ __forceinline__ bool drain_stage(int32_t* cnt, float* ck, int32_t* ci, int cap, float ksc, const float* sk,
                                             const int32_t* si, int n) {
-    if (n <= 0) return;
+    if (n <= 0) return false;
     const int base = atomicAdd(cnt, n);
     for (int i = 0; i < n; i++) {
         if (base + i < cap) {
@@ -392,6 +397,7 @@ __device__ __forceinline__ void drain_stage(int32_t* cnt, float* ck, int32_t* ci
             ci[base + i] = si[i * STAGE_LD];
         }
     }
+    return base + n > cap;
 }
 
 // NCH x 32 accumulator columns from taddr on, through `use(registers, chunk)`, a chunk while the next one is on its way;

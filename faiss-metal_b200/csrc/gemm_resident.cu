@@ -292,19 +292,24 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
             if (p.rowscale && row_live) ksc *= __ldcg(p.rowscale + (p.rowscale_map ? (int64_t)__ldcg(p.rowscale_map + grow) : grow));
             float thr = -CUDART_INF_F, radd = 0.f;
             if (FILTER) {
-                if (row_live) thr = filter_threshold(__ldcg(p.fthr + grow * p.fthr_stride + p.fthr_pos) / ksc);
+                if (row_live) {
+                    thr = filter_threshold(__ldcg(p.fthr + grow * p.fthr_stride + p.fthr_pos) / ksc);
+                    if (__ldcg(p.cand_cnt + grow) > p.cand_cap) thr = -CUDART_INF_F;   // see drain_hits
+                }
             } else if (row_live && p.rowadd) {
                 radd = p.rowadd[grow];
             }
             auto drain = [&]() {   // the stage
-                drain_stage(p.cand_cnt + grow, p.cand_key + grow * p.cand_cap, p.cand_idx + grow * p.cand_cap, p.cand_cap,
-                                          ksc, stage_key, stage_idx, nstaged);
+                if (drain_stage(p.cand_cnt + grow, p.cand_key + grow * p.cand_cap, p.cand_idx + grow * p.cand_cap, p.cand_cap,
+                                ksc, stage_key, stage_idx, nstaged))
+                    thr = -CUDART_INF_F;
                 nstaged = 0;
             };
             auto drain_queue = [&]() {
                 const int64_t row0 = grow - lane;
-                drain_hits(p.cand_cnt + row0, p.cand_key + row0 * p.cand_cap, p.cand_idx + row0 * p.cand_cap, p.cand_cap, ksc, hits.key,
-                           hits.col, hits.lane, nhits);
+                const unsigned over = drain_hits(p.cand_cnt + row0, p.cand_key + row0 * p.cand_cap, p.cand_idx + row0 * p.cand_cap,
+                                                 p.cand_cap, ksc, hits.key, hits.col, hits.lane, nhits);
+                if ((over >> lane) & 1u) thr = -CUDART_INF_F;
                 nhits = 0;
             };
             for (int64_t t = t0; t < t1; t++) {

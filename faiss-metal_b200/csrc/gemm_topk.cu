@@ -394,8 +394,9 @@ gemm_topk_kernel(const __grid_constant__ CUtensorMap tmap_a,
                 radd = p.rowadd[grow];
             }
             auto drain = [&]() {
-                drain_stage(p.cand_cnt + grow, p.cand_key + grow * p.cand_cap, p.cand_idx + grow * p.cand_cap, p.cand_cap, ksc,
-                            stage_key, stage_idx, nstaged);
+                if (drain_stage(p.cand_cnt + grow, p.cand_key + grow * p.cand_cap, p.cand_idx + grow * p.cand_cap, p.cand_cap, ksc,
+                                stage_key, stage_idx, nstaged))
+                    thr_eff = -CUDART_INF_F;
                 nstaged = 0;
             };
             for (int64_t t = t0; t < t1 && ok; t++) {

@@ -60,3 +60,31 @@ def test_filter(fm, res, storage, metric, d, nq, nb, k):
     for q in (slice(0, 8), slice(nq // 2, nq // 2 + 8), slice(nq - 8, nq)):
         H.check_against_oracle(metric, storage, True, xb, xq[q], k, D[q], I[q], loose=False)
     idx.close()
+
+
+@pytest.mark.parametrize("storage,nq,k", [(2, 129, 10), (1, 300, 100), (0, 257, 10), (2, 300, 1000)])
+def test_overflowed_rows_stop_filtering(fm, res, storage, nq, k):
+    # equal rows: every column is a hit of every query.  What a search over them pays for a filter that is in vain stays
+    # within what the redo without one takes; hits that no longer fit used to be worked off one by one (5 times as long)
+    nb, d = 1_000_000, 24
+    idx = fm.B200IndexFlat(res, d, O.METRIC_L2, storage)
+    idx.add(np.tile(H.gaussian(1, d, 1), (nb, 1)))
+    xq = torch.from_numpy(H.gaussian(nq, d, 2)).cuda()
+    best = {}
+    try:
+        for mode in (0, 2):   # auto, without the filter
+            assert fm.lib().b200f_set_selection_mode(mode) == 0
+            t = []
+            for _ in range(5):
+                t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                t0.record()
+                D, I = idx.search(xq, k)
+                t1.record()
+                torch.cuda.synchronize()
+                assert (I == torch.arange(k, device=I.device)).all()
+                t.append(t0.elapsed_time(t1))
+            best[mode] = min(t)
+    finally:
+        fm.lib().b200f_set_selection_mode(0)
+    assert best[0] <= 2 * best[2] + 0.2, best
+    idx.close()
