@@ -915,7 +915,15 @@ int launch_row_select(RowSelectParams& p, int64_t n_typical, const Launch& ln) {
     if (g > gcap) g = gcap;
     // rows counted on the device are usually few or none: idle CTAs leave at once
     if (p.nq_dev && g > sm) g = sm;
-    B200F_CUDA_TRY(launch_kernel(four ? row_select_kernel<4> : row_select_kernel<1>, dim3((unsigned)g), T, smem, ln, p));
+    // Launched before the distance kernel's SMs are idle the CTAs would keep its division of them, nearly all shared memory.
+    // That matters where a row of keys is read several times and fits the L1 of an SM with one CTA: on most SMs (the matrix of
+    // 148 queries on 32,000 rows, k = 10: 90 us a search, 79 launched plainly; 20 queries 62 and 65, 300 129 and 123 - 129), and
+    // in a redo, where every SM has one, if it is of many rows (1,000 queries on 100,000 rows ordered by cluster, k = 40: 1,600 and
+    // 1,330 us).  With nothing to redo the plain launch takes 2 us, and fewer than 600 queries are under 120.
+    const bool several = !p.ids && n_typical > RS_REGS * T;
+    const bool plain = several && (p.nq_dev ? p.nq >= 4 * sm : 2 * g > sm && g <= sm);
+    B200F_CUDA_TRY(launch_kernel(four ? row_select_kernel<4> : row_select_kernel<1>, dim3((unsigned)g), T, smem,
+                                 plain ? Launch(ln.stream) : ln, p));
     count_launch();
     B200F_LAUNCH_CHECK();
     return B200F_OK;
