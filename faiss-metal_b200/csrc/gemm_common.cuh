@@ -6,6 +6,7 @@
 
 #include "common.cuh"
 #include "ptx.cuh"
+#include "tensor_map.h"
 
 namespace b200f {
 
@@ -491,28 +492,6 @@ __device__ __forceinline__ void store_keys(const GemmParams& p, const uint32_t (
 }
 
 // ---- host side -------------------------------------------------------------------------
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
-                                  const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-inline EncodeTiledFn get_encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
-        void* ptr = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) ==
-                    cudaSuccess &&
-            qres == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(ptr);
-        else
-            (void)cudaGetLastError();
-    }
-    return fn;
-}
 
 // 3-D map {k, row, plane} over a [planes][rows][pitch] 16-bit array; box {64, box_rows, 1}.
 inline int make_operand_map(CUtensorMap* map, const uint16_t* base, int is_bf16, int64_t k_extent,
