@@ -62,6 +62,57 @@ def test_filter(fm, res, storage, metric, d, nq, nb, k):
     idx.close()
 
 
+def search_words(fm, xb, xq, storage, metric, k):
+    """Result and status words of a search whose fp32 rows are two fp16 planes, which is what the resident kernel takes."""
+    nb, d = xb.shape
+    st = Stored(fm, xb, storage)
+    xq_dev = torch.from_numpy(xq).cuda()
+    D = torch.empty((len(xq), k), dtype=torch.float32, device="cuda:0")
+    I = torch.empty((len(xq), k), dtype=torch.int64, device="cuda:0")
+    a = st.args(fm, xq_dev, metric, k, 2, D, I)
+    if storage == 0:
+        fm.abi.check_op(fm.lib().b200f_store_rows_fp32(vp(st.rows), st.pitch, nb, d, vp(st.rows), st.pitch, vp(st.planes),
+                                                       st.ppitch, nb * st.ppitch, 1, 4, None, None, 1, cur_stream()), "planes")
+        a.plane_format, a.plane_scale_log2 = 1, 4
+    fm.abi.check_op(fm.lib().b200f_search(ctypes.byref(a)), "search")
+    torch.cuda.synchronize()
+    return D.cpu().numpy(), I.cpu().numpy(), st.status.tolist()
+
+
+@pytest.mark.parametrize("storage,metric,d,nq,nb,k", [
+    (0, O.METRIC_L2, 96, 300, 140_001, 100), (0, O.METRIC_INNER_PRODUCT, 192, 129, 131_328, 10), (0, O.METRIC_L2, 128, 1000, 70_000, 5),
+    (0, O.METRIC_L2, 184, 200, 140_001, 1024), (1, O.METRIC_L2, 40, 513, 131_329, 1024), (2, O.METRIC_INNER_PRODUCT, 384, 257, 100_100, 32)])
+def test_no_hit_is_lost(fm, res, storage, metric, d, nq, nb, k):
+    # rows that lost hits, or took too many, would be redone and come out right all the same: none is
+    xb = H.gaussian(nb, d, 1)
+    xq = H.gaussian(nq, d, 2)
+    D, I, words = search_words(fm, xb, xq, storage, metric, k)
+    assert words[:2] == [0, 0]
+    for q in (slice(0, 8), slice(nq - 8, nq)):
+        H.check_against_oracle(metric, storage, True, xb, xq[q], k, D[q], I[q], loose=False)
+
+
+@pytest.mark.parametrize("storage", [0, 1, 2])
+@pytest.mark.parametrize("near,first", [(3, 0), (32, 0), (32, 17), (100, 5)])
+@pytest.mark.parametrize("nq", [129, 300])
+def test_hits_of_all_rows_in_one_chunk(fm, res, storage, near, first, nq):
+    # queries near one another and a block of rows near them, in a tile that no sample takes: every row of a warp hits every
+    # column of a chunk of 32, four turns of eight rows, and the queue is worked off in the middle of it.  What the
+    # threshold admits beside them still fits the buffers, so nothing is redone.  (Around the origin: elsewhere their
+    # distances would be small differences of large products.)
+    nb, d, k = 140_000, 64, 20
+    xb = H.gaussian(nb, d, 3)
+    at = 512 * 133 + first
+    xb[at:at + near] = H.gaussian(near, d, 5, scale=0.2)
+    xq = H.gaussian(nq, d, 6, scale=0.2)
+    D, I, words = search_words(fm, xb, xq, storage, O.METRIC_L2, k)
+    assert words[:2] == [0, 0]
+    m = min(near, k)
+    assert ((I[:, :m] >= at) & (I[:, :m] < at + near)).all()
+    for q in (slice(0, 4), slice(nq - 4, nq)):
+        H.check_against_oracle(O.METRIC_L2, storage, True, xb, xq[q], k, D[q], I[q], loose=False)
+
+
 @pytest.mark.parametrize("storage,nq,k", [(2, 129, 10), (1, 300, 100), (0, 257, 10), (2, 300, 1000)])
 def test_overflowed_rows_stop_filtering(fm, res, storage, nq, k):
     # equal rows: every column is a hit of every query.  What a search over them pays for a filter that is in vain stays
