@@ -648,8 +648,11 @@ def run_workload(ctx, name, w, steps, warmup, headline, with_e2e=True, with_labe
         launches_per_step = max(1.0, main_launches.value / max(1, steps))
         achieved = flops_per_launch / (main_avg_ms * launches_per_step * 1e-3) / 1e12 if main_avg_ms > 0 else 0.0
         peak = peaks["bf16_tflops_sustained"] if ms_step * steps > 1000 else peaks["bf16_tflops"]
+        # rows whose query block stays in shared memory, norm columns included
+        resident = nq > 128 and d + (8 if w["metric"] == 1 else 0) <= (192 if w["storage"] == 0 else 384)
         roofline = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-                    "frac": achieved / peak, "traffic": traffic, "traffic_unit": "bytes per step (scaled from an ncu capture)", "kernel": "gemm_topk_kernel",
+                    "frac": achieved / peak, "traffic": traffic, "traffic_unit": "bytes per step (scaled from an ncu capture)",
+                    "kernel": "gemm_resident_kernel" if resident else "gemm_topk_kernel",
                     "kernel_ms_avg": main_avg_ms, "kernel_launches": main_launches.value,
                     "kernel_launches_per_step": launches_per_step,
                     "peak_source": peaks["source"] + (" sustained" if peak == peaks["bf16_tflops_sustained"] else " burst"),

@@ -1,9 +1,10 @@
 // Distance GEMM for narrow rows: the query block stays in shared memory, X alone is streamed.
 //
-// Serves the filter and store launches of gemm_topk.cu (same operands, same outputs, bit for bit: every accumulator
+// Serves the filter, store and minima launches of gemm_topk.cu (same operands, same outputs, bit for bit: every accumulator
 // takes the same MMAs in the same order) where a query block and the k-blocks of one X tile fit shared memory
-// together (resident_fits): fp32 rows up to d = 192, 16-bit rows up to d = 384, more than 128 queries.  A
-// tile has so few MMAs there (7 to 30) that reading its accumulator takes as long, and the pair shape of
+// together (resident_blocks): inner product on fp32 rows up to d = 192 and 16-bit rows up to d = 384, L2 with its eight norm
+// columns up to 184 and 376; more than 128 queries.  A
+// tile has so few MMAs there (36 at most) that reading its accumulator takes as long, and the pair shape of
 // gemm_topk.cu, whose two accumulators fill the tensor memory, cannot do both at once.
 //
 // A cluster of two CTAs per 256 x 256 tile (cta_group::2, M = N = 256), persistent over work items (query block, range of

@@ -304,6 +304,9 @@ __device__ bool bucket_place(const RowSelectParams& p, int64_t qo, int c, float 
 // longer than placing 130 candidates.  False, with nothing written, where the keys do not spread (ties, infinities).
 // 50 rows of 3,900 candidates, k = 2048: 18 us with thread minima, radix digits and a second reading of the row;
 // the search 116 -> 102.5 us.
+// Ten words a thread, 64 registers (4 bytes of the longer way spilled): with eight 300 queries, k = 1024, on 300,000 rows take
+// 201 us instead of 191, 100 queries on 10,000 rows 69.6 instead of 66.5; with twelve shorter rows take 1 - 2 % more (50 queries,
+// k = 2048: 107.8 -> 109.3), 12,000 keys 59.0 instead of 62.8.
 constexpr int RS_REGS = 10;
 __device__ __forceinline__ bool register_select(const RowSelectParams& p, int64_t qo, const float* keys, const int32_t* ids, int n,
                                                 uint64_t* words, int* end, int* s_live, uint32_t* s_min, uint32_t* s_max,
