@@ -139,3 +139,34 @@ def test_overflowed_rows_stop_filtering(fm, res, storage, nq, k):
         fm.lib().b200f_set_selection_mode(0)
     assert best[0] <= 2 * best[2] + 0.2, best
     idx.close()
+
+
+@pytest.mark.parametrize("storage,d", [(1, 256), (0, 96)])
+def test_redos_of_few_rows_use_the_whole_gpu(fm, res, storage, d):
+    # 100 rows are one query block, whatever the number of queries: redoing them must not take longer because the others
+    # are more (ranges made for eight blocks left one to nine of 72 CTA pairs: 1,370 us instead of 590)
+    nb, k = 1_000_000, 100
+    xb = H.gaussian(nb, d, 1)
+    xb[5000:20000] = xb[7]
+    idx = fm.B200IndexFlat(res, d, O.METRIC_L2, storage)
+    idx.add(xb)
+    extra = []
+    for nq in (1000, 2048):
+        best = []
+        for redone in (0, 100):
+            xq = H.gaussian(nq, d, 2)
+            xq[:redone] = xb[7] + H.gaussian(redone, d, 3, scale=0.01)
+            xq = torch.from_numpy(xq).cuda()
+            t = []
+            for _ in range(8):
+                t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                t0.record()
+                D, I = idx.search(xq, k)
+                t1.record()
+                torch.cuda.synchronize()
+                t.append(1e3 * t0.elapsed_time(t1))
+            best.append(min(t))
+        assert (I[:100] == I[0]).all() and int(I[0, 0]) == 7 and int(I[0, 1]) == 5000
+        extra.append(best[1] - best[0])
+    assert extra[1] <= 1.4 * extra[0], extra
+    idx.close()
