@@ -7,8 +7,9 @@
 // tile has so few MMAs there (36 at most) that reading its accumulator takes as long, and the pair shape of
 // gemm_topk.cu, whose two accumulators fill the tensor memory, cannot do both at once.
 //
-// A cluster of two CTAs per 256 x 256 tile (cta_group::2, M = N = 256), persistent over work items (query block, range of
-// X tiles):
+// A cluster of two CTAs per 256 x 256 tile (cta_group::2, M = N = 256), persistent over work items (query block, every P-th
+// X tile; neighbouring tiles in one item would leave the hits of rows that are near one another and stored side by side to a
+// few CTAs: 100 of 1,000 queries near 15,000 equal rows in a row, 100,000 rows: 1,373 us a search, 866 so):
 //   warp 0     producer: the CTA's half of the query block once per item, then its half (128 rows) of the X k-blocks,
 //              16 KiB each, through a ring of barriers per block
 //   warp 1     of the even CTA: MMAs of one tile after another into two accumulators of 256 columns.  The whole warp walks through
@@ -47,7 +48,7 @@ constexpr int RES_TILE_N = 256;
 static_assert(RES_EPI_WARPS<MODE_FILTER> * HITS_BYTES <= RES_SM_BAR - RES_SM_STAGE && HITS_BYTES % 16 == 0, "hits share the transposes' area");
 
 struct ResidentParams {
-    GemmParams g;        // ntiles, tiles_per_range and P count tiles of 256 columns
+    GemmParams g;        // ntiles and P count tiles of 256 columns; an item takes every P-th
     int nkd, nkl;        // k-blocks of a plane without and with the norm columns (plane 0 has them)
     int n_blocks;        // blocks of the query block, and of an X tile
     int ring;            // X blocks in shared memory, >= n_blocks
@@ -129,7 +130,6 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
             bool ok = true;
             for (int64_t item = unit; item < nitems && ok; item += nunits) {
                 const int qb = (int)(item % nqb);
-                const int64_t t0 = item / nqb * p.tiles_per_range, t1 = min(t0 + p.tiles_per_range, p.ntiles);
                 if (qb != have_qb) {
                     if (!mbar_wait(bar_qempty, qphase ^ 1, abort_flag, p.status)) {
                         ok = false;
@@ -145,7 +145,7 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                     qphase ^= 1;
                     have_qb = qb;
                 }
-                for (int64_t t = t0; t < t1 && ok; t++) {
+                for (int64_t t = item / nqb; t < p.ntiles && ok; t += p.P) {
                     const int xrow = (int)tile_col(t) + (int)cta_rank * 128;
                     for (int i = 0; i < nb; i++) {
                         if (!mbar_wait(bar_empty + slot * 8, phase ^ 1, abort_flag, p.status)) {
@@ -202,14 +202,13 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
             };
             for (int64_t item = unit; item < nitems && ok; item += nunits) {
                 const int qb = (int)(item % nqb);
-                const int64_t t0 = item / nqb * p.tiles_per_range, t1 = min(t0 + p.tiles_per_range, p.ntiles);
                 if (qb != have_qb) {
                     ok = __all_sync(0xffffffffu, mbar_wait(bar_qfull, qphase, abort_flag, p.status));
                     if (!ok) break;
                     qphase ^= 1;
                     have_qb = qb;
                 }
-                for (int64_t t = t0; t < t1 && ok; t++) {
+                for (int64_t t = item / nqb; t < p.ntiles && ok; t += p.P) {
                     ok = mbar_wait(bar_tempty + acc * 8, acc_phase ^ 1, abort_flag, p.status);
                     tc_fence_after();
                     d_tmem = tmem_base + acc * RES_TILE_N;
@@ -285,7 +284,6 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         bool ok = true;
         for (int64_t item = unit; item < nitems && ok; item += nunits) {
             const int qb = (int)(item % nqb);
-            const int64_t t0 = item / nqb * p.tiles_per_range, t1 = min(t0 + p.tiles_per_range, p.ntiles);
             const int64_t grow = (int64_t)qb * 256 + (int64_t)cta_rank * BM + row;
             const bool row_live = grow < nq_live;
             float ksc = p.kscale;
@@ -313,7 +311,7 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                 if ((over >> lane) & 1u) thr = -CUDART_INF_F;
                 nhits = 0;
             };
-            for (int64_t t = t0; t < t1; t++) {
+            for (int64_t t = item / nqb; t < p.ntiles; t += p.P) {
                 const int64_t c_tile = tile_col(t);
                 {
                     const bool w = mbar_wait(bar_tfull + acc * 8, acc_phase, abort_flag, p.status);
@@ -406,7 +404,7 @@ int launch_resident(const GemmOperands& op, const GemmPlan& plan, GemmParams& g,
     // tiles of 256 columns; the second half of the last 512 may lie beyond the end
     int64_t ntiles = 2 * plan.ntiles;
     if (g.col0 + (plan.ntiles - 1) * g.tile_stride * 512 + RES_TILE_N >= g.ncols_end) ntiles--;
-    // Ranges that leave the last wave full; a range costs the query block's way from L2, about one tile.  Of query blocks that are
+    // Items ("ranges", of tpr tiles at most) that leave the last wave full; a range costs the query block's way from L2, about one tile.  Of query blocks that are
     // counted on the device any number may be live, one above all: ranges for that one as well (100 of 2,048 queries redone over
     // 1 M fp16 rows of d = 256, k = 1000: 4,232 us with ranges for all eight blocks, 2,506 so).
     int64_t tpr_best = 1;
@@ -421,7 +419,6 @@ int launch_resident(const GemmOperands& op, const GemmPlan& plan, GemmParams& g,
         }
     }
     g.ntiles = ntiles;
-    g.tiles_per_range = tpr_best;
     g.P = (int)ceil_div64(ntiles, tpr_best);
     p.g = g;
     const int64_t items = (int64_t)plan.nqb * g.P;

@@ -170,3 +170,32 @@ def test_redos_of_few_rows_use_the_whole_gpu(fm, res, storage, d):
         extra.append(best[1] - best[0])
     assert extra[1] <= 1.4 * extra[0], extra
     idx.close()
+
+
+def test_hits_side_by_side_are_shared_out(fm, res):
+    # 15,000 equal rows in a row: the hits of 100 queries near them lie in 59 neighbouring tiles.  Dealt out as ranges of
+    # neighbours these were the work of three CTA pairs of 72; scattered over the index the same rows are the measure
+    nb, d, nq, k = 100_000, 128, 1000, 1000
+    near = np.arange(5000, 20000)
+    scattered = np.sort(np.random.default_rng(1).permutation(nb)[:15000])
+    best = []
+    for where in (scattered, near):
+        xb = H.gaussian(nb, d, 1)
+        xb[where] = H.gaussian(1, d, 2)
+        idx = fm.B200IndexFlat(res, d, O.METRIC_L2, 0)
+        idx.add(xb)
+        xq = H.gaussian(nq, d, 3)
+        xq[:100] = xb[where[0]] + H.gaussian(100, d, 4, scale=0.01)
+        xq = torch.from_numpy(xq).cuda()
+        t = []
+        for _ in range(8):
+            t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            t0.record()
+            D, I = idx.search(xq, k)
+            t1.record()
+            torch.cuda.synchronize()
+            t.append(1e3 * t0.elapsed_time(t1))
+        best.append(min(t))
+        assert (I[:100].cpu().numpy() == where[:k]).all()
+        idx.close()
+    assert best[1] <= 1.15 * best[0], best
